@@ -252,7 +252,8 @@ static int gkr_common(const f128 *images, const f128 *columns, int log_cols, con
   gkr_build(columns, log_cols, images, sc, ctx.stream());
   f128 z[kMaxPointGkr], pt[kMaxPointGkr];
   for (int i = 0; i < log_cols; i++) z[i] = mk(zeta[2 * i], zeta[2 * i + 1]);
-  f128 claim = gkr_prove(log_cols, z, grinding_bits(security_bits, 3), t->t, sc, ctx.stream(), pt);
+  f128 claim = gkr_prove(columns, log_cols, images, z, grinding_bits(security_bits, 3), t->t, sc,
+                         ctx.stream(), pt);
   for (int i = 0; i < log_cols + 7; i++) {
     point_out[2 * i] = pt[i].lo;
     point_out[2 * i + 1] = pt[i].hi;

@@ -257,12 +257,8 @@ Context::Context() {
   BZ_CUDA(cudaMallocHost(&host_, 64 * sizeof(uint64_t)));
   pg_.acc = acc_.get();
   pg_.host = host_;
-  gk_pair_.resize(2);
   gk_.acc = acc_.get();
-  gk_.host = host_;
-  gk_.pair = gk_pair_.get();
   gk_ctl_.resize(kMaxPointGkr);
-  gk_.ctl = gk_ctl_.get();
   // the round mailbox: one mapped pinned page and a device block counter
   void *mb = nullptr;
   // one mapped allocation: mailbox (0), downbox (512), error word (1024),
@@ -286,7 +282,6 @@ Context::Context() {
   pg_.channel = &channel_;
   pg_.ctl = gk_ctl_.get();
   gk_.channel = &channel_;
-  gk_.mid_blocks = gkr_mid_blocks(false);
   sp_mid_blocks_ = ::bz::sp_mid_blocks(false);
   pg_.mid_blocks = ::bz::pg_mid_blocks(false);
   lane_bootstrap(*this);
@@ -309,12 +304,11 @@ std::atomic<unsigned long long> &launch_counter() {
 Context &Context::get() {
   // One default lane per process, created on first use on the current device.
   // It proves one statement at a time with the GPU to itself, so its resident
-  // middle rounds (GKR, Spartan, post-GKR and Ligerito) use grids of 128
+  // middle rounds (Spartan, post-GKR and Ligerito) use grids of 128
   // blocks; pool lanes, which share the GPU, run those rounds as queued
   // launches (or 32-block grids with BITZ_POOL_MID=1).
   static Context *ctx = [] {
     Context *c = new Context();
-    c->gk_.mid_blocks = gkr_mid_blocks(true);
     c->sp_mid_blocks_ = ::bz::sp_mid_blocks(true);
     c->pg_.mid_blocks = ::bz::pg_mid_blocks(true);
     return c;

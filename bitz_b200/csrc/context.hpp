@@ -136,18 +136,19 @@ class Context {
   GkrScratch &gkr_scratch(int s) {
     size_t leaves = (size_t)128 << s;
     if (gk_.capacity < leaves) {
-      size_t total = 0;
-      for (int j = 0; j < 8; j++) total += leaves >> j;
+      size_t total = leaves >> 6;
+      for (int j = 2; j < 8; j++) total += leaves >> j;
       gk_layers_.resize(total);
-      size_t off = 0;
-      for (int j = 0; j < 8; j++) {
+      gk_.bound = gk_layers_.get();
+      size_t off = leaves >> 6;
+      for (int j = 2; j < 8; j++) {
         gk_.layer[j] = gk_layers_.get() + off;
         off += leaves >> j;
       }
-      gk_eq_.resize(leaves / 4);
-      gk_eq_scratch_.resize(eq_scratch_entries(6 + s));
-      gk_.eq = gk_eq_.get();
-      gk_.eq_scratch = gk_eq_scratch_.get();
+      gk_gram_.resize(gkr_gram_words());
+      gk_mid_.resize(2304);
+      gk_.gram = gk_gram_.get();
+      gk_.mid = gk_mid_.get();
       gk_.capacity = leaves;
     }
     return gk_;
@@ -160,7 +161,8 @@ class Context {
   DeviceBuffer<unsigned long long> acc_;
   uint64_t *host_ = nullptr;
   GkrScratch gk_;
-  DeviceBuffer<f128> gk_layers_, gk_eq_, gk_eq_scratch_, gk_pair_;
+  DeviceBuffer<f128> gk_layers_, gk_mid_;
+  DeviceBuffer<unsigned long long> gk_gram_;
   DeviceBuffer<RoundCtl> gk_ctl_;
   RoundChannel channel_;
   DeviceBuffer<unsigned int> counter_;

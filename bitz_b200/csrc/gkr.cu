@@ -2,18 +2,31 @@
 //
 // Leaf (b << s) | c of the product tree is the row image b where column c has
 // bit b set, one elsewhere (crates/prover/src/reduce.rs:1-5); node k of each
-// layer multiplies nodes k and k + half of the layer below. The reference
-// keeps layers 0-2 in 16-entry lookup tables to save CPU memory traffic;
-// here every layer is a dense device table (2^(7+s) leaves at most, 512 MiB
-// at s = 18), built by one pass per layer. Round messages are exact field
-// values, so the dense sums equal the reference's bucketed ones bit for bit.
+// layer multiplies nodes k and k + half of the layer below. A node of layers 0
+// to 3 takes 2, 4, 16 or 256 values, by the column's bits in its rows (the
+// reference keeps layers 0-2 in 16-entry lookup tables for the same reason,
+// lib.rs:274-303). Layers 2 and 3 are looked up and stored, the layers above
+// are products of them; layers 0 and 1 are never stored, their sumchecks start
+// from the bits. Round messages are exact field values, so any order of sums
+// gives the reference's bytes.
 //
-// A layer sumcheck binds its point's top coordinate first. Round i splits
-// the children into L = C[0, 2^n) and R = C[2^n, 2^(n+1)), each into halves
-// at 2^i. One launch per round binds round i+1 in place, sums the eq table
-// down to round i's (eq_i[x] = eq_{i+1}[x] + eq_{i+1}[x + 2^i], summing out
-// coordinate i), and accumulates round i's two sums from the freshly bound
-// values; 32 bytes leave the device per round.
+// A layer sumcheck binds its point's top coordinate first: with L = C[0, 2^n)
+// and R = C[2^n, 2^(n+1)) it sums eq(x) L(x) R(x). Several rounds go through
+// the device as one pass. A pass over the top K coordinates X sums, for every
+// point p of {0, 1, infinity}^K (infinity: the coefficient of X^1, i.e. the
+// sum of the halves),
+//
+//   F(p) = sum over the lower coordinates x of eq(x) L(p, x) R(p, x),
+//
+// which determines the product polynomial (degree two in each coordinate), so
+// the host reads the 3^K values and runs K rounds by itself; the next pass
+// binds the K coordinates at once. What bounds a small round is its
+// host-device turn, and a pass of three rounds makes 8 + 27 products where
+// three rounds make 4 (4 + 2 + 1) = 28, so a turn per three rounds is the
+// better split at every size. Tables of 2^kHostLog entries or fewer go to the
+// host, which runs the remaining rounds. Measured for the seven layers, a
+// round a turn before and passes now: s = 18 8.59 -> 3.91 ms, s = 14 in a
+// proof of 64 blocks 1.52 -> 0.93 ms (77 turns -> 29).
 #include <algorithm>
 #include <chrono>
 #include <cstdio>
@@ -25,735 +38,785 @@
 
 namespace bz {
 
-__global__ void gkr_leaves(const f128 *__restrict__ cols, int s, const f128 *__restrict__ images,
-                           f128 *__restrict__ out) {
-  const size_t total = (size_t)128 << s;
-  const size_t cmask = ((size_t)1 << s) - 1;
-  for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < total;
-       k += (size_t)gridDim.x * blockDim.x) {
-    size_t c = k & cmask;
-    int b = (int)(k >> s);
-    f128 word = ld(cols + c);
-    st(out + k, bit128(word, b) ? ld(images + b) : mk(1, 0));
+// Layers 2 and 3 from the bits. Block row y holds nodes y and y + 16 of layer 2
+// and node y of layer 3, their product, so a column is 4 + 4 bits, three
+// lookups and three coalesced stores: the kernel is bound by its writes
+// (48 of the 63 entries a column has in the stored layers).
+__device__ __forceinline__ f128 row_value(const f128 *images, int row, int bit) {
+  return bit ? ld(images + row) : mk(1, 0);
+}
+
+__global__ void __launch_bounds__(kThreads) gkr_low_layers(const f128 *__restrict__ cols, int s,
+                                                           const f128 *__restrict__ images,
+                                                           f128 *__restrict__ layer2,
+                                                           f128 *__restrict__ layer3) {
+  __shared__ f128 two[2][16], three[256];
+  const int y = blockIdx.y, t = threadIdx.x;
+  if (t < 32) {
+    const int node = y + (t & 16), v = t & 15;
+    f128 p[2];
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+      p[i] = gmul(row_value(images, node + 64 * i, (v >> (2 * i)) & 1),
+                  row_value(images, node + 64 * i + 32, (v >> (2 * i + 1)) & 1));
+    two[t >> 4][v] = gmul(p[0], p[1]);
   }
+  __syncthreads();
+  three[t] = gmul(two[0][t & 15], two[1][t >> 4]);
+  __syncthreads();
+  const size_t n = (size_t)1 << s;
+  for (size_t c = blockIdx.x * (size_t)blockDim.x + t; c < n; c += (size_t)gridDim.x * blockDim.x) {
+    const uint4 w = __ldg(reinterpret_cast<const uint4 *>(cols + c));
+    auto four = [&](int r) {  // bits r, r + 32, r + 64, r + 96
+      return (int)(((w.x >> r) & 1) | ((w.y >> r) & 1) << 1 | ((w.z >> r) & 1) << 2 |
+                   ((w.w >> r) & 1) << 3);
+    };
+    const int i = four(y), j = four(y + 16);
+    st(layer2 + ((size_t)y << s) + c, two[0][i]);
+    st(layer2 + ((size_t)(y + 16) << s) + c, two[1][j]);
+    st(layer3 + ((size_t)y << s) + c, three[16 * j + i]);
+  }
+}
+
+// Layers 4 to 7: a thread takes a column's 16 nodes of layer 3 through the four
+// levels, 15 products. Padded columns have only ones.
+__global__ void __launch_bounds__(128) gkr_high_layers(const f128 *__restrict__ layer3, int s,
+                                                       f128 *__restrict__ l4, f128 *__restrict__ l5,
+                                                       f128 *__restrict__ l6, f128 *__restrict__ l7,
+                                                       size_t live) {
+  const size_t n = (size_t)1 << s;
+  for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < n;
+       c += (size_t)gridDim.x * blockDim.x) {
+    const bool one = c >= live;
+    f128 v[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      const size_t at = ((size_t)k << s) + c;
+      v[k] = one ? mk(1, 0) : gmul(ld(layer3 + at), ld(layer3 + at + ((size_t)8 << s)));
+      st(l4 + at, v[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      if (!one) v[k] = gmul(v[k], v[k + 4]);
+      st(l5 + ((size_t)k << s) + c, v[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      if (!one) v[k] = gmul(v[k], v[k + 2]);
+      st(l6 + ((size_t)k << s) + c, v[k]);
+    }
+    st(l7 + c, one ? v[0] : gmul(v[0], v[1]));
+  }
+}
+
+// ------------------------------------------------------------------ passes
+
+constexpr int kPassThreads = 288;  // nine warps: the 27 points of a tile in three turns
+constexpr int kPassMaxK = 3;
+constexpr int kPassMaxX = 32;  // positions per tile
+constexpr int kFacLog = 7;     // coordinates per eq factor
+
+constexpr int pow3(int k) { return k == 0 ? 1 : 3 * pow3(k - 1); }
+
+// eq(x) over the lower coordinates as a product of NF factor tables, factor g
+// over coordinates 7g .. 7g + 6. The host forms the layer's tables once (about
+// 130 products each) and they travel as a launch argument: no copy, no setup
+// launch before the layer's first pass.
+template <int NF>
+struct EqFactors {
+  f128 f[NF][1 << kFacLog];
+};
+
+// The challenges of the pass before: r[0] bound the top coordinate.
+struct PassBind {
+  f128 r[kPassMaxK];
+  int k;
+};
+
+// Products as calls: a pass is short for most sizes and starts with a cold
+// instruction cache (a product inlined 40 times costs more to fetch than to
+// run), and the larger ones are bound by the products themselves.
+static __device__ __noinline__ wide pass_wide(f128 a, f128 b) { return gmul_wide(a, b); }
+static __device__ __noinline__ f128 pass_table(const MulTable *T, f128 a) {
+  return mul_table(*T, a);
+}
+static __device__ __forceinline__ f128 pass_mul(f128 a, f128 b) { return greduce(pass_wide(a, b)); }
+
+// The window tables of b.r[0 .. b.k), every thread of the block taking part.
+static __device__ __forceinline__ void pass_tables(MulTable *T, const PassBind &b) {
+  for (int u = threadIdx.x; u < b.k * 128; u += blockDim.x) {
+    const int t = u >> 7, k = u & 127;
+    const f128 v = gmul_xk(b.r[t], k);
+    T[t].lo[k >> 2][1 << (k & 3)] = v.lo;
+    T[t].hi[k >> 2][1 << (k & 3)] = v.hi;
+  }
+  __syncthreads();
+  for (int u = threadIdx.x; u < b.k * 512; u += blockDim.x) {
+    const int t = u >> 9, j = (u >> 4) & 31, v = u & 15;
+    if (v != 0 && (v & (v - 1)) == 0) continue;  // written above
+    uint64_t lo = 0, hi = 0;
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+      if ((v >> q) & 1) {
+        lo ^= T[t].lo[j][1 << q];
+        hi ^= T[t].hi[j][1 << q];
+      }
+    T[t].lo[j][v] = lo;
+    T[t].hi[j][v] = hi;
+  }
+  __syncthreads();
+}
+
+static __device__ __forceinline__ f128 bind2(const MulTable *T, f128 a, f128 b) {
+  return gadd(a, pass_table(T, gadd(a, b)));
+}
+
+// Entry `pos` of a table of `n` entries after binding the k coordinates above
+// it: block b of the unbound table starts at b n, the first challenge bound
+// the top bit of b.
+static __device__ __forceinline__ f128 pass_bind(const f128 *tab, size_t pos, size_t n,
+                                                 const MulTable *T, int k) {
+  const f128 *p = tab + pos;
+  if (k == 0) return ld(p);
+  if (k == 1) return bind2(T, ld(p), ld(p + n));
+  if (k == 2) {
+    const f128 a = bind2(T, ld(p), ld(p + 2 * n)), b = bind2(T, ld(p + n), ld(p + 3 * n));
+    return bind2(T + 1, a, b);
+  }
+  const f128 a0 = bind2(T, ld(p), ld(p + 4 * n)), a2 = bind2(T, ld(p + 2 * n), ld(p + 6 * n));
+  const f128 a1 = bind2(T, ld(p + n), ld(p + 5 * n)), a3 = bind2(T, ld(p + 3 * n), ld(p + 7 * n));
+  return bind2(T + 2, bind2(T + 1, a0, a2), bind2(T + 1, a1, a3));
+}
+
+// Table t (2^K blocks of X positions) at point p, digit i of p (base 3) for
+// bit i of the block: 0, 1, or 2 for infinity (the sum over the bit).
+template <int K>
+static __device__ __forceinline__ f128 point_value(const f128 *t, int lx, int x, int p) {
+  int one = 0, inf = 0;
+#pragma unroll
+  for (int i = 0; i < K; i++) {
+    const int d = p % 3;
+    p /= 3;
+    one |= (d == 1) << i;
+    inf |= (d == 2) << i;
+  }
+  f128 v = t[(one << lx) + x];
+  for (int sub = inf; sub; sub = (sub - 1) & inf) v = gadd(v, t[((one | sub) << lx) + x]);
+  return v;
 }
 
 // Padding: the low s bits of every layer index are the column, and a column at
-// or beyond `live` has only one-valued nodes. Whenever entry x of a half is
-// such a column, so are x + h and x + 2h (same column, or a higher one below
-// 2^s), so a thread whose x is padded binds nothing (1 + r (1 + 1) = 1) and
-// adds e * 1 * 1 = e to the first sum and e * 0 * 0 = 0 to the second.
-__device__ __forceinline__ bool padded(size_t x, size_t colmask, size_t live) {
-  return (x & colmask) >= live;
-}
-
-__global__ void gkr_parent(const f128 *__restrict__ child, size_t half, f128 *__restrict__ out,
-                           size_t colmask, size_t live) {
-  for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < half;
-       k += (size_t)gridDim.x * blockDim.x)
-    st(out + k, padded(k, colmask, live) ? mk(1, 0) : gmul(ld(child + k), ld(child + half + k)));
-}
-
-// Queued rounds (the round link in device.cuh): every bind round of a layer
-// is queued at the layer's start, so no round waits for a launch from the
-// host.
-
-// Every thread calls it; false when the chain has stopped (the block returns).
-__device__ __forceinline__ bool round_begin(const RoundLink &lk, f128 r_arg, f128 &r) {
-  if (!lk.in) {
-    r = r_arg;
-    return true;
-  }
-  unsigned long long w0, w1;
-  const bool ok = link_begin(lk, w0, w1);
-  r = mk(w0, w1);
-  return ok;
-}
-
-// publish<4>, then the last block fetches the next challenge for `out`.
-__device__ __forceinline__ void round_end(unsigned long long *acc, const Publish &p,
-                                          const RoundLink &lk) {
-  publish_link<4>(acc, p, lk);
-}
-
-// A layer's start. The eq table over the n - 1 coordinates below the top one
-// is the product of two factor tables, lo over the first a coordinates and
-// hi over the other b: block 0 builds lo and clears the layer's round
-// accumulators, block 1 builds hi and clears the round controls; the top
-// sums kernel multiplies the factors out as it reads them.
-__global__ void __launch_bounds__(kThreads) gkr_layer_setup(Point p, int a, int b, f128 *lo,
-                                                            f128 *hi, unsigned long long *acc,
-                                                            int acc_words, RoundCtl *ctl,
-                                                            int nctl) {
-  __shared__ MulTable T;
-  if (blockIdx.x == 0) {
-    for (int k = threadIdx.x; k < acc_words; k += blockDim.x) acc[k] = 0;
-    eq_factor_block(p, 0, a, lo, T);
-  } else {
-    for (int k = threadIdx.x; k < nctl; k += blockDim.x) ctl[k] = RoundCtl{0, 0, 0, 0, 0};
-    eq_factor_block(p, a, b, hi, T);
-  }
-}
-
-// Round i's sums (round_sums, lib.rs:164-216) before any bind: the top round.
-// Entry x of the eq table is lo[x mod 2^a] * hi[x >> a]; it is stored for the
-// bind rounds as it is formed.
-__global__ void gkr_top_sums(const f128 *__restrict__ c, size_t n_half, size_t h,
-                             const f128 *__restrict__ lo, int a, const f128 *__restrict__ hi,
-                             f128 *__restrict__ eq, int at_one, unsigned long long *acc,
-                             Publish pub, RoundLink lk, size_t colmask, size_t live) {
-  const f128 *L = c, *R = c + n_half;
-  const size_t amask = ((size_t)1 << a) - 1;
-  wide sb = wzero(), si = wzero();
-  for (size_t x = blockIdx.x * (size_t)blockDim.x + threadIdx.x; x < h;
-       x += (size_t)gridDim.x * blockDim.x) {
-    const f128 e = gmul(ld(lo + (x & amask)), ld(hi + (x >> a)));
-    st(eq + x, e);
-    if (padded(x, colmask, live)) {
-      sb.w0 ^= e.lo;
-      sb.w1 ^= e.hi;
-      continue;
+// or beyond `live` has only one-valued nodes, before and after any bind
+// (1 + r (1 + 1) = 1). Whenever position x of a block is such a column, so is
+// the same position of the higher blocks (same column, or a higher one below
+// 2^s), so a pass leaves those positions out: they add eq(x) to F at the points
+// without infinity and nothing at the others.
+// One pass. Binds the coordinates of `b` (in place: the entry at pos comes from
+// pos + j N), then sums the 3^K points over the live positions of the 2^log_m
+// below the top K coordinates, and the eq weights of those positions. The last
+// block posts the 3^K + 1 sums as handover publication seq.
+//
+// A block works tiles of X = 2^lx positions: the 2 2^K X bound entries (and
+// the X weights) one per thread into shared memory, the 2^K X products of the
+// weights with L, then the 3^K X wide products, whose sums stay in registers
+// (thread t of turn q always has the same point). X shrinks with the number of
+// positions, so that a small pass still spreads over the SMs.
+template <int K, int NF>
+__global__ void __launch_bounds__(kPassThreads, 2) gkr_pass(
+    f128 *__restrict__ c, size_t n_half, int log_m, PassBind b,
+    const __grid_constant__ EqFactors<NF> eq, size_t colmask, uint32_t live, uint32_t count,
+    int lx, unsigned long long *acc, unsigned int *counter, unsigned long long *handover,
+    unsigned long long seq) {
+  constexpr int kPoints = pow3(K), kBlocks = 1 << K;
+  constexpr int kTurns = (kPoints * kPassMaxX + kPassThreads - 1) / kPassThreads;
+  __shared__ MulTable T[kPassMaxK];
+  __shared__ f128 G[kBlocks * kPassMaxX], R[kBlocks * kPassMaxX], E[kPassMaxX];
+  __shared__ f128 F[NF][1 << kFacLog];
+  __shared__ bool last;
+  const int t = threadIdx.x;
+  const size_t m = (size_t)1 << log_m, n = m << K;
+  const int X = 1 << lx;
+  for (int u = t; u < NF << kFacLog; u += kPassThreads) (&F[0][0])[u] = (&eq.f[0][0])[u];
+  if (b.k)
+    pass_tables(T, b);
+  else
+    __syncthreads();
+  // position of live index i: rows of `live` columns when a block spans whole
+  // rows of the column space, else i itself
+  const bool by_row = m > colmask;
+  auto position = [&](uint32_t i) -> size_t {
+    if (!by_row) return i;
+    const uint32_t row = i / live;
+    return (size_t)row * (colmask + 1) + (i - row * live);
+  };
+  wide sum[kTurns];
+#pragma unroll
+  for (int q = 0; q < kTurns; q++) sum[q] = wzero();
+  f128 sum_e = mk(0, 0);
+  for (uint32_t i0 = blockIdx.x << lx; i0 < count; i0 += gridDim.x << lx) {
+    const int nbind = 2 * kBlocks << lx;
+    for (int u = t; u < nbind + X; u += kPassThreads) {
+      const uint32_t i = i0 + (u & (X - 1));
+      const bool in = i < count;
+      const size_t x = in ? position(i) : 0;
+      if (u >= nbind) {  // the weight of position x
+        f128 e = mk(0, 0);
+        if (in) {
+          e = F[0][x & ((1 << kFacLog) - 1)];
+#pragma unroll 1
+          for (int g = 1; g < NF && g * kFacLog < log_m; g++)
+            e = pass_mul(e, F[g][(x >> (g * kFacLog)) & ((1 << kFacLog) - 1)]);
+        }
+        E[u - nbind] = e;
+        sum_e = gadd(sum_e, e);
+        continue;
+      }
+      const bool right = u >= nbind / 2;
+      const int slot = right ? u - nbind / 2 : u;
+      f128 v = mk(0, 0);
+      if (in) {
+        f128 *tab = right ? c + n_half : c;
+        const size_t pos = x + (size_t)(slot >> lx) * m;
+        v = pass_bind(tab, pos, n, T, b.k);
+        if (b.k) st(tab + pos, v);
+      }
+      (right ? R : G)[slot] = v;
     }
-    f128 l0 = ld(L + x), l1 = ld(L + h + x), r0 = ld(R + x), r1 = ld(R + h + x);
-    f128 lb = at_one ? l1 : l0, rb = at_one ? r1 : r0;
-    wacc(sb, gmul_wide(gmul(e, lb), rb));
-    wacc(si, gmul_wide(gmul(e, gadd(l1, l0)), gadd(r1, r0)));
-  }
-  f128 sa = greduce(sb), sbb = greduce(si);
-  uint64_t v[4] = {sa.lo, sa.hi, sbb.lo, sbb.hi};
-  block_xor_atomic<4>(v, acc);
-  round_end(acc, pub, lk);
-}
-
-// Bind round i+1 at r (halves of 2^(i+1)), derive eq_i in place, and sum
-// round i (halves of 2^i). Thread x < 2^i owns entries x and x + 2^i.
-__global__ void gkr_bind_sums(f128 *__restrict__ c, size_t n_half, size_t h, f128 r_arg,
-                              f128 *__restrict__ eq, int at_one, unsigned long long *acc,
-                              Publish pub, RoundLink lk, size_t colmask, size_t live) {
-  f128 r;
-  if (!round_begin(lk, r_arg, r)) return;
-  __shared__ MulTable T;  // the binds by r through r's window table
-  mul_table_build(T, r);
-  f128 *L = c, *R = c + n_half;
-  const size_t h2 = 2 * h;
-  wide sb = wzero(), si = wzero();
-  for (size_t x = blockIdx.x * (size_t)blockDim.x + threadIdx.x; x < h;
-       x += (size_t)gridDim.x * blockDim.x) {
-    if (padded(x, colmask, live)) {
-      f128 e = gadd(ld(eq + x), ld(eq + x + h));
-      st(eq + x, e);
-      sb.w0 ^= e.lo;
-      sb.w1 ^= e.hi;
-      continue;
+    __syncthreads();
+    for (int u = t; u < kBlocks << lx; u += kPassThreads) G[u] = pass_mul(E[u & (X - 1)], G[u]);
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kTurns; q++) {
+      const int u = t + q * kPassThreads;
+      if (u < kPoints << lx) {
+        const int p = u >> lx, x = u & (X - 1);
+        wacc(sum[q], pass_wide(point_value<K>(G, lx, x, p), point_value<K>(R, lx, x, p)));
+      }
     }
-    f128 a0 = ld(L + x), a1 = ld(L + x + h2), b0 = ld(L + x + h), b1 = ld(L + x + h + h2);
-    f128 l0 = gadd(a0, mul_table(T, gadd(a1, a0)));
-    f128 l1 = gadd(b0, mul_table(T, gadd(b1, b0)));
-    f128 c0 = ld(R + x), c1 = ld(R + x + h2), d0 = ld(R + x + h), d1 = ld(R + x + h + h2);
-    f128 r0 = gadd(c0, mul_table(T, gadd(c1, c0)));
-    f128 r1 = gadd(d0, mul_table(T, gadd(d1, d0)));
-    st(L + x, l0);
-    st(L + x + h, l1);
-    st(R + x, r0);
-    st(R + x + h, r1);
-    f128 e = gadd(ld(eq + x), ld(eq + x + h));
-    st(eq + x, e);
-    f128 lb = at_one ? l1 : l0, rb = at_one ? r1 : r0;
-    wacc(sb, gmul_wide(gmul(e, lb), rb));
-    wacc(si, gmul_wide(gmul(e, gadd(l1, l0)), gadd(r1, r0)));
+    __syncthreads();  // the tile's tables before the next tile's
   }
-  f128 a = greduce(sb), b = greduce(si);
-  uint64_t v[4] = {a.lo, a.hi, b.lo, b.hi};
-  block_xor_atomic<4>(v, acc);
-  round_end(acc, pub, lk);
+  // the block's sums: over the X lanes of each point, then into acc
+#pragma unroll
+  for (int q = 0; q < kTurns; q++) {
+    const int u = t + q * kPassThreads;
+    f128 v = greduce(sum[q]);
+    for (int off = X >> 1; off > 0; off >>= 1) {
+      v.lo ^= __shfl_xor_sync(0xffffffffu, v.lo, off);
+      v.hi ^= __shfl_xor_sync(0xffffffffu, v.hi, off);
+    }
+    if (u < kPoints << lx && (u & (X - 1)) == 0) {
+      atomicXor(acc + 2 * (u >> lx), (unsigned long long)v.lo);
+      atomicXor(acc + 2 * (u >> lx) + 1, (unsigned long long)v.hi);
+    }
+  }
+  for (int off = 16; off > 0; off >>= 1) {
+    sum_e.lo ^= __shfl_xor_sync(0xffffffffu, sum_e.lo, off);
+    sum_e.hi ^= __shfl_xor_sync(0xffffffffu, sum_e.hi, off);
+  }
+  if ((t & 31) == 0 && (sum_e.lo | sum_e.hi)) {
+    atomicXor(acc + 2 * kPoints, (unsigned long long)sum_e.lo);
+    atomicXor(acc + 2 * kPoints + 1, (unsigned long long)sum_e.hi);
+  }
+  __threadfence();
+  __syncthreads();
+  if (t == 0) {
+    last = atomicAdd(counter, 1u) == gridDim.x - 1;
+    __threadfence();
+  }
+  __syncthreads();
+  if (last) {
+    if (t < 2 * (kPoints + 1))
+      handover_post(handover, seq, t, atomicExch(acc + t, 0ull));
+    if (t == 0) *counter = 0;
+  }
 }
 
-// gkr_bind_sums by tiles, for rounds where few elements leave each thread's
-// chain of eight products (four binds, two with e, two wide) as the round's
-// latency. A block takes a tile of kMidTile elements and works it in three
-// levels, each product of a level on its own thread: the 4 * kMidTile binds
-// by r through the block's window table (2 per thread), then the
-// 2 * kMidTile products with e, then the 2 * kMidTile wide products. Same
-// values, same sums as gkr_bind_sums.
-constexpr int kTailH = 256;  // gkr_tail's first round binds at most 4 kTailH entries per half
-constexpr int kMidThreads = 256;
-constexpr int kMidTile = 128;
-constexpr size_t kMidMaxH = (size_t)1 << 15;  // larger rounds are issue bound: gkr_bind_sums
-static_assert(kMidThreads == 2 * kMidTile && kMidThreads == kThreads, "one product per thread");
+// The layer's last tables to the host: L, then R, of n entries each after the
+// binds of `b`, as handover publication seq (two words per entry).
+constexpr int kHandThreads = 256, kHandEntries = 64;  // threads build the tables, entries bind
+__global__ void __launch_bounds__(kHandThreads) gkr_handover(const f128 *__restrict__ c,
+                                                             size_t n_half, int n, PassBind b,
+                                                             unsigned long long *handover,
+                                                             unsigned long long seq) {
+  __shared__ MulTable T[kPassMaxK];
+  pass_tables(T, b);
+  const int k = blockIdx.x * kHandEntries + threadIdx.x;
+  if (threadIdx.x >= kHandEntries || k >= 2 * n) return;
+  const f128 v = k < n ? pass_bind(c, k, n, T, b.k) : pass_bind(c + n_half, k - n, n, T, b.k);
+  handover_post(handover, seq, 2 * k, v.lo);
+  handover_post(handover, seq, 2 * k + 1, v.hi);
+}
 
-// Shared memory of one tile: the window table of r, the tile's bound
-// entries L[x], L[x+h], R[x], R[x+h], its eq entries and the products with e.
-struct TileShared {
-  MulTable T;
-  f128 B[4][kMidTile];
-  f128 E[kMidTile], P[kMidTile], Q[kMidTile];
+// ------------------------------------------ the two lowest layers' row rounds
+//
+// A node of layer 0 or 1 is a sum over features of the column's bits: layer 0
+// has 1 + bit d (d: the row's image plus one), layer 1, with rows a and a + 64,
+// 1 + p d + q d' + p q d d'. So the sums of all rounds over row coordinates
+// (6 of layer 0, 5 of layer 1) come from the weighted counts
+//
+//   X[i][j] = sum over the columns with features i and j of eq(column),
+//
+// i over the features of the rows below the top coordinate and j over those
+// above it: 64 x 64 and 96 x 96. Over 128 columns such a sum is one product
+// through a window table whose single-bit entries are the columns' weights,
+// with the two features' common bits as the other factor. That is 13,600
+// lookup products per 128 columns for both layers, where the dense rounds make
+// 127 - 31 = 96 x 9 general ones per column.
+
+template <int NFEAT>
+struct GramShape {
+  static constexpr int kGroups = NFEAT == 64 ? 4 : 3;  // thread groups over j
+  static constexpr int kThreadsPer = NFEAT * kGroups;
+  static constexpr int kRow = NFEAT + 1;  // X's row; index NFEAT is the constant feature
 };
 
-// L2 loads: a resident kernel reads entries that other blocks wrote in its
-// previous round, which this SM's L1 may hold stale.
-__device__ __forceinline__ f128 ld_cg(const f128 *p) {
-  const ulonglong2 v = __ldcg(reinterpret_cast<const ulonglong2 *>(p));
-  return mk(v.x, v.y);
+template <int NFEAT>
+__device__ __forceinline__ uint4 feature(const uint4 *rows, int i, bool upper) {
+  if (NFEAT == 64) return rows[i + (upper ? 64 : 0)];
+  const int at = (i & 31) + (upper ? 32 : 0);
+  const uint4 p = rows[at], q = rows[at + 64];
+  if (i < 32) return p;
+  if (i < 64) return q;
+  return make_uint4(p.x & q.x, p.y & q.y, p.z & q.z, p.w & q.w);
 }
 
-// Elements [x0, x0 + kMidTile) of a bind round with S.T built for r: the
-// three levels, the tile's share of the first message summed by even
-// threads into acc_w, of the second by odd ones. Every thread calls it; it
-// ends with the block synchronised.
-__device__ __forceinline__ void bind_tile(TileShared &S, f128 *L, f128 *R, f128 *eq, size_t h,
-                                          size_t x0, int at_one, size_t colmask, size_t live,
-                                          wide &acc_w) {
-  const size_t h2 = 2 * h;
-  const int t = threadIdx.x;
-  // level 1: entry (k, q) of the tile is L[x], L[x+h], R[x], R[x+h] for q = 0..3
-#pragma unroll
-  for (int it = 0; it < 4 * kMidTile / kMidThreads; it++) {
-    const int u = t + it * kMidThreads;
-    const int k = u >> 2, q = u & 3;
-    const size_t x = x0 + k;
-    if (x >= h) continue;
-    if (q == 0) {
-      const f128 e = gadd(ld_cg(eq + x), ld_cg(eq + x + h));
-      st(eq + x, e);
-      S.E[k] = e;
-    }
-    f128 v = mk(1, 0);  // a padded column stays one
-    if (!padded(x, colmask, live)) {
-      f128 *tab = q < 2 ? L : R;
-      const size_t at = x + (q & 1) * h;
-      const f128 a0 = ld_cg(tab + at), a1 = ld_cg(tab + at + h2);
-      v = gadd(a0, mul_table(S.T, gadd(a1, a0)));
-      st(tab + at, v);
-    }
-    S.B[q][k] = v;
-  }
-  __syncthreads();
-  // level 2: P = e * L_b, Q = e * (L_1 + L_0)
-  {
-    const int k = t >> 1;
-    const size_t x = x0 + k;
-    if (x < h) {
-      const f128 e = S.E[k];
-      if (padded(x, colmask, live)) {  // e * 1 and e * 0
-        if (t & 1)
-          S.Q[k] = mk(0, 0);
-        else
-          S.P[k] = e;
-      } else if (t & 1) {
-        S.Q[k] = gmul(e, gadd(S.B[1][k], S.B[0][k]));
-      } else {
-        S.P[k] = gmul(e, at_one ? S.B[1][k] : S.B[0][k]);
-      }
-    }
-  }
-  __syncthreads();
-  // level 3: P * R_b into the first sum, Q * (R_1 + R_0) into the second
-  {
-    const int k = t >> 1;
-    const size_t x = x0 + k;
-    if (x < h) {
-      if (padded(x, colmask, live)) {  // P * 1 and Q * 0
-        if (!(t & 1)) {
-          acc_w.w0 ^= S.P[k].lo;
-          acc_w.w1 ^= S.P[k].hi;
-        }
-      } else if (t & 1) {
-        wacc(acc_w, gmul_wide(S.Q[k], gadd(S.B[3][k], S.B[2][k])));
-      } else {
-        wacc(acc_w, gmul_wide(S.P[k], at_one ? S.B[3][k] : S.B[2][k]));
-      }
-    }
-  }
-  __syncthreads();  // the tile's tables before the next tile overwrites them
+static __device__ __forceinline__ f128 and_bits(uint4 a, uint4 b) {
+  return mk((uint64_t)(a.x & b.x) | (uint64_t)(a.y & b.y) << 32,
+            (uint64_t)(a.z & b.z) | (uint64_t)(a.w & b.w) << 32);
 }
 
-// The block's four words of the round's sums (even threads hold the first
-// message, odd ones the second).
-__device__ __forceinline__ void tile_words(const wide &acc_w, uint64_t (&v)[4]) {
-  const f128 s = greduce(acc_w);
-  const bool odd = threadIdx.x & 1;
-  v[0] = odd ? 0 : s.lo;
-  v[1] = odd ? 0 : s.hi;
-  v[2] = odd ? s.lo : 0;
-  v[3] = odd ? s.hi : 0;
-}
-
-__global__ void __launch_bounds__(kMidThreads) gkr_round(
-    f128 *__restrict__ c, size_t n_half, size_t h, f128 r_arg, f128 *__restrict__ eq, int at_one,
-    unsigned long long *acc, Publish pub, RoundLink lk, size_t colmask, size_t live) {
-  f128 r;
-  if (!round_begin(lk, r_arg, r)) return;
-  __shared__ TileShared S;
-  mul_table_build(S.T, r);
-  wide acc_w = wzero();
-  for (size_t x0 = (size_t)blockIdx.x * kMidTile; x0 < h; x0 += (size_t)gridDim.x * kMidTile)
-    bind_tile(S, c, c + n_half, eq, h, x0, at_one, colmask, live, acc_w);
-  uint64_t v[4];
-  tile_words(acc_w, v);
-  block_xor_atomic<4>(v, acc);
-  round_end(acc, pub, lk);
-}
-
-// The middle rounds of a layer (bind r_i for i = i_hi .. i_lo) in one
-// cooperative launch of B blocks that stays resident, with the layer's live
-// entries in shared memory from the first round to the last. With the period
-// P = B kMidRuns, block b owns the positions whose residue mod P lies in
-// [b kMidRuns, (b + 1) kMidRuns); slot m of the block is position
-// P (m / kMidRuns) + b kMidRuns + m % kMidRuns. Every h of these rounds is a
-// multiple of P, so positions y, y + h, y + 2h, y + 3h belong to one block and
-// sit at slots m, m + E, m + 2E, m + 3E (E = h / B elements per block): each
-// round binds slot m < 2E from slots m and m + 2E in place and sums elements
-// j < E from slots j and j + E. Blocks share nothing but the challenge and the
-// sums: block 0 reads r_i from the downbox (publication d0 + n - 1 - i) and
-// relays it through ctl; each block adds its share of the sums into acc and
-// the last one through the round posts them as publication p0 + n - i. The
-// entries the tail kernel reads are written back at the end. All blocks are
-// resident together (cooperative launch), so the relay waits end; each is
-// bounded all the same. A lane proving alone uses kMidBlocks blocks; a pooled
-// lane, which shares the GPU with other lanes' kernels, kMidPoolBlocks (each
-// block then holds four times the entries, 192 KB of shared memory at the
-// largest round).
-constexpr int kMidBlocks = 128;      // a lane proving alone
-constexpr int kMidPoolBlocks = 32;   // a pooled lane, sharing the GPU with others
-constexpr int kMidRuns = 4;
-static_assert((size_t)kMidBlocks * kMidRuns <= 2 * (size_t)kTailH,
-              "the tail starts below the middle rounds");
-
-// The period is gridDim.x kMidRuns positions: the grid is kMidBlocks blocks
-// or fewer.
-__device__ __forceinline__ size_t mid_pos(size_t m) {
-  const size_t period = (size_t)gridDim.x * kMidRuns;
-  return period * (m / kMidRuns) + (size_t)blockIdx.x * kMidRuns + m % kMidRuns;
-}
-
-// Dynamic shared memory for e0 elements: L and R at slots < 2 e0 (lo) and
-// [2 e0, 4 e0) (hi), eq at slots < 2 e0, and the products with e.
-__host__ __device__ constexpr size_t mid_smem_bytes(size_t e0) { return 12 * e0 * sizeof(f128); }
-
-__global__ void __launch_bounds__(kMidThreads) gkr_mid(
-    f128 *__restrict__ c, size_t n_half, int n, int i_hi, int i_lo, f128 *__restrict__ eq,
-    unsigned long long at_one_mask, unsigned long long *acc_base, Mailbox *mb,
-    unsigned long long p0, const Mailbox *down, unsigned long long d0, RoundCtl *ctl,
-    size_t colmask, size_t live) {
-  extern __shared__ f128 dyn[];
+// Thread (i, group) sums J features j of its group over the block's chunks of
+// 128 columns; blockIdx.y takes the other j. J = 16 uses a chunk's table 16
+// times per thread; J = 4 spreads few chunks over the chip.
+template <int NFEAT, int J>
+__global__ void __launch_bounds__(GramShape<NFEAT>::kThreadsPer) gkr_gram(
+    const f128 *__restrict__ cols, uint32_t live, int log_cols,
+    const __grid_constant__ EqFactors<5> eq, unsigned long long *X) {
+  using S = GramShape<NFEAT>;
   __shared__ MulTable T;
+  __shared__ uint4 rows[128];  // row r's bits of the chunk's 128 columns
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int i = t % NFEAT, group = t / NFEAT;
+  const int j0 = (blockIdx.y * S::kGroups + group) * J;
+  f128 sum[J], one = mk(0, 0);
+#pragma unroll
+  for (int q = 0; q < J; q++) sum[q] = mk(0, 0);
+  const uint32_t chunks = (live + 127) / 128;
+  for (uint32_t ch = blockIdx.x; ch < chunks; ch += gridDim.x) {
+    if (t < 128) {
+      f128 e = eq.f[0][t];
+#pragma unroll 1
+      for (int g = 1; g < 5 && g * kFacLog < log_cols; g++)
+        e = pass_mul(e, eq.f[g][(ch >> ((g - 1) * kFacLog)) & ((1 << kFacLog) - 1)]);
+      T.lo[t >> 2][1 << (t & 3)] = e.lo;
+      T.hi[t >> 2][1 << (t & 3)] = e.hi;
+    }
+    if (warp < 8) {  // 32 columns by 64 rows per warp, transposed by ballots
+      const uint32_t c = ch * 128 + (warp & 3) * 32 + lane;
+      const ulonglong2 w =
+          c < live ? __ldg(reinterpret_cast<const ulonglong2 *>(cols + c)) : make_ulonglong2(0, 0);
+      const uint64_t half = warp < 4 ? w.x : w.y;
+      uint32_t r0 = 0, r1 = 0;
+#pragma unroll 8
+      for (int r = 0; r < 32; r++) {
+        const uint32_t a = __ballot_sync(0xffffffffu, (half >> r) & 1);
+        const uint32_t b = __ballot_sync(0xffffffffu, (half >> (r + 32)) & 1);
+        if (lane == r) r0 = a, r1 = b;
+      }
+      uint32_t *out = reinterpret_cast<uint32_t *>(rows + (warp < 4 ? 0 : 64));
+      out[4 * lane + (warp & 3)] = r0;
+      out[4 * (lane + 32) + (warp & 3)] = r1;
+    }
+    __syncthreads();
+    for (int e = t; e < 512; e += S::kThreadsPer) {
+      const int k = e >> 4, v = e & 15;
+      if (v != 0 && (v & (v - 1)) == 0) continue;  // written above
+      uint64_t lo = 0, hi = 0;
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        if ((v >> q) & 1) {
+          lo ^= T.lo[k][1 << q];
+          hi ^= T.hi[k][1 << q];
+        }
+      T.lo[k][v] = lo;
+      T.hi[k][v] = hi;
+    }
+    __syncthreads();
+    const uint4 fa = feature<NFEAT>(rows, i, false);
+#pragma unroll
+    for (int q = 0; q < J; q++)
+      sum[q] = gadd(sum[q], pass_table(&T, and_bits(fa, feature<NFEAT>(rows, j0 + q, true))));
+    if (blockIdx.y == 0 && group < 2) {  // the features by themselves
+      const uint4 f = group ? feature<NFEAT>(rows, i, true) : fa;
+      one = gadd(one, pass_table(&T, and_bits(f, f)));
+    }
+    __syncthreads();  // the chunk's table before the next chunk's
+  }
+  auto add = [&](int a, int b, f128 v) {
+    unsigned long long *x = X + 2 * (a * S::kRow + b);
+    if (v.lo) atomicXor(x, (unsigned long long)v.lo);
+    if (v.hi) atomicXor(x + 1, (unsigned long long)v.hi);
+  };
+#pragma unroll
+  for (int q = 0; q < J; q++) add(i, j0 + q, sum[q]);
+  if (blockIdx.y == 0 && group < 2) group ? add(NFEAT, i, one) : add(i, NFEAT, one);
+}
+
+// From the counts to the point sums of all row rounds: first
+// H[a][b] = sum over the columns of eq L(a) R(b) for every pair of rows, then,
+// a coordinate at a time, {0, 1, infinity} from the pairs of its bit: the
+// entries (0,0), (1,1) and the sum of all four. 16 blocks of 256 threads form H
+// and the top coordinates (two, or one) by lane exchanges; the last block to
+// finish does the other four in shared memory and posts the 729 or 243 sums.
+template <int LAYER>
+__global__ void __launch_bounds__(256) gkr_moments(const unsigned long long *__restrict__ X,
+                                                   const f128 *__restrict__ images,
+                                                   f128 *__restrict__ mid, unsigned int *counter,
+                                                   unsigned long long *handover,
+                                                   unsigned long long seq) {
+  constexpr int kDone = LAYER == 0 ? 9 : 3;  // digit values formed by the lanes
+  constexpr int kFeat = LAYER == 0 ? 64 : 96, kRow = GramShape<kFeat>::kRow;
+  __shared__ f128 A[27 * 64], B[81 * 16];
+  __shared__ bool last;
+  const int t = threadIdx.x, u = blockIdx.x * 256 + t;
+  const int w = (u >> 4) & 255, a_low = w & 15, b_low = w >> 4;
+  auto delta = [&](int row) {
+    f128 d = ld(images + row);
+    d.lo ^= 1;
+    return d;
+  };
+  auto x_at = [&](int a, int b) {
+    if (a == kFeat && b == kFeat) return mk(1, 0);
+    const ulonglong2 v = __ldcg(reinterpret_cast<const ulonglong2 *>(X) + (a * kRow + b));
+    return mk(v.x, v.y);
+  };
+  auto lanes_xor = [](f128 v, int m) {
+    v.lo ^= __shfl_xor_sync(0xffffffffu, v.lo, m);
+    v.hi ^= __shfl_xor_sync(0xffffffffu, v.hi, m);
+    return v;
+  };
+  auto digit = [](int role) { return role == 0 ? 0 : role == 3 ? 1 : 2; };
+  const int role2 = (u >> 2) & 3;
+  f128 v;
+  if (LAYER == 0) {
+    const int a = a_low | (role2 & 1) << 4 | (u & 1) << 5;
+    const int b = b_low | (role2 >> 1) << 4 | ((u >> 1) & 1) << 5;
+    const f128 da = delta(a), db = delta(64 + b);
+    v = gadd(gadd(mk(1, 0), pass_mul(da, x_at(a, kFeat))),
+             pass_mul(db, gadd(x_at(kFeat, b), pass_mul(da, x_at(a, b)))));
+  } else {
+    // lane f of four: the terms with feature f of R (none, r, s, r s)
+    const int f = u & 3;
+    const int a = a_low | (role2 & 1) << 4, b = b_low | (role2 >> 1) << 4;
+    const f128 da = delta(a), da2 = delta(a + 64), db = delta(b + 32), db2 = delta(b + 96);
+    const int jb = f == 0 ? kFeat : 32 * (f - 1) + b;
+    v = gadd(gadd(x_at(kFeat, jb), pass_mul(da, x_at(a, jb))),
+             pass_mul(da2, gadd(x_at(32 + a, jb), pass_mul(da, x_at(64 + a, jb)))));
+    if (f & 1) v = pass_mul(v, db);
+    if (f & 2) v = pass_mul(v, db2);
+  }
+  // features are ordered r, s, r s: lane 1 has r, lane 2 s, lane 3 both
+  const f128 s1 = lanes_xor(lanes_xor(v, 1), 2);
+  const int role1 = u & 3;
+  if (LAYER == 1 || role1 == 1) v = s1;
+  const f128 s2 = lanes_xor(lanes_xor(v, 4), 8);
+  if (role2 == 1) v = s2;
+  if (role2 != 2) {
+    if (LAYER == 0) {
+      if (role1 != 2) st(mid + (3 * digit(role1) + digit(role2)) * 256 + w, v);
+    } else if (role1 == 0) {
+      st(mid + digit(role2) * 256 + w, v);
+    }
+  }
+  __threadfence();
+  __syncthreads();
+  if (t == 0) {
+    last = atomicAdd(counter, 1u) == gridDim.x - 1;
+    __threadfence();
+  }
+  __syncthreads();
+  if (!last) return;
+  auto ld_mid = [&](int k) {
+    const ulonglong2 q = __ldcg(reinterpret_cast<const ulonglong2 *>(mid) + k);
+    return mk(q.x, q.y);
+  };
+  // [done][2^r][2^r] (b, then a) -> [3 done][2^(r-1)][2^(r-1)]
+  auto step = [&](auto in, f128 *out, int done, int r) {
+    const int q = r - 1, per = 1 << (2 * q);
+    for (int k = t; k < 3 * done * per; k += 256) {
+      const int d = (k >> (2 * q)) % 3, base = ((k >> (2 * q)) / 3) << (2 * r);
+      const int a = k & ((1 << q) - 1), b = (k >> q) & ((1 << q) - 1);
+      const int e00 = base + (b << r) + a, e01 = e00 + (1 << q), e10 = e00 + (1 << (q + r)),
+                e11 = e10 + (1 << q);
+      out[k] = d == 0 ? in(e00) : d == 1 ? in(e11)
+                                         : gadd(gadd(in(e00), in(e01)), gadd(in(e10), in(e11)));
+    }
+    __syncthreads();
+  };
+  step(ld_mid, A, kDone, 4);
+  step([&](int k) { return A[k]; }, B, 3 * kDone, 3);
+  step([&](int k) { return B[k]; }, A, 9 * kDone, 2);
+  step([&](int k) { return A[k]; }, B, 27 * kDone, 1);
+  for (int k = t; k < 2 * 81 * kDone; k += 256)
+    handover_post(handover, seq, k, k & 1 ? B[k >> 1].hi : B[k >> 1].lo);
+  if (t == 0) *counter = 0;
+}
+
+// The layer's tables once its row coordinates are bound: L(c) and R(c) are one
+// plus sums over the features of column c of their coefficients (the bound
+// row's eq weight times the feature's), through 4-bit windows of the column's
+// bits.
+struct RowWeights {
+  f128 e[64];
+};
+
+template <int LAYER>
+__global__ void __launch_bounds__(kThreads) gkr_bound_rows(const f128 *__restrict__ cols, int s,
+                                                           const f128 *__restrict__ images,
+                                                           const __grid_constant__ RowWeights eps,
+                                                           f128 *__restrict__ L,
+                                                           f128 *__restrict__ R) {
+  constexpr int kFeat = LAYER == 0 ? 64 : 96, kWin = kFeat / 4;
+  __shared__ uint64_t lo[2 * kWin][16], hi[2 * kWin][16];
   const int t = threadIdx.x;
-  const size_t e0 = ((size_t)1 << (i_hi - 1)) / gridDim.x;
-  f128 *SL = dyn, *SL1 = dyn + 2 * e0, *SR = dyn + 4 * e0, *SR1 = dyn + 6 * e0;
-  f128 *EQ = dyn + 8 * e0, *P = dyn + 10 * e0, *Q = dyn + 11 * e0;
-  f128 *L = c, *R = c + n_half;
-  {
-    const size_t h0 = (size_t)1 << (i_hi - 1);
-    for (size_t m = t; m < 2 * e0; m += kMidThreads) {
-      const size_t y = mid_pos(m);
-      SL[m] = ld(L + y);
-      SL1[m] = ld(L + y + 2 * h0);
-      SR[m] = ld(R + y);
-      SR1[m] = ld(R + y + 2 * h0);
-      EQ[m] = ld(eq + y);
-    }
-  }
-  for (int i = i_hi; i >= i_lo; i--) {
-    RoundCtl *cl = ctl + (n - 1 - i);
-    unsigned long long rw[2];
-    if (!resident_challenge(down, d0 + (n - 1 - i), cl, rw)) return;
-    mul_table_build(T, mk(rw[0], rw[1]));
-    const size_t e = ((size_t)1 << (i - 1)) / gridDim.x;
-    const int at_one = (int)((at_one_mask >> (i - 1)) & 1);
-    // the upper half of the live slots: separate arrays in the first round,
-    // slots [2e, 4e) of the lower ones after it
-    const f128 *hl = i == i_hi ? SL1 : SL + 2 * e, *hr = i == i_hi ? SR1 : SR + 2 * e;
-    // level 1: the 2e slots of L and of R bound at r; the eq table summed down
-    for (size_t u = t; u < 4 * e; u += kMidThreads) {
-      const bool right = u >= 2 * e;
-      const size_t m = right ? u - 2 * e : u;
-      if (padded(mid_pos(m), colmask, live)) continue;  // stays one
-      f128 *lo = right ? SR : SL;
-      const f128 a0 = lo[m];
-      lo[m] = gadd(a0, mul_table(T, gadd((right ? hr : hl)[m], a0)));
-    }
-    for (size_t j = t; j < e; j += kMidThreads) EQ[j] = gadd(EQ[j], EQ[j + e]);
-    __syncthreads();
-    // level 2: P = e * L_b, Q = e * (L_1 + L_0) for the e elements
-    for (size_t u = t; u < 2 * e; u += kMidThreads) {
-      const size_t j = u >> 1;
-      const f128 ev = EQ[j];
-      if (padded(mid_pos(j), colmask, live)) {  // e * 1 and e * 0
-        if (u & 1)
-          Q[j] = mk(0, 0);
-        else
-          P[j] = ev;
-      } else if (u & 1) {
-        Q[j] = gmul(ev, gadd(SL[j + e], SL[j]));
-      } else {
-        P[j] = gmul(ev, at_one ? SL[j + e] : SL[j]);
-      }
-    }
-    __syncthreads();
-    // level 3: P * R_b into the first sum, Q * (R_1 + R_0) into the second
-    wide acc_w = wzero();
-    for (size_t u = t; u < 2 * e; u += kMidThreads) {
-      const size_t j = u >> 1;
-      if (padded(mid_pos(j), colmask, live)) {  // P * 1 and Q * 0
-        if (!(u & 1)) {
-          acc_w.w0 ^= P[j].lo;
-          acc_w.w1 ^= P[j].hi;
-        }
-      } else if (u & 1) {
-        wacc(acc_w, gmul_wide(Q[j], gadd(SR[j + e], SR[j])));
-      } else {
-        wacc(acc_w, gmul_wide(P[j], at_one ? SR[j + e] : SR[j]));
-      }
-    }
-    uint64_t v[4];
-    tile_words(acc_w, v);  // kMidThreads is even: thread parity = u parity
-    unsigned long long *acc = acc_base + 4 * (n - i);
-    block_xor_atomic<4>(v, acc);  // synchronises the block: P, Q, SL, SR free again
-    if (t == 0) {
-      __threadfence();
-      const unsigned int prev = atomicAdd(&cl->done, 1u);
-      if (prev == gridDim.x - 1) {
-        __threadfence();
-#pragma unroll
-        for (int k = 0; k < 4; k++) mailbox_post(mb, p0 + (n - i), k, atomicExch(acc + k, 0ull));
-      }
-    }
-  }
-  // the live entries after round i_lo: L and R below 2 h, eq below h
-  const size_t e = ((size_t)1 << (i_lo - 1)) / gridDim.x;
-  for (size_t m = t; m < 2 * e; m += kMidThreads) {
-    const size_t y = mid_pos(m);
-    st(L + y, SL[m]);
-    st(R + y, SR[m]);
-  }
-  for (size_t j = t; j < e; j += kMidThreads) st(eq + mid_pos(j), EQ[j]);
-}
-
-// The bind after round 0: one pair left in each half. Delivered through the
-// mailbox when publishing, else to out[0..2).
-__global__ void gkr_final_bind(const f128 *__restrict__ c, size_t n_half, f128 r, f128 *out,
-                               Publish pub) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    f128 l0 = ld(c), l1 = ld(c + 1), r0 = ld(c + n_half), r1 = ld(c + n_half + 1);
-    f128 lr = gadd(l0, gmul(r, gadd(l1, l0)));
-    f128 rr = gadd(r0, gmul(r, gadd(r1, r0)));
-    if (pub.counter) {
-      mailbox_post(pub.mailbox, pub.seq, 0, lr.lo);
-      mailbox_post(pub.mailbox, pub.seq, 1, lr.hi);
-      mailbox_post(pub.mailbox, pub.seq, 2, rr.lo);
-      mailbox_post(pub.mailbox, pub.seq, 3, rr.hi);
+  for (int u = t; u < 2 * kFeat; u += kThreads) {
+    const int side = u / kFeat, i = u % kFeat;
+    f128 k;
+    if (LAYER == 0) {
+      f128 d = ld(images + 64 * side + i);
+      d.lo ^= 1;
+      k = pass_mul(eps.e[i], d);
     } else {
-      st(out, lr);
-      st(out + 1, rr);
+      const int a = i & 31, row = a + 32 * side;
+      f128 d = ld(images + row), d2 = ld(images + row + 64);
+      d.lo ^= 1;
+      d2.lo ^= 1;
+      k = pass_mul(eps.e[a], i < 32 ? d : d2);
+      if (i >= 64) k = pass_mul(k, d);
     }
+    lo[u >> 2][1 << (u & 3)] = k.lo;
+    hi[u >> 2][1 << (u & 3)] = k.hi;
   }
-}
-
-// The last rounds of a layer in one resident block. From iteration i0 (where
-// the live halves hold 4h0 = 2^(i0+1) entries, h0 <= kTailH) down to 0 the
-// block keeps both halves and the eq table in shared memory; each iteration
-// waits for the host's challenge r_i in the lane's downbox (bounded), binds
-// and sums exactly as gkr_bind_sums / gkr_final_bind, and posts the round's
-// four words to the mailbox (publication seq0 + i0 - i). A missing challenge
-// ends the kernel without a post, which the host reads as a failed round.
-// At iteration i_host (-1: none) the block hands its tables to the host
-// instead and ends: rounds whose tables are that small cost the host about a
-// microsecond each, against a PCIe round trip and a device step per round.
-//
-// A round is a chain of three dependent products per element (the bind,
-// e * L, then * R); with few elements one thread per element leaves the
-// block idle behind that chain, so the round is spread by product instead:
-// the 4h binds (and the eq update) across the block, then the 2h products
-// with e, then the 2h wide products, each level one product per thread.
-constexpr int kTailThreads = 512;
-constexpr unsigned long long kTailWaitNs = 2000000000ull;  // 2 s per challenge
-
-__global__ void __launch_bounds__(kTailThreads) gkr_tail(const f128 *__restrict__ c,
-                                                         size_t n_half, int i0,
-                                                         const f128 *__restrict__ eq,
-                                                         uint32_t at_one_mask, Mailbox *mb,
-                                                         unsigned long long seq0,
-                                                         const Mailbox *down,
-                                                         unsigned long long dseq0, size_t colmask,
-                                                         size_t live_cols, int i_host,
-                                                         unsigned long long *handover,
-                                                         unsigned long long hseq) {
-  __shared__ f128 L[4 * kTailH], R[4 * kTailH], E[2 * kTailH];
-  __shared__ uint64_t red[4][kTailThreads / 32];
-  __shared__ unsigned long long chal[2];
-  __shared__ int ok;
-  const int h0 = i0 > 0 ? 1 << (i0 - 1) : 1;
-  const int live = i0 > 0 ? 4 * h0 : 2;
-  for (int k = threadIdx.x; k < live; k += blockDim.x) {
-    L[k] = ld(c + k);
-    R[k] = ld(c + n_half + k);
+  __syncthreads();
+  for (int e = t; e < 2 * kWin * 16; e += kThreads) {
+    const int k = e >> 4, v = e & 15;
+    if (v != 0 && (v & (v - 1)) == 0) continue;  // written above
+    uint64_t a = 0, b = 0;
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+      if ((v >> q) & 1) {
+        a ^= lo[k][1 << q];
+        b ^= hi[k][1 << q];
+      }
+    lo[k][v] = a;
+    hi[k][v] = b;
   }
-  for (int k = threadIdx.x; k < 2 * h0 && i0 > 0; k += blockDim.x) E[k] = ld(eq + k);
-  for (int i = i0; i >= 0; i--) {
-    if (i == i_host) {
-      // the layer's last rounds run on the host: the tables as they stand
-      // before r_i's bind (L and R: 4h entries each, then E: 2h) go out as
-      // handover publication hseq, two words per entry, and the block ends
-      const int h = 1 << (i - 1), nl = 4 * h;
-      __syncthreads();  // the tables as loaded (a first iteration has no barrier yet)
-      for (int k = threadIdx.x; k < 2 * nl + 2 * h; k += blockDim.x) {
-        const f128 v = k < nl ? L[k] : k < 2 * nl ? R[k - nl] : E[k - 2 * nl];
-        handover_post(handover, hseq, 2 * k, v.lo);
-        handover_post(handover, hseq, 2 * k + 1, v.hi);
-      }
-      return;
-    }
-    if (threadIdx.x == 0) ok = mailbox_wait_device(down, dseq0 + (i0 - i), 2, chal, kTailWaitNs);
-    __syncthreads();
-    if (!ok) return;
-    const f128 r = mk(chal[0], chal[1]);
-    const unsigned long long seq = seq0 + (i0 - i);
-    if (i == 0) {
-      if (threadIdx.x == 0) {
-        f128 lr = gadd(L[0], gmul(r, gadd(L[1], L[0])));
-        f128 rr = gadd(R[0], gmul(r, gadd(R[1], R[0])));
-        mailbox_post(mb, seq, 0, lr.lo);
-        mailbox_post(mb, seq, 1, lr.hi);
-        mailbox_post(mb, seq, 2, rr.lo);
-        mailbox_post(mb, seq, 3, rr.hi);
-      }
-      return;
-    }
-    const int h = 1 << (i - 1), h2 = 2 * h;
-    const int at_one = (at_one_mask >> (i - 1)) & 1;
-    // level 1: the binds of round i+1 at r; entry (x, q) is L[x], L[x+h],
-    // R[x], R[x+h] for q = 0..3, each read and written by one thread only;
-    // the q = 0 thread also sums the eq table down
-    for (int t = threadIdx.x; t < 4 * h; t += blockDim.x) {
-      const int x = t >> 2, q = t & 3;
-      if (q == 0) E[x] = gadd(E[x], E[x + h]);
-      if (padded((size_t)x, colmask, live_cols)) continue;  // stays one
-      f128 *T = q < 2 ? L : R;
-      const int at = x + (q & 1) * h;
-      T[at] = gadd(T[at], gmul(r, gadd(T[at + h2], T[at])));
-    }
-    __syncthreads();
-    // level 2: P = e * L_b, Q = e * (L_1 + L_0), kept in the halves' upper
-    // quarters [2h, 3h), which the binds above have consumed
-    f128 *P = L + h2, *Q = R + h2;
-    for (int t = threadIdx.x; t < 2 * h; t += blockDim.x) {
-      const int x = t >> 1;
-      const f128 e = E[x];
-      if (padded((size_t)x, colmask, live_cols)) {  // e * 1 and e * 0
-        if (t & 1)
-          Q[x] = mk(0, 0);
-        else
-          P[x] = e;
-        continue;
-      }
-      if (t & 1)
-        Q[x] = gmul(e, gadd(L[x + h], L[x]));
-      else
-        P[x] = gmul(e, at_one ? L[x + h] : L[x]);
-    }
-    __syncthreads();
-    // level 3: P * R_b into the first sum, Q * (R_1 + R_0) into the second
-    uint64_t v[4] = {0, 0, 0, 0};
-    for (int t = threadIdx.x; t < 2 * h; t += blockDim.x) {
-      const int x = t >> 1;
-      if (padded((size_t)x, colmask, live_cols)) {  // P * 1 and Q * 0
-        if (!(t & 1)) {
-          v[0] ^= P[x].lo;
-          v[1] ^= P[x].hi;
-        }
-        continue;
-      }
-      if (t & 1) {
-        f128 p = gmul(Q[x], gadd(R[x + h], R[x]));
-        v[2] ^= p.lo;
-        v[3] ^= p.hi;
+  __syncthreads();
+  const size_t n = (size_t)1 << s;
+  for (size_t c = blockIdx.x * (size_t)blockDim.x + t; c < n; c += (size_t)gridDim.x * blockDim.x) {
+    const uint4 w = __ldg(reinterpret_cast<const uint4 *>(cols + c));
+#pragma unroll
+    for (int side = 0; side < 2; side++) {
+      uint32_t bits[kFeat / 32];
+      if (LAYER == 0) {
+        bits[0] = side ? w.z : w.x;
+        bits[1] = side ? w.w : w.y;
       } else {
-        f128 p = gmul(P[x], at_one ? R[x + h] : R[x]);
-        v[0] ^= p.lo;
-        v[1] ^= p.hi;
+        bits[0] = side ? w.y : w.x;
+        bits[1] = side ? w.w : w.z;
+        bits[kFeat / 32 - 1] = bits[0] & bits[1];
       }
-    }
-    // block XOR-reduction of the four words; thread 0 posts
+      uint64_t a = 1, b = 0;
 #pragma unroll
-    for (int k = 0; k < 4; k++)
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) v[k] ^= __shfl_xor_sync(0xffffffffu, v[k], off);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0)
-      for (int k = 0; k < 4; k++) red[k][warp] = v[k];
-    __syncthreads();
-    if (warp == 0) {
-      const int nw = blockDim.x >> 5;
-      for (int k = 0; k < 4; k++) {
-        uint64_t x = lane < nw ? red[k][lane] : 0;
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) x ^= __shfl_xor_sync(0xffffffffu, x, off);
-        v[k] = x;
+      for (int k = 0; k < kWin; k++) {
+        const uint32_t v = (bits[k / 8] >> (4 * (k % 8))) & 15u;
+        a ^= lo[side * kWin + k][v];
+        b ^= hi[side * kWin + k][v];
       }
-      if (lane == 0)
-        for (int k = 0; k < 4; k++) mailbox_post(mb, seq, k, v[k]);
+      st((side ? R : L) + c, mk(a, b));
     }
-    __syncthreads();  // this round's tables before the next round's reads
   }
 }
 
-static Publish arm(GkrScratch &sc) {
-  return sc.channel ? sc.channel->arm() : Publish{nullptr, nullptr, 0};
+// Tables of this many entries or fewer (per half) go to the host: a round on
+// them costs the host a few microseconds, a device turn about 14.
+constexpr int kHostLog = 8;
+static_assert(4 << kHostLog <= kHandoverWords, "the last tables fit one handover");
+// A layer's first pass binds nothing, so three rounds of it make 4.4 products
+// per entry where two make 3.25 (and leave a table 4 times the size for the
+// next pass): two rounds from this size on, where products are the cost.
+constexpr int kFirstLog = 17;
+
+// Prefix tables of eq over up to kFacLog coordinates: entries [2^i, 2^(i+1))
+// hold eq over the first i of them.
+struct EqHeap {
+  f128 v[2 << kFacLog];
+  void build(const f128 *z, int n) {
+    v[1] = mk(1, 0);
+    for (int i = 0; i < n; i++) {
+      const f128 *p = v + ((size_t)1 << i);
+      f128 *q = v + ((size_t)2 << i);
+      for (int k = 0; k < 1 << i; k++) {
+        const f128 one = gmul(p[k], z[i]);
+        q[k] = gadd(p[k], one);
+        q[k + (1 << i)] = one;
+      }
+    }
+  }
+  const f128 *prefix(int n) const { return v + ((size_t)1 << n); }
+};
+
+static unsigned int pass_grid(uint32_t count, int lx) {
+  const uint32_t tiles = (count + (1u << lx) - 1) >> lx;
+  return std::max(1u, std::min(tiles, 2u * kSMs));
 }
 
-// The round's four words, from the mailbox or by a copy of `src`.
-static void round_read(GkrScratch &sc, const void *src, cudaStream_t s) {
-  if (sc.channel) {
-    sc.channel->wait(s, sc.host, 4);
-    return;
+template <int K, int NF>
+static void launch_pass_nf(f128 *c, size_t n_half, int log_m, const PassBind &b, const EqHeap *heap,
+                           size_t colmask, uint32_t live, uint32_t count, GkrScratch &sc,
+                           unsigned long long seq, cudaStream_t st) {
+  EqFactors<NF> eq;
+  for (int g = 0; g < NF; g++) {
+    const int have = std::min(kFacLog, std::max(0, log_m - g * kFacLog));
+    memcpy(eq.f[g], heap[g].prefix(have), sizeof(f128) << have);
   }
-  BZ_CUDA(cudaMemcpyAsync(sc.host, src, 32, cudaMemcpyDeviceToHost, s));
-  BZ_CUDA(stream_wait(s));
+  // the largest tile that still gives every SM one: wide tiles fill the turns
+  // (27 points of 32 positions are three per thread), narrow ones the chip
+  int lx = 5;
+  while (lx > 2 && (count >> lx) < (uint32_t)kSMs) lx--;
+  gkr_pass<K, NF><<<pass_grid(count, lx), kPassThreads, 0, st>>>(
+      c, n_half, log_m, b, eq, colmask, live, count, lx, sc.acc, sc.channel->counter,
+      sc.channel->handover_dev, seq);
+  BZ_LAUNCH_CHECK();
+}
+
+template <int K>
+static void launch_pass(f128 *c, size_t n_half, int log_m, const PassBind &b, const EqHeap *heap,
+                        size_t colmask, uint32_t live, uint32_t count, GkrScratch &sc,
+                        unsigned long long seq, cudaStream_t st) {
+  if (log_m <= 2 * kFacLog)
+    launch_pass_nf<K, 2>(c, n_half, log_m, b, heap, colmask, live, count, sc, seq, st);
+  else
+    launch_pass_nf<K, 5>(c, n_half, log_m, b, heap, colmask, live, count, sc, seq, st);
 }
 
 void gkr_build(const f128 *cols, int s, const f128 *images, GkrScratch &sc, cudaStream_t st_) {
-  size_t total = (size_t)128 << s;
-  if (sc.capacity < total) throw CudaError("gkr_build: scratch too small");
-  gkr_leaves<<<grid_for(total), kThreads, 0, st_>>>(cols, s, images, sc.layer[0]);
+  if (sc.capacity < (size_t)128 << s) throw CudaError("gkr_build: scratch too small");
+  const size_t n = (size_t)1 << s, live = sc.live_cols ? sc.live_cols : n;
+  const dim3 grid(grid_for(n, kThreads, kSMs / 2), 16);
+  gkr_low_layers<<<grid, kThreads, 0, st_>>>(cols, s, images, sc.layer[2], sc.layer[3]);
   BZ_LAUNCH_CHECK();
-  size_t len = total;
-  const size_t colmask = ((size_t)1 << s) - 1;
-  const size_t live = sc.live_cols ? sc.live_cols : colmask + 1;
-  for (int j = 0; j < 7; j++) {
-    gkr_parent<<<grid_for(len / 2), kThreads, 0, st_>>>(sc.layer[j], len / 2, sc.layer[j + 1],
-                                                         colmask, live);
-    BZ_LAUNCH_CHECK();
-    len /= 2;
+  gkr_high_layers<<<grid_for(n, 128, kSMs * 16), 128, 0, st_>>>(
+      sc.layer[3], s, sc.layer[4], sc.layer[5], sc.layer[6], sc.layer[7], live);
+  BZ_LAUNCH_CHECK();
+}
+
+// X of layer 0 or 1 (zeroed before) over the live columns.
+template <int NFEAT>
+static void launch_gram(const f128 *cols, uint32_t live, int s, const EqHeap *heap,
+                        unsigned long long *X, cudaStream_t st) {
+  using S = GramShape<NFEAT>;
+  EqFactors<5> eq;
+  for (int g = 0; g < 5; g++) {
+    const int have = std::min(kFacLog, std::max(0, s - g * kFacLog));
+    memcpy(eq.f[g], heap[g].prefix(have), sizeof(f128) << have);
   }
+  if (s < kFacLog)  // weights of columns that do not exist
+    memset(eq.f[0] + ((size_t)1 << s), 0, sizeof(f128) * ((1 << kFacLog) - ((size_t)1 << s)));
+  const uint32_t chunks = (live + 127) / 128;
+  // with J = 16 a block takes 64 x 64 (or 48 x 96) sums of a chunk; below two
+  // chunks per SM that leaves SMs idle, so four times the blocks take a quarter
+  if (chunks >= 2 * kSMs)
+    gkr_gram<NFEAT, 16><<<dim3(std::min(chunks, (uint32_t)(4 * kSMs)), NFEAT / (16 * S::kGroups)),
+                          S::kThreadsPer, 0, st>>>(cols, live, s, eq, X);
+  else
+    gkr_gram<NFEAT, 4><<<dim3(chunks, NFEAT / (4 * S::kGroups)), S::kThreadsPer, 0, st>>>(
+        cols, live, s, eq, X);
+  BZ_LAUNCH_CHECK();
 }
 
 static f128 eq_factor(f128 r, f128 z) { return gadd(gadd(mk(1, 0), r), z); }
 
-// One bind round of hh elements per half: by tiles up to kMidMaxH, one
-// element per thread above (issue bound there).
-// Grid of the resident middle rounds for a lane: kMidBlocks for a lane proving
-// alone; for a pooled lane none (every middle round a queued launch), or
-// kMidPoolBlocks with BITZ_POOL_MID=1. On the batched mix the pooled grids cut
-// a proof's launches from 189 to 130 but not its time: at 24 lanes and more
-// the cooperative grids of different lanes compete for SMs and the mix ran
-// 10-20 % slower, so they are off by default.
-int gkr_mid_blocks(bool alone) {
-  if (alone) return kMidBlocks;
-  static const bool pool = [] {
-    const char *e = getenv("BITZ_POOL_MID");
-    return e && e[0] == '1';
-  }();
-  return pool ? kMidPoolBlocks : 0;
-}
+// One layer's rounds: the transcript's side of round i from its two sums (at
+// zero, or at one when the point's coordinate is zero, and at infinity).
+struct LayerRounds {
+  const f128 *point;
+  f128 *next;
+  uint32_t grind_bits;
+  Transcript &ts;
+  f128 eq_bound = mk(1, 0);
 
-// Elements below h whose packed column holds bits of h (the rest are padding).
-static double live_threads(size_t h, size_t colmask, size_t live) {
-  return h > colmask ? (double)(h / (colmask + 1)) * (double)live : (double)std::min(h, live);
-}
-
-static void launch_bind(f128 *c, size_t n_half, size_t hh, f128 r, f128 *eq, int at_one,
-                        unsigned long long *acc, const Publish &pub, const RoundLink &lk,
-                        size_t colmask, size_t live, cudaStream_t st) {
-  if (hh <= kMidMaxH)
-    gkr_round<<<(unsigned)((hh + kMidTile - 1) / kMidTile), kMidThreads, 0, st>>>(
-        c, n_half, hh, r, eq, at_one, acc, pub, lk, colmask, live);
-  else
-    gkr_bind_sums<<<grid_for(hh), kThreads, 0, st>>>(c, n_half, hh, r, eq, at_one, acc, pub, lk,
-                                                      colmask, live);
-  BZ_LAUNCH_CHECK();
-}
-
-// gkr_mid over bind rounds i_hi .. i_lo as a cooperative launch of
-// sc.mid_blocks blocks (every block must be resident together).
-static void launch_mid(f128 *c, size_t n_half, int n, int i_hi, int i_lo, const f128 *point,
-                       GkrScratch &sc, unsigned long long p0, unsigned long long d0,
-                       size_t colmask, size_t live, cudaStream_t st) {
-  const int nb = sc.mid_blocks;
-  const size_t e0 = ((size_t)1 << (i_hi - 1)) / nb;
-  const size_t smem = mid_smem_bytes(e0);
-  // residency for the largest rounds of each grid size (the kernel's shared
-  // memory limit raised once to the largest, the pooled grid's)
-  static const int capacity[2] = {[] {
-    int dev = 0, sms = 0, per_sm = 0;
-    BZ_CUDA(cudaGetDevice(&dev));
-    BZ_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    BZ_CUDA(cudaFuncSetAttribute(gkr_mid, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)mid_smem_bytes(kMidMaxH / kMidPoolBlocks)));
-    BZ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gkr_mid, kMidThreads,
-                                                          mid_smem_bytes(kMidMaxH / kMidBlocks)));
-    return sms * per_sm;
-  }(), [] {
-    int dev = 0, sms = 0, per_sm = 0;
-    BZ_CUDA(cudaGetDevice(&dev));
-    BZ_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    BZ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &per_sm, gkr_mid, kMidThreads, mid_smem_bytes(kMidMaxH / kMidPoolBlocks)));
-    return sms * per_sm;
-  }()};
-  if (nb != kMidBlocks && nb != kMidPoolBlocks) throw CudaError("gkr_mid: unsupported grid");
-  if (capacity[nb == kMidBlocks ? 0 : 1] < nb)
-    throw CudaError("gkr_mid: the blocks do not fit resident together");
-  if (((size_t)1 << (i_lo - 1)) < (size_t)nb * kMidRuns || ((size_t)1 << (i_hi - 1)) > kMidMaxH)
-    throw CudaError("gkr_mid: round sizes outside the resident range");
-  unsigned long long mask = 0;
-  for (int i = i_lo; i <= i_hi; i++) mask |= (unsigned long long)gis_zero(point[i - 1]) << (i - 1);
-  RoundChannel *ch = sc.channel;
-  f128 *eq = sc.eq;
-  unsigned long long *acc = sc.acc;
-  Mailbox *mb = ch->dev;
-  const Mailbox *down = ch->down_dev;
-  RoundCtl *ctl = sc.ctl;
-  void *args[] = {&c,  &n_half, &n,    &i_hi, &i_lo, &eq,      &mask,  &acc,
-                  &mb, &p0,     &down, &d0,   &ctl,  &colmask, &live};
-  BZ_CUDA(cudaLaunchCooperativeKernel((const void *)gkr_mid, dim3(nb), dim3(kMidThreads), args,
-                                      smem, st));
-  BZ_LAUNCH_CHECK();
-}
-
-// The rounds from this iteration down run on the host once gkr_tail has
-// handed over its tables (h <= 2^(kHostTailI - 1) = 64 pairs).
-constexpr int kHostTailI = 7;
-
-// One iteration of gkr_tail on the host, with the same arithmetic: bind the
-// tables (L, R: 4h entries, E: 2h, h = 2^(i-1)) at r and leave the sums of
-// the next round in out, or, at i == 0, the bound pair (lr, rr).
-static void host_tail_round(std::vector<f128> &L, std::vector<f128> &R, std::vector<f128> &E,
-                            int i, f128 r, uint32_t at_one_mask, size_t colmask, size_t live,
-                            f128 out[2]) {
-  if (i == 0) {
-    out[0] = gadd(L[0], gmul(r, gadd(L[1], L[0])));
-    out[1] = gadd(R[0], gmul(r, gadd(R[1], R[0])));
-    return;
+  f128 round(int i, f128 at_zero, f128 at_one, f128 at_inf) {
+    const f128 z = point[i];
+    f128 msg[2] = {gmul(eq_bound, gis_zero(z) ? at_one : at_zero), gmul(eq_bound, at_inf)};
+    ts.prover_message(msg, 32);
+    ts.grind("gkr/cubic/v1", grind_bits);
+    const f128 r = ts.challenge_f128();
+    next[i] = r;
+    eq_bound = gmul(eq_bound, eq_factor(r, z));
+    return r;
   }
-  const size_t h = (size_t)1 << (i - 1), h2 = 2 * h;
-  const bool at_one = (at_one_mask >> (i - 1)) & 1;
-  for (size_t x = 0; x < h; x++) {
-    E[x] = gadd(E[x], E[x + h]);
-    if ((x & colmask) >= live) continue;  // a padded column stays one
-    for (int q = 0; q < 4; q++) {
-      std::vector<f128> &T = q < 2 ? L : R;
-      const size_t at = x + (q & 1) * h;
-      T[at] = gadd(T[at], gmul(r, gadd(T[at + h2], T[at])));
+
+  // k rounds from the 3^k point sums F (digit k - 1 of the index is coordinate
+  // `top`); the challenges go to r.
+  void from_points(std::vector<f128> &F, int top, int k, f128 *r) {
+    f128 e[32];   // eq over the coordinates below the current one, at zeros and ones
+    int at[32];   // and the index of that point
+    size_t block = F.size() / 3;
+    for (int t = 0; t < k; t++, block /= 3) {
+      const int rest = k - 1 - t;
+      e[0] = mk(1, 0);
+      at[0] = 0;
+      for (int q = 0, p = 1; q < rest; q++, p *= 3)
+        for (int x = 0; x < 1 << q; x++) {
+          const f128 one = gmul(e[x], point[top - k + 1 + q]);
+          e[x | 1 << q] = one;
+          e[x] = gadd(e[x], one);
+          at[x | 1 << q] = at[x] + p;
+        }
+      f128 s[3];
+      for (int d = 0; d < 3; d++) {
+        wide a = wzero();
+        for (int x = 0; x < 1 << rest; x++) wacc(a, gmul_wide(e[x], F[d * block + at[x]]));
+        s[d] = greduce(a);
+      }
+      r[t] = round(top - t, s[0], s[1], s[2]);
+      for (size_t x = 0; x < block; x++) {  // h0 + r (h1 + h0 + hinf) + r^2 hinf
+        const f128 h0 = F[x], h1 = F[block + x], hi = F[2 * block + x];
+        F[x] = gadd(h0, gmul(r[t], gadd(gadd(h0, h1), gadd(hi, gmul(r[t], hi)))));
+      }
     }
   }
-  f128 s0 = mk(0, 0), s1 = mk(0, 0);
-  for (size_t x = 0; x < h; x++) {
-    const f128 e = E[x];
-    if ((x & colmask) >= live) {  // e * 1 * 1 and e * 0 * 0
-      s0 = gadd(s0, e);
-      continue;
-    }
-    const f128 p = gmul(e, at_one ? L[x + h] : L[x]);
-    const f128 q = gmul(e, gadd(L[x + h], L[x]));
-    s0 = gadd(s0, gmul(p, at_one ? R[x + h] : R[x]));
-    s1 = gadd(s1, gmul(q, gadd(R[x + h], R[x])));
-  }
-  out[0] = s0;
-  out[1] = s1;
-}
 
-f128 gkr_prove(int s, const f128 *zeta, uint32_t grind_bits, Transcript &ts, GkrScratch &sc,
-               cudaStream_t st_, f128 *point_out) {
+  // The remaining n rounds on tables of 2^n entries; leaves the bound pair.
+  void from_tables(f128 *L, f128 *R, int n, const f128 *eq_prefix, f128 out[2]) {
+    for (int i = n - 1; i >= 0; i--) {
+      const int h = 1 << i;
+      const f128 *e = eq_prefix + h;  // eq over the i coordinates below
+      const bool one = gis_zero(point[i]);
+      wide sb = wzero(), si = wzero();
+      for (int x = 0; x < h; x++) {
+        const f128 lb = one ? L[x + h] : L[x], rb = one ? R[x + h] : R[x];
+        wacc(sb, gmul_wide(gmul(e[x], lb), rb));
+        wacc(si, gmul_wide(gmul(e[x], gadd(L[x], L[x + h])), gadd(R[x], R[x + h])));
+      }
+      const f128 b = greduce(sb);
+      const f128 r = round(i, b, b, greduce(si));
+      for (int x = 0; x < h; x++) {
+        L[x] = gadd(L[x], gmul(r, gadd(L[x], L[x + h])));
+        R[x] = gadd(R[x], gmul(r, gadd(R[x], R[x + h])));
+      }
+    }
+    out[0] = L[0];
+    out[1] = R[0];
+  }
+};
+
+constexpr size_t kGram0Words = 2 * 65 * 65, kGram1Words = 2 * 97 * 97;
+size_t gkr_gram_words() { return kGram0Words + kGram1Words; }
+
+f128 gkr_prove(const f128 *cols, int s, const f128 *images, const f128 *zeta, uint32_t grind_bits,
+               Transcript &ts, GkrScratch &sc, cudaStream_t st_, f128 *point_out) {
   f128 point[kMaxPoint], next[kMaxPoint];
   for (int i = 0; i < s; i++) point[i] = zeta[i];
   int n = s;
@@ -762,186 +825,122 @@ f128 gkr_prove(int s, const f128 *zeta, uint32_t grind_bits, Transcript &ts, Gkr
   f128 claim = mk(0, 0);
   KernelProbe &probe = KernelProbe::get();
   RoundChannel *ch = sc.channel;
-  bool tail = false;  // a tail kernel of this layer is resident and waiting
-  // without resident rounds every round is its own launch (same results)
-  const bool resident = resident_rounds_enabled();
-  // BITZ_ROUND_TRACE=1 prints the host time between consecutive round results
+  // BITZ_ROUND_TRACE=1 prints the host time of every device turn
   static const bool trace = getenv("BITZ_ROUND_TRACE") != nullptr;
-  auto t_prev = std::chrono::steady_clock::now();
-  // no other thread's device allocation while a round kernel waits for this one
-  ResidentScope gate(ch && resident);
-  try {
+  BZ_CUDA(cudaMemsetAsync(sc.acc, 0, 2 * (pow3(kPassMaxK) + 1) * sizeof(unsigned long long), st_));
+  std::vector<EqHeap> heap(5);
+  std::vector<uint64_t> words(kHandoverWords);
+  std::vector<f128> F, L, R;
+  BZ_CUDA(cudaMemsetAsync(sc.gram, 0, gkr_gram_words() * sizeof(unsigned long long), st_));
   for (int j = 6; j >= 0; j--) {
-    f128 *c = sc.layer[j];
-    size_t n_half = (size_t)1 << n;
-    int rounds = n;
-    // eq over the coordinates below the top one (2^(n-1) entries) as the
-    // factors over the lower a and the upper b of them; the accumulators and
-    // round controls of the layer cleared
-    const int a = (n - 1) / 2, b = (n - 1) - a;
-    f128 *lo = sc.eq_scratch, *hi = sc.eq_scratch + ((size_t)1 << a);
-    {
-      Point pt;
-      pt.n = n - 1;
-      for (int k = 0; k < n - 1; k++) pt.c[k] = point[k];
-      gkr_layer_setup<<<2, kThreads, 0, st_>>>(pt, a, b, lo, hi, sc.acc, 4 * (rounds + 1),
-                                               sc.ctl, rounds);
+    // layers 0 and 1 have tables only over the columns, once their rows are bound
+    f128 *c = j >= 2 ? sc.layer[j] : sc.bound;
+    const size_t n_half = (size_t)1 << (j >= 2 ? n : s);
+    for (int g = 0; g * kFacLog < n - 1 || g == 0; g++)
+      heap[g].build(point + g * kFacLog, std::min(kFacLog, std::max(0, n - 1 - g * kFacLog)));
+    for (int g = (n - 2) / kFacLog + 1; g < 5; g++) heap[g].v[1] = mk(1, 0);
+    LayerRounds rounds{point, next, grind_bits, ts};
+    PassBind b{};
+    int rem = n;  // coordinates not bound yet (b's are bound by the next pass)
+    auto t_prev = std::chrono::steady_clock::now();
+    auto mark = [&](const char *what) {
+      if (!trace) return;
+      const auto now = std::chrono::steady_clock::now();
+      fprintf(stderr, "[gkr] layer %d %s, %d coordinates: %7.2f us\n", j, what, rem,
+              std::chrono::duration<double, std::micro>(now - t_prev).count());
+      t_prev = now;
+    };
+    if (j < 2) {  // the rounds over the row coordinates, from the bits
+      const int k = 6 - j, points = pow3(k);
+      unsigned long long *X = sc.gram + (j == 0 ? 0 : kGram0Words);
+      if (j == 0)
+        launch_gram<64>(cols, (uint32_t)live, s, heap.data(), X, st_);
+      else
+        launch_gram<96>(cols, (uint32_t)live, s, heap.data(), X, st_);
+      const unsigned long long seq = ch->arm().seq;
+      (j == 0 ? gkr_moments<0> : gkr_moments<1>)<<<16, 256, 0, st_>>>(
+          X, images, sc.mid, ch->counter, ch->handover_dev, seq);
+      BZ_LAUNCH_CHECK();
+      ch->wait_handover(st_, seq, words.data(), 2 * points);
+      mark("rows");
+      F.resize(points);
+      for (int p = 0; p < points; p++) F[p] = mk(words[2 * p], words[2 * p + 1]);
+      f128 r[6];
+      rounds.from_points(F, rem - 1, k, r);
+      rem -= k;
+      RowWeights eps{};  // r[t] bound row bit k - 1 - t
+      eps.e[0] = mk(1, 0);
+      for (int q = 0; q < k; q++)
+        for (int x = 0; x < 1 << q; x++) {
+          const f128 one = gmul(eps.e[x], r[k - 1 - q]);
+          eps.e[x | 1 << q] = one;
+          eps.e[x] = gadd(eps.e[x], one);
+        }
+      (j == 0 ? gkr_bound_rows<0> : gkr_bound_rows<1>)<<<grid_for(colmask + 1), kThreads, 0, st_>>>(
+          cols, s, images, eps, c, c + n_half);
       BZ_LAUNCH_CHECK();
     }
-    size_t h = n_half / 2;
-    // Queued mode: the bind rounds above the tail's first (h <= kTailH) and
-    // the tail itself are all queued behind the top sums, each round's
-    // challenge fetched on the device. Publication p0 + (n - i) carries the
-    // sums after binding r_i, which the host posts as downbox publication
-    // d0 + (n - 1 - i). The kernel probe times kernels alone, so it runs
-    // every round as its own launch.
-    const bool queued = ch && resident;
-    int i_tail = n - 1;
-    while (i_tail > 0 && ((size_t)1 << (i_tail - 1)) > (size_t)kTailH) i_tail--;
-    const Publish top = arm(sc);
-    const unsigned long long p0 = top.seq, d0 = ch ? ch->down_next + 1 : 0;
-    // Queued mode: the tail hands its tables over at iteration i_host and the
-    // host runs the rounds from there down (handover publication hseq).
-    const int i_host =
-        queued && ch->handover_host && i_tail >= 1 ? std::min(kHostTailI, i_tail) : -1;
-    const unsigned long long hseq = p0 + (n - i_host);
-    uint32_t tail_mask = 0;
-    for (int k = 1; k <= i_tail; k++) tail_mask |= (uint32_t)gis_zero(point[k - 1]) << (k - 1);
-    std::vector<f128> HL, HR, HE;
-    f128 host_out[2] = {mk(0, 0), mk(0, 0)};  // sums (or the pair) the host computed
-    RoundLink none{nullptr, nullptr, nullptr, 0};
-    // Bind round i > i_tail runs in gkr_mid (which reads r_i from the downbox
-    // itself) when the lane keeps the middle rounds resident and 2^(i-1) <=
-    // kMidMaxH; otherwise as a queued launch that reads r_i from ctl, left
-    // there by the kernel before it.
-    auto in_mid = [&](int i) {
-      return sc.mid_blocks > 0 && ((size_t)1 << (i - 1)) <= kMidMaxH;
-    };
-    auto link_for = [&](int i) {  // where the kernel before bind round i leaves r_i
-      return queued && i > i_tail && !in_mid(i) ? sc.ctl + (n - 1 - i) : nullptr;
-    };
-    RoundLink top_link = none;
-    if (queued && n - 1 > i_tail) top_link = RoundLink{nullptr, link_for(n - 1), ch->down_dev, d0};
-    if (queued) tail = true;  // from here a kernel of the lane may wait for this thread
-    const bool probe_top = probe.on("gkr_top_sums");
-    if (probe_top) probe.before(st_);
-    gkr_top_sums<<<grid_for(h), kThreads, 0, st_>>>(c, n_half, h, lo, a, hi, sc.eq,
-                                                    gis_zero(point[n - 1]), sc.acc, top, top_link,
-                                                    colmask, live);
+    while (rem > kHostLog) {
+      const int k = b.k == 0 && rem >= kFirstLog ? 2 : 3;
+      const int log_m = rem - k;
+      const size_t m = (size_t)1 << log_m;
+      const uint32_t count = (uint32_t)(m > colmask ? (m >> s) * live : std::min(m, live));
+      const int points = pow3(k);
+      const bool probed = probe.on("gkr_pass");
+      if (probed) probe.before(st_);
+      const unsigned long long seq = ch->arm().seq;
+      if (k == 2)
+        launch_pass<2>(c, n_half, log_m, b, heap.data(), colmask, (uint32_t)live, count, sc, seq, st_);
+      else
+        launch_pass<3>(c, n_half, log_m, b, heap.data(), colmask, (uint32_t)live, count, sc, seq, st_);
+      if (probed) {
+        // per live position: 2^(k+1) entries of the bound tables, each from
+        // 2^kb read and one written (none written without a bind), 2^kb - 1
+        // products through window tables each; the weight, 2^k products by it
+        // and 3^k wide ones
+        const double e = (double)count * (2 << k), in = (double)(1 << b.k);
+        probe.after(st_, "gkr_pass", 16.0 * e * (in + (b.k ? 1.0 : 0.0)),
+                    (double)count * ((1 << k) + (log_m - 1) / kFacLog), (double)count * points,
+                    e * (in - 1));
+      }
+      ch->wait_handover(st_, seq, words.data(), 2 * (points + 1));
+      mark("pass");
+      F.resize(points);
+      for (int p = 0; p < points; p++) F[p] = mk(words[2 * p], words[2 * p + 1]);
+      // the padded positions' weights (all of them sum to one) at the points
+      // of zeros and ones
+      const f128 pad = mk(words[2 * points] ^ 1, words[2 * points + 1]);
+      if (!gis_zero(pad))
+        for (int x = 0; x < 1 << k; x++) {
+          int p = 0;
+          for (int q = k - 1; q >= 0; q--) p = 3 * p + ((x >> q) & 1);
+          F[p] = gadd(F[p], pad);
+        }
+      rounds.from_points(F, rem - 1, k, b.r);
+      b.k = k;
+      rem -= k;
+    }
+    const int len = 1 << rem;
+    const unsigned long long seq = ch->arm().seq;
+    gkr_handover<<<(2 * len + kHandEntries - 1) / kHandEntries, kHandThreads, 0, st_>>>(
+        c, n_half, len, b, ch->handover_dev, seq);
     BZ_LAUNCH_CHECK();
-    if (probe_top) {
-      // each thread forms e = lo * hi and writes it; a live one also reads its
-      // four child entries and multiplies e by two of them and the results by two more
-      const double nl = live_threads(h, colmask, live);
-      probe.after(st_, "gkr_top_sums", 16.0 * (double)h + 64.0 * nl, (double)h + 2.0 * nl,
-                  2.0 * nl);
-    }
-    if (queued) {
-      int i = n - 1;
-      for (; i > i_tail && !in_mid(i); i--) {
-        const size_t hh = (size_t)1 << (i - 1);
-        RoundLink lk{sc.ctl + (n - 1 - i), link_for(i - 1), ch->down_dev, d0 + (n - i)};
-        const Publish pub{ch->counter, ch->dev, p0 + (n - i)};
-        launch_bind(c, n_half, hh, mk(0, 0), sc.eq, gis_zero(point[i - 1]),
-                    sc.acc + 4 * (n - i), pub, lk, colmask, live, st_);
-      }
-      if (i > i_tail) launch_mid(c, n_half, n, i, i_tail + 1, point, sc, p0, d0, colmask, live, st_);
-      gkr_tail<<<1, kTailThreads, 0, st_>>>(c, n_half, i_tail, sc.eq, tail_mask, ch->dev,
-                                            p0 + (n - i_tail), ch->down_dev,
-                                            d0 + (n - 1 - i_tail), colmask, live, i_host,
-                                            ch->handover_dev, hseq);
-      BZ_LAUNCH_CHECK();
-      tail = true;
-    }
-    f128 eq_bound = mk(1, 0);
-    for (int i = n - 1; i >= 0; i--) {
-      unsigned long long *acc = sc.acc + 4 * (n - 1 - i);
-      if (i_host >= 0 && i < i_host) {  // the host's own round
-        sc.host[0] = host_out[0].lo;
-        sc.host[1] = host_out[0].hi;
-        sc.host[2] = host_out[1].lo;
-        sc.host[3] = host_out[1].hi;
-      } else {
-        round_read(sc, acc, st_);
-      }
-      if (trace) {
-        const auto now = std::chrono::steady_clock::now();
-        fprintf(stderr, "[gkr] layer %d round %2d h %8zu %s %7.2f us\n", j, i, (size_t)1 << i,
-                i == n - 1 ? "top " : (queued && i < i_tail) ? "tail" : "bind",
-                std::chrono::duration<double, std::micro>(now - t_prev).count());
-        t_prev = now;
-      }
-      f128 sb = mk(sc.host[0], sc.host[1]), si = mk(sc.host[2], sc.host[3]);
-      f128 msg[2] = {gmul(eq_bound, sb), gmul(eq_bound, si)};
-      ts.prover_message(msg, 32);
-      ts.grind("gkr/cubic/v1", grind_bits);
-      f128 r = ts.challenge_f128();
-      next[i] = r;
-      eq_bound = gmul(eq_bound, eq_factor(r, point[i]));
-      const uint64_t rw[2] = {r.lo, r.hi};
-      if (queued && i_host >= 0 && i <= i_host) {
-        if (i == i_host) {  // the tail's tables, as it stood before binding r_i
-          const int h = 1 << (i - 1), nl = 4 * h;
-          std::vector<uint64_t> w(2 * (2 * nl + 2 * h));
-          ch->wait_handover(st_, hseq, w.data(), (int)w.size());
-          tail = false;  // the tail kernel ends after the handover
-          auto take = [&](std::vector<f128> &v, int at, int cnt) {
-            v.resize(cnt);
-            for (int k = 0; k < cnt; k++) v[k] = mk(w[2 * (at + k)], w[2 * (at + k) + 1]);
-          };
-          take(HL, 0, nl);
-          take(HR, nl, nl);
-          take(HE, 2 * nl, 2 * h);
-        }
-        host_tail_round(HL, HR, HE, i, r, tail_mask, colmask, live, host_out);
-        ch->arm();  // publication numbering as if the device had posted
-      } else if (queued) {
-        ch->send(rw, 2);
-        ch->arm();
-      } else if (i > 0) {
-        size_t hh = (size_t)1 << (i - 1);
-        const char *name = hh <= kMidMaxH ? "gkr_round" : "gkr_bind_sums";
-        const bool probed = probe.on(name);
-        if (probed) probe.before(st_);
-        launch_bind(c, n_half, hh, r, sc.eq, gis_zero(point[i - 1]), acc + 4, arm(sc), none,
-                    colmask, live, st_);
-        if (probed) {
-          // a live element reads 8 child and 2 eq entries and writes 4 and 1
-          // (240 B), binds four entries by r through r's window table and
-          // makes four general products (two by e, two wide); a padded one
-          // moves the eq table's 3 entries (48 B)
-          const double nl = live_threads(hh, colmask, live);
-          probe.after(st_, name, 240.0 * nl + 48.0 * ((double)hh - nl), 2.0 * nl, 2.0 * nl,
-                      4.0 * nl);
-        }
-      } else {
-        gkr_final_bind<<<1, 32, 0, st_>>>(c, n_half, r, sc.pair, arm(sc));
-        BZ_LAUNCH_CHECK();
-      }
+    if ((int)L.size() < len) L.resize(len), R.resize(len);
+    ch->wait_handover(st_, seq, words.data(), 4 * len);
+    mark("tables");
+    for (int k = 0; k < len; k++) {
+      L[k] = mk(words[2 * k], words[2 * k + 1]);
+      R[k] = mk(words[2 * (len + k)], words[2 * (len + k) + 1]);
     }
     f128 lr[2];
-    if (i_host >= 0) {
-      lr[0] = host_out[0];
-      lr[1] = host_out[1];
-    } else {
-      round_read(sc, sc.pair, st_);
-      tail = false;  // the tail kernel ends after posting the pair
-      memcpy(lr, sc.host, 32);
-    }
+    rounds.from_tables(L.data(), R.data(), rem, heap[0].v, lr);
     ts.prover_message(lr, 32);
-    f128 t = ts.challenge_f128();
+    const f128 t = ts.challenge_f128();
     next[n] = t;
     claim = gadd(lr[0], gmul(t, gadd(lr[1], lr[0])));
     n++;
     for (int i = 0; i < n; i++) point[i] = next[i];
-  }
-  } catch (...) {
-    if (tail) {  // release the waiting kernel before the lane is reused
-      ch->abort();
-      stream_wait(st_);
-      ch->clear_down();
-    }
-    throw;
+    mark("host rounds");
   }
   for (int i = 0; i < n; i++) point_out[i] = point[i];
   return claim;
@@ -950,15 +949,21 @@ f128 gkr_prove(int s, const f128 *zeta, uint32_t grind_bits, Transcript &ts, Gkr
 // Every kernel of this file, loaded when the process's first lane on a device
 // is made (lane_bootstrap, context.cpp).
 void preload_gkr_kernels() {
-  load_kernels({(const void *)gkr_leaves,
-                (const void *)gkr_parent,
-                (const void *)gkr_layer_setup,
-                (const void *)gkr_top_sums,
-                (const void *)gkr_bind_sums,
-                (const void *)gkr_round,
-                (const void *)gkr_mid,
-                (const void *)gkr_final_bind,
-                (const void *)gkr_tail});
+  load_kernels({(const void *)gkr_low_layers,
+                (const void *)gkr_high_layers,
+                (const void *)gkr_gram<64, 4>,
+                (const void *)gkr_gram<64, 16>,
+                (const void *)gkr_gram<96, 4>,
+                (const void *)gkr_gram<96, 16>,
+                (const void *)gkr_moments<0>,
+                (const void *)gkr_moments<1>,
+                (const void *)gkr_bound_rows<0>,
+                (const void *)gkr_bound_rows<1>,
+                (const void *)gkr_pass<2, 2>,
+                (const void *)gkr_pass<2, 5>,
+                (const void *)gkr_pass<3, 2>,
+                (const void *)gkr_pass<3, 5>,
+                (const void *)gkr_handover});
 }
 
 }  // namespace bz

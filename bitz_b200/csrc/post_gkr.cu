@@ -248,7 +248,7 @@ static bool host_pg_round(std::vector<f128> &W, std::vector<f128> &V, f128 r, f1
 }
 
 // The last rounds in one resident block, fed through the lane's downbox like
-// the GKR tail: the tables (at most 2 * kPgTailN entries each) sit in shared
+// the Spartan tails: the tables (at most 2 * kPgTailN entries each) sit in shared
 // memory; each round waits (bounded) for the host's challenge, folds both
 // tables at it and posts the next round's (a0, a2), or, after the last fold,
 // the closing pair (w, v). A missing challenge ends the kernel without a post.

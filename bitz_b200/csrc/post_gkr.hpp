@@ -54,7 +54,7 @@ void launch_pg_mid(const f128 *w_in, const f128 *v_in, size_t n_in, int km, int 
                    int nb, cudaStream_t s);
 // The grid of a lane's resident post-GKR and Ligerito folds
 // (PostGkrScratch::mid_blocks): 128 for a lane proving alone; for a pooled
-// lane none, or 32 with BITZ_POOL_MID=1 (as for the GKR middle rounds).
+// lane none, or 32 with BITZ_POOL_MID=1.
 int pg_mid_blocks(bool alone);
 
 // The quadratic sumcheck round of <W, V> (shared with the Ligerito folds):

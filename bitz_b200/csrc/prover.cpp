@@ -820,8 +820,8 @@ int ProofSystem::prove_after_commit(cudaStream_t s, std::vector<uint8_t> &proof)
   ph.mark("fold");
   // gkr_reduce (crates/prover/src/reduce.rs:17-47); the layers were built above
   std::vector<f128> gpt(sc_cols + 7);
-  f128 gclaim = gkr_prove(sc_cols, zeta.data(), grinding_bits((uint32_t)security_, 3), t, gs, s,
-                          gpt.data());
+  f128 gclaim = gkr_prove(hpk, sc_cols, W.images.get(), zeta.data(),
+                          grinding_bits((uint32_t)security_, 3), t, gs, s, gpt.data());
   f128 ip_target = gadd(gclaim, mk(1, 0));
   ph.mark("gkr");
   std::vector<f128> eqb(128), u1(128);

@@ -280,7 +280,7 @@ int bitz_server_stop(bitz_server *srv);
  * probe off, "*" probes every instrumented launch site, else a comma-separated
  * list of kernel names; enabling resets the totals. While the probe is on,
  * every sumcheck round is its own launch (as under a kernel profiler).
- * Instrumented: gkr_top_sums, gkr_round, gkr_bind_sums, pg_round,
+ * Instrumented: gkr_pass, pg_round,
  * k_outer_round, k_inner_round, k_fp_finalize. */
 int bitz_probe_kernel(const char *spec);
 /* One kernel's totals since the probe was enabled: out[0] milliseconds,
