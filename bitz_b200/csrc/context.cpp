@@ -256,7 +256,6 @@ Context::Context() {
   acc_.resize(8 * 128);
   BZ_CUDA(cudaMallocHost(&host_, 64 * sizeof(uint64_t)));
   pg_.acc = acc_.get();
-  pg_.host = host_;
   gk_.acc = acc_.get();
   gk_ctl_.resize(kMaxPointGkr);
   // the round mailbox: one mapped pinned page and a device block counter
@@ -280,10 +279,8 @@ Context::Context() {
   BZ_CUDA(cudaMemset(counter_.get(), 0, sizeof(unsigned int)));
   channel_.counter = counter_.get();
   pg_.channel = &channel_;
-  pg_.ctl = gk_ctl_.get();
   gk_.channel = &channel_;
   sp_mid_blocks_ = ::bz::sp_mid_blocks(false);
-  pg_.mid_blocks = ::bz::pg_mid_blocks(false);
   lane_bootstrap(*this);
 }
 
@@ -304,13 +301,12 @@ std::atomic<unsigned long long> &launch_counter() {
 Context &Context::get() {
   // One default lane per process, created on first use on the current device.
   // It proves one statement at a time with the GPU to itself, so its resident
-  // middle rounds (Spartan, post-GKR and Ligerito) use grids of 128
+  // middle rounds (Spartan) use grids of 128
   // blocks; pool lanes, which share the GPU, run those rounds as queued
   // launches (or 32-block grids with BITZ_POOL_MID=1).
   static Context *ctx = [] {
     Context *c = new Context();
     c->sp_mid_blocks_ = ::bz::sp_mid_blocks(true);
-    c->pg_.mid_blocks = ::bz::pg_mid_blocks(true);
     return c;
   }();
   return *ctx;

@@ -113,8 +113,6 @@ class Context {
   RoundCtl *round_ctl() { return gk_ctl_.get(); }
   // Grid of the resident Spartan grid rounds on this lane (0: none).
   int sp_mid_blocks() const { return sp_mid_blocks_; }
-  // Grid of the resident post-GKR and Ligerito folds on this lane (0: none).
-  int pg_mid_blocks() const { return pg_.mid_blocks; }
   // Prover workspace slot, owned by the lane (created by the prover).
   std::shared_ptr<Workspace> workspace;
 

@@ -35,6 +35,7 @@
 #include "context.hpp"
 #include "eq.cuh"
 #include "gkr.hpp"
+#include "passes.cuh"
 
 namespace bz {
 
@@ -111,98 +112,12 @@ __global__ void __launch_bounds__(128) gkr_high_layers(const f128 *__restrict__ 
 
 // ------------------------------------------------------------------ passes
 
-constexpr int kPassThreads = 288;  // nine warps: the 27 points of a tile in three turns
-constexpr int kPassMaxK = 3;
-constexpr int kPassMaxX = 32;  // positions per tile
-constexpr int kFacLog = 7;     // coordinates per eq factor
-
-constexpr int pow3(int k) { return k == 0 ? 1 : 3 * pow3(k - 1); }
-
-// eq(x) over the lower coordinates as a product of NF factor tables, factor g
-// over coordinates 7g .. 7g + 6. The host forms the layer's tables once (about
-// 130 products each) and they travel as a launch argument: no copy, no setup
-// launch before the layer's first pass.
-template <int NF>
-struct EqFactors {
-  f128 f[NF][1 << kFacLog];
-};
-
-// The challenges of the pass before: r[0] bound the top coordinate.
-struct PassBind {
-  f128 r[kPassMaxK];
-  int k;
-};
-
-// Products as calls: a pass is short for most sizes and starts with a cold
-// instruction cache (a product inlined 40 times costs more to fetch than to
-// run), and the larger ones are bound by the products themselves.
-static __device__ __noinline__ wide pass_wide(f128 a, f128 b) { return gmul_wide(a, b); }
-static __device__ __noinline__ f128 pass_table(const MulTable *T, f128 a) {
-  return mul_table(*T, a);
-}
-static __device__ __forceinline__ f128 pass_mul(f128 a, f128 b) { return greduce(pass_wide(a, b)); }
-
-// The window tables of b.r[0 .. b.k), every thread of the block taking part.
-static __device__ __forceinline__ void pass_tables(MulTable *T, const PassBind &b) {
-  for (int u = threadIdx.x; u < b.k * 128; u += blockDim.x) {
-    const int t = u >> 7, k = u & 127;
-    const f128 v = gmul_xk(b.r[t], k);
-    T[t].lo[k >> 2][1 << (k & 3)] = v.lo;
-    T[t].hi[k >> 2][1 << (k & 3)] = v.hi;
-  }
-  __syncthreads();
-  for (int u = threadIdx.x; u < b.k * 512; u += blockDim.x) {
-    const int t = u >> 9, j = (u >> 4) & 31, v = u & 15;
-    if (v != 0 && (v & (v - 1)) == 0) continue;  // written above
-    uint64_t lo = 0, hi = 0;
-#pragma unroll
-    for (int q = 0; q < 4; q++)
-      if ((v >> q) & 1) {
-        lo ^= T[t].lo[j][1 << q];
-        hi ^= T[t].hi[j][1 << q];
-      }
-    T[t].lo[j][v] = lo;
-    T[t].hi[j][v] = hi;
-  }
-  __syncthreads();
-}
-
-static __device__ __forceinline__ f128 bind2(const MulTable *T, f128 a, f128 b) {
-  return gadd(a, pass_table(T, gadd(a, b)));
-}
-
 // Entry `pos` of a table of `n` entries after binding the k coordinates above
 // it: block b of the unbound table starts at b n, the first challenge bound
 // the top bit of b.
-static __device__ __forceinline__ f128 pass_bind(const f128 *tab, size_t pos, size_t n,
-                                                 const MulTable *T, int k) {
-  const f128 *p = tab + pos;
-  if (k == 0) return ld(p);
-  if (k == 1) return bind2(T, ld(p), ld(p + n));
-  if (k == 2) {
-    const f128 a = bind2(T, ld(p), ld(p + 2 * n)), b = bind2(T, ld(p + n), ld(p + 3 * n));
-    return bind2(T + 1, a, b);
-  }
-  const f128 a0 = bind2(T, ld(p), ld(p + 4 * n)), a2 = bind2(T, ld(p + 2 * n), ld(p + 6 * n));
-  const f128 a1 = bind2(T, ld(p + n), ld(p + 5 * n)), a3 = bind2(T, ld(p + 3 * n), ld(p + 7 * n));
-  return bind2(T + 2, bind2(T + 1, a0, a2), bind2(T + 1, a1, a3));
-}
-
-// Table t (2^K blocks of X positions) at point p, digit i of p (base 3) for
-// bit i of the block: 0, 1, or 2 for infinity (the sum over the bit).
-template <int K>
-static __device__ __forceinline__ f128 point_value(const f128 *t, int lx, int x, int p) {
-  int one = 0, inf = 0;
-#pragma unroll
-  for (int i = 0; i < K; i++) {
-    const int d = p % 3;
-    p /= 3;
-    one |= (d == 1) << i;
-    inf |= (d == 2) << i;
-  }
-  f128 v = t[(one << lx) + x];
-  for (int sub = inf; sub; sub = (sub - 1) & inf) v = gadd(v, t[((one | sub) << lx) + x]);
-  return v;
+static __device__ __forceinline__ f128 bind_above(const f128 *tab, size_t pos, size_t n,
+                                                  const MulTable *T, int k) {
+  return pass_bind<false>([&](int b) { return ld(tab + pos + b * n); }, T, k);
 }
 
 // Padding: the low s bits of every layer index are the column, and a column at
@@ -232,7 +147,6 @@ __global__ void __launch_bounds__(kPassThreads, 2) gkr_pass(
   __shared__ MulTable T[kPassMaxK];
   __shared__ f128 G[kBlocks * kPassMaxX], R[kBlocks * kPassMaxX], E[kPassMaxX];
   __shared__ f128 F[NF][1 << kFacLog];
-  __shared__ bool last;
   const int t = threadIdx.x;
   const size_t m = (size_t)1 << log_m, n = m << K;
   const int X = 1 << lx;
@@ -277,7 +191,7 @@ __global__ void __launch_bounds__(kPassThreads, 2) gkr_pass(
       if (in) {
         f128 *tab = right ? c + n_half : c;
         const size_t pos = x + (size_t)(slot >> lx) * m;
-        v = pass_bind(tab, pos, n, T, b.k);
+        v = bind_above(tab, pos, n, T, b.k);
         if (b.k) st(tab + pos, v);
       }
       (right ? R : G)[slot] = v;
@@ -289,26 +203,15 @@ __global__ void __launch_bounds__(kPassThreads, 2) gkr_pass(
     for (int q = 0; q < kTurns; q++) {
       const int u = t + q * kPassThreads;
       if (u < kPoints << lx) {
-        const int p = u >> lx, x = u & (X - 1);
-        wacc(sum[q], pass_wide(point_value<K>(G, lx, x, p), point_value<K>(R, lx, x, p)));
+        int one, inf;
+        point_bits<K, false>(u >> lx, one, inf);
+        const int x = u & (X - 1);
+        wacc(sum[q], pass_wide(point_value(G + x, X, one, inf), point_value(R + x, X, one, inf)));
       }
     }
     __syncthreads();  // the tile's tables before the next tile's
   }
-  // the block's sums: over the X lanes of each point, then into acc
-#pragma unroll
-  for (int q = 0; q < kTurns; q++) {
-    const int u = t + q * kPassThreads;
-    f128 v = greduce(sum[q]);
-    for (int off = X >> 1; off > 0; off >>= 1) {
-      v.lo ^= __shfl_xor_sync(0xffffffffu, v.lo, off);
-      v.hi ^= __shfl_xor_sync(0xffffffffu, v.hi, off);
-    }
-    if (u < kPoints << lx && (u & (X - 1)) == 0) {
-      atomicXor(acc + 2 * (u >> lx), (unsigned long long)v.lo);
-      atomicXor(acc + 2 * (u >> lx) + 1, (unsigned long long)v.hi);
-    }
-  }
+  pass_reduce<kPoints, kTurns>(sum, lx, acc);
   for (int off = 16; off > 0; off >>= 1) {
     sum_e.lo ^= __shfl_xor_sync(0xffffffffu, sum_e.lo, off);
     sum_e.hi ^= __shfl_xor_sync(0xffffffffu, sum_e.hi, off);
@@ -317,18 +220,7 @@ __global__ void __launch_bounds__(kPassThreads, 2) gkr_pass(
     atomicXor(acc + 2 * kPoints, (unsigned long long)sum_e.lo);
     atomicXor(acc + 2 * kPoints + 1, (unsigned long long)sum_e.hi);
   }
-  __threadfence();
-  __syncthreads();
-  if (t == 0) {
-    last = atomicAdd(counter, 1u) == gridDim.x - 1;
-    __threadfence();
-  }
-  __syncthreads();
-  if (last) {
-    if (t < 2 * (kPoints + 1))
-      handover_post(handover, seq, t, atomicExch(acc + t, 0ull));
-    if (t == 0) *counter = 0;
-  }
+  pass_publish(acc, 2 * (kPoints + 1), counter, handover, seq);
 }
 
 // The layer's last tables to the host: L, then R, of n entries each after the
@@ -342,7 +234,7 @@ __global__ void __launch_bounds__(kHandThreads) gkr_handover(const f128 *__restr
   pass_tables(T, b);
   const int k = blockIdx.x * kHandEntries + threadIdx.x;
   if (threadIdx.x >= kHandEntries || k >= 2 * n) return;
-  const f128 v = k < n ? pass_bind(c, k, n, T, b.k) : pass_bind(c + n_half, k - n, n, T, b.k);
+  const f128 v = k < n ? bind_above(c, k, n, T, b.k) : bind_above(c + n_half, k - n, n, T, b.k);
   handover_post(handover, seq, 2 * k, v.lo);
   handover_post(handover, seq, 2 * k + 1, v.hi);
 }
@@ -428,19 +320,7 @@ __global__ void __launch_bounds__(GramShape<NFEAT>::kThreadsPer) gkr_gram(
       out[4 * (lane + 32) + (warp & 3)] = r1;
     }
     __syncthreads();
-    for (int e = t; e < 512; e += S::kThreadsPer) {
-      const int k = e >> 4, v = e & 15;
-      if (v != 0 && (v & (v - 1)) == 0) continue;  // written above
-      uint64_t lo = 0, hi = 0;
-#pragma unroll
-      for (int q = 0; q < 4; q++)
-        if ((v >> q) & 1) {
-          lo ^= T.lo[k][1 << q];
-          hi ^= T.hi[k][1 << q];
-        }
-      T.lo[k][v] = lo;
-      T.hi[k][v] = hi;
-    }
+    fill_windows(T.lo, T.hi, 32);
     __syncthreads();
     const uint4 fa = feature<NFEAT>(rows, i, false);
 #pragma unroll
@@ -598,19 +478,7 @@ __global__ void __launch_bounds__(kThreads) gkr_bound_rows(const f128 *__restric
     hi[u >> 2][1 << (u & 3)] = k.hi;
   }
   __syncthreads();
-  for (int e = t; e < 2 * kWin * 16; e += kThreads) {
-    const int k = e >> 4, v = e & 15;
-    if (v != 0 && (v & (v - 1)) == 0) continue;  // written above
-    uint64_t a = 0, b = 0;
-#pragma unroll
-    for (int q = 0; q < 4; q++)
-      if ((v >> q) & 1) {
-        a ^= lo[k][1 << q];
-        b ^= hi[k][1 << q];
-      }
-    lo[k][v] = a;
-    hi[k][v] = b;
-  }
+  fill_windows(lo, hi, 2 * kWin);
   __syncthreads();
   const size_t n = (size_t)1 << s;
   for (size_t c = blockIdx.x * (size_t)blockDim.x + t; c < n; c += (size_t)gridDim.x * blockDim.x) {
@@ -647,30 +515,6 @@ static_assert(4 << kHostLog <= kHandoverWords, "the last tables fit one handover
 // next pass): two rounds from this size on, where products are the cost.
 constexpr int kFirstLog = 17;
 
-// Prefix tables of eq over up to kFacLog coordinates: entries [2^i, 2^(i+1))
-// hold eq over the first i of them.
-struct EqHeap {
-  f128 v[2 << kFacLog];
-  void build(const f128 *z, int n) {
-    v[1] = mk(1, 0);
-    for (int i = 0; i < n; i++) {
-      const f128 *p = v + ((size_t)1 << i);
-      f128 *q = v + ((size_t)2 << i);
-      for (int k = 0; k < 1 << i; k++) {
-        const f128 one = gmul(p[k], z[i]);
-        q[k] = gadd(p[k], one);
-        q[k + (1 << i)] = one;
-      }
-    }
-  }
-  const f128 *prefix(int n) const { return v + ((size_t)1 << n); }
-};
-
-static unsigned int pass_grid(uint32_t count, int lx) {
-  const uint32_t tiles = (count + (1u << lx) - 1) >> lx;
-  return std::max(1u, std::min(tiles, 2u * kSMs));
-}
-
 template <int K, int NF>
 static void launch_pass_nf(f128 *c, size_t n_half, int log_m, const PassBind &b, const EqHeap *heap,
                            size_t colmask, uint32_t live, uint32_t count, GkrScratch &sc,
@@ -680,10 +524,7 @@ static void launch_pass_nf(f128 *c, size_t n_half, int log_m, const PassBind &b,
     const int have = std::min(kFacLog, std::max(0, log_m - g * kFacLog));
     memcpy(eq.f[g], heap[g].prefix(have), sizeof(f128) << have);
   }
-  // the largest tile that still gives every SM one: wide tiles fill the turns
-  // (27 points of 32 positions are three per thread), narrow ones the chip
-  int lx = 5;
-  while (lx > 2 && (count >> lx) < (uint32_t)kSMs) lx--;
+  const int lx = pass_tile_log(count);
   gkr_pass<K, NF><<<pass_grid(count, lx), kPassThreads, 0, st>>>(
       c, n_half, log_m, b, eq, colmask, live, count, lx, sc.acc, sc.channel->counter,
       sc.channel->handover_dev, seq);

@@ -1,0 +1,225 @@
+// What the multi-round sumcheck passes share (GKR, post-GKR, Ligerito): several
+// rounds go through the device at once, as the product polynomial's values at
+// the points {0, 1, infinity}^K of the K coordinates to be bound next.
+#pragma once
+#include <vector>
+
+#include "device.cuh"
+
+namespace bz {
+
+constexpr int kPassThreads = 288;  // nine warps: the 27 points of a tile in three turns
+constexpr int kPassMaxK = 3;
+constexpr int kPassMaxX = 32;  // positions per tile
+
+constexpr int pow3(int k) { return k == 0 ? 1 : 3 * pow3(k - 1); }
+
+// The challenges that the next pass binds, the first one drawn in r[0].
+struct PassBind {
+  f128 r[kPassMaxK];
+  int k;
+};
+
+// eq(x) over many coordinates as a product of NF factor tables, factor g over
+// coordinates 7g .. 7g + 6. The host forms a layer's tables once (about 130
+// products each) and they travel as a launch argument: no copy, no setup
+// launch before the first pass.
+constexpr int kFacLog = 7;
+template <int NF>
+struct EqFactors {
+  f128 f[NF][1 << kFacLog];
+};
+
+// Prefix tables of eq over up to kFacLog coordinates: entries [2^i, 2^(i+1))
+// hold eq over the first i of them.
+struct EqHeap {
+  f128 v[2 << kFacLog];
+  void build(const f128 *z, int n) {
+    v[1] = mk(1, 0);
+    for (int i = 0; i < n; i++) {
+      const f128 *p = v + ((size_t)1 << i);
+      f128 *q = v + ((size_t)2 << i);
+      for (int k = 0; k < 1 << i; k++) {
+        const f128 one = gmul(p[k], z[i]);
+        q[k] = gadd(p[k], one);
+        q[k + (1 << i)] = one;
+      }
+    }
+  }
+  const f128 *prefix(int n) const { return v + ((size_t)1 << n); }
+};
+
+// Where a pass sums and posts.
+struct PassPost {
+  unsigned long long *acc;       // zero before, zero after
+  unsigned int *counter;         // finished blocks, likewise
+  unsigned long long *handover;  // tagged slots
+  unsigned long long seq;        // their publication
+};
+
+// k rounds of a quadratic sumcheck from its point sums F (the first round's
+// coordinate is the top digit): `round` takes a message's (a0, a2) and returns
+// the challenge.
+template <class Round>
+inline void quad_rounds(std::vector<f128> &F, int k, f128 *r, Round round) {
+  size_t block = F.size() / 3;
+  for (int t = 0; t < k; t++, block /= 3) {
+    const int rest = k - 1 - t;
+    f128 a0 = mk(0, 0), a2 = mk(0, 0);
+    for (int x = 0; x < 1 << rest; x++) {
+      size_t at = 0;
+      for (int q = rest - 1; q >= 0; q--) at = 3 * at + ((x >> q) & 1);
+      a0 = gadd(a0, F[at]);
+      a2 = gadd(a2, F[2 * block + at]);
+    }
+    r[t] = round(a0, a2);
+    for (size_t x = 0; x < block; x++) {  // h0 + r (h1 + h0 + hinf) + r^2 hinf
+      const f128 h0 = F[x], h1 = F[block + x], hi = F[2 * block + x];
+      F[x] = gadd(h0, gmul(r[t], gadd(gadd(h0, h1), gadd(hi, gmul(r[t], hi)))));
+    }
+  }
+}
+
+// A pass's grid for `count` positions in tiles of 2^lx, and the tile: the
+// largest that still gives every SM one. Wide tiles fill the turns (27 points
+// of 32 positions are three per thread), narrow ones the chip.
+inline int pass_tile_log(uint32_t count) {
+  int lx = 5;
+  while (lx > 2 && (count >> lx) < (uint32_t)kSMs) lx--;
+  return lx;
+}
+inline unsigned int pass_grid(uint32_t count, int lx) {
+  const uint32_t tiles = (count + (1u << lx) - 1) >> lx;
+  return tiles < 1 ? 1 : tiles < 2u * kSMs ? tiles : 2u * kSMs;
+}
+
+#if defined(__CUDACC__)
+// Products as calls: a pass is short for most sizes and starts with a cold
+// instruction cache (a product inlined 40 times costs more to fetch than to
+// run), and the larger ones are bound by the products themselves.
+static __device__ __noinline__ wide pass_wide(f128 a, f128 b) { return gmul_wide(a, b); }
+static __device__ __noinline__ f128 pass_table(const MulTable *T, f128 a) {
+  return mul_table(*T, a);
+}
+static __device__ __forceinline__ f128 pass_mul(f128 a, f128 b) { return greduce(pass_wide(a, b)); }
+
+// The other entries of `n` windows whose single-bit entries are in place: every
+// thread of the block takes part; the caller synchronises around it.
+static __device__ __forceinline__ void fill_windows(uint64_t (*lo)[16], uint64_t (*hi)[16],
+                                                    int n) {
+  for (int u = threadIdx.x; u < n * 16; u += blockDim.x) {
+    const int j = u >> 4, v = u & 15;
+    if (v != 0 && (v & (v - 1)) == 0) continue;
+    uint64_t a = 0, b = 0;
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+      if ((v >> q) & 1) {
+        a ^= lo[j][1 << q];
+        b ^= hi[j][1 << q];
+      }
+    lo[j][v] = a;
+    hi[j][v] = b;
+  }
+}
+
+// The window tables of b.r[0 .. b.k), every thread of the block taking part.
+static __device__ __forceinline__ void pass_tables(MulTable *T, const PassBind &b) {
+  for (int u = threadIdx.x; u < b.k * 128; u += blockDim.x) {
+    const int t = u >> 7, k = u & 127;
+    const f128 v = gmul_xk(b.r[t], k);
+    T[t].lo[k >> 2][1 << (k & 3)] = v.lo;
+    T[t].hi[k >> 2][1 << (k & 3)] = v.hi;
+  }
+  __syncthreads();
+  for (int t = 0; t < b.k; t++) fill_windows(T[t].lo, T[t].hi, 32);
+  __syncthreads();
+}
+
+static __device__ __forceinline__ f128 bind2(const MulTable *T, f128 a, f128 b) {
+  return gadd(a, pass_table(T, gadd(a, b)));
+}
+
+// 2^k entries in(0), in(1), ... bound at k challenges, the first one bound by
+// index bit `first` (0: the lowest bit first; k - 1: the highest first).
+template <bool kLowFirst, class In>
+static __device__ __forceinline__ f128 pass_bind(In in, const MulTable *T, int k) {
+  if (k == 0) return in(0);
+  if (k == 1) return bind2(T, in(0), in(1));
+  if (k == 2) {
+    const f128 a = kLowFirst ? bind2(T, in(0), in(1)) : bind2(T, in(0), in(2));
+    const f128 b = kLowFirst ? bind2(T, in(2), in(3)) : bind2(T, in(1), in(3));
+    return bind2(T + 1, a, b);
+  }
+  const f128 a = kLowFirst ? bind2(T, in(0), in(1)) : bind2(T, in(0), in(4));
+  const f128 b = kLowFirst ? bind2(T, in(2), in(3)) : bind2(T, in(2), in(6));
+  const f128 ab = bind2(T + 1, a, b);
+  const f128 c = kLowFirst ? bind2(T, in(4), in(5)) : bind2(T, in(1), in(5));
+  const f128 d = kLowFirst ? bind2(T, in(6), in(7)) : bind2(T, in(3), in(7));
+  return bind2(T + 2, ab, bind2(T + 1, c, d));
+}
+
+// Which block bits point p has at one and at infinity (the sum over the bit):
+// digit i of p (base 3) is bit i of the block, or bit K - 1 - i when the lowest
+// bit is bound first (the first round's coordinate is always the top digit).
+template <int K, bool kLowFirst>
+static __device__ __forceinline__ void point_bits(int p, int &one, int &inf) {
+  one = inf = 0;
+#pragma unroll
+  for (int i = 0; i < K; i++) {
+    const int d = p % 3, bit = kLowFirst ? K - 1 - i : i;
+    p /= 3;
+    one |= (d == 1) << bit;
+    inf |= (d == 2) << bit;
+  }
+}
+
+// A table's value at a point: blocks `stride` entries apart.
+static __device__ __forceinline__ f128 point_value(const f128 *t, int stride, int one, int inf) {
+  f128 v = t[one * stride];
+  for (int sub = inf; sub; sub = (sub - 1) & inf) v = gadd(v, t[(one | sub) * stride]);
+  return v;
+}
+
+// A pass's sums over the X lanes of each point, then into acc: turn q of thread
+// t has point (t + q kPassThreads) / X.
+template <int kPoints, int kTurns>
+static __device__ __forceinline__ void pass_reduce(const wide (&sum)[kTurns], int lx,
+                                                   unsigned long long *acc) {
+  const int X = 1 << lx;
+#pragma unroll
+  for (int q = 0; q < kTurns; q++) {
+    const int u = threadIdx.x + q * kPassThreads;
+    f128 v = greduce(sum[q]);
+    for (int off = X >> 1; off > 0; off >>= 1) {
+      v.lo ^= __shfl_xor_sync(0xffffffffu, v.lo, off);
+      v.hi ^= __shfl_xor_sync(0xffffffffu, v.hi, off);
+    }
+    if (u < kPoints << lx && (u & (X - 1)) == 0) {
+      atomicXor(acc + 2 * (u >> lx), (unsigned long long)v.lo);
+      atomicXor(acc + 2 * (u >> lx) + 1, (unsigned long long)v.hi);
+    }
+  }
+}
+
+// Every thread calls it after its atomics: the last block to finish posts the
+// first `words` words of acc (and clears them) as handover publication seq.
+static __device__ __forceinline__ void pass_publish(unsigned long long *acc, int words,
+                                                    unsigned int *counter,
+                                                    unsigned long long *handover,
+                                                    unsigned long long seq) {
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last = atomicAdd(counter, 1u) == gridDim.x - 1;
+    __threadfence();
+  }
+  __syncthreads();
+  if (!last) return;
+  for (int k = threadIdx.x; k < words; k += blockDim.x)
+    handover_post(handover, seq, k, atomicExch(acc + k, 0ull));
+  if (threadIdx.x == 0) *counter = 0;
+}
+#endif
+
+}  // namespace bz

@@ -5,6 +5,7 @@
 #include <string>
 
 #include "device.cuh"
+#include "passes.cuh"
 #include "status.hpp"
 #include "transcript.hpp"
 
@@ -21,49 +22,27 @@ struct PostGkrArgs {
 };
 
 // Device scratch, reusable across proofs: four tables of `capacity` entries,
-// a round-accumulator array and a pinned host staging buffer.
+// the passes' sums, and where they are posted: the lane's channel, or (without
+// one) tagged slots in device memory that the host copies and waits for.
 struct PostGkrScratch {
   size_t capacity = 0;
   f128 *w0 = nullptr, *v0 = nullptr, *w1 = nullptr, *v1 = nullptr;
-  unsigned long long *acc = nullptr;  // 8 words per round, 64 rounds
-  uint64_t *host = nullptr;           // pinned, 8 words
+  unsigned long long *acc = nullptr;  // 130 words
   f128 claim_seen{0, 0};              // the weighted sum found when a claim fails
-  RoundChannel *channel = nullptr;    // mailbox for round results; null: copy + sync
-  RoundCtl *ctl = nullptr;            // round controls for queued rounds; null: none
-  // blocks of the cooperative kernel that runs the rounds above the tail
-  // resident (128 for a lane proving alone, fewer for a pooled lane); 0: queued
-  // launches
-  int mid_blocks = 0;
+  RoundChannel *channel = nullptr;
+  unsigned int *counter = nullptr;         // without a channel
+  unsigned long long *handover = nullptr;  // 2 kHandoverWords slots
+  unsigned long long seq = 0;
 };
 
-// Folds k = km .. t0-1 of a quadratic sumcheck over <W, V> (n_in entries
-// each) in one resident cooperative launch of nb blocks: fold
-// k takes its challenge from downbox publication d0 + k (relayed through
-// ctl[k], which must start zeroed), XORs the next message into
-// acc + 8 (k + acc_off) and posts it as publication p0 + k + 1 (the last fold
-// only with emit_last); the folded tables end in (w_out, v_out).
-// pg_mid_start gives the first fold it can take (t0 when none).
-// nb is the grid (0: none fits).
-int pg_mid_start(size_t n1, int t0, int nb);
-// All `rounds` folds of n-entry tables fit launch_pg_mid with nb blocks (the
-// last without a message).
-bool pg_mid_fits_folds(size_t n, int rounds, int nb);
-void launch_pg_mid(const f128 *w_in, const f128 *v_in, size_t n_in, int km, int t0,
-                   int emit_last, int acc_off, f128 *w_out, f128 *v_out, unsigned long long *acc,
-                   RoundChannel *ch, unsigned long long p0, unsigned long long d0, RoundCtl *ctl,
-                   int nb, cudaStream_t s);
-// The grid of a lane's resident post-GKR and Ligerito folds
-// (PostGkrScratch::mid_blocks): 128 for a lane proving alone; for a pooled
-// lane none, or 32 with BITZ_POOL_MID=1.
-int pg_mid_blocks(bool alone);
-
-// The quadratic sumcheck round of <W, V> (shared with the Ligerito folds):
-// quad_sums accumulates (a0, a2) over the pairs as they are; quad_fold folds
-// both tables at r and, with emit, accumulates the next round's sums.
-void quad_sums(const f128 *w, const f128 *v, size_t n, unsigned long long *acc, Publish pub,
+// The quadratic sumcheck of <W, V> (shared with the Ligerito folds), low
+// coordinate first. quad_pass binds both tables at b's challenges (into w2 and
+// v2, when there are any), n entries each after that, and posts the 3^k point
+// sums of the next k rounds; quad_bind only binds (v may be null).
+void quad_pass(int k, const f128 *w, const f128 *v, f128 *w2, f128 *v2, size_t n,
+               const PassBind &b, const PassPost &post, cudaStream_t s);
+void quad_bind(const f128 *w, const f128 *v, f128 *w2, f128 *v2, size_t n, const PassBind &b,
                cudaStream_t s);
-void quad_fold(const f128 *w, const f128 *v, f128 r, f128 *w2, f128 *v2, size_t n, int emit,
-               unsigned long long *acc, Publish pub, cudaStream_t s);
 
 // Runs the whole reduction: writes t+s challenges to point_out and the
 // closing evaluation to value_out, appending every message to `ts`.

@@ -8,7 +8,7 @@
 // their request path (an allocation can block behind work on the whole
 // device). They pass device pointers to the inputs and host pointers for the
 // outputs, and nothing else is needed. The call is not for stream capture:
-// every round copies its message to the host and synchronises the stream so
+// every pass copies its sums to the host and synchronises the stream so
 // that the host transcript can draw the next challenge, and neither is
 // allowed while a stream is being captured.
 //
@@ -27,12 +27,15 @@
 namespace bz {
 
 // Largest claim served: 2^20 bits (log_rows + log_cols <= 20), so four tables
-// of 2^19 F128 each (32 MiB) and round accumulators for up to 64 rounds.
+// of 2^19 F128 each (32 MiB), and the passes' sums with their slots (26 KiB).
 constexpr int kNoAllocMaxLogBits = 20;
 constexpr size_t kNoAllocTable = (size_t)1 << (kNoAllocMaxLogBits - 1);
 
 static __device__ __align__(256) f128 g_noalloc_tables[4 * kNoAllocTable];
-static __device__ __align__(256) unsigned long long g_noalloc_acc[8 * 64];
+// the passes' sums, the block counter (one word behind them) and the tagged
+// slots that the host copies
+constexpr size_t kNoAllocSums = 256;
+static __device__ __align__(256) unsigned long long g_noalloc_acc[kNoAllocSums + 2 * kHandoverWords];
 
 constexpr int kMaxDevices = 64;
 static f128 *s_tables[kMaxDevices];
@@ -100,15 +103,15 @@ int post_gkr_prove_noalloc(const PostGkrArgs &a, Transcript &ts, cudaStream_t s,
   }
   int rc = noalloc_setup(dev, err);
   if (rc) return rc;
-  uint64_t host[8];  // pageable: the round messages copy back synchronously
   PostGkrScratch sc;
   sc.capacity = kNoAllocTable;
   sc.w0 = s_tables[dev];
   sc.v0 = s_tables[dev] + kNoAllocTable;
   sc.w1 = s_tables[dev] + 2 * kNoAllocTable;
   sc.v1 = s_tables[dev] + 3 * kNoAllocTable;
-  sc.acc = s_acc[dev];  // zeroed by post_gkr_prove before its first round
-  sc.host = host;
+  sc.acc = s_acc[dev];  // zeroed by post_gkr_prove before its first pass
+  sc.counter = reinterpret_cast<unsigned int *>(s_acc[dev] + kNoAllocSums - 1);
+  sc.handover = s_acc[dev] + kNoAllocSums;
   return post_gkr_prove(a, ts, sc, s, point_out, value_out);
 }
 

@@ -547,7 +547,6 @@ int ProofSystem::verify(const uint8_t *proof, size_t proof_len, Context *lane) {
   W.bw.upload(bw.data(), 128, s);
   W.lb.resize(np);
   W.lb2.resize(np);
-  W.lf2.resize(np);
   W.eq.resize(np);
   f128 coef = mk(0, 0);
   if (security_ == 100) {
@@ -605,16 +604,20 @@ int ProofSystem::verify(const uint8_t *proof, size_t proof_len, Context *lane) {
   for (int i = 0; i < cfg.nlevels; i++) {
     const PcsLevel &L = cfg.levels[i];
     std::vector<f128> rs;
+    PassBind pb{};
     for (int r = 0; r < L.k; r++) {
       const f128 a0 = rd.f(), a2 = rd.f();
       BZ_VERIFY(lig_grind(), "Ligerito fold grinding nonce");
       const f128 c = t.challenge_f128();
       rs.push_back(c);
       lclaim = advance(lclaim, a0, a2, c);
-      // the basis folds at c (both tables of the fold kernel are the basis)
-      quad_fold(b, b, c, b2, W.lf2.get(), n, 0, W.acc.get(), Publish{nullptr, nullptr, 0}, s);
+      pb.r[pb.k++] = c;
+      if (pb.k < kPassMaxK && r + 1 < L.k) continue;
+      // the basis folds at up to three challenges at once
+      n >>= pb.k;
+      quad_bind(b, nullptr, b2, nullptr, n, pb, s);
       std::swap(b, b2);
-      n /= 2;
+      pb.k = 0;
     }
     const int l = L.log_msg_cols;
     const bool last = i + 1 == cfg.nlevels;

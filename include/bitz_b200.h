@@ -77,7 +77,7 @@ int bitz_post_gkr_prove_dev(const uint64_t *rows_dev, int log_rows, const uint64
  * the library's device memory (32 MiB on every GPU that loads the library,
  * held until the process exits), so log_rows + log_cols must be at most 20:
  * larger claims return BZ_ERR_SCRATCH. Every call shares that array: calls
- * that overlap on the GPU race, so serialise them. Each round copies its
+ * that overlap on the GPU race, so serialise them. Each device pass copies its
  * message to the host and synchronises the stream (the host transcript draws
  * the next challenge), so the call cannot run while a stream is being
  * captured. The first call on a device (and the first after the device's
@@ -280,7 +280,7 @@ int bitz_server_stop(bitz_server *srv);
  * probe off, "*" probes every instrumented launch site, else a comma-separated
  * list of kernel names; enabling resets the totals. While the probe is on,
  * every sumcheck round is its own launch (as under a kernel profiler).
- * Instrumented: gkr_pass, pg_round,
+ * Instrumented: gkr_pass, pg_pass,
  * k_outer_round, k_inner_round, k_fp_finalize. */
 int bitz_probe_kernel(const char *spec);
 /* One kernel's totals since the probe was enabled: out[0] milliseconds,
