@@ -112,14 +112,6 @@ __global__ void __launch_bounds__(128) gkr_high_layers(const f128 *__restrict__ 
 
 // ------------------------------------------------------------------ passes
 
-// Entry `pos` of a table of `n` entries after binding the k coordinates above
-// it: block b of the unbound table starts at b n, the first challenge bound
-// the top bit of b.
-static __device__ __forceinline__ f128 bind_above(const f128 *tab, size_t pos, size_t n,
-                                                  const MulTable *T, int k) {
-  return pass_bind<false>([&](int b) { return ld(tab + pos + b * n); }, T, k);
-}
-
 // Padding: the low s bits of every layer index are the column, and a column at
 // or beyond `live` has only one-valued nodes, before and after any bind
 // (1 + r (1 + 1) = 1). Whenever position x of a block is such a column, so is
@@ -140,21 +132,16 @@ template <int K, int NF>
 __global__ void __launch_bounds__(kPassThreads, 2) gkr_pass(
     f128 *__restrict__ c, size_t n_half, int log_m, PassBind b,
     const __grid_constant__ EqFactors<NF> eq, size_t colmask, uint32_t live, uint32_t count,
-    int lx, unsigned long long *acc, unsigned int *counter, unsigned long long *handover,
-    unsigned long long seq) {
-  constexpr int kPoints = pow3(K), kBlocks = 1 << K;
+    int lx, PassPost post) {
+  constexpr int kPoints = pow3(K), kBlocks = 1 << K, kWords = 2 * (kPoints + 1);
   constexpr int kTurns = (kPoints * kPassMaxX + kPassThreads - 1) / kPassThreads;
+  constexpr int kEqWarp = kPassThreads / 32 - 1;  // the warp that forms a tile's weights
   __shared__ MulTable T[kPassMaxK];
   __shared__ f128 G[kBlocks * kPassMaxX], R[kBlocks * kPassMaxX], E[kPassMaxX];
-  __shared__ f128 F[NF][1 << kFacLog];
   const int t = threadIdx.x;
   const size_t m = (size_t)1 << log_m, n = m << K;
   const int X = 1 << lx;
-  for (int u = t; u < NF << kFacLog; u += kPassThreads) (&F[0][0])[u] = (&eq.f[0][0])[u];
-  if (b.k)
-    pass_tables(T, b);
-  else
-    __syncthreads();
+  pass_tables(T, b.r, b.k);
   // position of live index i: rows of `live` columns when a block spans whole
   // rows of the column space, else i itself
   const bool by_row = m > colmask;
@@ -168,36 +155,55 @@ __global__ void __launch_bounds__(kPassThreads, 2) gkr_pass(
   for (int q = 0; q < kTurns; q++) sum[q] = wzero();
   f128 sum_e = mk(0, 0);
   for (uint32_t i0 = blockIdx.x << lx; i0 < count; i0 += gridDim.x << lx) {
-    const int nbind = 2 * kBlocks << lx;
-    for (int u = t; u < nbind + X; u += kPassThreads) {
-      const uint32_t i = i0 + (u & (X - 1));
-      const bool in = i < count;
-      const size_t x = in ? position(i) : 0;
-      if (u >= nbind) {  // the weight of position x
-        f128 e = mk(0, 0);
-        if (in) {
-          e = F[0][x & ((1 << kFacLog) - 1)];
+    if (t >> 5 == kEqWarp && (t & 31) < X) {
+      const uint32_t i = i0 + (t & 31);
+      f128 e = mk(0, 0);
+      if (i < count) {
+        const size_t x = position(i);
+        e = eq.f[0][x & ((1 << kFacLog) - 1)];
 #pragma unroll 1
-          for (int g = 1; g < NF && g * kFacLog < log_m; g++)
-            e = pass_mul(e, F[g][(x >> (g * kFacLog)) & ((1 << kFacLog) - 1)]);
+        for (int g = 1; g < NF && g * kFacLog < log_m; g++)
+          e = pass_mul(e, eq.f[g][(x >> (g * kFacLog)) & ((1 << kFacLog) - 1)]);
+      }
+      E[t & 31] = e;
+      sum_e = gadd(sum_e, e);
+    }
+    // entry `slot` (block slot >> lx, position slot mod X) of the tile of L,
+    // then of R
+    const int half = kBlocks << lx;
+    auto entry = [&](int slot, f128 *&at) {
+      const uint32_t i = i0 + (slot & (X - 1));
+      at = nullptr;
+      if (i < count)
+        at = (slot >= half ? c + n_half : c) + position(i) +
+             (size_t)((slot & (half - 1)) >> lx) * m;
+    };
+    if (b.k && lx <= kLaneTileLog) {
+      const int gl = b.k - 1;
+      for (int u = t; u < 2 * half << gl; u += kPassThreads) {
+        const int slot = u >> gl;
+        f128 *at;
+        entry(slot, at);
+        f128 v = pass_bind_lanes<false>(
+            [&](int j) { return at ? ld(at + j * n) : mk(0, 0); }, T, b.k, u & ((1 << gl) - 1));
+        if (u & ((1 << gl) - 1)) continue;
+        if (at) st(at, v);
+        (slot >= half ? R : G)[slot & (half - 1)] = v;
+      }
+    } else {
+      for (int slot = t; slot < 2 * half; slot += kPassThreads) {
+        f128 *at;
+        entry(slot, at);
+        f128 v = mk(0, 0);
+        if (at) {
+          v = pass_bind<false>([&](int j) { return ld(at + j * n); }, T, b.k);
+          if (b.k) st(at, v);
         }
-        E[u - nbind] = e;
-        sum_e = gadd(sum_e, e);
-        continue;
+        (slot >= half ? R : G)[slot & (half - 1)] = v;
       }
-      const bool right = u >= nbind / 2;
-      const int slot = right ? u - nbind / 2 : u;
-      f128 v = mk(0, 0);
-      if (in) {
-        f128 *tab = right ? c + n_half : c;
-        const size_t pos = x + (size_t)(slot >> lx) * m;
-        v = bind_above(tab, pos, n, T, b.k);
-        if (b.k) st(tab + pos, v);
-      }
-      (right ? R : G)[slot] = v;
     }
     __syncthreads();
-    for (int u = t; u < kBlocks << lx; u += kPassThreads) G[u] = pass_mul(E[u & (X - 1)], G[u]);
+    for (int u = t; u < half; u += kPassThreads) G[u] = pass_mul(E[u & (X - 1)], G[u]);
     __syncthreads();
 #pragma unroll
     for (int q = 0; q < kTurns; q++) {
@@ -211,30 +217,43 @@ __global__ void __launch_bounds__(kPassThreads, 2) gkr_pass(
     }
     __syncthreads();  // the tile's tables before the next tile's
   }
-  pass_reduce<kPoints, kTurns>(sum, lx, acc);
-  for (int off = 16; off > 0; off >>= 1) {
-    sum_e.lo ^= __shfl_xor_sync(0xffffffffu, sum_e.lo, off);
-    sum_e.hi ^= __shfl_xor_sync(0xffffffffu, sum_e.hi, off);
+  const bool direct = pass_direct(gridDim.x, kWords);
+  pass_reduce<kPoints, kTurns>(sum, lx, kWords, direct, post);
+  if (t >> 5 == kEqWarp) {
+    for (int off = 16; off > 0; off >>= 1) {
+      sum_e.lo ^= __shfl_xor_sync(0xffffffffu, sum_e.lo, off);
+      sum_e.hi ^= __shfl_xor_sync(0xffffffffu, sum_e.hi, off);
+    }
+    if ((t & 31) == 0) {
+      const int at = 2 * kPoints;
+      if (direct) {
+        handover_post(post.handover, post.seq, blockIdx.x * kWords + at, sum_e.lo);
+        handover_post(post.handover, post.seq, blockIdx.x * kWords + at + 1, sum_e.hi);
+      } else {
+        atomicXor(post.acc + at, (unsigned long long)sum_e.lo);
+        atomicXor(post.acc + at + 1, (unsigned long long)sum_e.hi);
+      }
+    }
   }
-  if ((t & 31) == 0 && (sum_e.lo | sum_e.hi)) {
-    atomicXor(acc + 2 * kPoints, (unsigned long long)sum_e.lo);
-    atomicXor(acc + 2 * kPoints + 1, (unsigned long long)sum_e.hi);
-  }
-  pass_publish(acc, 2 * (kPoints + 1), counter, handover, seq);
+  if (!direct) pass_publish(post.acc, kWords, post.counter, post.handover, post.seq);
 }
 
 // The layer's last tables to the host: L, then R, of n entries each after the
 // binds of `b`, as handover publication seq (two words per entry).
-constexpr int kHandThreads = 256, kHandEntries = 64;  // threads build the tables, entries bind
+constexpr int kHandThreads = 256, kHandEntries = 64;  // up to four lanes per entry
 __global__ void __launch_bounds__(kHandThreads) gkr_handover(const f128 *__restrict__ c,
                                                              size_t n_half, int n, PassBind b,
                                                              unsigned long long *handover,
                                                              unsigned long long seq) {
   __shared__ MulTable T[kPassMaxK];
-  pass_tables(T, b);
-  const int k = blockIdx.x * kHandEntries + threadIdx.x;
-  if (threadIdx.x >= kHandEntries || k >= 2 * n) return;
-  const f128 v = k < n ? bind_above(c, k, n, T, b.k) : bind_above(c + n_half, k - n, n, T, b.k);
+  pass_tables(T, b.r, b.k);
+  const int gl = b.k > 1 ? b.k - 1 : 0, q = threadIdx.x & ((1 << gl) - 1);
+  if (threadIdx.x >> 5 >= (kHandEntries << gl) >> 5) return;  // whole warps
+  const int k = blockIdx.x * kHandEntries + (threadIdx.x >> gl);
+  const f128 *at = k < n ? c + k : c + n_half + (k - n);
+  auto in = [&](int j) { return k < 2 * n ? ld(at + (size_t)j * n) : mk(0, 0); };
+  const f128 v = b.k ? pass_bind_lanes<false>(in, T, b.k, q) : in(0);
+  if (q || k >= 2 * n) return;
   handover_post(handover, seq, 2 * k, v.lo);
   handover_post(handover, seq, 2 * k + 1, v.hi);
 }
@@ -515,30 +534,31 @@ static_assert(4 << kHostLog <= kHandoverWords, "the last tables fit one handover
 // next pass): two rounds from this size on, where products are the cost.
 constexpr int kFirstLog = 17;
 
+// Returns how many blocks post sums of their own.
 template <int K, int NF>
-static void launch_pass_nf(f128 *c, size_t n_half, int log_m, const PassBind &b, const EqHeap *heap,
-                           size_t colmask, uint32_t live, uint32_t count, GkrScratch &sc,
-                           unsigned long long seq, cudaStream_t st) {
+static int launch_pass_nf(f128 *c, size_t n_half, int log_m, const PassBind &b, const EqHeap *heap,
+                           size_t colmask, uint32_t live, uint32_t count, const PassPost &post,
+                           cudaStream_t st) {
   EqFactors<NF> eq;
   for (int g = 0; g < NF; g++) {
     const int have = std::min(kFacLog, std::max(0, log_m - g * kFacLog));
     memcpy(eq.f[g], heap[g].prefix(have), sizeof(f128) << have);
   }
   const int lx = pass_tile_log(count);
-  gkr_pass<K, NF><<<pass_grid(count, lx), kPassThreads, 0, st>>>(
-      c, n_half, log_m, b, eq, colmask, live, count, lx, sc.acc, sc.channel->counter,
-      sc.channel->handover_dev, seq);
+  const unsigned int grid = pass_grid(count, lx);
+  gkr_pass<K, NF><<<grid, kPassThreads, 0, st>>>(c, n_half, log_m, b, eq, colmask, live, count, lx,
+                                                 post);
   BZ_LAUNCH_CHECK();
+  return pass_direct(grid, 2 * (pow3(K) + 1)) ? (int)grid : 1;
 }
 
 template <int K>
-static void launch_pass(f128 *c, size_t n_half, int log_m, const PassBind &b, const EqHeap *heap,
-                        size_t colmask, uint32_t live, uint32_t count, GkrScratch &sc,
-                        unsigned long long seq, cudaStream_t st) {
+static int launch_pass(f128 *c, size_t n_half, int log_m, const PassBind &b, const EqHeap *heap,
+                        size_t colmask, uint32_t live, uint32_t count, const PassPost &post,
+                        cudaStream_t st) {
   if (log_m <= 2 * kFacLog)
-    launch_pass_nf<K, 2>(c, n_half, log_m, b, heap, colmask, live, count, sc, seq, st);
-  else
-    launch_pass_nf<K, 5>(c, n_half, log_m, b, heap, colmask, live, count, sc, seq, st);
+    return launch_pass_nf<K, 2>(c, n_half, log_m, b, heap, colmask, live, count, post, st);
+  return launch_pass_nf<K, 5>(c, n_half, log_m, b, heap, colmask, live, count, post, st);
 }
 
 void gkr_build(const f128 *cols, int s, const f128 *images, GkrScratch &sc, cudaStream_t st_) {
@@ -729,11 +749,9 @@ f128 gkr_prove(const f128 *cols, int s, const f128 *images, const f128 *zeta, ui
       const int points = pow3(k);
       const bool probed = probe.on("gkr_pass");
       if (probed) probe.before(st_);
-      const unsigned long long seq = ch->arm().seq;
-      if (k == 2)
-        launch_pass<2>(c, n_half, log_m, b, heap.data(), colmask, (uint32_t)live, count, sc, seq, st_);
-      else
-        launch_pass<3>(c, n_half, log_m, b, heap.data(), colmask, (uint32_t)live, count, sc, seq, st_);
+      const PassPost post{sc.acc, ch->counter, ch->handover_dev, ch->arm().seq};
+      const int blocks = (k == 2 ? launch_pass<2> : launch_pass<3>)(
+          c, n_half, log_m, b, heap.data(), colmask, (uint32_t)live, count, post, st_);
       if (probed) {
         // per live position: 2^(k+1) entries of the bound tables, each from
         // 2^kb read and one written (none written without a bind), 2^kb - 1
@@ -744,7 +762,8 @@ f128 gkr_prove(const f128 *cols, int s, const f128 *images, const f128 *zeta, ui
                     (double)count * ((1 << k) + (log_m - 1) / kFacLog), (double)count * points,
                     e * (in - 1));
       }
-      ch->wait_handover(st_, seq, words.data(), 2 * (points + 1));
+      ch->wait_handover(st_, post.seq, words.data(), 2 * (points + 1) * blocks);
+      pass_combine(words.data(), 2 * (points + 1), blocks);
       mark("pass");
       F.resize(points);
       for (int p = 0; p < points; p++) F[p] = mk(words[2 * p], words[2 * p + 1]);

@@ -88,6 +88,16 @@ inline int pass_tile_log(uint32_t count) {
   while (lx > 2 && (count >> lx) < (uint32_t)kSMs) lx--;
   return lx;
 }
+// Few blocks post their sums by themselves (the host adds them up) instead of
+// through atomics and a last block: three trips to the L2 less, 1.4 us.
+__host__ __device__ inline bool pass_direct(unsigned int grid, int words) {
+  return grid * (unsigned int)words <= (unsigned int)kHandoverWords;
+}
+// Adds the blocks' words up into the first `words`.
+inline void pass_combine(uint64_t *w, int words, int blocks) {
+  for (int b = 1; b < blocks; b++)
+    for (int k = 0; k < words; k++) w[k] ^= w[b * words + k];
+}
 inline unsigned int pass_grid(uint32_t count, int lx) {
   const uint32_t tiles = (count + (1u << lx) - 1) >> lx;
   return tiles < 1 ? 1 : tiles < 2u * kSMs ? tiles : 2u * kSMs;
@@ -122,16 +132,33 @@ static __device__ __forceinline__ void fill_windows(uint64_t (*lo)[16], uint64_t
   }
 }
 
-// The window tables of b.r[0 .. b.k), every thread of the block taking part.
-static __device__ __forceinline__ void pass_tables(MulTable *T, const PassBind &b) {
-  for (int u = threadIdx.x; u < b.k * 128; u += blockDim.x) {
-    const int t = u >> 7, k = u & 127;
-    const f128 v = gmul_xk(b.r[t], k);
-    T[t].lo[k >> 2][1 << (k & 3)] = v.lo;
-    T[t].hi[k >> 2][1 << (k & 3)] = v.hi;
+// v X, reduced.
+static __device__ __forceinline__ f128 times_x(f128 v) {
+  return mk((v.lo << 1) ^ ((0 - (v.hi >> 63)) & 0x87), (v.hi << 1) | (v.lo >> 63));
+}
+
+// The window tables of r[0 .. k), every thread of the block taking part: a
+// thread forms a window's four single-bit entries in registers and writes four
+// entries of the window, so the build is one step without a barrier inside.
+static __device__ __forceinline__ void pass_tables(MulTable *T, const f128 *r, int k) {
+  for (int u = threadIdx.x; u < k * 128; u += blockDim.x) {
+    const int t = u >> 7, j = (u >> 2) & 31, top = u & 3;
+    const f128 v = r[t];
+    const int s = (4 * j) & 63;
+    const uint64_t w0 = v.lo << s, w1 = (v.hi << s) | ((v.lo >> 1) >> (63 - s)),
+                   w2 = (v.hi >> 1) >> (63 - s);
+    f128 b[4];
+    b[0] = greduce(j >= 16 ? wide{0, w0, w1, w2} : wide{w0, w1, w2, 0});  // r X^(4j)
+#pragma unroll
+    for (int q = 1; q < 4; q++) b[q] = times_x(b[q - 1]);
+    f128 e = mk(0, 0);
+    if (top & 1) e = b[2];
+    if (top & 2) e = gadd(e, b[3]);
+    uint64_t *lo = T[t].lo[j] + 4 * top, *hi = T[t].hi[j] + 4 * top;
+    const f128 e1 = gadd(e, b[0]), e2 = gadd(e, b[1]), e3 = gadd(e1, b[1]);
+    lo[0] = e.lo, lo[1] = e1.lo, lo[2] = e2.lo, lo[3] = e3.lo;
+    hi[0] = e.hi, hi[1] = e1.hi, hi[2] = e2.hi, hi[3] = e3.hi;
   }
-  __syncthreads();
-  for (int t = 0; t < b.k; t++) fill_windows(T[t].lo, T[t].hi, 32);
   __syncthreads();
 }
 
@@ -146,17 +173,40 @@ static __device__ __forceinline__ f128 pass_bind(In in, const MulTable *T, int k
   if (k == 0) return in(0);
   if (k == 1) return bind2(T, in(0), in(1));
   if (k == 2) {
-    const f128 a = kLowFirst ? bind2(T, in(0), in(1)) : bind2(T, in(0), in(2));
-    const f128 b = kLowFirst ? bind2(T, in(2), in(3)) : bind2(T, in(1), in(3));
+    const f128 x[4] = {in(0), in(kLowFirst ? 1 : 2), in(kLowFirst ? 2 : 1), in(3)};
+    const f128 a = bind2(T, x[0], x[1]), b = bind2(T, x[2], x[3]);
     return bind2(T + 1, a, b);
   }
-  const f128 a = kLowFirst ? bind2(T, in(0), in(1)) : bind2(T, in(0), in(4));
-  const f128 b = kLowFirst ? bind2(T, in(2), in(3)) : bind2(T, in(2), in(6));
-  const f128 ab = bind2(T + 1, a, b);
-  const f128 c = kLowFirst ? bind2(T, in(4), in(5)) : bind2(T, in(1), in(5));
-  const f128 d = kLowFirst ? bind2(T, in(6), in(7)) : bind2(T, in(3), in(7));
+  // pairs of the first challenge, in the order the second one joins them; all
+  // loads before the first product
+  f128 x[8];
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    constexpr int kLow[8] = {0, 1, 2, 3, 4, 5, 6, 7}, kHigh[8] = {0, 4, 2, 6, 1, 5, 3, 7};
+    x[i] = in(kLowFirst ? kLow[i] : kHigh[i]);
+  }
+  const f128 a = bind2(T, x[0], x[1]), b = bind2(T, x[2], x[3]), ab = bind2(T + 1, a, b);
+  const f128 c = bind2(T, x[4], x[5]), d = bind2(T, x[6], x[7]);
   return bind2(T + 2, ab, bind2(T + 1, c, d));
 }
+
+// The same by 2^(k-1) neighbouring lanes, lane q of them: one pair per lane,
+// then joined by exchanges. Three products deep instead of seven (0.9 against
+// 6.2 us for a small pass); it makes 12 lane products for 7, so only where a
+// block has few entries. k >= 1, every lane of the warp.
+template <bool kLowFirst, class In>
+static __device__ __forceinline__ f128 pass_bind_lanes(In in, const MulTable *T, int k, int q) {
+  const int g = 1 << (k - 1);
+  f128 v = kLowFirst ? bind2(T, in(2 * q), in(2 * q + 1)) : bind2(T, in(q), in(q + g));
+  for (int l = 1; l < k; l++) {
+    const int m = kLowFirst ? 1 << (l - 1) : g >> l;
+    const f128 o = mk(__shfl_xor_sync(0xffffffffu, v.lo, m), __shfl_xor_sync(0xffffffffu, v.hi, m));
+    v = (q & m) ? bind2(T + l, o, v) : bind2(T + l, v, o);
+  }
+  return v;
+}
+// Tiles up to this size (log) bind by lanes.
+constexpr int kLaneTileLog = 3;
 
 // Which block bits point p has at one and at infinity (the sum over the bit):
 // digit i of p (base 3) is bit i of the block, or bit K - 1 - i when the lowest
@@ -180,23 +230,30 @@ static __device__ __forceinline__ f128 point_value(const f128 *t, int stride, in
   return v;
 }
 
-// A pass's sums over the X lanes of each point, then into acc: turn q of thread
-// t has point (t + q kPassThreads) / X.
+// A pass's sums over the X lanes of each point: turn q of thread t has point
+// (t + q kPassThreads) / X. Into acc, or, where every block posts by itself,
+// to words 2 p and 2 p + 1 of the block's `words` handover words.
 template <int kPoints, int kTurns>
-static __device__ __forceinline__ void pass_reduce(const wide (&sum)[kTurns], int lx,
-                                                   unsigned long long *acc) {
+static __device__ __forceinline__ void pass_reduce(const wide (&sum)[kTurns], int lx, int words,
+                                                   bool direct, const PassPost &post) {
   const int X = 1 << lx;
 #pragma unroll
   for (int q = 0; q < kTurns; q++) {
-    const int u = threadIdx.x + q * kPassThreads;
+    const int u = threadIdx.x + q * kPassThreads, p = u >> lx;
+    if ((u & ~31) >= kPoints << lx) break;  // the whole warp
     f128 v = greduce(sum[q]);
     for (int off = X >> 1; off > 0; off >>= 1) {
       v.lo ^= __shfl_xor_sync(0xffffffffu, v.lo, off);
       v.hi ^= __shfl_xor_sync(0xffffffffu, v.hi, off);
     }
-    if (u < kPoints << lx && (u & (X - 1)) == 0) {
-      atomicXor(acc + 2 * (u >> lx), (unsigned long long)v.lo);
-      atomicXor(acc + 2 * (u >> lx) + 1, (unsigned long long)v.hi);
+    if (p < kPoints && (u & (X - 1)) == 0) {
+      if (direct) {
+        handover_post(post.handover, post.seq, blockIdx.x * words + 2 * p, v.lo);
+        handover_post(post.handover, post.seq, blockIdx.x * words + 2 * p + 1, v.hi);
+      } else {
+        atomicXor(post.acc + 2 * p, (unsigned long long)v.lo);
+        atomicXor(post.acc + 2 * p + 1, (unsigned long long)v.hi);
+      }
     }
   }
 }

@@ -179,7 +179,7 @@ static __device__ __forceinline__ void bit_values(f128 *V8, const BitWeights &e)
 static __device__ __forceinline__ f128 bind_low(const f128 *tab, size_t o, const MulTable *T,
                                                 int k) {
   const f128 *p = tab + (o << k);
-  return pass_bind<true>([&](int b) { return ld(p + b); }, T, k);
+  return pass_bind<true>([&](int j) { return ld(p + j); }, T, k);
 }
 
 // One pass over the low K coordinates of W and V (n entries each after the binds
@@ -195,8 +195,7 @@ template <int K, bool kBits>
 __global__ void __launch_bounds__(kPassThreads, 2) pg_pass(
     const f128 *__restrict__ w_in, const f128 *__restrict__ v_in, f128 *__restrict__ w_out,
     f128 *__restrict__ v_out, uint32_t count, PassBind b, const __grid_constant__ BitWeights e8,
-    int lx, unsigned long long *acc, unsigned int *counter, unsigned long long *handover,
-    unsigned long long seq) {
+    int lx, PassPost post) {
   constexpr int kPoints = pow3(K), kBlocks = 1 << K;
   constexpr int kTurns = (kPoints * kPassMaxX + kPassThreads - 1) / kPassThreads;
   __shared__ MulTable T[kPassMaxK];
@@ -204,13 +203,31 @@ __global__ void __launch_bounds__(kPassThreads, 2) pg_pass(
   __shared__ f128 V8[kBits ? 256 : 1];
   const int t = threadIdx.x, X = 1 << lx;
   if (kBits) bit_values(V8, e8);
-  pass_tables(T, b);
+  pass_tables(T, b.r, b.k);
   wide sum[kTurns];
 #pragma unroll
   for (int q = 0; q < kTurns; q++) sum[q] = wzero();
   for (uint32_t i0 = blockIdx.x << lx; i0 < count; i0 += gridDim.x << lx) {
     const int half = kBlocks << lx;
-    for (int u = t; u < 2 * half; u += kPassThreads) {
+    const bool lanes = b.k && lx <= kLaneTileLog;
+    if (lanes) {
+      const int gl = b.k - 1, total = (kBits ? half : 2 * half) << gl;
+      for (int u = t; u < total; u += kPassThreads) {
+        const int at = u >> gl, q = u & ((1 << gl) - 1);
+        const bool right = at >= half;
+        const int slot = at & (half - 1), x = slot >> K;
+        const bool in = i0 + x < count;
+        const size_t o = ((size_t)i0 << K) + slot;
+        const f128 *p = (right ? v_in : w_in) + (o << b.k);
+        const f128 v = pass_bind_lanes<true>([&](int j) { return in ? ld(p + j) : mk(0, 0); }, T,
+                                             b.k, q);
+        if (q) continue;
+        if (in) st((right ? v_out : w_out) + o, v);
+        (right ? R : G)[(slot & (kBlocks - 1)) * (X + 1) + x] = v;
+      }
+    }
+    // one thread per entry (with lanes, only V's bytes are left)
+    for (int u = lanes ? t + half : t; u < 2 * half && (!lanes || kBits); u += kPassThreads) {
       const bool right = u >= half;
       const int slot = right ? u - half : u, x = slot >> K, a = slot & (kBlocks - 1);
       f128 v = mk(0, 0);
@@ -238,8 +255,9 @@ __global__ void __launch_bounds__(kPassThreads, 2) pg_pass(
     }
     __syncthreads();  // the tile's tables before the next tile's
   }
-  pass_reduce<kPoints, kTurns>(sum, lx, acc);
-  pass_publish(acc, 2 * kPoints, counter, handover, seq);
+  const bool direct = pass_direct(gridDim.x, 2 * kPoints);
+  pass_reduce<kPoints, kTurns>(sum, lx, 2 * kPoints, direct, post);
+  if (!direct) pass_publish(post.acc, 2 * kPoints, post.counter, post.handover, post.seq);
 }
 
 // The binds of b alone: n entries of each table.
@@ -249,7 +267,7 @@ __global__ void __launch_bounds__(kThreads) pg_bind(const f128 *__restrict__ w_i
                                                     f128 *__restrict__ v_out, size_t n,
                                                     PassBind b) {
   __shared__ MulTable T[kPassMaxK];
-  pass_tables(T, b);
+  pass_tables(T, b.r, b.k);
   const size_t total = v_in ? 2 * n : n;
   for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < total;
        k += (size_t)gridDim.x * blockDim.x) {
@@ -260,7 +278,7 @@ __global__ void __launch_bounds__(kThreads) pg_bind(const f128 *__restrict__ w_i
 }
 
 // The last tables to the host: W, then V, of n entries each after the binds of b.
-constexpr int kHandThreads = 256, kHandEntries = 64;  // threads build the tables, entries bind
+constexpr int kHandThreads = 256, kHandEntries = 64;  // up to four lanes per entry
 template <bool kBits>
 __global__ void __launch_bounds__(kHandThreads) pg_handover(const f128 *__restrict__ w_in,
                                                             const f128 *__restrict__ v_in, int n,
@@ -270,16 +288,16 @@ __global__ void __launch_bounds__(kHandThreads) pg_handover(const f128 *__restri
   __shared__ MulTable T[kPassMaxK];
   __shared__ f128 V8[kBits ? 256 : 1];
   if (kBits) bit_values(V8, e8);
-  pass_tables(T, b);
-  const int k = blockIdx.x * kHandEntries + threadIdx.x;
-  if (threadIdx.x >= kHandEntries || k >= 2 * n) return;
-  f128 v;
-  if (k < n)
-    v = bind_low(w_in, k, T, b.k);
-  else if (kBits)
-    v = V8[reinterpret_cast<const uint8_t *>(v_in)[k - n]];
-  else
-    v = bind_low(v_in, k - n, T, b.k);
+  pass_tables(T, b.r, b.k);
+  const int gl = b.k > 1 ? b.k - 1 : 0, q = threadIdx.x & ((1 << gl) - 1);
+  if (threadIdx.x >> 5 >= (kHandEntries << gl) >> 5) return;  // whole warps
+  const int k = blockIdx.x * kHandEntries + (threadIdx.x >> gl);
+  const f128 *at = k < n ? w_in + ((size_t)k << b.k) : v_in + ((size_t)(k - n) << b.k);
+  const bool byte = kBits && k >= n;
+  auto in = [&](int j) { return k < 2 * n && !byte ? ld(at + j) : mk(0, 0); };
+  f128 v = b.k ? pass_bind_lanes<true>(in, T, b.k, q) : in(0);
+  if (q || k >= 2 * n) return;
+  if (byte) v = V8[reinterpret_cast<const uint8_t *>(v_in)[k - n]];
   handover_post(handover, seq, 2 * k, v.lo);
   handover_post(handover, seq, 2 * k + 1, v.hi);
 }
@@ -329,31 +347,30 @@ __global__ void __launch_bounds__(kThreads) pg_bound_cols(const f128 *__restrict
   }
 }
 
+// Returns how many blocks post sums of their own.
 template <int K, bool kBits>
-static void launch_quad(const f128 *w, const f128 *v, f128 *w2, f128 *v2, size_t n,
+static int launch_quad(const f128 *w, const f128 *v, f128 *w2, f128 *v2, size_t n,
                         const PassBind &b, const BitWeights &e8, const PassPost &post,
                         cudaStream_t s) {
   const uint32_t count = (uint32_t)(n >> K);
   const int lx = pass_tile_log(count);
-  pg_pass<K, kBits><<<pass_grid(count, lx), kPassThreads, 0, s>>>(
-      w, v, w2, v2, count, b, e8, lx, post.acc, post.counter, post.handover, post.seq);
+  const unsigned int grid = pass_grid(count, lx);
+  pg_pass<K, kBits><<<grid, kPassThreads, 0, s>>>(w, v, w2, v2, count, b, e8, lx, post);
   BZ_LAUNCH_CHECK();
+  return pass_direct(grid, 2 * pow3(K)) ? (int)grid : 1;
 }
 
-static void quad_pass_from(bool bits, int k, const f128 *w, const f128 *v, f128 *w2, f128 *v2,
+static int quad_pass_from(bool bits, int k, const f128 *w, const f128 *v, f128 *w2, f128 *v2,
                            size_t n, const PassBind &b, const BitWeights &e8,
                            const PassPost &post, cudaStream_t s) {
   KernelProbe &probe = KernelProbe::get();
   const bool probed = probe.on("pg_pass");
   if (probed) probe.before(s);
-  if (bits)
-    launch_quad<3, true>(w, v, w2, v2, n, b, e8, post, s);
-  else if (k == 3)
-    launch_quad<3, false>(w, v, w2, v2, n, b, e8, post, s);
-  else if (k == 2)
-    launch_quad<2, false>(w, v, w2, v2, n, b, e8, post, s);
-  else
-    launch_quad<1, false>(w, v, w2, v2, n, b, e8, post, s);
+  const auto launch = bits     ? launch_quad<3, true>
+                      : k == 3 ? launch_quad<3, false>
+                      : k == 2 ? launch_quad<2, false>
+                               : launch_quad<1, false>;
+  const int blocks = launch(w, v, w2, v2, n, b, e8, post, s);
   if (probed) {
     // an entry of each table comes from 2^kb (a byte of f for V with bits)
     // and is written when there is a bind; 2^kb - 1 products through window
@@ -363,11 +380,12 @@ static void quad_pass_from(bool bits, int k, const f128 *w, const f128 *v, f128 
                 (double)n * (16.0 * (tabs * in + (b.k ? 2.0 : 0.0)) + (bits ? 1.0 : 0.0)), 0.0,
                 (double)(n >> k) * pow3(k), tabs * (double)n * (in - 1));
   }
+  return blocks;
 }
 
-void quad_pass(int k, const f128 *w, const f128 *v, f128 *w2, f128 *v2, size_t n,
+int quad_pass(int k, const f128 *w, const f128 *v, f128 *w2, f128 *v2, size_t n,
                const PassBind &b, const PassPost &post, cudaStream_t s) {
-  quad_pass_from(false, k, w, v, w2, v2, n, b, BitWeights{}, post, s);
+  return quad_pass_from(false, k, w, v, w2, v2, n, b, BitWeights{}, post, s);
 }
 
 void quad_bind(const f128 *w, const f128 *v, f128 *w2, f128 *v2, size_t n, const PassBind &b,
@@ -459,14 +477,16 @@ struct PostGkrRun {
       // entry, three 3.4, and above 2^17 entries the products are the cost
       const int k = b.k == 0 && rem >= 17 ? 2 : 3;
       const PassPost post = arm();
-      quad_pass_from(bits, k, w, v, bufs[set][0], bufs[set][1], (size_t)1 << rem, b, e8, post, s);
+      const int blocks = quad_pass_from(bits, k, w, v, bufs[set][0], bufs[set][1], (size_t)1 << rem,
+                                        b, e8, post, s);
       if (b.k) {
         w = bufs[set][0];
         v = bufs[set][1];
         set ^= 1;
         bits = false;
       }
-      wait(post, 2 * pow3(k));
+      wait(post, 2 * pow3(k) * blocks);
+      pass_combine(words.data(), 2 * pow3(k), blocks);
       F.resize(pow3(k));
       for (int p = 0; p < pow3(k); p++) F[p] = mk(words[2 * p], words[2 * p + 1]);
       if (!from_points(k, b.r)) return BZ_ERR_CLAIM;

@@ -38,8 +38,9 @@ struct PostGkrScratch {
 // The quadratic sumcheck of <W, V> (shared with the Ligerito folds), low
 // coordinate first. quad_pass binds both tables at b's challenges (into w2 and
 // v2, when there are any), n entries each after that, and posts the 3^k point
-// sums of the next k rounds; quad_bind only binds (v may be null).
-void quad_pass(int k, const f128 *w, const f128 *v, f128 *w2, f128 *v2, size_t n,
+// sums of the next k rounds (it returns how many blocks post sums of their own,
+// to be added up); quad_bind only binds (v may be null).
+int quad_pass(int k, const f128 *w, const f128 *v, f128 *w2, f128 *v2, size_t n,
                const PassBind &b, const PassPost &post, cudaStream_t s);
 void quad_bind(const f128 *w, const f128 *v, f128 *w2, f128 *v2, size_t n, const PassBind &b,
                cudaStream_t s);

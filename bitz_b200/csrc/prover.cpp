@@ -493,13 +493,14 @@ std::vector<uint8_t> ProofSystem::ligerito(cudaStream_t s, f128 target) {
       const int k = std::min(kPassMaxK, L.k - r), points = pow3(k);
       const PassPost post{acc, ch->counter, ch->handover_dev, ch->arm().seq};
       n >>= pb.k;
-      quad_pass(k, b, f, b2, f2, n, pb, post, s);
+      const int blocks = quad_pass(k, b, f, b2, f2, n, pb, post, s);
       if (pb.k) {
         std::swap(f, f2);
         std::swap(b, b2);
       }
-      std::vector<uint64_t> words(2 * points);
-      ch->wait_handover(s, post.seq, words.data(), 2 * points);
+      std::vector<uint64_t> words(2 * points * blocks);
+      ch->wait_handover(s, post.seq, words.data(), 2 * points * blocks);
+      pass_combine(words.data(), 2 * points, blocks);
       std::vector<f128> F(points);
       for (int p = 0; p < points; p++) F[p] = mk(words[2 * p], words[2 * p + 1]);
       quad_rounds(F, k, pb.r, [&](f128 a0, f128 a2) {
