@@ -280,7 +280,6 @@ Context::Context() {
   channel_.counter = counter_.get();
   pg_.channel = &channel_;
   gk_.channel = &channel_;
-  sp_mid_blocks_ = ::bz::sp_mid_blocks(false);
   lane_bootstrap(*this);
 }
 
@@ -306,7 +305,6 @@ Context &Context::get() {
   // launches (or 32-block grids with BITZ_POOL_MID=1).
   static Context *ctx = [] {
     Context *c = new Context();
-    c->sp_mid_blocks_ = ::bz::sp_mid_blocks(true);
     return c;
   }();
   return *ctx;

@@ -111,8 +111,6 @@ class Context {
   RoundChannel *channel() { return &channel_; }
   // The lane's round controls (kMaxPointGkr entries), used by one phase at a time.
   RoundCtl *round_ctl() { return gk_ctl_.get(); }
-  // Grid of the resident Spartan grid rounds on this lane (0: none).
-  int sp_mid_blocks() const { return sp_mid_blocks_; }
   // Prover workspace slot, owned by the lane (created by the prover).
   std::shared_ptr<Workspace> workspace;
 
@@ -164,7 +162,6 @@ class Context {
   DeviceBuffer<RoundCtl> gk_ctl_;
   RoundChannel channel_;
   DeviceBuffer<unsigned int> counter_;
-  int sp_mid_blocks_ = 0;
 };
 
 // Loads kernels now (cudaFuncGetAttributes), so no kernel is loaded on its

@@ -670,7 +670,7 @@ int ProofSystem::prove_after_commit(cudaStream_t s, std::vector<uint8_t> &proof)
   W.sp_t.resize(8 * R);
   W.sp_d.resize(4 * Cn);
   W.sp_eqs.resize(4096 * 2 + ((size_t)1 << ((std::max(nr, nc) + 1) / 2 + 1)));
-  W.sp_part.resize(3 * kSMs * 8 + 16);
+  W.sp_part.resize(kSpPartials);
   W.sp_sums.resize(4);
   W.sp_tab.resize(dev_->ntab + 1);
   if (bit_rows_.empty())
@@ -686,8 +686,6 @@ int ProofSystem::prove_after_commit(cudaStream_t s, std::vector<uint8_t> &proof)
   sc.tab = W.sp_tab.get();
   sc.host = W.host_fp;
   sc.channel = ctx.channel();
-  sc.ctl = ctx.round_ctl();
-  sc.mid_blocks = ctx.sp_mid_blocks();
   SpartanArgs sa;
   sa.ctx = fc;
   sa.q = q;

@@ -2,13 +2,20 @@
 // transcript-drawn prime (crates/spartan/src/piop.rs:67-113,
 // sumcheck.rs:252-553, matrix.rs:336-467).
 //
-// Tables hold Montgomery residues. Each round is one launch that folds the
-// previous round's challenge into every table and accumulates the next
-// round's coefficients from the folded values in registers (the reference's
-// fold/round fusion, sumcheck.rs:963-1026), then one single-block launch adds
-// the per-block partial sums; 48 (outer) or 32 (inner) bytes go to the host.
+// Tables hold Montgomery residues. Both sumchecks bind their lowest coordinate
+// first and go through the device in passes of up to three rounds (passes.cuh):
+// a pass posts the summed polynomial's values at the points {0, 1, infinity}^K
+// (infinity: the coefficient of X^2, from the differences of the halves) and
+// the host runs K rounds from them. The outer polynomial is
+// eq(tau) (A B - C); eq is a product over the coordinates, so the passes sum
+// only A B - C, weighted by eq over the coordinates above, and the host
+// multiplies the round's own linear factor in. The inner one is D W with W the
+// packed bits of h: its first three rounds need 64 sums of D by position and
+// bit position within groups of eight, and W after their binds is a 256-entry
+// table of the group's byte.
 #include "device.cuh"
 #include "context.hpp"
+#include "passes.cuh"
 #include "spartan.hpp"
 
 #include <chrono>
@@ -100,184 +107,11 @@ BZ_HD void cubic(fp e0, fp e1, fp a0, fp a1, fp b0, fp b1, fp c0, fp c1, const F
   acc[2] = fp_add(acc[2], fp_mul(ed, rq, c), c);
 }
 
-// The round's message from the blocks' partial sums (block_fp_sum<N> left
-// them at partial[block * N + k], written by thread 0): the last block to
-// count itself in `counter` adds every block's partials (mod q, in any order)
-// and posts the N totals as words 2k (low half) and 2k + 1 (high half) of
-// publication seq. Every thread calls it; true in the last block (whose
-// threads are still together), false in the others.
-template <int N>
-__device__ bool fp_last_block_post(const fp *partial, const FpCtx &c, unsigned int *counter,
-                                   Mailbox *mb, unsigned long long seq) {
-  static_assert(2 * N <= kMailboxWords, "mailbox too small");
-  __shared__ int last_s;
-  __shared__ fp red[N][kThreads / 32];
-  if (threadIdx.x == 0) {
-    __threadfence();
-    last_s = atomicAdd(counter, 1u) == gridDim.x - 1;
-  }
-  __syncthreads();
-  if (!last_s) return false;
-  __threadfence();
-  fp v[N];
-#pragma unroll
-  for (int k = 0; k < N; k++) v[k] = fp_zero();
-  for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x)
-#pragma unroll
-    for (int k = 0; k < N; k++) {
-      const ulonglong2 w = __ldcg(reinterpret_cast<const ulonglong2 *>(partial + b * N + k));
-      v[k] = fp_add(v[k], fp{w.x, w.y}, c);
-    }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int k = 0; k < N; k++) {
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-      fp o;
-      o.lo = __shfl_xor_sync(0xffffffffu, v[k].lo, off);
-      o.hi = __shfl_xor_sync(0xffffffffu, v[k].hi, off);
-      v[k] = fp_add(v[k], o, c);
-    }
-    if (lane == 0) red[k][warp] = v[k];
-  }
-  __syncthreads();
-  if (threadIdx.x == 0)
-    for (int k = 0; k < N; k++) {
-      fp x = red[k][0];
-      for (int w = 1; w < (int)(blockDim.x >> 5); w++) x = fp_add(x, red[k][w], c);
-      mailbox_post(mb, seq, 2 * k, x.lo);
-      mailbox_post(mb, seq, 2 * k + 1, x.hi);
-    }
-  return true;
-}
-
-// fp_last_block_post through the lane's shared counter (reset by the last
-// block), then the last block fetches the next challenge for the round link.
-template <int N>
-__device__ void fp_round_end(const fp *partial, const FpCtx &c, const Publish &p,
-                             const RoundLink &lk) {
-  if (!fp_last_block_post<N>(partial, c, p.counter, p.mailbox, p.seq)) return;
-  if (threadIdx.x == 0) {
-    *p.counter = 0;
-    link_fetch(lk);
-  }
-}
-
-// One outer round. fold = 0: sums over the pairs of the tables as they are.
-// fold = 1: fold every table at r (output at half length) and sum over the
-// folded pairs. emit = 0 only folds (the last fold).
-__global__ void k_outer_round(const fp *E, const fp *A, const fp *B, const fp *C, fp *E2, fp *A2,
-                              fp *B2, fp *C2, size_t n, int fold, int emit, fp r, FpCtx c,
-                              fp *partial, Publish pub, RoundLink lk) {
-  if (lk.in) {
-    unsigned long long w0, w1;
-    if (!link_begin(lk, w0, w1)) return;
-    r = fp{w0, w1};
-  }
-  fp acc[3] = {fp_zero(), fp_zero(), fp_zero()};
-  size_t npairs = fold ? (n / 2 + 1) / 2 : n / 2;
-  for (size_t j = blockIdx.x * (size_t)blockDim.x + threadIdx.x; j < npairs;
-       j += (size_t)gridDim.x * blockDim.x) {
-    fp e[2], a[2], b[2], cc[2];
-    if (fold) {
-      for (int t = 0; t < 2; t++) {
-        size_t o = 2 * j + t;
-        if (o >= n / 2) {
-          e[t] = a[t] = b[t] = cc[t] = fp_zero();
-          continue;
-        }
-        e[t] = interp(E[2 * o], E[2 * o + 1], r, c);
-        a[t] = interp(A[2 * o], A[2 * o + 1], r, c);
-        b[t] = interp(B[2 * o], B[2 * o + 1], r, c);
-        cc[t] = interp(C[2 * o], C[2 * o + 1], r, c);
-        E2[o] = e[t];
-        A2[o] = a[t];
-        B2[o] = b[t];
-        C2[o] = cc[t];
-      }
-    } else {
-      for (int t = 0; t < 2; t++) {
-        e[t] = E[2 * j + t];
-        a[t] = A[2 * j + t];
-        b[t] = B[2 * j + t];
-        cc[t] = C[2 * j + t];
-      }
-    }
-    if (emit) cubic(e[0], e[1], a[0], a[1], b[0], b[1], cc[0], cc[1], c, acc);
-  }
-  if (emit) {
-    block_fp_sum<3>(acc, c, partial);
-    if (pub.counter) fp_round_end<3>(partial, c, pub, lk);
-  }
-}
-
-// One inner round over D and the assignment W. W is read from the packed h
-// bits while w_bits is set (round 0, and the input of round 1's fold).
-__global__ void k_inner_round(const fp *D, const fp *W, const uint32_t *hbits, int w_bits, fp *D2,
-                              fp *W2, size_t n, int fold, int emit, fp r, FpCtx c, fp *partial,
-                              Publish pub, RoundLink lk) {
-  if (lk.in) {
-    unsigned long long w0, w1;
-    if (!link_begin(lk, w0, w1)) return;
-    r = fp{w0, w1};
-  }
-  fp acc[2] = {fp_zero(), fp_zero()};
-  size_t npairs = fold ? (n / 2 + 1) / 2 : n / 2;
-  for (size_t j = blockIdx.x * (size_t)blockDim.x + threadIdx.x; j < npairs;
-       j += (size_t)gridDim.x * blockDim.x) {
-    fp d[2], w[2];
-    for (int t = 0; t < 2; t++) {
-      size_t o = 2 * j + t;
-      if (fold) {
-        if (o >= n / 2) {
-          d[t] = w[t] = fp_zero();
-          continue;
-        }
-        fp w0, w1;
-        if (w_bits) {
-          size_t i0 = 2 * o;
-          w0 = ((hbits[i0 >> 5] >> (i0 & 31)) & 1) ? c.one : fp_zero();
-          w1 = ((hbits[(i0 + 1) >> 5] >> ((i0 + 1) & 31)) & 1) ? c.one : fp_zero();
-        } else {
-          w0 = W[2 * o];
-          w1 = W[2 * o + 1];
-        }
-        d[t] = interp(D[2 * o], D[2 * o + 1], r, c);
-        w[t] = interp(w0, w1, r, c);
-        D2[o] = d[t];
-        W2[o] = w[t];
-      } else {
-        d[t] = D[o];
-        w[t] = ((hbits[o >> 5] >> (o & 31)) & 1) ? c.one : fp_zero();
-      }
-    }
-    if (emit) {
-      acc[0] = fp_add(acc[0], fp_mul(d[0], w[0], c), c);
-      acc[1] = fp_add(acc[1], fp_mul(fp_sub(d[1], d[0], c), fp_sub(w[1], w[0], c), c), c);
-    }
-  }
-  if (emit) {
-    block_fp_sum<2>(acc, c, partial);
-    if (pub.counter) fp_round_end<2>(partial, c, pub, lk);
-  }
-}
-
-// One block adds the per-block partials; the totals go to out and, when
-// publishing, to the mailbox (written by the thread that wrote out).
-template <int N>
-__global__ void k_fp_finalize(const fp *partial, int nblocks, FpCtx c, fp *out, Publish pub) {
-  fp acc[N];
-  for (int k = 0; k < N; k++) acc[k] = fp_zero();
-  for (int b = threadIdx.x; b < nblocks; b += blockDim.x)
-    for (int k = 0; k < N; k++) acc[k] = fp_add(acc[k], partial[b * N + k], c);
-  block_fp_sum<N>(acc, c, out);
-  static_assert(2 * N <= kMailboxWords, "mailbox too small");
-  if (pub.counter && threadIdx.x == 0) {
-    for (int k = 0; k < N; k++) {
-      mailbox_post(pub.mailbox, pub.seq, 2 * k, out[k].lo);
-      mailbox_post(pub.mailbox, pub.seq, 2 * k + 1, out[k].hi);
-    }
-  }
+// One block adds the per-block partials into out.
+__global__ void k_fp_finalize(const fp *partial, int nblocks, FpCtx c, fp *out) {
+  fp acc[1] = {fp_zero()};
+  for (int b = threadIdx.x; b < nblocks; b += blockDim.x) acc[0] = fp_add(acc[0], partial[b], c);
+  block_fp_sum<1>(acc, c, out);
 }
 
 // The coefficient table of the bind: scale_k * coefficient for every distinct
@@ -337,192 +171,395 @@ __global__ void k_bind_col0_finish(const fp *partial, int nblocks, FpCtx c, fp *
 }
 
 
-// The last rounds of each sumcheck in one resident block, fed through the
-// lane's downbox (bounded waits; a missing challenge ends the kernel without
-// a post). The tables (at most kSpTailN entries each) sit in shared memory.
-// Each round folds at the previous round's challenge (when `fold`), sums the
-// round's coefficients and posts them; after the last round the final fold's
-// single entries are posted.
-constexpr int kSpTailN = 512;
-constexpr unsigned long long kSpWaitNs = 2000000000ull;
+// ------------------------------------------------------------------ passes
 
-// Folds T tables of len entries in place at r (all reads, then all writes).
-template <int T>
-__device__ __forceinline__ int sp_fold(fp (*tab)[kSpTailN], int len, fp r, const FpCtx &c) {
-  const int nout = len / 2;
-  fp f[T][2];
-  int cnt = 0;
-  for (int o = threadIdx.x; o < nout; o += blockDim.x, cnt++)
-    for (int t = 0; t < T; t++) f[t][cnt] = interp(tab[t][2 * o], tab[t][2 * o + 1], r, c);
-  __syncthreads();
-  cnt = 0;
-  for (int o = threadIdx.x; o < nout; o += blockDim.x, cnt++)
-    for (int t = 0; t < T; t++) tab[t][o] = f[t][cnt];
-  __syncthreads();
-  return nout;
+// 256-bit sums of products of residues, reduced once. With q < 2^126, eight
+// products fit.
+struct FpWide {
+  uint64_t w[4];
+};
+
+__device__ __forceinline__ void fp_mac(FpWide &t, fp a, fp b) {
+  typedef unsigned __int128 u128;
+  u128 s = (u128)a.lo * b.lo + t.w[0];
+  t.w[0] = (uint64_t)s;
+  s = (u128)a.lo * b.hi + t.w[1] + (uint64_t)(s >> 64);
+  t.w[1] = (uint64_t)s;
+  const uint64_t top = (uint64_t)(s >> 64);
+  s = (u128)a.hi * b.lo + t.w[1];
+  t.w[1] = (uint64_t)s;
+  s = (u128)a.hi * b.hi + t.w[2] + (uint64_t)(s >> 64);
+  u128 r = (u128)(uint64_t)s + top;
+  t.w[2] = (uint64_t)r;
+  t.w[3] += (uint64_t)(s >> 64) + (uint64_t)(r >> 64);
 }
 
-__device__ __forceinline__ bool sp_challenge(const Mailbox *down, unsigned long long dseq,
-                                             const FpCtx &c, fp &r) {
-  __shared__ unsigned long long chal[2];
-  __shared__ int ok;
-  if (threadIdx.x == 0) ok = mailbox_wait_device(down, dseq, 2, chal, kSpWaitNs);
-  __syncthreads();
-  r = fp{chal[0], chal[1]};
-  bool good = ok;
-  __syncthreads();
-  return good;
+// t 2^-128 mod q for t < 8 q^2: two reduction steps leave less than 3q.
+__device__ __forceinline__ fp fp_reduce(const FpWide &t, const FpCtx &c) {
+  typedef unsigned __int128 u128;
+  uint64_t m = t.w[0] * c.qinv;
+  u128 s = (u128)m * c.q0 + t.w[0];
+  s = (u128)m * c.q1 + t.w[1] + (uint64_t)(s >> 64);
+  const uint64_t w1 = (uint64_t)s;
+  s = (u128)t.w[2] + (uint64_t)(s >> 64);
+  const uint64_t w2 = (uint64_t)s;
+  const uint64_t w3 = t.w[3] + (uint64_t)(s >> 64);
+  m = w1 * c.qinv;
+  s = (u128)m * c.q0 + w1;
+  s = (u128)m * c.q1 + w2 + (uint64_t)(s >> 64);
+  fp r{(uint64_t)s, w3 + (uint64_t)(s >> 64)};
+  if (fp_ge(r, c.q0, c.q1)) r = fp_sub_raw(r, c.q0, c.q1);
+  if (fp_ge(r, c.q0, c.q1)) r = fp_sub_raw(r, c.q0, c.q1);
+  return r;
 }
 
-// The T tables (len entries each, one after another) as handover
-// publication seq: the host runs the sumcheck's remaining rounds.
-template <int T>
-__device__ __forceinline__ void sp_handover(fp (*tab)[kSpTailN], int len,
-                                            unsigned long long *handover,
-                                            unsigned long long seq) {
-  for (int k = threadIdx.x; k < T * len; k += blockDim.x) {
-    const fp v = tab[k / len][k % len];
-    handover_post(handover, seq, 2 * k, v.lo);
-    handover_post(handover, seq, 2 * k + 1, v.hi);
-  }
+static __device__ __noinline__ fp pass_fp_mul(fp a, fp b, const FpCtx &c) {
+  return fp_mul(a, b, c);
 }
 
-template <int N>
-__device__ __forceinline__ void sp_post(fp (&acc)[N], const FpCtx &c, Mailbox *mb,
-                                        unsigned long long seq) {
-  __shared__ fp red[N];
-  block_fp_sum<N>(acc, c, red);
-  if (threadIdx.x == 0)
-    for (int k = 0; k < N; k++) {
-      mailbox_post(mb, seq, 2 * k, red[k].lo);
-      mailbox_post(mb, seq, 2 * k + 1, red[k].hi);
-    }
-  __syncthreads();
+// The eq weights (Montgomery) of the 2^k entries that a bind joins.
+struct FpBind {
+  fp e[8];
+  int k;
+};
+
+// eq over the coordinates above a pass as a product of factor tables: factor 0
+// over the lowest `low` of them, each further one over seven.
+struct FpFactors {
+  fp f[4][1 << kFacLog];
+  int low, n;
+};
+
+// Entry o of a table after the binds, from the 2^k entries it joins; entries at
+// or beyond `live` are zero.
+__device__ __forceinline__ fp fp_bound(const fp *in, size_t o, size_t live, const FpBind &b,
+                                       const FpCtx &c) {
+  const fp *p = in + (o << b.k);
+  const size_t left = live > (o << b.k) ? live - (o << b.k) : 0;
+  auto at = [&](int j) {
+    if ((size_t)j >= left) return fp_zero();
+    const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(p + j);
+    return fp{v.x, v.y};
+  };
+  if (b.k == 0) return at(0);
+  FpWide t{{0, 0, 0, 0}};
+#pragma unroll 2
+  for (int j = 0; j < 1 << b.k; j++) fp_mac(t, b.e[j], at(j));
+  return fp_reduce(t, c);
 }
 
-// Outer rounds round0 .. rounds-1 over E, A, B, C (len0 entries each).
-__global__ void __launch_bounds__(kThreads) sp_outer_tail(const fp *E, const fp *A, const fp *B,
-                                                          const fp *C, int len0, int fold0,
-                                                          int nrounds, FpCtx c, Mailbox *mb,
-                                                          unsigned long long seq0,
-                                                          const Mailbox *down,
-                                                          unsigned long long dseq0,
-                                                          int hand_round,
-                                                          unsigned long long *handover,
-                                                          unsigned long long hseq) {
-  __shared__ fp tab[4][kSpTailN];
-  for (int k = threadIdx.x; k < len0; k += blockDim.x) {
-    tab[0][k] = E[k];
-    tab[1][k] = A[k];
-    tab[2][k] = B[k];
-    tab[3][k] = C[k];
+// A table's value at a point: the difference of the halves at infinity.
+__device__ __forceinline__ fp fp_point(const fp *t, int stride, int one, int inf, const FpCtx &c) {
+  fp v = t[(one | inf) * stride];
+  for (int sub = inf; sub;) {
+    sub = (sub - 1) & inf;
+    const fp x = t[(one | sub) * stride];
+    v = __popc(inf ^ sub) & 1 ? fp_sub(v, x, c) : fp_add(v, x, c);
+    if (!sub) break;
   }
-  __syncthreads();
-  int len = len0, nd = 0, np = 0;
-  for (int round = 0; round < nrounds; round++) {
-    if (round == hand_round) {  // the remaining rounds run on the host
-      sp_handover<4>(tab, len, handover, hseq);
-      return;
-    }
-    if (round > 0 || fold0) {
-      fp r;
-      if (!sp_challenge(down, dseq0 + nd++, c, r)) return;
-      len = sp_fold<4>(tab, len, r, c);
-    }
-    fp acc[3] = {fp_zero(), fp_zero(), fp_zero()};
-    for (int j = threadIdx.x; j < len / 2; j += blockDim.x)
-      cubic(tab[0][2 * j], tab[0][2 * j + 1], tab[1][2 * j], tab[1][2 * j + 1], tab[2][2 * j],
-            tab[2][2 * j + 1], tab[3][2 * j], tab[3][2 * j + 1], c, acc);
-    sp_post<3>(acc, c, mb, seq0 + np++);
-  }
-  fp r;
-  if (!sp_challenge(down, dseq0 + nd, c, r)) return;
-  sp_fold<4>(tab, len, r, c);
-  if (threadIdx.x == 0)
-    for (int k = 0; k < 3; k++) {
-      mailbox_post(mb, seq0 + np, 2 * k, tab[k + 1][0].lo);
-      mailbox_post(mb, seq0 + np, 2 * k + 1, tab[k + 1][0].hi);
-    }
+  return v;
 }
 
-// Inner rounds over D and W (W from the packed h bits when w_bits).
-__global__ void __launch_bounds__(kThreads) sp_inner_tail(const fp *D, const fp *W,
-                                                          const uint32_t *hbits, int w_bits,
-                                                          int len0, int fold0, int nrounds,
-                                                          FpCtx c, Mailbox *mb,
-                                                          unsigned long long seq0,
-                                                          const Mailbox *down,
-                                                          unsigned long long dseq0,
-                                                          int hand_round,
-                                                          unsigned long long *handover,
-                                                          unsigned long long hseq) {
-  __shared__ fp tab[2][kSpTailN];
-  for (int k = threadIdx.x; k < len0; k += blockDim.x) {
-    tab[0][k] = D[k];
-    tab[1][k] = w_bits ? (((hbits[k >> 5] >> (k & 31)) & 1) ? c.one : fp_zero()) : W[k];
+// A pass's sums over the X lanes of each point, posted by each block (few
+// blocks) or left in partial[block][point] for the last block, which adds them
+// up (lanes over the blocks) and posts them.
+template <int kPoints, int kTurns>
+__device__ __forceinline__ void fp_pass_end(fp (&sum)[kTurns], int lx, const FpCtx &c, fp *partial,
+                                            const PassPost &post) {
+  __shared__ bool last;
+  const int X = 1 << lx, t = threadIdx.x;
+  const bool direct = pass_direct(gridDim.x, 2 * kPoints);
+  auto exchange = [](fp v, int off) {
+    return fp{__shfl_xor_sync(0xffffffffu, v.lo, off), __shfl_xor_sync(0xffffffffu, v.hi, off)};
+  };
+  auto put = [&](int at, fp v) {
+    handover_post(post.handover, post.seq, 2 * at, v.lo);
+    handover_post(post.handover, post.seq, 2 * at + 1, v.hi);
+  };
+#pragma unroll
+  for (int q = 0; q < kTurns; q++) {
+    const int u = t + q * kPassThreads, p = u >> lx;
+    if ((u & ~31) >= kPoints << lx) break;  // the whole warp
+    fp v = sum[q];
+    for (int off = X >> 1; off > 0; off >>= 1) v = fp_add(v, exchange(v, off), c);
+    if (p < kPoints && (u & (X - 1)) == 0) {
+      if (direct)
+        put(blockIdx.x * kPoints + p, v);
+      else
+        partial[(size_t)blockIdx.x * kPoints + p] = v;
+    }
+  }
+  if (direct) return;
+  __threadfence();
+  __syncthreads();
+  if (t == 0) {
+    last = atomicAdd(post.counter, 1u) == gridDim.x - 1;
+    __threadfence();
   }
   __syncthreads();
-  int len = len0, nd = 0, np = 0;
-  for (int round = 0; round < nrounds; round++) {
-    if (round == hand_round) {  // the remaining rounds run on the host
-      sp_handover<2>(tab, len, handover, hseq);
-      return;
+  if (!last) return;
+  for (int p = t >> 5; p < kPoints; p += kPassThreads / 32) {
+    fp v = fp_zero();
+    for (unsigned b = t & 31; b < gridDim.x; b += 32) {
+      const ulonglong2 w = __ldcg(reinterpret_cast<const ulonglong2 *>(partial + (size_t)b * kPoints + p));
+      v = fp_add(v, fp{w.x, w.y}, c);
     }
-    if (round > 0 || fold0) {
-      fp r;
-      if (!sp_challenge(down, dseq0 + nd++, c, r)) return;
-      len = sp_fold<2>(tab, len, r, c);
-    }
-    fp acc[2] = {fp_zero(), fp_zero()};
-    for (int j = threadIdx.x; j < len / 2; j += blockDim.x) {
-      fp d0 = tab[0][2 * j], d1 = tab[0][2 * j + 1], w0 = tab[1][2 * j], w1 = tab[1][2 * j + 1];
-      acc[0] = fp_add(acc[0], fp_mul(d0, w0, c), c);
-      acc[1] = fp_add(acc[1], fp_mul(fp_sub(d1, d0, c), fp_sub(w1, w0, c), c), c);
-    }
-    sp_post<2>(acc, c, mb, seq0 + np++);
+    for (int off = 16; off > 0; off >>= 1) v = fp_add(v, exchange(v, off), c);
+    if ((t & 31) == 0) put(p, v);
   }
-  fp r;
-  if (!sp_challenge(down, dseq0 + nd, c, r)) return;
-  sp_fold<2>(tab, len, r, c);
-  if (threadIdx.x == 0) {
-    mailbox_post(mb, seq0 + np, 0, tab[0][0].lo);
-    mailbox_post(mb, seq0 + np, 1, tab[0][0].hi);
-    mailbox_post(mb, seq0 + np, 2, tab[1][0].lo);
-    mailbox_post(mb, seq0 + np, 3, tab[1][0].hi);
+  if (t == 0) *post.counter = 0;
+}
+
+// One pass of the outer sumcheck over A, B, C: binds (to `out` when b.k > 0),
+// then the 3^K sums of eq (A B - C) over the positions above the low K
+// coordinates (C is linear, so it only counts at the points without infinity).
+// `live` entries of each input table are not known to be zero. Tiles and
+// threads as in the GKR's passes (gkr.cu): bound entries, weighted A and C,
+// then the points.
+struct SpTabs {
+  fp *t[3];
+};
+
+template <int K>
+__global__ void __launch_bounds__(kPassThreads, 2) sp_outer_pass(
+    SpTabs in, SpTabs out, size_t live, uint32_t count, const __grid_constant__ FpBind b,
+    const __grid_constant__ FpFactors eq, FpCtx c, int lx, fp *partial, PassPost post) {
+  constexpr int kPoints = pow3(K), kBlocks = 1 << K;
+  constexpr int kTurns = (kPoints * kPassMaxX + kPassThreads - 1) / kPassThreads;
+  constexpr int kRow = kPassMaxX + 1;
+  __shared__ fp S[3][kBlocks * kRow], E[kPassMaxX];
+  const int t = threadIdx.x, X = 1 << lx;
+  fp sum[kTurns];
+#pragma unroll
+  for (int q = 0; q < kTurns; q++) sum[q] = fp_zero();
+  for (uint32_t i0 = blockIdx.x << lx; i0 < count; i0 += gridDim.x << lx) {
+    if (t >= kPassThreads - 32 && (t & 31) < X) {  // the last warp: the weights
+      const uint32_t x = i0 + (t & 31);
+      fp e = fp_zero();
+      if (x < count) {
+        e = eq.f[0][x & ((1u << eq.low) - 1)];
+#pragma unroll 1
+        for (int g = 1; g < eq.n; g++)
+          e = pass_fp_mul(e, eq.f[g][(x >> (eq.low + kFacLog * (g - 1))) & ((1 << kFacLog) - 1)], c);
+      }
+      E[t & 31] = e;
+    }
+    const int size = kBlocks << lx;
+    for (int u = t; u < 3 * size; u += kPassThreads) {
+      const int tab = u / size, slot = u - tab * size, x = slot >> K, a = slot & (kBlocks - 1);
+      fp v = fp_zero();
+      if (i0 + x < count) {
+        const size_t o = ((size_t)i0 << K) + slot;
+        v = fp_bound(in.t[tab], o, live, b, c);
+        if (b.k) out.t[tab][o] = v;
+      }
+      S[tab][a * kRow + x] = v;
+    }
+    __syncthreads();
+    for (int u = t; u < 2 * size; u += kPassThreads) {
+      const int tab = u >= size ? 2 : 0, slot = u & (size - 1), x = slot & (X - 1);
+      fp *p = &S[tab][(slot >> lx) * kRow + x];
+      *p = pass_fp_mul(E[x], *p, c);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kTurns; q++) {
+      const int u = t + q * kPassThreads;
+      if (u < kPoints << lx) {
+        int one, inf;
+        point_bits<K, true>(u >> lx, one, inf);
+        const int x = u & (X - 1);
+        fp v = pass_fp_mul(fp_point(S[0] + x, kRow, one, inf, c),
+                           fp_point(S[1] + x, kRow, one, inf, c), c);
+        if (!inf) v = fp_sub(v, S[2][one * kRow + x], c);
+        sum[q] = fp_add(sum[q], v, c);
+      }
+    }
+    __syncthreads();  // the tile's tables before the next tile's
   }
+  fp_pass_end<kPoints, kTurns>(sum, lx, c, partial, post);
+}
+
+// One pass of the inner sumcheck over D and W; with kBits, W comes from h's
+// bytes (b.k = 3).
+template <int K, bool kBits>
+__global__ void __launch_bounds__(kPassThreads, 2) sp_inner_pass(
+    const fp *D, const fp *W, fp *D2, fp *W2, size_t live, uint32_t count,
+    const __grid_constant__ FpBind b, FpCtx c, int lx, fp *partial, PassPost post) {
+  constexpr int kPoints = pow3(K), kBlocks = 1 << K;
+  constexpr int kTurns = (kPoints * kPassMaxX + kPassThreads - 1) / kPassThreads;
+  constexpr int kRow = kPassMaxX + 1;
+  __shared__ fp S[2][kBlocks * kRow], W8[kBits ? 256 : 1];
+  const int t = threadIdx.x, X = 1 << lx;
+  if (kBits) {
+    if (t < 256) {
+      fp v = fp_zero();
+#pragma unroll 1
+      for (int j = 0; j < 8; j++)
+        if ((t >> j) & 1) v = fp_add(v, b.e[j], c);
+      W8[t] = v;
+    }
+    __syncthreads();
+  }
+  fp sum[kTurns];
+#pragma unroll
+  for (int q = 0; q < kTurns; q++) sum[q] = fp_zero();
+  for (uint32_t i0 = blockIdx.x << lx; i0 < count; i0 += gridDim.x << lx) {
+    const int size = kBlocks << lx;
+    for (int u = t; u < 2 * size; u += kPassThreads) {
+      const int tab = u >= size, slot = u & (size - 1), x = slot >> K, a = slot & (kBlocks - 1);
+      fp v = fp_zero();
+      if (i0 + x < count) {
+        const size_t o = ((size_t)i0 << K) + slot;
+        if (kBits && tab)
+          v = W8[reinterpret_cast<const uint8_t *>(W)[o]];
+        else
+          v = fp_bound(tab ? W : D, o, live, b, c);
+        if (b.k) (tab ? W2 : D2)[o] = v;
+      }
+      S[tab][a * kRow + x] = v;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kTurns; q++) {
+      const int u = t + q * kPassThreads;
+      if (u < kPoints << lx) {
+        int one, inf;
+        point_bits<K, true>(u >> lx, one, inf);
+        const int x = u & (X - 1);
+        sum[q] = fp_add(sum[q], pass_fp_mul(fp_point(S[0] + x, kRow, one, inf, c),
+                                            fp_point(S[1] + x, kRow, one, inf, c), c), c);
+      }
+    }
+    __syncthreads();  // the tile's tables before the next tile's
+  }
+  fp_pass_end<kPoints, kTurns>(sum, lx, c, partial, post);
+}
+
+// A residue sum of up to 2^32 terms.
+struct FpSum160 {
+  uint64_t lo, hi;
+  uint32_t top;
+  __device__ __forceinline__ void add(fp v) {
+    asm("add.cc.u64 %0, %0, %3;\n\taddc.cc.u64 %1, %1, %4;\n\taddc.u32 %2, %2, 0;"
+        : "+l"(lo), "+l"(hi), "+r"(top)
+        : "l"(v.lo), "l"(v.hi));
+  }
+  // mod q: the low 128 bits times one and the rest times 2^128
+  __device__ __forceinline__ fp reduce(const FpCtx &c) const {
+    return fp_add(fp_mul(fp{lo, hi}, c.one, c), fp_mul(fp{top, 0}, c.r2, c), c);
+  }
+};
+
+// The inner sumcheck's first three rounds: H[a][b], the sum over the groups of
+// eight columns of D's entry a where h's bit b is set. One lane per column, so
+// D is read once, coalesced; 32 columns without a set bit are skipped. The sums
+// stay unreduced (160 bits) until the end. 2^25 columns: 0.5 GB.
+constexpr int kSpBitsBlocks = 4 * kSMs;
+__global__ void __launch_bounds__(kThreads) sp_bits(const fp *__restrict__ D,
+                                                    const uint32_t *__restrict__ bits, size_t words,
+                                                    FpCtx c, fp *partial, PassPost post) {
+  __shared__ fp sums[kThreads / 32][64];
+  __shared__ bool last;
+  const int t = threadIdx.x, lane = t & 31;
+  const size_t warps = (size_t)gridDim.x * (kThreads / 32);
+  FpSum160 h[8];
+#pragma unroll
+  for (int b = 0; b < 8; b++) h[b] = FpSum160{0, 0, 0};
+#pragma unroll 2
+  for (size_t k = blockIdx.x * (size_t)(kThreads / 32) + (t >> 5); k < words; k += warps) {
+    const uint32_t word = __ldg(bits + k);
+    if (!word) continue;
+    const ulonglong2 w = *reinterpret_cast<const ulonglong2 *>(D + 32 * k + lane);
+    const uint32_t byte = word >> (lane & 24);
+#pragma unroll
+    for (int b = 0; b < 8; b++)
+      if ((byte >> b) & 1) h[b].add(fp{w.x, w.y});
+  }
+#pragma unroll
+  for (int b = 0; b < 8; b++) {
+    fp v = h[b].reduce(c);
+    for (int off = 8; off < 32; off <<= 1)
+      v = fp_add(v, fp{__shfl_xor_sync(0xffffffffu, v.lo, off), __shfl_xor_sync(0xffffffffu, v.hi, off)}, c);
+    if (lane < 8) sums[t >> 5][8 * lane + b] = v;
+  }
+  __syncthreads();
+  if (t < 64) {
+    fp v = sums[0][t];
+    for (int w = 1; w < kThreads / 32; w++) v = fp_add(v, sums[w][t], c);
+    partial[(size_t)blockIdx.x * 64 + t] = v;
+  }
+  __threadfence();
+  __syncthreads();
+  if (t == 0) {
+    last = atomicAdd(post.counter, 1u) == gridDim.x - 1;
+    __threadfence();
+  }
+  __syncthreads();
+  if (!last) return;
+  {  // four threads per sum over the blocks
+    fp v = fp_zero();
+    for (unsigned b = t & 3; b < gridDim.x; b += 4) {
+      const ulonglong2 w = __ldcg(reinterpret_cast<const ulonglong2 *>(partial + (size_t)b * 64 + (t >> 2)));
+      v = fp_add(v, fp{w.x, w.y}, c);
+    }
+    for (int off = 1; off < 4; off <<= 1)
+      v = fp_add(v, fp{__shfl_xor_sync(0xffffffffu, v.lo, off), __shfl_xor_sync(0xffffffffu, v.hi, off)}, c);
+    if ((t & 3) == 0) {
+      handover_post(post.handover, post.seq, 2 * (t >> 2), v.lo);
+      handover_post(post.handover, post.seq, 2 * (t >> 2) + 1, v.hi);
+    }
+  }
+  if (t == 0) *post.counter = 0;
+}
+
+// The last tables to the host, `tables` of n entries each after the binds; W
+// from h's bytes with kBits (then b.k = 3) or from its bits (w_bits).
+template <bool kBits>
+__global__ void __launch_bounds__(64) sp_handover(SpTabs in, int tables, int n, size_t live,
+                                                  const uint32_t *w_bits,
+                                                  const __grid_constant__ FpBind b, FpCtx c,
+                                                  unsigned long long *handover,
+                                                  unsigned long long seq) {
+  const int k = blockIdx.x * 64 + threadIdx.x, tab = k / n, o = k % n;
+  if (tab >= tables) return;
+  fp v = fp_zero();
+  if (kBits && tab == 1) {
+    const int byte = reinterpret_cast<const uint8_t *>(w_bits)[o];
+#pragma unroll 1
+    for (int j = 0; j < 8; j++)
+      if ((byte >> j) & 1) v = fp_add(v, b.e[j], c);
+  } else {
+    v = fp_bound(in.t[tab], o, live, b, c);
+  }
+  handover_post(handover, seq, 2 * k, v.lo);
+  handover_post(handover, seq, 2 * k + 1, v.hi);
 }
 
 // ------------------------------------------------------------------- host
 
-// The tail hands its tables to the host at the first round whose input is at
-// most this long; each round after that costs the host a few microseconds,
-// against a PCIe round trip and a device step.
-constexpr size_t kSpHostLen = 64;
+// Tables of this many entries or fewer go to the host.
+constexpr int kSpHostLog = 7;
+static_assert(6 << kSpHostLog <= kHandoverWords, "the last tables fit one handover");
 
-// The first round (at or after the tail's first, t0) whose input of
-// n0 >> (k - 1) entries (n0 at k = 0) is at most kSpHostLen; -1 without a
-// handover area or a round that small.
-static int sp_host_round(const RoundChannel *ch, size_t n0, int t0, int nrounds) {
-  if (!ch->handover_host) return -1;
-  for (int k = t0; k < nrounds; k++)
-    if ((k == 0 ? n0 : n0 >> (k - 1)) <= kSpHostLen) return k;
-  return -1;
+static std::vector<fp> sp_words(const std::vector<uint64_t> &w, size_t n) {
+  std::vector<fp> v(n);
+  for (size_t k = 0; k < n; k++) v[k] = fp{w[2 * k], w[2 * k + 1]};
+  return v;
 }
 
-// The handover's T tables of len entries each.
-static void sp_take_handover(RoundChannel *ch, cudaStream_t s, unsigned long long seq, int T,
-                             size_t len, std::vector<fp> *tab) {
-  std::vector<uint64_t> w(2 * T * len);
-  ch->wait_handover(s, seq, w.data(), (int)w.size());
-  for (int t = 0; t < T; t++) {
-    tab[t].resize(len);
-    for (size_t k = 0; k < len; k++)
-      tab[t][k] = fp{w[2 * (t * len + k)], w[2 * (t * len + k) + 1]};
-  }
+// Adds the blocks' points up into the first `points`.
+static std::vector<fp> sp_combine(const std::vector<uint64_t> &w, int points, int blocks,
+                                  const FpCtx &c) {
+  std::vector<fp> v = sp_words(w, (size_t)points * blocks);
+  for (int b = 1; b < blocks; b++)
+    for (int p = 0; p < points; p++) v[p] = fp_add(v[p], v[b * points + p], c);
+  v.resize(points);
+  return v;
 }
 
-// sp_fold on the host: each table folded at r in place (entry o from 2o and
-// 2o + 1, read before it is overwritten).
+// Each table folded at r in place (entry o from 2o and 2o + 1, read before it
+// is overwritten).
 static void host_sp_fold(std::vector<fp> *tab, int T, fp r, const FpCtx &c) {
   for (int t = 0; t < T; t++) {
     const size_t n = tab[t].size() / 2;
@@ -531,45 +568,53 @@ static void host_sp_fold(std::vector<fp> *tab, int T, fp r, const FpCtx &c) {
   }
 }
 
-// The outer and inner rounds' sums, as the tail kernels form them.
-static void host_outer_sums(const std::vector<fp> *tab, const FpCtx &c, fp *out) {
-  fp acc[3] = {fp_zero(), fp_zero(), fp_zero()};
-  for (size_t j = 0; j < tab[0].size() / 2; j++)
-    cubic(tab[0][2 * j], tab[0][2 * j + 1], tab[1][2 * j], tab[1][2 * j + 1], tab[2][2 * j],
-          tab[2][2 * j + 1], tab[3][2 * j], tab[3][2 * j + 1], c, acc);
-  for (int k = 0; k < 3; k++) out[k] = acc[k];
+// A sumcheck's point sums at the first coordinate's three values, summed over
+// the others at zeros and ones with weights e.
+static void sp_round_sums(const std::vector<fp> &F, int rest, const std::vector<fp> &e,
+                          const FpCtx &c, fp (&s)[3]) {
+  const size_t block = F.size() / 3;
+  for (int d = 0; d < 3; d++) {
+    s[d] = fp_zero();
+    for (int x = 0; x < 1 << rest; x++) {
+      size_t at = 0;  // the next coordinate is the next digit from the top
+      for (int q = 0; q < rest; q++) at = 3 * at + ((x >> q) & 1);
+      const fp v = F[d * block + at];
+      s[d] = fp_add(s[d], e.empty() ? v : fp_mul(e[x], v, c), c);
+    }
+  }
 }
 
-static void host_inner_sums(const std::vector<fp> *tab, const FpCtx &c, fp *out) {
-  fp acc[2] = {fp_zero(), fp_zero()};
-  for (size_t j = 0; j < tab[0].size() / 2; j++) {
-    const fp d0 = tab[0][2 * j], d1 = tab[0][2 * j + 1], w0 = tab[1][2 * j], w1 = tab[1][2 * j + 1];
-    acc[0] = fp_add(acc[0], fp_mul(d0, w0, c), c);
-    acc[1] = fp_add(acc[1], fp_mul(fp_sub(d1, d0, c), fp_sub(w1, w0, c), c), c);
+static void sp_fold_points(std::vector<fp> &F, fp r, const FpCtx &c) {
+  const size_t block = F.size() / 3;
+  for (size_t x = 0; x < block; x++) {  // h0 + r (h1 - h0 - hinf) + r^2 hinf
+    const fp h0 = F[x], h1 = F[block + x], hi = F[2 * block + x];
+    const fp mid = fp_sub(fp_sub(h1, h0, c), hi, c);
+    F[x] = fp_add(h0, fp_mul(r, fp_add(mid, fp_mul(r, hi, c), c), c), c);
   }
-  out[0] = acc[0];
-  out[1] = acc[1];
+  F.resize(block);
 }
 
-static fp host_partial_sum(const fp *d_partial, int nblocks, int N, fp *d_out, fp *h_out,
-                           const FpCtx &c, cudaStream_t s, RoundChannel *ch) {
-  Publish pub = ch ? ch->arm() : Publish{nullptr, nullptr, 0};
-  KernelProbe &probe = KernelProbe::get();
-  const bool probed = probe.on("k_fp_finalize");
-  if (probed) probe.before(s);
-  if (N == 3)
-    k_fp_finalize<3><<<1, kThreads, 0, s>>>(d_partial, nblocks, c, d_out, pub);
-  else
-    k_fp_finalize<2><<<1, kThreads, 0, s>>>(d_partial, nblocks, c, d_out, pub);
-  BZ_LAUNCH_CHECK();
-  if (probed) probe.after(s, "k_fp_finalize", 16.0 * N * (nblocks + 1));
-  if (ch) {
-    ch->wait(s, reinterpret_cast<uint64_t *>(h_out), 2 * N);
-  } else {
-    BZ_CUDA(cudaMemcpyAsync(h_out, d_out, N * sizeof(fp), cudaMemcpyDeviceToHost, s));
-    BZ_CUDA(stream_wait(s));
+// eq over a run of coordinates, coordinate 0 in the lowest bit.
+static std::vector<fp> sp_eq(const fp *z, int n, const FpCtx &c, fp scale) {
+  std::vector<fp> e{scale};
+  for (int i = 0; i < n; i++) {
+    const size_t h = e.size();
+    e.resize(2 * h);
+    for (size_t k = 0; k < h; k++) {
+      const fp one = fp_mul(e[k], z[i], c);
+      e[k + h] = one;
+      e[k] = fp_sub(e[k], one, c);
+    }
   }
-  return h_out[0];
+  return e;
+}
+
+static FpBind sp_bind_weights(const fp *r, int k, const FpCtx &c) {
+  FpBind b{};
+  const std::vector<fp> e = sp_eq(r, k, c, c.one);
+  for (size_t j = 0; j < e.size(); j++) b.e[j] = e[j];
+  b.k = k;
+  return b;
 }
 
 static void put_canonical(uint8_t *b, fp mont, const FpCtx &c) {
@@ -600,151 +645,6 @@ static fp round_message(Transcript &ts, const FpCtx &c, fp &claim, const fp *wl,
   return r;
 }
 
-// The grid rounds k0 .. k1-1 of a sumcheck (outer: T = 4 tables E, A, B, C
-// and the cubic message, N = 3; inner: T = 2 tables D, W and N = 2) in one
-// cooperative launch that stays resident. Tables fold on their low
-// coordinate (pairs 2o, 2o + 1), so block b owns the contiguous chunk [b m,
-// (b + 1) m) of each input table (m = n_in / kSpMidBlocks) and, after each
-// fold, the first half of what it held: the chunk stays in the block's shared
-// memory from the first round to the last, and blocks share nothing but the
-// challenge (block 0 reads r_{k-1} from the downbox as publication
-// d0 + k - 1 and relays it through ctl[k - 1]) and the message (per-block
-// partial sums; the last block through round k, counted in ctl[k].done, adds
-// them and posts publication p0 + k). At the end each block writes its chunk
-// to `out` for the tail kernel. All blocks are resident together
-// (cooperative launch), so the relay waits end; each is bounded all the same.
-constexpr int kSpMidBlocks = 128;     // a lane proving alone
-constexpr int kSpMidPoolBlocks = 32;  // a pooled lane, sharing the GPU with others
-constexpr size_t kSpMidMaxChunk = 2048;  // entries per table per block
-struct SpTabs {
-  fp *t[4];
-};
-
-template <int T, int N>
-__global__ void __launch_bounds__(kThreads) sp_mid(SpTabs in, SpTabs out, size_t n_in, int k0,
-                                                   int k1, FpCtx c, fp *partial, Mailbox *mb,
-                                                   unsigned long long p0, const Mailbox *down,
-                                                   unsigned long long d0, RoundCtl *ctl) {
-  extern __shared__ fp chunk[];
-  const size_t m = n_in / gridDim.x;
-  fp *tab[T];
-#pragma unroll
-  for (int t = 0; t < T; t++) tab[t] = chunk + t * m;
-  const size_t base = (size_t)blockIdx.x * m;
-  for (size_t i = threadIdx.x; i < m; i += blockDim.x)
-#pragma unroll
-    for (int t = 0; t < T; t++) tab[t][i] = in.t[t][base + i];
-  __syncthreads();
-  size_t len = m;
-  for (int k = k0; k < k1; k++) {
-    if (k > 0) {
-      unsigned long long rw[2];
-      if (!resident_challenge(down, d0 + (k - 1), ctl + (k - 1), rw)) return;
-      const fp r = fp{rw[0], rw[1]};
-      // fold in place: every read of the level, then every write
-      constexpr int kPer = (int)(kSpMidMaxChunk / 2 / kThreads);
-      fp f[T][kPer];
-      const size_t nout = len / 2;
-#pragma unroll
-      for (int q = 0; q < kPer; q++) {
-        const size_t o = threadIdx.x + (size_t)q * kThreads;
-        if (o < nout)
-#pragma unroll
-          for (int t = 0; t < T; t++) f[t][q] = interp(tab[t][2 * o], tab[t][2 * o + 1], r, c);
-      }
-      __syncthreads();
-#pragma unroll
-      for (int q = 0; q < kPer; q++) {
-        const size_t o = threadIdx.x + (size_t)q * kThreads;
-        if (o < nout)
-#pragma unroll
-          for (int t = 0; t < T; t++) tab[t][o] = f[t][q];
-      }
-      __syncthreads();
-      len = nout;
-    }
-    fp acc[N];
-#pragma unroll
-    for (int q = 0; q < N; q++) acc[q] = fp_zero();
-    for (size_t j = threadIdx.x; j < len / 2; j += blockDim.x) {
-      if constexpr (T == 4) {
-        cubic(tab[0][2 * j], tab[0][2 * j + 1], tab[1][2 * j], tab[1][2 * j + 1], tab[2][2 * j],
-              tab[2][2 * j + 1], tab[3][2 * j], tab[3][2 * j + 1], c, acc);
-      } else {
-        const fp d0v = tab[0][2 * j], d1v = tab[0][2 * j + 1];
-        const fp w0v = tab[1][2 * j], w1v = tab[1][2 * j + 1];
-        acc[0] = fp_add(acc[0], fp_mul(d0v, w0v, c), c);
-        acc[1] = fp_add(acc[1], fp_mul(fp_sub(d1v, d0v, c), fp_sub(w1v, w0v, c), c), c);
-      }
-    }
-    block_fp_sum<N>(acc, c, partial);
-    fp_last_block_post<N>(partial, c, &ctl[k].done, mb, p0 + k);
-    __syncthreads();  // the chunk's reads of this round before the next fold
-  }
-  const size_t ob = (size_t)blockIdx.x * len;
-  for (size_t i = threadIdx.x; i < len; i += blockDim.x)
-#pragma unroll
-    for (int t = 0; t < T; t++) out.t[t][ob + i] = tab[t][i];
-}
-
-// sp_mid over rounds k0 .. k1-1 as a cooperative launch of sc.mid_blocks
-// blocks; n_in entries per input table.
-template <int T, int N>
-static void launch_sp_mid(const SpTabs &in, const SpTabs &out, size_t n_in, int k0, int k1,
-                          const FpCtx &c, const SpartanScratch &sc, unsigned long long p0,
-                          unsigned long long d0, cudaStream_t s) {
-  const int nb = sc.mid_blocks;
-  const size_t smem = T * (n_in / nb) * sizeof(fp);
-  static const int capacity = [] {
-    int dev = 0, sms = 0, per_sm = 0;
-    const size_t most = T * kSpMidMaxChunk * sizeof(fp);
-    BZ_CUDA(cudaGetDevice(&dev));
-    BZ_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    BZ_CUDA(cudaFuncSetAttribute(sp_mid<T, N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)most));
-    BZ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sp_mid<T, N>, kThreads, most));
-    return sms * per_sm;
-  }();
-  if (nb < 1 || nb > kSpMidBlocks || capacity < nb)
-    throw CudaError("sp_mid: the blocks do not fit resident together");
-  RoundChannel *ch = sc.channel;
-  SpTabs a = in, b = out;
-  FpCtx cc = c;
-  fp *partial = sc.partial;
-  Mailbox *mb = ch->dev;
-  const Mailbox *down = ch->down_dev;
-  RoundCtl *ctl = sc.ctl;
-  void *args[] = {&a, &b, &n_in, &k0, &k1, &cc, &partial, &mb, &p0, &down, &d0, &ctl};
-  BZ_CUDA(cudaLaunchCooperativeKernel((const void *)sp_mid<T, N>, dim3(nb), dim3(kThreads), args,
-                                      smem, s));
-  BZ_LAUNCH_CHECK();
-}
-
-// The first round (>= kmin) from which sp_mid can run the rounds up to t0:
-// its input fits the blocks' chunks, and the last resident round still sums
-// whole pairs in every block. t0 when there is none.
-static int sp_mid_start(size_t n0, int kmin, int t0, int nb) {
-  if (nb <= 0) return t0;
-  for (int k = kmin; k < t0; k++) {
-    const size_t n_in = k == 0 ? n0 : n0 >> (k - 1);
-    const size_t last = (n0 >> (t0 - 1)) / nb;  // per block after the last fold
-    if (n_in % nb == 0 && n_in / nb <= kSpMidMaxChunk && last >= 2) return k;
-  }
-  return t0;
-}
-
-// Grid of the resident grid rounds for a lane: kSpMidBlocks for a lane proving
-// alone; for a pooled lane none, or kSpMidPoolBlocks with BITZ_POOL_MID=1 (as
-// for the GKR middle rounds, gkr.cu).
-int sp_mid_blocks(bool alone) {
-  if (alone) return kSpMidBlocks;
-  static const bool pool = [] {
-    const char *e = getenv("BITZ_POOL_MID");
-    return e && e[0] == '1';
-  }();
-  return pool ? kSpMidPoolBlocks : 0;
-}
-
 void spartan_prove(const SpartanArgs &a, Transcript &ts, SpartanScratch &sc, cudaStream_t s,
                    SpartanOut &out) {
   const FpCtx &c = a.ctx;
@@ -756,190 +656,133 @@ void spartan_prove(const SpartanArgs &a, Transcript &ts, SpartanScratch &sc, cud
     u128 t = ts.challenge_fp(a.q);
     tau[i] = fp_mul(fp{(uint64_t)t, (uint64_t)(t >> 64)}, c.r2, c);
   }
-  fp *E = sc.t[0], *A = sc.t[1], *B = sc.t[2], *C = sc.t[3];
-  fp *E2 = sc.t[4], *A2 = sc.t[5], *B2 = sc.t[6], *C2 = sc.t[7];
-  fp_eq_table(tau, nr, c, E, sc.eq_scratch, s);
-  k_products_to_fp<<<grid_for(R), kThreads, 0, s>>>(a.prod, a.rows, R, c, A, B, C);
+  SpTabs in{{sc.t[1], sc.t[2], sc.t[3]}};
+  k_products_to_fp<<<grid_for(R), kThreads, 0, s>>>(a.prod, a.rows, R, c, in.t[0], in.t[1],
+                                                    in.t[2]);
   BZ_LAUNCH_CHECK();
   fp claim = fp_zero();
   out.outer.resize(4 * (size_t)nr);
   out.rx.resize(nr);
-  size_t len = R;
-  fp r = fp_zero();
   RoundChannel *ch = sc.channel;
-  const bool resident = resident_rounds_enabled();
-  bool tail = false;  // a resident tail kernel runs the remaining rounds
-  // no other thread's device allocation while a tail kernel waits for this one
-  ResidentScope gate(ch && resident);
-  auto send_r = [&](fp x) {
-    const uint64_t w[2] = {x.lo, x.hi};
-    ch->send(w, 2);
-  };
-  // BITZ_ROUND_TRACE=1 prints the host time between consecutive round results
+  KernelProbe &probe = KernelProbe::get();
+  std::vector<uint64_t> words(kHandoverWords);
+  std::vector<fp> F;
+  auto arm = [&] { return PassPost{nullptr, ch->counter, ch->handover_dev, ch->arm().seq}; };
+  // BITZ_ROUND_TRACE=1 prints the host time of every device turn
   static const bool trace = getenv("BITZ_ROUND_TRACE") != nullptr;
   auto t_prev = std::chrono::steady_clock::now();
-  auto trace_round = [&](const char *what, int round, bool queued_kernel) {
+  auto mark = [&](const char *what, int left) {
     if (!trace) return;
     const auto now = std::chrono::steady_clock::now();
-    fprintf(stderr, "[spartan] %s round %2d %s %7.2f us\n", what, round,
-            queued_kernel ? "grid" : "tail",
+    fprintf(stderr, "[spartan] %s, %d coordinates: %7.2f us\n", what, left,
             std::chrono::duration<double, std::micro>(now - t_prev).count());
     t_prev = now;
   };
   fp fin[3];
-  // Queued mode: every outer round is queued now, then the tail. Round k > 0
-  // folds at r_{k-1}, which the host posts as downbox publication d0 + k - 1
-  // and the round before fetches into ctl[k-1] (the tail reads its first
-  // challenge from the downbox itself); round k posts its message as
-  // publication p0 + k.
-  const bool queued = ch && resident && sc.ctl;
-  try {
-  if (queued) {
-    int t0 = 0;  // the tail's first round: its table fits in shared memory
-    while (t0 < nr && (t0 == 0 ? R : R >> (t0 - 1)) > (size_t)kSpTailN) t0++;
-    const unsigned long long p0 = ch->next + 1, d0 = ch->down_next + 1;
-    tail = true;  // from here a kernel of the lane may wait for this thread
-    fp *set[2][4] = {{E, A, B, C}, {E2, A2, B2, C2}};
-    // rounds km .. t0-1 resident (sp_mid, a grid of sc.mid_blocks blocks) when
-    // a round's input fits the blocks' shared memory; the rounds before them
-    // are queued launches
-    const int km = sp_mid_start(R, 0, t0, sc.mid_blocks);
-    BZ_CUDA(cudaMemsetAsync(sc.ctl, 0, sizeof(RoundCtl) * (nr + 1), s));
-    for (int k = 0; k < km; k++) {
-      const int fold = k > 0;
-      const size_t n = k == 0 ? R : R >> (k - 1);
-      fp *const *in = set[fold ? (k - 1) % 2 : 0];
-      fp *const *to = set[k % 2];
-      const size_t npairs = fold ? (n / 2 + 1) / 2 : n / 2;
-      RoundLink lk{fold ? sc.ctl + (k - 1) : nullptr, k + 1 < km ? sc.ctl + k : nullptr,
-                   ch->down_dev, d0 + k};
-      k_outer_round<<<grid_for(npairs), kThreads, 0, s>>>(
-          in[0], in[1], in[2], in[3], to[0], to[1], to[2], to[3], n, fold, 1, fp_zero(), c,
-          sc.partial, Publish{ch->counter, ch->dev, p0 + k}, lk);
-      BZ_LAUNCH_CHECK();
+  {
+    // eq(tau) over the coordinates above a pass: groups of seven from the top,
+    // group[g][n] over the lowest n... of the group's highest coordinates
+    std::vector<std::vector<fp>> group[4];
+    for (int g = 0, hi = nr; hi > 0; g++, hi -= kFacLog) {
+      if (g == 4) throw CudaError("spartan: too many row variables");
+      const int lo = std::max(0, hi - kFacLog);
+      for (int at = hi; at >= lo; at--) group[g].push_back(sp_eq(tau + at, hi - at, c, c.one));
     }
-    int cur_set = t0 > 0 ? (t0 - 1) % 2 : 0;
-    if (km < t0) {
-      const int si = km > 0 ? (km - 1) % 2 : 0;
-      const size_t n_in = km == 0 ? R : R >> (km - 1);
-      launch_sp_mid<4, 3>(SpTabs{{set[si][0], set[si][1], set[si][2], set[si][3]}},
-                          SpTabs{{set[1 - si][0], set[1 - si][1], set[1 - si][2], set[1 - si][3]}},
-                          n_in, km, t0, c, sc, p0, d0, s);
-      cur_set = 1 - si;
-    }
-    // rounds kh .. nr-1 on the host, from the tail's handover
-    const int kh = sp_host_round(ch, R, t0, nr);
-    const unsigned long long hseq = p0 + (kh >= 0 ? kh : 0);
-    std::vector<fp> host_tab[4];
-    {
-      fp *const *cur = set[cur_set];
-      const size_t n = t0 == 0 ? R : R >> (t0 - 1);
-      sp_outer_tail<<<1, kThreads, 0, s>>>(cur[0], cur[1], cur[2], cur[3], (int)n, t0 > 0,
-                                           nr - t0, c, ch->dev, p0 + t0, ch->down_dev,
-                                           d0 + (t0 > 0 ? t0 - 1 : 0), kh >= 0 ? kh - t0 : -1,
-                                           ch->handover_dev, hseq);
-      BZ_LAUNCH_CHECK();
-      tail = true;
-    }
-    for (int round = 0; round < nr; round++) {
-      if (kh >= 0 && round >= kh) {
-        if (round == kh) {
-          sp_take_handover(ch, s, hseq, 4, round == 0 ? R : R >> (round - 1), host_tab);
-          tail = false;  // the tail kernel ends after the handover
-        }
-        if (round > 0) host_sp_fold(host_tab, 4, r, c);
-        host_outer_sums(host_tab, c, sc.host);
-        ch->arm();  // publication numbering as if the device had posted
-      } else {
-        if (round > 0) send_r(r);
-        ch->arm();
-        ch->wait(s, reinterpret_cast<uint64_t *>(sc.host), 6);
+    auto factors = [&](int n) {  // over the top n coordinates
+      FpFactors f{};
+      const int groups = n == 0 ? 1 : (n + kFacLog - 1) / kFacLog;
+      f.n = groups;
+      f.low = n - kFacLog * (groups - 1);
+      for (int g = 0; g < groups; g++) {
+        const std::vector<fp> &v = group[groups - 1 - g][g == 0 ? f.low : kFacLog];
+        std::copy(v.begin(), v.end(), f.f[g]);
       }
-      trace_round("outer", round, round < t0);
+      return f;
+    };
+    // the outer message from t(0), t(1) and t's X^2 coefficient, times the
+    // round's eq factor and the bound coordinates' scale
+    fp scale = c.one;
+    int round = 0;
+    auto message = [&](const fp (&t)[3]) {
+      const fp l0 = fp_sub(c.one, tau[round], c), l1 = fp_sub(tau[round], l0, c);
+      const fp mid = fp_sub(fp_sub(t[1], t[0], c), t[2], c);
+      const fp wl[3] = {fp_mul(scale, fp_mul(l0, t[0], c), c),
+                        fp_mul(scale, fp_add(fp_mul(l0, t[2], c), fp_mul(l1, mid, c), c), c),
+                        fp_mul(scale, fp_mul(l1, t[2], c), c)};
       fp co[4];
-      r = round_message(ts, c, claim, sc.host, 4, a.q, co);
+      const fp r = round_message(ts, c, claim, wl, 4, a.q, co);
       for (int i = 0; i < 4; i++) out.outer[4 * round + i] = co[i];
-      out.rx[round] = r;
-    }
-    if (kh >= 0) {  // the last fold leaves one entry per table
-      host_sp_fold(host_tab, 4, r, c);
-      for (int k = 0; k < 3; k++) fin[k] = host_tab[k + 1][0];
-      ch->arm();
-    } else {
-      // the tail's last publication: the single entries of A, B and C
-      send_r(r);
-      ch->arm();
-      ch->wait(s, reinterpret_cast<uint64_t *>(fin), 6);
-    }
-  } else {
-  for (int round = 0; round < nr; round++) {
-    int fold = round > 0;
-    if (!tail && ch && resident && len <= (size_t)kSpTailN) {
-      sp_outer_tail<<<1, kThreads, 0, s>>>(E, A, B, C, (int)len, fold, nr - round, c, ch->dev,
-                                           ch->next + 1, ch->down_dev, ch->down_next + 1, -1,
-                                           nullptr, 0);
-      BZ_LAUNCH_CHECK();
-      tail = true;
-    }
-    if (tail) {
-      if (fold) {
-        send_r(r);
-        len /= 2;
-      }
-      ch->arm();
-      ch->wait(s, reinterpret_cast<uint64_t *>(sc.host), 6);
-    } else {
-      size_t npairs = fold ? (len / 2 + 1) / 2 : len / 2;
-      int g = grid_for(npairs);
-      KernelProbe &probe = KernelProbe::get();
-      const bool probed = probe.on("k_outer_round");
+      out.rx[round++] = r;
+      scale = fp_mul(scale, fp_add(l0, fp_mul(l1, r, c), c), c);
+      return r;
+    };
+    size_t live = a.rows;
+    SpTabs spare[2] = {{{sc.t[4], sc.t[5], sc.t[6]}}, {{sc.t[1], sc.t[2], sc.t[3]}}};
+    int to = 0;
+    FpBind b{};
+    int rem = nr;
+    while (rem > kSpHostLog) {
+      const int k = std::min(kPassMaxK, rem), points = pow3(k);
+      const size_t live_out = (live + (((size_t)1 << b.k) - 1)) >> b.k;
+      // positions past the live entries add nothing
+      const uint32_t count = (uint32_t)((live_out + ((size_t)1 << k) - 1) >> k);
+      const int lx = pass_tile_log(count);
+      const unsigned int grid = pass_grid(count, lx);
+      const bool probed = probe.on("sp_outer_pass");
       if (probed) probe.before(s);
-      k_outer_round<<<g, kThreads, 0, s>>>(E, A, B, C, E2, A2, B2, C2, len, fold, 1, r, c,
-                                           sc.partial, Publish{nullptr, nullptr, 0},
-                                           RoundLink{nullptr, nullptr, nullptr, 0});
+      const PassPost post = arm();
+      sp_outer_pass<3><<<grid, kPassThreads, 0, s>>>(in, spare[to], live, count, b,
+                                                     factors(rem - k), c, lx, sc.partial, post);
       BZ_LAUNCH_CHECK();
-      // four tables of 16-byte residues: read whole, written folded to half
-      if (probed) probe.after(s, "k_outer_round", 16.0 * 4 * (double)len * (fold ? 1.5 : 1.0));
-      host_partial_sum(sc.partial, g, 3, sc.sums, sc.host, c, s, sc.channel);
-      if (fold) {
-        std::swap(E, E2);
-        std::swap(A, A2);
-        std::swap(B, B2);
-        std::swap(C, C2);
-        len /= 2;
+      // three tables of 16-byte residues read, and written bound
+      if (probed)
+        probe.after(s, "sp_outer_pass",
+                    48.0 * ((double)live + (b.k ? (double)live_out : 0.0)));
+      if (b.k) {
+        in = spare[to];
+        to ^= 1;
+        live = (size_t)count << k;
       }
+      const int blocks = pass_direct(grid, 2 * points) ? (int)grid : 1;
+      ch->wait_handover(s, post.seq, words.data(), 2 * points * blocks);
+      mark("outer pass", rem);
+      F = sp_combine(words, points, blocks, c);
+      fp r[kPassMaxK];
+      for (int t = 0; t < k; t++) {
+        fp sums[3];
+        sp_round_sums(F, k - 1 - t, sp_eq(tau + round + 1, k - 1 - t, c, c.one), c, sums);
+        r[t] = message(sums);
+        sp_fold_points(F, r[t], c);
+      }
+      b = sp_bind_weights(r, k, c);
+      rem -= k;
     }
-    fp co[4];
-    r = round_message(ts, c, claim, sc.host, 4, a.q, co);
-    for (int i = 0; i < 4; i++) out.outer[4 * round + i] = co[i];
-    out.rx[round] = r;
-  }
-  if (tail) {
-    // the tail's last publication: the single entries of A, B and C
-    send_r(r);
-    ch->arm();
-    ch->wait(s, reinterpret_cast<uint64_t *>(fin), 6);
-  } else {
-    // the last fold leaves one entry per table
-    k_outer_round<<<1, kThreads, 0, s>>>(E, A, B, C, E2, A2, B2, C2, len, 1, 0, r, c, sc.partial,
-                                         Publish{nullptr, nullptr, 0},
-                                         RoundLink{nullptr, nullptr, nullptr, 0});
+    const int n = 1 << rem;
+    const PassPost post = arm();
+    sp_handover<false><<<(3 * n + 63) / 64, 64, 0, s>>>(in, 3, n, live, nullptr, b, c,
+                                                        post.handover, post.seq);
     BZ_LAUNCH_CHECK();
-    BZ_CUDA(cudaMemcpyAsync(&fin[0], A2, sizeof(fp), cudaMemcpyDeviceToHost, s));
-    BZ_CUDA(cudaMemcpyAsync(&fin[1], B2, sizeof(fp), cudaMemcpyDeviceToHost, s));
-    BZ_CUDA(cudaMemcpyAsync(&fin[2], C2, sizeof(fp), cudaMemcpyDeviceToHost, s));
-    BZ_CUDA(stream_wait(s));
-  }
-  }
-  } catch (...) {
-    if (tail) {  // release the waiting kernel before the lane is reused
-      ch->abort();
-      stream_wait(s);
-      ch->clear_down();
+    ch->wait_handover(s, post.seq, words.data(), 6 * n);
+    mark("outer tables", rem);
+    const std::vector<fp> all = sp_words(words, 3 * (size_t)n);
+    std::vector<fp> tab[3];
+    for (int t = 0; t < 3; t++) tab[t].assign(all.begin() + t * n, all.begin() + (t + 1) * n);
+    while (round < nr) {
+      const std::vector<fp> e = sp_eq(tau + round + 1, nr - round - 1, c, c.one);
+      fp sums[3] = {fp_zero(), fp_zero(), fp_zero()};
+      for (size_t j = 0; j < e.size(); j++) {
+        const fp a0 = tab[0][2 * j], a1 = tab[0][2 * j + 1], b0 = tab[1][2 * j],
+                 b1 = tab[1][2 * j + 1];
+        sums[0] = fp_add(sums[0], fp_mul(e[j], fp_sub(fp_mul(a0, b0, c), tab[2][2 * j], c), c), c);
+        sums[1] =
+            fp_add(sums[1], fp_mul(e[j], fp_sub(fp_mul(a1, b1, c), tab[2][2 * j + 1], c), c), c);
+        sums[2] = fp_add(sums[2], fp_mul(e[j], fp_mul(fp_sub(a1, a0, c), fp_sub(b1, b0, c), c), c), c);
+      }
+      host_sp_fold(tab, 3, message(sums), c);
     }
-    throw;
+    for (int k = 0; k < 3; k++) fin[k] = tab[k][0];
+    mark("outer host rounds", 0);
   }
-  tail = false;
   uint8_t msg[48];
   for (int k = 0; k < 3; k++) {
     out.abc[k] = fin[k];
@@ -956,7 +799,7 @@ void spartan_prove(const SpartanArgs &a, Transcript &ts, SpartanScratch &sc, cud
   k_bind_table<<<(a.ntab + 127) / 128, 128, 0, s>>>(a.tab_vals, a.tab_which, a.ntab, rho, rho2, c,
                                                      sc.tab);
   BZ_LAUNCH_CHECK();
-  fp *D = sc.d[0], *W = sc.d[1], *D2 = sc.d[2], *W2 = sc.d[3];
+  fp *D = sc.d[0];
   k_bind<<<grid_for(Cn), kThreads, 0, s>>>(a.csc_off, a.csc_row, a.csc_idx, sc.tab, eq, a.cols, Cn,
                                            c, D);
   BZ_LAUNCH_CHECK();
@@ -971,156 +814,120 @@ void spartan_prove(const SpartanArgs &a, Transcript &ts, SpartanScratch &sc, cud
   // inner sumcheck
   out.inner.resize(3 * (size_t)nc);
   out.ry.resize(nc);
-  len = Cn;
-  int w_bits = 1;
   fp dw[2];
-  try {
-  if (queued) {
-    // as the outer rounds: round k > 0 folds at r_{k-1} (downbox publication
-    // d0 + k - 1, fetched into ctl[k-1] by round k - 1) and posts p0 + k; W
-    // comes from the packed bits of h until round 1 has folded them
-    int t0 = 0;
-    while (t0 < nc && (t0 == 0 ? Cn : Cn >> (t0 - 1)) > (size_t)kSpTailN) t0++;
-    const unsigned long long p0 = ch->next + 1, d0 = ch->down_next + 1;
-    tail = true;  // from here a kernel of the lane may wait for this thread
-    fp *set[2][2] = {{D, W}, {D2, W2}};
-    // W is read from the packed bits of h through round 1: resident rounds
-    // start at 2 at the earliest
-    const int km = sp_mid_start(Cn, 2, t0, sc.mid_blocks);
-    BZ_CUDA(cudaMemsetAsync(sc.ctl, 0, sizeof(RoundCtl) * (nc + 1), s));
-    for (int k = 0; k < km; k++) {
-      const int fold = k > 0;
-      const size_t n = k == 0 ? Cn : Cn >> (k - 1);
-      fp *const *in = set[fold ? (k - 1) % 2 : 0];
-      fp *const *to = set[k % 2];
-      const size_t npairs = fold ? (n / 2 + 1) / 2 : n / 2;
-      RoundLink lk{fold ? sc.ctl + (k - 1) : nullptr, k + 1 < km ? sc.ctl + k : nullptr,
-                   ch->down_dev, d0 + k};
-      k_inner_round<<<grid_for(npairs), kThreads, 0, s>>>(
-          in[0], in[1], a.hbits, k <= 1 ? 1 : 0, to[0], to[1], n, fold, 1, fp_zero(), c,
-          sc.partial, Publish{ch->counter, ch->dev, p0 + k}, lk);
-      BZ_LAUNCH_CHECK();
-    }
-    int cur_set = t0 > 0 ? (t0 - 1) % 2 : 0;
-    if (km < t0) {
-      const int si = (km - 1) % 2;
-      launch_sp_mid<2, 2>(SpTabs{{set[si][0], set[si][1], nullptr, nullptr}},
-                          SpTabs{{set[1 - si][0], set[1 - si][1], nullptr, nullptr}},
-                          Cn >> (km - 1), km, t0, c, sc, p0, d0, s);
-      cur_set = 1 - si;
-    }
-    // rounds kh .. nc-1 on the host, from the tail's handover
-    const int kh = sp_host_round(ch, Cn, t0, nc);
-    const unsigned long long hseq = p0 + (kh >= 0 ? kh : 0);
-    std::vector<fp> host_tab[2];
-    {
-      fp *const *cur = set[cur_set];
-      const size_t n = t0 == 0 ? Cn : Cn >> (t0 - 1);
-      sp_inner_tail<<<1, kThreads, 0, s>>>(cur[0], cur[1], a.hbits, t0 <= 1 ? 1 : 0, (int)n,
-                                           t0 > 0, nc - t0, c, ch->dev, p0 + t0, ch->down_dev,
-                                           d0 + (t0 > 0 ? t0 - 1 : 0), kh >= 0 ? kh - t0 : -1,
-                                           ch->handover_dev, hseq);
-      BZ_LAUNCH_CHECK();
-      tail = true;
-    }
-    for (int round = 0; round < nc; round++) {
-      if (kh >= 0 && round >= kh) {
-        if (round == kh) {
-          sp_take_handover(ch, s, hseq, 2, round == 0 ? Cn : Cn >> (round - 1), host_tab);
-          tail = false;  // the tail kernel ends after the handover
-        }
-        if (round > 0) host_sp_fold(host_tab, 2, r, c);
-        host_inner_sums(host_tab, c, sc.host);
-        ch->arm();  // publication numbering as if the device had posted
-      } else {
-        if (round > 0) send_r(r);
-        ch->arm();
-        ch->wait(s, reinterpret_cast<uint64_t *>(sc.host), 4);
-      }
-      trace_round("inner", round, round < t0);
+  {
+    int round = 0;
+    auto message = [&](fp at_zero, fp at_inf) {
+      const fp wl[2] = {at_zero, at_inf};
       fp co[3];
-      r = round_message(ts, c, claim, sc.host, 3, a.q, co);
+      const fp r = round_message(ts, c, claim, wl, 3, a.q, co);
       for (int i = 0; i < 3; i++) out.inner[3 * round + i] = co[i];
-      out.ry[round] = r;
-    }
-    if (kh >= 0) {  // the last fold leaves one entry per table
-      host_sp_fold(host_tab, 2, r, c);
-      dw[0] = host_tab[0][0];
-      dw[1] = host_tab[1][0];
-      ch->arm();
-    } else {
-      send_r(r);
-      ch->arm();
-      ch->wait(s, reinterpret_cast<uint64_t *>(dw), 4);
-    }
-  } else {
-  for (int round = 0; round < nc; round++) {
-    int fold = round > 0;
-    if (!tail && ch && resident && len <= (size_t)kSpTailN) {
-      sp_inner_tail<<<1, kThreads, 0, s>>>(D, W, a.hbits, w_bits, (int)len, fold, nc - round, c,
-                                           ch->dev, ch->next + 1, ch->down_dev,
-                                           ch->down_next + 1, -1, nullptr, 0);
-      BZ_LAUNCH_CHECK();
-      tail = true;
-    }
-    if (tail) {
-      if (fold) {
-        send_r(r);
-        len /= 2;
+      out.ry[round++] = r;
+      return r;
+    };
+    auto from_points = [&](int k) {
+      fp r[kPassMaxK];
+      for (int t = 0; t < k; t++) {
+        fp sums[3];
+        sp_round_sums(F, k - 1 - t, {}, c, sums);
+        r[t] = message(sums[0], sums[2]);
+        sp_fold_points(F, r[t], c);
       }
-      ch->arm();
-      ch->wait(s, reinterpret_cast<uint64_t *>(sc.host), 4);
-    } else {
-      size_t npairs = fold ? (len / 2 + 1) / 2 : len / 2;
-      int g = grid_for(npairs);
-      KernelProbe &probe = KernelProbe::get();
-      const bool probed = probe.on("k_inner_round");
+      return sp_bind_weights(r, k, c);
+    };
+    FpBind b{};
+    int rem = nc;
+    size_t live = a.cols;
+    bool bits = true;
+    const fp *d = D, *w = nullptr;
+    // every circuit has a compression's 20,456 columns
+    if (rem <= kSpHostLog + kPassMaxK) throw CudaError("spartan: too few columns");
+    {
+      const PassPost post = arm();
+      const size_t n = (a.cols + 31) / 32;
+      const bool probed = probe.on("sp_bits");
       if (probed) probe.before(s);
-      k_inner_round<<<g, kThreads, 0, s>>>(D, W, a.hbits, w_bits, D2, W2, len, fold, 1, r, c,
-                                           sc.partial, Publish{nullptr, nullptr, 0},
-                                           RoundLink{nullptr, nullptr, nullptr, 0});
+      sp_bits<<<grid_for(n, kThreads / 32, kSpBitsBlocks), kThreads, 0, s>>>(D, a.hbits, n, c,
+                                                                             sc.partial, post);
       BZ_LAUNCH_CHECK();
-      // D (16-byte residues) and W (16-byte residues, or bits while w_bits is
-      // set): read whole, written folded to half
-      if (probed) {
-        const double wbytes = w_bits ? (double)len / 8.0 : 16.0 * (double)len;
-        probe.after(s, "k_inner_round",
-                    16.0 * (double)len + wbytes + (fold ? 16.0 * (double)len : 0.0));
+      if (probed) probe.after(s, "sp_bits", (16.0 + 1.0 / 8) * (double)a.cols);
+      ch->wait_handover(s, post.seq, words.data(), 128);
+      mark("inner bits", rem);
+      const std::vector<fp> H = sp_words(words, 64);
+      F.assign(27, fp_zero());
+      for (int p = 0; p < 27; p++) {
+        int one = 0, inf = 0;
+        for (int i = 0, q = p; i < 3; i++, q /= 3) {
+          one |= (q % 3 == 1) << (2 - i);
+          inf |= (q % 3 == 2) << (2 - i);
+        }
+        for (int x = 0; x < 8; x++)  // signs: a difference of halves at infinity
+          for (int y = 0; y < 8; y++)
+            if ((x & ~inf) == one && (y & ~inf) == one)
+              F[p] = __builtin_popcount((x ^ y) & inf) & 1 ? fp_sub(F[p], H[8 * x + y], c)
+                                                           : fp_add(F[p], H[8 * x + y], c);
       }
-      host_partial_sum(sc.partial, g, 2, sc.sums, sc.host, c, s, sc.channel);
-      if (fold) {
-        std::swap(D, D2);
-        std::swap(W, W2);
-        len /= 2;
-        w_bits = 0;
-      }
+      b = from_points(3);
+      rem -= 3;
     }
-    fp co[3];
-    r = round_message(ts, c, claim, sc.host, 3, a.q, co);
-    for (int i = 0; i < 3; i++) out.inner[3 * round + i] = co[i];
-    out.ry[round] = r;
-  }
-  if (tail) {
-    send_r(r);
-    ch->arm();
-    ch->wait(s, reinterpret_cast<uint64_t *>(dw), 4);
-  } else {
-    k_inner_round<<<1, kThreads, 0, s>>>(D, W, a.hbits, w_bits, D2, W2, len, 1, 0, r, c,
-                                         sc.partial, Publish{nullptr, nullptr, 0},
-                                         RoundLink{nullptr, nullptr, nullptr, 0});
+    fp *set[2][2] = {{sc.d[2], sc.d[3]}, {sc.d[0], sc.d[1]}};
+    int to = 0;
+    while (rem > kSpHostLog) {
+      const int k = kPassMaxK, points = pow3(k);
+      const size_t live_out = (live + (((size_t)1 << b.k) - 1)) >> b.k;
+      const uint32_t count = (uint32_t)((live_out + ((size_t)1 << k) - 1) >> k);
+      const int lx = pass_tile_log(count);
+      const unsigned int grid = pass_grid(count, lx);
+      const bool probed = probe.on("sp_inner_pass");
+      if (probed) probe.before(s);
+      const PassPost post = arm();
+      if (bits)
+        sp_inner_pass<3, true><<<grid, kPassThreads, 0, s>>>(
+            d, reinterpret_cast<const fp *>(a.hbits), set[to][0], set[to][1], live, count, b, c, lx,
+            sc.partial, post);
+      else
+        sp_inner_pass<3, false><<<grid, kPassThreads, 0, s>>>(d, w, set[to][0], set[to][1], live,
+                                                              count, b, c, lx, sc.partial, post);
+      BZ_LAUNCH_CHECK();
+      if (probed)
+        probe.after(s, "sp_inner_pass",
+                    (bits ? 16.125 : 32.0) * (double)live + 32.0 * (double)live_out);
+      bits = false;
+      d = set[to][0];
+      w = set[to][1];
+      to ^= 1;
+      live = (size_t)count << k;
+      const int blocks = pass_direct(grid, 2 * points) ? (int)grid : 1;
+      ch->wait_handover(s, post.seq, words.data(), 2 * points * blocks);
+      mark("inner pass", rem);
+      F = sp_combine(words, points, blocks, c);
+      b = from_points(k);
+      rem -= k;
+    }
+    const int n = 1 << rem;
+    const PassPost post = arm();
+    const SpTabs last{{const_cast<fp *>(d), const_cast<fp *>(w), nullptr}};
+    (bits ? sp_handover<true> : sp_handover<false>)<<<(2 * n + 63) / 64, 64, 0, s>>>(
+        last, 2, n, live, a.hbits, b, c, post.handover, post.seq);
     BZ_LAUNCH_CHECK();
-    BZ_CUDA(cudaMemcpyAsync(&dw[0], D2, sizeof(fp), cudaMemcpyDeviceToHost, s));
-    BZ_CUDA(cudaMemcpyAsync(&dw[1], W2, sizeof(fp), cudaMemcpyDeviceToHost, s));
-    BZ_CUDA(stream_wait(s));
-  }
-  }
-  } catch (...) {
-    if (tail) {
-      ch->abort();
-      stream_wait(s);
-      ch->clear_down();
+    ch->wait_handover(s, post.seq, words.data(), 4 * n);
+    mark("inner tables", rem);
+    const std::vector<fp> all = sp_words(words, 2 * (size_t)n);
+    std::vector<fp> tab[2];
+    for (int t = 0; t < 2; t++) tab[t].assign(all.begin() + t * n, all.begin() + (t + 1) * n);
+    while (round < nc) {
+      fp s0 = fp_zero(), si = fp_zero();
+      for (size_t j = 0; j < tab[0].size() / 2; j++) {
+        const fp d0 = tab[0][2 * j], d1 = tab[0][2 * j + 1], w0 = tab[1][2 * j],
+                 w1 = tab[1][2 * j + 1];
+        s0 = fp_add(s0, fp_mul(d0, w0, c), c);
+        si = fp_add(si, fp_mul(fp_sub(d1, d0, c), fp_sub(w1, w0, c), c), c);
+      }
+      host_sp_fold(tab, 2, message(s0, si), c);
     }
-    throw;
+    dw[0] = tab[0][0];
+    dw[1] = tab[1][0];
+    mark("inner host rounds", 0);
   }
   out.d_at_ry = dw[0];
   out.final_claim = claim;
@@ -1166,7 +973,7 @@ fp spartan_matrix_eval(const SpartanArgs &a, const fp *rx, fp rho, const fp *ry,
   const int g = grid_for(Cn);
   k_fp_dot<<<g, kThreads, 0, s>>>(D, EY, Cn, c, sc.partial);
   BZ_LAUNCH_CHECK();
-  k_fp_finalize<1><<<1, kThreads, 0, s>>>(sc.partial, g, c, sc.sums, Publish{nullptr, nullptr, 0});
+  k_fp_finalize<<<1, kThreads, 0, s>>>(sc.partial, g, c, sc.sums);
   BZ_LAUNCH_CHECK();
   BZ_CUDA(cudaMemcpyAsync(sc.host, sc.sums, sizeof(fp), cudaMemcpyDeviceToHost, s));
   BZ_CUDA(stream_wait(s));
@@ -1218,19 +1025,17 @@ void preload_spartan_kernels() {
   load_kernels({(const void *)k_fp_eq_factor,
                 (const void *)k_fp_eq_expand,
                 (const void *)k_products_to_fp,
-                (const void *)k_outer_round,
-                (const void *)k_inner_round,
-                (const void *)k_fp_finalize<1>,
-                (const void *)k_fp_finalize<2>,
-                (const void *)k_fp_finalize<3>,
+                (const void *)k_fp_finalize,
+                (const void *)sp_outer_pass<3>,
+                (const void *)sp_inner_pass<3, true>,
+                (const void *)sp_inner_pass<3, false>,
+                (const void *)sp_bits,
+                (const void *)sp_handover<true>,
+                (const void *)sp_handover<false>,
                 (const void *)k_bind_table,
                 (const void *)k_bind,
                 (const void *)k_bind_col0,
                 (const void *)k_bind_col0_finish,
-                (const void *)sp_outer_tail,
-                (const void *)sp_inner_tail,
-                (const void *)sp_mid<4, 3>,
-                (const void *)sp_mid<2, 2>,
                 (const void *)k_fp_dot,
                 (const void *)k_fp_canonical});
 }

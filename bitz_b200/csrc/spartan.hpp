@@ -34,19 +34,18 @@ struct SpartanArgs {
 };
 
 struct SpartanScratch {
-  fp *t[8];        // outer tables: E, A, B, C and their fold targets (2^rows each)
-  fp *d[4];        // inner tables: D, W and fold targets (2^cols each)
+  fp *t[8];        // eq over the rows (0), A, B, C (1-3) and their bound forms (4-6), 2^rows each
+  fp *d[4];        // D (0) and the bound D and W (2, 3, then 0, 1), 2^cols each
   fp *eq_scratch;  // factor tables
-  fp *partial;     // per-block partial sums
+  fp *partial;     // per-block partial sums, kSpPartials entries
   fp *sums;        // device, 3 entries
   fp *tab;         // coefficient table, ntab entries
   fp *host;        // pinned, 4 entries
-  RoundChannel *channel = nullptr;  // mailbox for round results; null: copy + sync
-  RoundCtl *ctl = nullptr;          // the lane's round controls (queued rounds)
-  // blocks of the cooperative kernel that runs the grid rounds resident (128
-  // for a lane proving alone, fewer for a pooled lane); 0: queued launches
-  int mid_blocks = 0;
+  RoundChannel *channel = nullptr;  // carries the passes' sums and the last tables
 };
+
+// Entries `partial` holds: the passes' blocks times their points.
+constexpr size_t kSpPartials = 4 * kSMs * 64;
 
 struct SpartanOut {
   std::vector<fp> outer, inner, rx, ry;  // Montgomery
@@ -55,8 +54,6 @@ struct SpartanOut {
   bool ok = false;
 };
 
-// The grid of a lane's resident Spartan rounds (SpartanScratch::mid_blocks).
-int sp_mid_blocks(bool alone);
 FpCtx make_fp_ctx(u128 q);
 u128 fp_canonical(fp mont, const FpCtx &c);
 // out[k] = canonical value of in[k] (as two LE words), on the device.

@@ -298,7 +298,7 @@ int ProofSystem::verify(const uint8_t *proof, size_t proof_len, Context *lane) {
   W.sp_t.resize(8 * R);
   W.sp_d.resize(4 * Cn);
   W.sp_eqs.resize(4096 * 2 + ((size_t)1 << ((std::max(nr, nc) + 1) / 2 + 1)));
-  W.sp_part.resize(3 * kSMs * 8 + 16);
+  W.sp_part.resize(kSpPartials);
   W.sp_sums.resize(4);
   W.sp_tab.resize(dev_->ntab + 1);
   if (bit_rows_.empty())

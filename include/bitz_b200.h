@@ -279,9 +279,8 @@ int bitz_server_stop(bitz_server *srv);
  * and counts each launch's algorithmic work. spec: NULL or "" turns the
  * probe off, "*" probes every instrumented launch site, else a comma-separated
  * list of kernel names; enabling resets the totals. While the probe is on,
- * every sumcheck round is its own launch (as under a kernel profiler).
- * Instrumented: gkr_pass, pg_pass,
- * k_outer_round, k_inner_round, k_fp_finalize. */
+ * every sumcheck pass is timed alone.
+ * Instrumented: gkr_pass, pg_pass, sp_outer_pass, sp_inner_pass, sp_bits. */
 int bitz_probe_kernel(const char *spec);
 /* One kernel's totals since the probe was enabled: out[0] milliseconds,
  * out[1] algorithmic bytes, and its GF(2^128) products: out[2] reduced
