@@ -71,4 +71,9 @@ void spartan_prove(const SpartanArgs &a, Transcript &ts, SpartanScratch &sc, cud
 fp spartan_matrix_eval(const SpartanArgs &a, const fp *rx, fp rho, const fp *ry,
                        SpartanScratch &sc, cudaStream_t s);
 
+// The verifier's sum over the columns of cols[j] (Montgomery) times fold_j mod
+// q into sc.host[0], once the stream is waited for; uses partial and sums.
+void fold_claim(const u128 *folds, const fp *cols, size_t n, const FpCtx &c, SpartanScratch &sc,
+                cudaStream_t s);
+
 }  // namespace bz

@@ -335,7 +335,7 @@ int ProofSystem::verify(const uint8_t *proof, size_t proof_len, Context *lane) {
   const size_t ncol = (size_t)1 << sc_cols;
   std::vector<fp> pt(7 + sc_cols, fp_zero());
   for (int i = 0; i < nc && i < 7 + sc_cols; i++) pt[i] = ry[i];
-  std::vector<u128> rows_w(128), cols_w(ncol);
+  std::vector<u128> rows_w(128);
   {
     fp e[128];
     fp_eq_small(pt.data(), 7, fc, e);
@@ -345,7 +345,8 @@ int ProofSystem::verify(const uint8_t *proof, size_t proof_len, Context *lane) {
   W.cols_canon.resize(ncol);
   fp_eq_table(pt.data() + 7, sc_cols, fc, W.cols_fp.get(), sc.eq_scratch, s);
   fp_canonical_device(W.cols_fp.get(), ncol, fc, W.cols_canon.get(), s);
-  BZ_CUDA(cudaMemcpyAsync(cols_w.data(), W.cols_canon.get(), ncol * 16, cudaMemcpyDeviceToHost, s));
+  u128 *cols_w = W.host_cols.get(ncol);
+  BZ_CUDA(cudaMemcpyAsync(cols_w, W.cols_canon.get(), ncol * 16, cudaMemcpyDeviceToHost, s));
   BZ_CUDA(stream_wait(s));
   const u128 fin_c = fp_canonical(fin, fc);
   t.public_message("bitz/virtual-statement/v1", 25);
@@ -358,42 +359,42 @@ int ProofSystem::verify(const uint8_t *proof, size_t proof_len, Context *lane) {
   }
   t.public_message(S.map_digest, 32);
   {
+    // one message, absorbed in pieces as the prover does
     std::vector<uint8_t> ce;
-    ce.reserve(16 * (129 + ncol) + 16);
+    ce.reserve(16 * 129 + 8);
     put_u64(ce, 128);
     for (auto w : rows_w) put_u128(ce, w);
     put_u64(ce, ncol);
-    for (auto w : cols_w) put_u128(ce, w);
+    t.public_message(ce.data(), ce.size());
+    t.public_message(cols_w, ncol * 16);
+    ce.clear();
     put_u128(ce, fin_c);
     t.public_message(ce.data(), ce.size());
   }
   t.public_message(pcs_enc_.data(), pcs_enc_.size());
   // ---- receive_fold (crates/verifier/src/fold.rs:42-77): every fold is at
-  // most 128 (q - 1), and sum_j cols_w[j] fold_j = the claim mod q
-  std::vector<u128> folds(ncol);
+  // most 128 (q - 1), and sum_j cols_w[j] fold_j = the claim mod q (summed on
+  // the device, read with the GKR's first claim)
+  u128 *folds = W.host_folds.get(ncol + 128);
   {
+    rd.take(folds, ncol * 16);
     const u128 bound = (u128)128 * (q - 1);
-    fp acc = fp_zero();
-    for (size_t j = 0; j < ncol; j++) {
-      uint8_t b[16];
-      rd.take(b, 16);
-      folds[j] = get_u128(b);
-      BZ_VERIFY(folds[j] <= bound, "a column fold exceeds 128 (q - 1)");
-      acc = fp_add(acc, fp_mul(mont(cols_w[j], fc), mont(folds[j] % q, fc), fc), fc);
-    }
+    bool over = false;
+    for (size_t j = 0; j < ncol; j++) over |= folds[j] > bound;
+    BZ_VERIFY(!over, "a column fold exceeds 128 (q - 1)");
     BZ_VERIFY(!rd.short_read, "the proof ends inside the column folds");
-    BZ_VERIFY(fp_canonical(acc, fc) == fin_c, "the column folds do not meet the Spartan claim");
   }
   // the images g^fold on the device (the prover's comb)
-  W.folds.upload(folds.data(), ncol, s);
+  W.folds.upload(folds, ncol, s);
+  fold_claim(W.folds.get(), W.cols_fp.get(), ncol, fc, sc, s);
   W.images.resize(ncol + 128);
   comb_pow(T.comb.get(), W.folds.get(), (int)ncol, W.images.get() + 128, s);
   W.exps.upload(rows_w.data(), 128, s);
   comb_pow(T.comb.get(), W.exps.get(), 128, W.images.get(), s);
   std::vector<f128> row_images(128);
   BZ_CUDA(cudaMemcpyAsync(row_images.data(), W.images.get(), 128 * 16, cudaMemcpyDeviceToHost, s));
-  BZ_VERIFY(rd.grind("bitz/columns/v1", grinding_bits((uint32_t)security_, (uint64_t)sc_cols)),
-            "column-fold grinding nonce");
+  const bool ground =
+      rd.grind("bitz/columns/v1", grinding_bits((uint32_t)security_, (uint64_t)sc_cols));
   std::vector<f128> point(sc_cols);
   for (auto &z : point) z = t.challenge_f128();
   // ---- gpgkr_verify (crates/gkr/src/lib.rs:717-772) from e0 = MLE(images)(zeta)
@@ -405,12 +406,23 @@ int ProofSystem::verify(const uint8_t *proof, size_t proof_len, Context *lane) {
   dot(W.u2.get(), W.images.get() + 128, ncol, W.acc.get(), Publish{nullptr, nullptr, 0}, s);
   BZ_CUDA(cudaMemcpyAsync(W.host_acc, W.acc.get(), 16, cudaMemcpyDeviceToHost, s));
   BZ_CUDA(stream_wait(s));
+  BZ_VERIFY(fp_canonical(sc.host[0], fc) == fin_c, "the column folds do not meet the Spartan claim");
+  BZ_VERIFY(ground, "column-fold grinding nonce");
   f128 gclaim = mk(W.host_acc[0], W.host_acc[1]);
   const uint32_t gkr_bits = grinding_bits((uint32_t)security_, 3);
   for (int layer = 0; layer < 7; layer++) {
     const int n = (int)point.size();
     std::vector<f128> next(n + 1);
     f128 eq_bound = kOne;
+    // the coordinates' inverses from one inversion of their product
+    std::vector<f128> inv(n), pre(n + 1, kOne);
+    for (int i = 0; i < n; i++) pre[i + 1] = gis_zero(point[i]) ? pre[i] : gmul(pre[i], point[i]);
+    f128 left_inv = gf_inv_host(pre[n]);
+    for (int i = n - 1; i >= 0; i--) {
+      if (gis_zero(point[i])) continue;
+      inv[i] = gmul(left_inv, pre[i]);
+      left_inv = gmul(left_inv, point[i]);
+    }
     for (int i = n - 1; i >= 0; i--) {
       const f128 z = point[i];
       const f128 sum_b = rd.f(), sum_inf = rd.f();
@@ -421,7 +433,7 @@ int ProofSystem::verify(const uint8_t *proof, size_t proof_len, Context *lane) {
         sum1 = sum_b;
       } else {
         sum0 = sum_b;
-        sum1 = gmul(gadd(gclaim, gmul(gadd(kOne, z), sum_b)), gf_inv_host(z));
+        sum1 = gmul(gadd(gclaim, gmul(gadd(kOne, z), sum_b)), inv[i]);
       }
       BZ_VERIFY(rd.grind("gkr/cubic/v1", gkr_bits), "GKR grinding nonce");
       const f128 r = t.challenge_f128();
