@@ -627,6 +627,67 @@ __global__ void k_merkle_parents(uint32_t *nodes, size_t lo, size_t hi) {
   }
 }
 
+// The verifier's openings of one level, a warp per query: lane 0 hashes the
+// row and climbs its path (a serial chain of about 30 compressions, 15 us, but
+// for every query at once), and every lane takes its share of the row's
+// combination. `proof` holds the openings at word `at`, each width * 4 words of
+// the row, then 8 per sibling. vals[q] is the combination; *bad is set when a
+// path does not reach the root.
+constexpr int kOpeningThreads = 64;
+__global__ void __launch_bounds__(kOpeningThreads) k_check_openings(
+    const uint32_t *__restrict__ proof, size_t at, int width, int depth,
+    const uint64_t *__restrict__ idx, int nq, const f128 *__restrict__ eqr, B3Root root,
+    f128 *__restrict__ vals, unsigned int *bad) {
+  const uint32_t IV[8] = {0x6A09E667, 0xBB67AE85, 0x3C6EF372, 0xA54FF53A,
+                          0x510E527F, 0x9B05688C, 0x1F83D9AB, 0x5BE0CD19};
+  const int q = (blockIdx.x * kOpeningThreads + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (q >= nq) return;
+  const uint32_t *row = proof + at + (size_t)q * (4 * width + 8 * depth);
+  wide sum = wzero();
+  for (int c = lane; c < width; c += 32) {
+    const uint32_t *p = row + 4 * c;
+    wacc(sum, gmul_wide(mk((uint64_t)p[0] | (uint64_t)p[1] << 32, (uint64_t)p[2] | (uint64_t)p[3] << 32),
+                        ld(eqr + c)));
+  }
+  f128 v = greduce(sum);
+  for (int off = 16; off > 0; off >>= 1) {
+    v.lo ^= __shfl_xor_sync(0xffffffffu, v.lo, off);
+    v.hi ^= __shfl_xor_sync(0xffffffffu, v.hi, off);
+  }
+  if (lane) return;
+  st(vals + q, v);
+  uint32_t cv[8], m[16];
+  for (int j = 0; j < 8; j++) cv[j] = IV[j];
+  const int nblk = (16 * width + 63) / 64;
+  for (int b = 0; b < nblk; b++) {
+    const int left = 4 * width - 16 * b;
+    for (int j = 0; j < 16; j++) m[j] = j < left ? row[16 * b + j] : 0;
+    const uint32_t fl = (b == 0 ? B3_CHUNK_START : 0) | (b == nblk - 1 ? B3_CHUNK_END | B3_ROOT : 0);
+    b3_compress(cv, m, 0, (uint32_t)(left < 16 ? 4 * left : 64), fl, cv);
+  }
+  const uint32_t *sib = row + 4 * width;
+  uint64_t node = idx[q];
+  for (int d = 0; d < depth; d++, sib += 8, node >>= 1) {
+    for (int j = 0; j < 8; j++) {
+      m[(node & 1 ? 0 : 8) + j] = sib[j];
+      m[(node & 1 ? 8 : 0) + j] = cv[j];
+    }
+    b3_compress(IV, m, 0, 64, B3_CHUNK_START | B3_CHUNK_END | B3_ROOT, cv);
+  }
+  uint32_t diff = 0;
+  for (int j = 0; j < 8; j++) diff |= cv[j] ^ root.w[j];
+  if (diff) *bad = 1;
+}
+
+void check_openings(const uint32_t *proof, size_t at, int width, int depth, const uint64_t *idx,
+                    int nq, const f128 *eqr, const B3Root &root, f128 *vals, unsigned int *bad,
+                    cudaStream_t s) {
+  if (16 * width > 1024) throw CudaError("check_openings: a row longer than one hash chunk");
+  k_check_openings<<<(32 * nq + kOpeningThreads - 1) / kOpeningThreads, kOpeningThreads, 0, s>>>(
+      proof, at, width, depth, idx, nq, eqr, root, vals, bad);
+  BZ_LAUNCH_CHECK();
+}
+
 void merkle_build(const f128 *cw, size_t rows, int k, uint32_t *nodes, cudaStream_t s) {
   k_merkle_leaves<<<grid_for(rows), kThreads, 0, s>>>(cw, rows, k, nodes);
   BZ_LAUNCH_CHECK();
@@ -777,6 +838,7 @@ void preload_pcs_kernels() {
                 (const void *)k_b3_chunks,
                 (const void *)k_b3_parents,
                 (const void *)k_b3_top,
+                (const void *)k_check_openings,
                 (const void *)k_ring_claims,
                 (const void *)k_packed_basis,
                 (const void *)k_dot,

@@ -53,6 +53,17 @@ void query_basis(const uint64_t *idx, const f128 *wh, const f128 *scale, int nq,
 void gather_openings(const f128 *cw, const uint32_t *nodes, size_t rows, int width, int depth,
                      const uint64_t *idx, int nq, f128 *out, cudaStream_t s);
 
+// A level's openings in a proof: `at` counts 32-bit words from `proof`, each of
+// the nq openings is the row (width 16-byte entries) and `depth` siblings.
+// vals[q] = sum over the row of entry c times eqr[c]; *bad is set (it starts
+// zero) when a path from leaf idx[q] does not reach the root.
+struct B3Root {
+  uint32_t w[8];
+};
+void check_openings(const uint32_t *proof, size_t at, int width, int depth, const uint64_t *idx,
+                    int nq, const f128 *eqr, const B3Root &root, f128 *vals, unsigned int *bad,
+                    cudaStream_t s);
+
 // Host helpers (GF(2^128) on the CPU for the few scalar steps).
 f128 gf_inv_host(f128 a);
 // wh[t * kMaxRsDim + s] = Wh_t(X^s): the normalised subspace polynomial of

@@ -57,6 +57,14 @@ struct Workspace {
   DeviceBuffer<f128> lig_cw[2], openings;
   DeviceBuffer<uint32_t> lig_nodes[2];
   DeviceBuffer<uint64_t> qidx;
+  // the verifier: the hint bytes, the openings' combinations and each level's
+  // path flag
+  DeviceBuffer<uint32_t> v_hints;
+  DeviceBuffer<f128> v_vals, v_eqr;
+  DeviceBuffer<unsigned int> v_bad;
+  PinnedBuffer<uint32_t> pin_hints;
+  PinnedBuffer<f128> pin_vals;
+  PinnedBuffer<unsigned int> pin_bad;
   PinnedBuffer<uint64_t> pin_idx;
   PinnedBuffer<f128> pin_open, pin_f, pin_b, pin_qw, pin_small;
   // the proof's own state: the staged statement, the witness, the level-0

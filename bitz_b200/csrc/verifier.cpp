@@ -199,13 +199,6 @@ f128 advance(f128 claim, f128 a0, f128 a2, f128 r) {
   return gadd(a0, gmul(r, gadd(gadd(claim, a2), gmul(r, a2))));
 }
 
-// BLAKE3 of one message, default mode.
-void blake3_once(const uint8_t *in, size_t len, uint8_t out[32]) {
-  Blake3 h;
-  h.update(in, len);
-  h.finalize(out);
-}
-
 }  // namespace
 
 // One failed check: its message, and the reference's verification error.
@@ -607,6 +600,45 @@ int ProofSystem::verify(const uint8_t *proof, size_t proof_len, Context *lane) {
   t.public_message("flock-ligerito-basis-v0", 23);
   t.public_f128(ptarget);
   f128 lclaim = ptarget;
+  // Every level's openings are checked on the device while the replay goes on:
+  // nothing that is absorbed depends on them. A level's combined openings enter
+  // the claim with the product of the fold challenges drawn after it.
+  size_t total_queries = 0;
+  for (int i = 0; i < cfg.nlevels; i++) total_queries += (size_t)cfg.levels[i].queries;
+  struct Opened {
+    std::vector<f128> weights;
+    size_t first;
+    f128 mult;
+  };
+  std::vector<Opened> opened;
+  size_t opened_queries = 0;
+  const size_t hint_words = (hs.len + 3) / 4;
+  {
+    uint32_t *ph = W.pin_hints.get(hint_words);
+    memcpy(ph, hs.p, hs.len);
+    W.v_hints.upload(ph, hint_words, s);
+    W.v_vals.resize(total_queries);
+    W.v_bad.resize((size_t)cfg.nlevels);
+    BZ_CUDA(cudaMemsetAsync(W.v_bad.get(), 0, sizeof(unsigned int) * (size_t)cfg.nlevels, s));
+  }
+  // the levels' path flags so far (waits for the device)
+  auto paths_hold = [&] {
+    unsigned int *bad = W.pin_bad.get((size_t)cfg.nlevels);
+    BZ_CUDA(cudaMemcpyAsync(bad, W.v_bad.get(), sizeof(unsigned int) * (size_t)cfg.nlevels,
+                            cudaMemcpyDeviceToHost, s));
+    BZ_CUDA(stream_wait(s));
+    bool ok = true;
+    for (size_t k = 0; k < opened.size(); k++) ok &= !bad[k];
+    return ok;
+  };
+// A failed check of the opening: an earlier level's path comes before it.
+#define BZ_VERIFY_OPENING(cond, what)                                                  \
+  do {                                                                                 \
+    if (!(cond)) {                                                                     \
+      error = paths_hold() ? (what) : "a Merkle path does not reach the root";         \
+      return BZ_ERR_VERIFY;                                                            \
+    }                                                                                  \
+  } while (0)
   uint8_t cur_root[32];
   memcpy(cur_root, root, 32);
   int cur_k = cfg.levels[0].k, cur_rate = cfg.levels[0].log_inv_rate, cur_log_n = log_n;
@@ -619,10 +651,11 @@ int ProofSystem::verify(const uint8_t *proof, size_t proof_len, Context *lane) {
     PassBind pb{};
     for (int r = 0; r < L.k; r++) {
       const f128 a0 = rd.f(), a2 = rd.f();
-      BZ_VERIFY(lig_grind(), "Ligerito fold grinding nonce");
+      BZ_VERIFY_OPENING(lig_grind(), "Ligerito fold grinding nonce");
       const f128 c = t.challenge_f128();
       rs.push_back(c);
       lclaim = advance(lclaim, a0, a2, c);
+      for (auto &o : opened) o.mult = gmul(o.mult, c);
       pb.r[pb.k++] = c;
       if (pb.k < kPassMaxK && r + 1 < L.k) continue;
       // the basis folds at up to three challenges at once
@@ -638,7 +671,7 @@ int ProofSystem::verify(const uint8_t *proof, size_t proof_len, Context *lane) {
       const PcsLevel &N = cfg.levels[i + 1];
       uint8_t rb[36];
       rd.take(rb, 36);
-      BZ_VERIFY(!rd.short_read && rb[0] == 32 && !rb[1] && !rb[2] && !rb[3],
+      BZ_VERIFY_OPENING(!rd.short_read && rb[0] == 32 && !rb[1] && !rb[2] && !rb[3],
                 "a Ligerito level's root");
       memcpy(next_root, rb + 4, 32);
       if (N.ood_samples) {
@@ -654,61 +687,48 @@ int ProofSystem::verify(const uint8_t *proof, size_t proof_len, Context *lane) {
       rd.take(nb, 4);
       const uint32_t fl = (uint32_t)nb[0] | ((uint32_t)nb[1] << 8) | ((uint32_t)nb[2] << 16) |
                           ((uint32_t)nb[3] << 24);
-      BZ_VERIFY(!rd.short_read && fl == (1u << l), "the final vector's length");
+      BZ_VERIFY_OPENING(!rd.short_read && fl == (1u << l), "the final vector's length");
       f_final.resize(fl);
       for (auto &x : f_final) x = rd.f();
     }
-    BZ_VERIFY(lig_grind(), "Ligerito query grinding nonce");
+    BZ_VERIFY_OPENING(lig_grind(), "Ligerito query grinding nonce");
     const std::vector<f128> qs = sample_vec((size_t)L.queries);
     const size_t rows = (size_t)1 << (cur_log_n - cur_k + cur_rate);
     const int width = 1 << cur_k, depth = ceil_log2(rows);
     const uint8_t *qh = hs.take(8);
-    BZ_VERIFY(qh, "the hint stream ends before a level's openings");
+    BZ_VERIFY_OPENING(qh, "the hint stream ends before a level's openings");
     uint64_t nq = 0;
     for (int k = 7; k >= 0; k--) nq = (nq << 8) | qh[k];
-    BZ_VERIFY(nq == (uint64_t)L.queries, "a level's query count");
+    BZ_VERIFY_OPENING(nq == (uint64_t)L.queries, "a level's query count");
     std::vector<f128> eqr((size_t)1 << L.k);
     eq_table_host(rs.data(), L.k, eqr.data());
-    std::vector<f128> vals(L.queries);
     std::vector<uint64_t> idx(L.queries);
-    for (int qi = 0; qi < L.queries; qi++) {
-      idx[qi] = qs[qi].lo & (rows - 1);
-      const uint8_t *row = hs.take((size_t)width * 16);
-      BZ_VERIFY(row, "the hint stream ends inside an opened row");
-      uint8_t node[32];
-      blake3_once(row, (size_t)width * 16, node);
-      size_t at_node = rows + idx[qi];
-      for (int d = 0; d < depth; d++) {
-        const uint8_t *sib = hs.take(32);
-        BZ_VERIFY(sib, "the hint stream ends inside a Merkle path");
-        uint8_t pair[64];
-        memcpy(pair, (at_node & 1) ? sib : node, 32);
-        memcpy(pair + 32, (at_node & 1) ? node : sib, 32);
-        blake3_once(pair, 64, node);
-        at_node >>= 1;
-      }
-      BZ_VERIFY(memcmp(node, cur_root, 32) == 0, "a Merkle path does not reach the root");
-      wide acc = wzero();
-      for (int c = 0; c < width; c++) {
-        f128 e;
-        memcpy(&e, row + 16 * c, 16);
-        wacc(acc, gmul_wide(e, eqr[c]));
-      }
-      vals[qi] = greduce(acc);
+    for (int qi = 0; qi < L.queries; qi++) idx[qi] = qs[qi].lo & (rows - 1);
+    const size_t level_at = hs.pos, row_bytes = (size_t)width * 16;
+    const size_t whole = (hs.len - hs.pos) / (row_bytes + 32 * (size_t)depth);
+    if (whole < (size_t)L.queries) {  // the stream ends at an opening's row or path
+      const size_t rest = hs.len - hs.pos - whole * (row_bytes + 32 * (size_t)depth);
+      BZ_VERIFY_OPENING(rest >= row_bytes, "the hint stream ends inside an opened row");
+      BZ_VERIFY_OPENING(false, "the hint stream ends inside a Merkle path");
     }
+    hs.take((size_t)L.queries * (row_bytes + 32 * (size_t)depth));
+    W.qidx.upload(idx.data(), idx.size(), s);
+    W.v_eqr.upload(eqr.data(), eqr.size(), s);
+    B3Root want;
+    b3_load_le(cur_root, want.w, 8);
+    check_openings(W.v_hints.get(), level_at / 4, width, depth, W.qidx.get(), L.queries,
+                   W.v_eqr.get(), want, W.v_vals.get() + opened_queries, W.v_bad.get() + i, s);
     const int av = ceil_log2((size_t)L.queries);
     const std::vector<f128> alpha = sample_vec((size_t)av);
     const f128 mu = t.challenge_f128();
     std::vector<f128> beta((size_t)1 << av), sq(L.queries);
     eq_table_host(alpha.data(), av, beta.data());
-    for (int qi = 0; qi < L.queries; qi++) {
-      sq[qi] = gmul(mu, beta[qi]);
-      lclaim = gadd(lclaim, gmul(sq[qi], vals[qi]));
-    }
+    for (int qi = 0; qi < L.queries; qi++) sq[qi] = gmul(mu, beta[qi]);
     // the glue on the device: basis += sum_q s_q X(x_q)
-    W.qidx.upload(idx.data(), idx.size(), s);
     W.qs.upload(sq.data(), sq.size(), s);
     query_basis(W.qidx.get(), T.wh.get(), W.qs.get(), L.queries, l, b, s);
+    opened.push_back(Opened{std::move(sq), opened_queries, kOne});
+    opened_queries += (size_t)L.queries;
     if (!last) {
       memcpy(cur_root, next_root, 32);
       cur_log_n = l;
@@ -716,16 +736,25 @@ int ProofSystem::verify(const uint8_t *proof, size_t proof_len, Context *lane) {
       cur_rate = cfg.levels[i + 1].log_inv_rate;
     }
   }
-  BZ_VERIFY(!rd.short_read, "the proof ends inside the opening");
+  BZ_VERIFY_OPENING(!rd.short_read, "the proof ends inside the opening");
   {
     std::vector<f128> hb(n);
+    f128 *vals = W.pin_vals.get(total_queries);
+    BZ_CUDA(cudaMemcpyAsync(vals, W.v_vals.get(), total_queries * 16, cudaMemcpyDeviceToHost, s));
     BZ_CUDA(cudaMemcpyAsync(hb.data(), b, n * 16, cudaMemcpyDeviceToHost, s));
-    BZ_CUDA(stream_wait(s));
+    BZ_VERIFY(paths_hold(), "a Merkle path does not reach the root");
+    for (const auto &o : opened) {
+      wide sum = wzero();
+      for (size_t q = 0; q < o.weights.size(); q++)
+        wacc(sum, gmul_wide(o.weights[q], vals[o.first + q]));
+      lclaim = gadd(lclaim, gmul(o.mult, greduce(sum)));
+    }
     BZ_VERIFY(f_final.size() == n, "the final vector's length");
     wide chk = wzero();
     for (size_t j = 0; j < n; j++) wacc(chk, gmul_wide(hb[j], f_final[j]));
     BZ_VERIFY(geq(greduce(chk), lclaim), "the final vector against its basis");
   }
+#undef BZ_VERIFY_OPENING
   // both streams spent (crates/verifier/src/verify.rs:69-71, check_eof)
   BZ_VERIFY(rd.pos == rd.len && hs.pos == hs.len, "leftover proof bytes");
   return BZ_OK;
