@@ -138,6 +138,14 @@ size_t bitz_transcript_hints(const bitz_transcript *t, uint8_t *out, size_t cap)
 
 // ------------------------------------------------------------- post-GKR
 
+// The host arrays' device copies stay with the lane (up to a bound) when the
+// call that filled them returns or throws.
+struct HeldInputs {
+  Context &ctx;
+  explicit HeldInputs(Context &c) : ctx(c) {}
+  ~HeldInputs() { ctx.release_inputs(); }
+};
+
 static int post_gkr_common(const f128 *rows, int log_rows, const f128 *cols, int log_cols,
                            const uint64_t target[2], const f128 *packed, uint32_t security_bits,
                            bitz_transcript *t, uint64_t *point_out, uint64_t value_out[2]) {
@@ -187,12 +195,12 @@ int bitz_post_gkr_prove(const uint64_t *rows, int log_rows, const uint64_t *cols
     Context &ctx = Context::get();
     size_t nr = (size_t)1 << log_rows, nc = (size_t)1 << log_cols;
     size_t np = (nr >> 7) * nc;
-    DeviceBuffer<f128> d_rows(nr), d_cols(nc), d_packed(np);
-    d_rows.upload((const f128 *)rows, nr, ctx.stream());
-    d_cols.upload((const f128 *)cols, nc, ctx.stream());
-    d_packed.upload((const f128 *)packed, np, ctx.stream());
-    return post_gkr_common(d_rows.get(), log_rows, d_cols.get(), log_cols, target, d_packed.get(),
-                           security_bits, t, point_out, value_out);
+    HeldInputs held(ctx);
+    ctx.in_a.upload((const f128 *)rows, nr, ctx.stream());
+    ctx.in_b.upload((const f128 *)cols, nc, ctx.stream());
+    ctx.in_c.upload((const f128 *)packed, np, ctx.stream());
+    return post_gkr_common(ctx.in_a.get(), log_rows, ctx.in_b.get(), log_cols, target,
+                           ctx.in_c.get(), security_bits, t, point_out, value_out);
   });
 }
 
@@ -279,10 +287,10 @@ int bitz_gkr_prove(const uint64_t *row_images, const uint64_t *columns, int log_
   return guarded([&] {
     Context &ctx = Context::get();
     size_t nc = (size_t)1 << log_cols;
-    DeviceBuffer<f128> d_img(128), d_cols(nc);
-    d_img.upload((const f128 *)row_images, 128, ctx.stream());
-    d_cols.upload((const f128 *)columns, nc, ctx.stream());
-    return gkr_common(d_img.get(), d_cols.get(), log_cols, zeta, security_bits, t, point_out,
+    HeldInputs held(ctx);
+    ctx.in_a.upload((const f128 *)row_images, 128, ctx.stream());
+    ctx.in_b.upload((const f128 *)columns, nc, ctx.stream());
+    return gkr_common(ctx.in_a.get(), ctx.in_b.get(), log_cols, zeta, security_bits, t, point_out,
                       claim_out);
   });
 }
@@ -306,12 +314,12 @@ int bitz_gkr_outputs(const uint64_t *row_images, const uint64_t *columns, int lo
   return guarded([&] {
     Context &ctx = Context::get();
     size_t nc = (size_t)1 << log_cols;
-    DeviceBuffer<f128> d_img(128), d_cols(nc);
-    d_img.upload((const f128 *)row_images, 128, ctx.stream());
-    d_cols.upload((const f128 *)columns, nc, ctx.stream());
+    HeldInputs held(ctx);
+    ctx.in_a.upload((const f128 *)row_images, 128, ctx.stream());
+    ctx.in_b.upload((const f128 *)columns, nc, ctx.stream());
     GkrScratch &sc = ctx.gkr_scratch(log_cols);
     sc.live_cols = 0;
-    gkr_build(d_cols.get(), log_cols, d_img.get(), sc, ctx.stream());
+    gkr_build(ctx.in_b.get(), log_cols, ctx.in_a.get(), sc, ctx.stream());
     BZ_CUDA(cudaMemcpyAsync(out, sc.layer[7], nc * 16, cudaMemcpyDeviceToHost, ctx.stream()));
     BZ_CUDA(cudaStreamSynchronize(ctx.stream()));
     return BZ_OK;

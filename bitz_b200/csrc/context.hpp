@@ -129,6 +129,15 @@ class Context {
     return pg_;
   }
 
+  // Device copies of a call's host arrays, kept between calls so that a call
+  // allocates nothing; release_inputs gives them back when they are large.
+  DeviceBuffer<f128> in_a, in_b, in_c;
+  static constexpr size_t kKeptInput = (size_t)1 << 22;  // entries: 64 MiB
+  void release_inputs() {
+    for (DeviceBuffer<f128> *b : {&in_a, &in_b, &in_c})
+      if (b->size() > kKeptInput) b->release();
+  }
+
   GkrScratch &gkr_scratch(int s) {
     size_t leaves = (size_t)128 << s;
     if (gk_.capacity < leaves) {
