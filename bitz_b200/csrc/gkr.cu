@@ -35,6 +35,7 @@
 #include "context.hpp"
 #include "eq.cuh"
 #include "gkr.hpp"
+#include "host_tail.hpp"
 #include "passes.cuh"
 
 namespace bz {
@@ -525,9 +526,10 @@ __global__ void __launch_bounds__(kThreads) gkr_bound_rows(const f128 *__restric
   }
 }
 
-// Tables of this many entries or fewer (per half) go to the host: a round on
-// them costs the host a few microseconds, a device turn about 14.
-constexpr int kHostLog = 8;
+// Tables of this many entries or fewer (per half) go to the host: all rounds on
+// 2^10 entries cost it about 8 us and their way there 8 more than one of 2^7,
+// a device turn of three rounds about 20.
+constexpr int kHostLog = 10;
 static_assert(4 << kHostLog <= kHandoverWords, "the last tables fit one handover");
 // A layer's first pass binds nothing, so three rounds of it make 4.4 products
 // per entry where two make 3.25 (and leave a table 4 times the size for the
@@ -652,21 +654,13 @@ struct LayerRounds {
   // The remaining n rounds on tables of 2^n entries; leaves the bound pair.
   void from_tables(f128 *L, f128 *R, int n, const f128 *eq_prefix, f128 out[2]) {
     for (int i = n - 1; i >= 0; i--) {
-      const int h = 1 << i;
-      const f128 *e = eq_prefix + h;  // eq over the i coordinates below
-      const bool one = gis_zero(point[i]);
-      wide sb = wzero(), si = wzero();
-      for (int x = 0; x < h; x++) {
-        const f128 lb = one ? L[x + h] : L[x], rb = one ? R[x + h] : R[x];
-        wacc(sb, gmul_wide(gmul(e[x], lb), rb));
-        wacc(si, gmul_wide(gmul(e[x], gadd(L[x], L[x + h])), gadd(R[x], R[x + h])));
-      }
-      const f128 b = greduce(sb);
-      const f128 r = round(i, b, b, greduce(si));
-      for (int x = 0; x < h; x++) {
-        L[x] = gadd(L[x], gmul(r, gadd(L[x], L[x + h])));
-        R[x] = gadd(R[x], gmul(r, gadd(R[x], R[x + h])));
-      }
+      const size_t h = (size_t)1 << i;
+      f128 sums[2];
+      // eq_prefix + h: eq over the i coordinates below
+      host_cubic_sums(eq_prefix + h, L, R, h, gis_zero(point[i]), sums);
+      const f128 r = round(i, sums[0], sums[0], sums[1]);
+      host_bind_high(L, h, r);
+      host_bind_high(R, h, r);
     }
     out[0] = L[0];
     out[1] = R[0];
@@ -793,7 +787,10 @@ f128 gkr_prove(const f128 *cols, int s, const f128 *images, const f128 *zeta, ui
       R[k] = mk(words[2 * (len + k)], words[2 * (len + k) + 1]);
     }
     f128 lr[2];
-    rounds.from_tables(L.data(), R.data(), rem, heap[0].v, lr);
+        std::vector<f128> prefix((size_t)1 << std::max(1, rem));
+    prefix[1] = mk(1, 0);
+    for (int i = 0; i + 1 < rem; i++) eq_double(prefix.data() + ((size_t)1 << i), (size_t)1 << i, point[i]);
+    rounds.from_tables(L.data(), R.data(), rem, prefix.data(), lr);
     ts.prover_message(lr, 32);
     const f128 t = ts.challenge_f128();
     next[n] = t;

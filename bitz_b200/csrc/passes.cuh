@@ -5,6 +5,7 @@
 #include <vector>
 
 #include "device.cuh"
+#include "host_tail.hpp"
 
 namespace bz {
 
@@ -30,21 +31,20 @@ struct EqFactors {
   f128 f[NF][1 << kFacLog];
 };
 
+// From eq over some coordinates at p[0, n) to eq over one more, z, at p[n, 3n).
+inline void eq_double(f128 *p, size_t n, f128 z) {
+  f128 *q = p + n;
+  host_scale(p, z, n, q + n);
+  for (size_t k = 0; k < n; k++) q[k] = gadd(p[k], q[k + n]);
+}
+
 // Prefix tables of eq over up to kFacLog coordinates: entries [2^i, 2^(i+1))
 // hold eq over the first i of them.
 struct EqHeap {
   f128 v[2 << kFacLog];
   void build(const f128 *z, int n) {
     v[1] = mk(1, 0);
-    for (int i = 0; i < n; i++) {
-      const f128 *p = v + ((size_t)1 << i);
-      f128 *q = v + ((size_t)2 << i);
-      for (int k = 0; k < 1 << i; k++) {
-        const f128 one = gmul(p[k], z[i]);
-        q[k] = gadd(p[k], one);
-        q[k + (1 << i)] = one;
-      }
-    }
+    for (int i = 0; i < n; i++) eq_double(v + ((size_t)1 << i), (size_t)1 << i, z[i]);
   }
   const f128 *prefix(int n) const { return v + ((size_t)1 << n); }
 };
@@ -91,7 +91,7 @@ inline int pass_tile_log(uint32_t count) {
 // Few blocks post their sums by themselves (the host adds them up) instead of
 // through atomics and a last block: three trips to the L2 less, 1.4 us.
 __host__ __device__ inline bool pass_direct(unsigned int grid, int words) {
-  return grid * (unsigned int)words <= (unsigned int)kHandoverWords;
+  return grid * (unsigned int)words <= 1536u;
 }
 // Adds the blocks' words up into the first `words`.
 inline void pass_combine(uint64_t *w, int words, int blocks) {

@@ -21,12 +21,13 @@
 #include <vector>
 
 #include "context.hpp"
+#include "host_tail.hpp"
 #include "post_gkr.hpp"
 
 namespace bz {
 
 // Tables of this many entries or fewer go to the host.
-constexpr int kHostLog = 8;
+constexpr int kHostLog = 10;
 static_assert(4 << kHostLog <= kHandoverWords, "the last tables fit one handover");
 
 // Y for few columns: a thread per row, its bit of every column.
@@ -510,16 +511,11 @@ struct PostGkrRun {
     }
     if (!claim_holds(greduce(total))) return BZ_ERR_CLAIM;
     for (int len = n / 2; len > 0; len /= 2) {
-      wide a0 = wzero(), a2 = wzero();
-      for (int j = 0; j < len; j++) {
-        wacc(a0, gmul_wide(W[2 * j], V[2 * j]));
-        wacc(a2, gmul_wide(gadd(W[2 * j], W[2 * j + 1]), gadd(V[2 * j], V[2 * j + 1])));
-      }
-      const f128 r = round(greduce(a0), greduce(a2));
-      for (int o = 0; o < len; o++) {
-        W[o] = gadd(W[2 * o], gmul(r, gadd(W[2 * o], W[2 * o + 1])));
-        V[o] = gadd(V[2 * o], gmul(r, gadd(V[2 * o], V[2 * o + 1])));
-      }
+      f128 sums[2];
+      host_quad_sums(W.data(), V.data(), len, sums);
+      const f128 r = round(sums[0], sums[1]);
+      host_bind_low(W.data(), len, r);
+      host_bind_low(V.data(), len, r);
     }
     out[0] = W[0];
     out[1] = V[0];

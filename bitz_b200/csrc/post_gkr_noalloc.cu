@@ -27,7 +27,7 @@
 namespace bz {
 
 // Largest claim served: 2^20 bits (log_rows + log_cols <= 20), so four tables
-// of 2^19 F128 each (32 MiB), and the passes' sums with their slots (26 KiB).
+// of 2^19 F128 each (32 MiB), and the passes' sums with their slots (66 KiB).
 constexpr int kNoAllocMaxLogBits = 20;
 constexpr size_t kNoAllocTable = (size_t)1 << (kNoAllocMaxLogBits - 1);
 

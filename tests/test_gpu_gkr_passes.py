@@ -58,3 +58,36 @@ def test_zero_and_one_coordinates(s, at):
     gt = bz.build_prover(b"z", b"z")
     _, gclaim = bz.gkr_prove(images, cols, zeta, 100, gt)
     assert gt.narg() == ot.narg() and np.array_equal(gclaim, oclaim)
+
+
+def test_scalar_host_rounds_give_the_same_transcript():
+    """BITZ_HOST_SIMD=0 runs the host's last rounds with one product at a time."""
+    import hashlib
+    import os
+    import subprocess
+    import sys
+    code = """
+import hashlib
+import numpy as np
+import bitz_b200 as bz
+from oracle import ffi as of
+rng = np.random.default_rng(12)
+draw = lambda n: rng.integers(0, 2**64, size=(n, 2), dtype=np.uint64)
+h = hashlib.sha256()
+for s in (1, 2, 9, 11):
+    t = bz.build_prover(b"simd", b"gkr")
+    bz.gkr_prove(draw(128), draw(1 << s), draw(s), 100, t)
+    h.update(t.narg())
+of.lib().o_set_clmul_mode(1)
+for lr, lc in ((8, 0), (13, 0), (7, 1), (7, 9)):
+    rows, cols, packed = draw(1 << lr), draw(1 << lc), draw(1 << (lr + lc - 7))
+    t = bz.build_prover(b"simd", b"post")
+    bz.post_gkr_prove(rows, cols, of.weighted_sum(rows, cols, packed), packed, 100, t)
+    h.update(t.narg())
+print(h.hexdigest())
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    got = [subprocess.run([sys.executable, "-c", code], cwd=root, check=True, capture_output=True,
+                          text=True, env=dict(os.environ, BITZ_HOST_SIMD=flag)).stdout.strip()
+           for flag in ("0", "1")]
+    assert got[0] == got[1] and len(got[0]) == 2 * hashlib.sha256().digest_size
