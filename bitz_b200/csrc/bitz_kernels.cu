@@ -114,17 +114,20 @@ __global__ void k_mt_col0(const uint32_t *__restrict__ off, const uint32_t *__re
 }
 
 // The dense eq table of the rows, dense[lo << log_u2 | hi] = u1[lo] * u2[hi]
-// (row r = hi * 128 + lo): block (lo, part) takes a slice of hi through
-// u1[lo]'s window table, writing along hi.
-constexpr int kMtParts = 2;
-__global__ void k_mt_dense(const f128 *__restrict__ u1, const f128 *__restrict__ u2, int log_u2,
-                           f128 *__restrict__ dense) {
+// (row r = hi * 128 + lo), for the `live` values of hi that rows exist for:
+// block (lo, part) takes a slice of hi through u1[lo]'s window table, writing
+// along hi. Bound by the table lookups (72 G/s), so rows that are only padding
+// are left out (38 % of them at 64 and 1024 blocks, 98 % at one) and the slices
+// are as many as keep the SMs level.
+__global__ void __launch_bounds__(kThreads) k_mt_dense(const f128 *__restrict__ u1,
+                                                       const f128 *__restrict__ u2, int log_u2,
+                                                       size_t live, f128 *__restrict__ dense) {
   __shared__ MulTable T;
-  const int lo = blockIdx.x / kMtParts, part = blockIdx.x % kMtParts;
+  const int lo = blockIdx.x;
   mul_table_build(T, ld(u1 + lo));
-  const size_t per = ((size_t)1 << log_u2) / kMtParts;
   f128 *out = dense + ((size_t)lo << log_u2);
-  for (size_t hi = part * per + threadIdx.x; hi < (part + 1) * per; hi += blockDim.x)
+  for (size_t hi = blockIdx.y * (size_t)kThreads + threadIdx.x; hi < live;
+       hi += (size_t)gridDim.y * kThreads)
     st(out + hi, mul_table(T, ld(u2 + hi)));
 }
 
@@ -147,9 +150,11 @@ __global__ void k_mt_gather(const uint32_t *__restrict__ off, const uint32_t *__
 
 void mt_transpose(const uint32_t *off, const uint32_t *row, size_t ncols, const f128 *u1,
                   const f128 *u2, f128 *weights, size_t padded, f128 *w0, cudaStream_t s,
-                  f128 *dense, int log_u2) {
+                  f128 *dense, int log_u2, size_t rows) {
   if (dense && log_u2 >= 8) {
-    k_mt_dense<<<128 * kMtParts, kThreads, 0, s>>>(u1, u2, log_u2, dense);
+    const size_t live = (rows + 127) / 128;
+    const dim3 grid(128, grid_for(live, kThreads, 8));
+    k_mt_dense<<<grid, kThreads, 0, s>>>(u1, u2, log_u2, live, dense);
     BZ_LAUNCH_CHECK();
     k_mt_gather<<<grid_for(padded + 1), kThreads, 0, s>>>(off, row, ncols, dense, log_u2, weights,
                                                           padded);

@@ -151,9 +151,10 @@ class Context {
         off += leaves >> j;
       }
       gk_gram_.resize(gkr_gram_words());
-      gk_mid_.resize(2304);
+      gk_mid_.resize(2304 + (1 << 14));
       gk_.gram = gk_gram_.get();
       gk_.mid = gk_mid_.get();
+      gk_.eq_low = gk_mid_.get() + 2304;
       gk_.capacity = leaves;
     }
     return gk_;

@@ -119,108 +119,163 @@ __global__ void __launch_bounds__(128) gkr_high_layers(const f128 *__restrict__ 
 // the same position of the higher blocks (same column, or a higher one below
 // 2^s), so a pass leaves those positions out: they add eq(x) to F at the points
 // without infinity and nothing at the others.
+// eq over the lowest 14 coordinates, the product of the first two factors, for
+// passes over more: one product per position instead of one per factor.
+constexpr int kEqLowLog = 2 * kFacLog;
+__global__ void __launch_bounds__(kThreads) gkr_eq_low(const __grid_constant__ EqFactors<2> eq,
+                                                       f128 *__restrict__ out) {
+  const int x = blockIdx.x * kThreads + threadIdx.x;
+  st(out + x, gmul(eq.f[0][x & ((1 << kFacLog) - 1)], eq.f[1][x >> kFacLog]));
+}
+
 // One pass. Binds the coordinates of `b` (in place: the entry at pos comes from
 // pos + j N), then sums the 3^K points over the live positions of the 2^log_m
 // below the top K coordinates, and the eq weights of those positions. The last
 // block posts the 3^K + 1 sums as handover publication seq.
 //
-// A block works tiles of X = 2^lx positions: the 2 2^K X bound entries (and
-// the X weights) one per thread into shared memory, the 2^K X products of the
-// weights with L, then the 3^K X wide products, whose sums stay in registers
-// (thread t of turn q always has the same point). X shrinks with the number of
-// positions, so that a small pass still spreads over the SMs.
-template <int K, int NF>
-__global__ void __launch_bounds__(kPassThreads, 2) gkr_pass(
-    f128 *__restrict__ c, size_t n_half, int log_m, PassBind b,
-    const __grid_constant__ EqFactors<NF> eq, size_t colmask, uint32_t live, uint32_t count,
-    int lx, PassPost post) {
+// A block works tiles of X = 2^lx positions: the 2 2^K X bound entries, one per
+// thread into shared memory, the 2^K X products of the weights with L, then the
+// 3^K X wide products, whose sums stay in registers (thread t of turn q always
+// has the same point). A tenth warp forms the next tile's weights meanwhile: in
+// line, their two or three dependent products left nine warps waiting for half
+// of a tile's time (layer of 2^22 entries, first pass: 618 us). X shrinks with
+// the number of positions, so that a small pass still spreads over the SMs; the
+// first pass of a large layer (K = 2, nothing to bind) takes tiles of 64, which
+// fill its turns. kLow: the weights' lowest 14 coordinates come from eq_low.
+template <int K, bool kLow>
+struct PassShape {
+  static constexpr int kMaxLx = K == 2 ? 6 : 5, kMaxX = 1 << kMaxLx;
+  static constexpr int kFactors = kLow ? 3 : 2, kBlocksPerSm = K == 2 ? 3 : 2;
+  static constexpr int kThreadsAll = kPassThreads + 32;
+};
+
+__device__ __forceinline__ void main_warps_sync() {
+  asm volatile("bar.sync 1, %0;" ::"n"(kPassThreads) : "memory");
+}
+
+template <int K, bool kLow>
+__global__ void __launch_bounds__(PassShape<K, kLow>::kThreadsAll, PassShape<K, kLow>::kBlocksPerSm)
+    gkr_pass(f128 *__restrict__ c, size_t n_half, int log_m, PassBind b,
+             const __grid_constant__ EqFactors<PassShape<K, kLow>::kFactors> eq,
+             const f128 *__restrict__ eq_low, size_t colmask, uint32_t live, uint32_t count, int lx,
+             PassPost post) {
+  using S = PassShape<K, kLow>;
   constexpr int kPoints = pow3(K), kBlocks = 1 << K, kWords = 2 * (kPoints + 1);
-  constexpr int kTurns = (kPoints * kPassMaxX + kPassThreads - 1) / kPassThreads;
-  constexpr int kEqWarp = kPassThreads / 32 - 1;  // the warp that forms a tile's weights
-  __shared__ MulTable T[kPassMaxK];
-  __shared__ f128 G[kBlocks * kPassMaxX], R[kBlocks * kPassMaxX], E[kPassMaxX];
+  constexpr int kTurns = (kPoints * S::kMaxX + kPassThreads - 1) / kPassThreads;
+  __shared__ MulTable T[K == 2 ? 1 : kPassMaxK];
+  __shared__ f128 G[kBlocks * S::kMaxX], R[kBlocks * S::kMaxX], E[2][S::kMaxX];
+  __shared__ uint32_t P[2][S::kMaxX];  // a tile's positions; kNone past the last
+  constexpr uint32_t kNone = 0xffffffffu;
   const int t = threadIdx.x;
   const size_t m = (size_t)1 << log_m, n = m << K;
   const int X = 1 << lx;
-  pass_tables(T, b.r, b.k);
+  const bool eq_warp = t >= kPassThreads;
+  if (K > 2) pass_tables(T, b.r, b.k);
   // position of live index i: rows of `live` columns when a block spans whole
   // rows of the column space, else i itself
   const bool by_row = m > colmask;
-  auto position = [&](uint32_t i) -> size_t {
+  auto position = [&](uint32_t i) -> uint32_t {
     if (!by_row) return i;
     const uint32_t row = i / live;
-    return (size_t)row * (colmask + 1) + (i - row * live);
+    return row * (uint32_t)(colmask + 1) + (i - row * live);
+  };
+  auto positions = [&](uint32_t i0, uint32_t *out) {
+    for (int k = t & 31; k < X; k += 32) out[k] = i0 + k < count ? position(i0 + k) : kNone;
+  };
+  f128 sum_e = mk(0, 0);
+  auto weights = [&](const uint32_t *at, f128 *out) {  // a tile's weights
+    for (int k = t & 31; k < X; k += 32) {
+      f128 e = mk(0, 0);
+      const uint32_t x = at[k];
+      if (x != kNone) {
+        constexpr int kMask = (1 << kFacLog) - 1;
+        if (kLow) {
+          e = pass_mul(ld(eq_low + (x & ((1 << kEqLowLog) - 1))),
+                       eq.f[0][(x >> kEqLowLog) & kMask]);
+#pragma unroll 1
+          for (int g = 1; g < S::kFactors && kEqLowLog + g * kFacLog < log_m; g++)
+            e = pass_mul(e, eq.f[g][(x >> (kEqLowLog + g * kFacLog)) & kMask]);
+        } else {
+          e = eq.f[0][x & kMask];
+          if (log_m > kFacLog) e = pass_mul(e, eq.f[1][(x >> kFacLog) & kMask]);
+        }
+      }
+      out[k] = e;
+      sum_e = gadd(sum_e, e);
+    }
   };
   wide sum[kTurns];
 #pragma unroll
   for (int q = 0; q < kTurns; q++) sum[q] = wzero();
-  f128 sum_e = mk(0, 0);
-  for (uint32_t i0 = blockIdx.x << lx; i0 < count; i0 += gridDim.x << lx) {
-    if (t >> 5 == kEqWarp && (t & 31) < X) {
-      const uint32_t i = i0 + (t & 31);
-      f128 e = mk(0, 0);
-      if (i < count) {
-        const size_t x = position(i);
-        e = eq.f[0][x & ((1 << kFacLog) - 1)];
-#pragma unroll 1
-        for (int g = 1; g < NF && g * kFacLog < log_m; g++)
-          e = pass_mul(e, eq.f[g][(x >> (g * kFacLog)) & ((1 << kFacLog) - 1)]);
-      }
-      E[t & 31] = e;
-      sum_e = gadd(sum_e, e);
+  const uint32_t step = gridDim.x << lx;
+  if (eq_warp) positions(blockIdx.x << lx, P[0]);
+  __syncthreads();
+  if (eq_warp) {  // weights of the tile and positions of the next one
+    int buf = 0;
+    weights(P[0], E[0]);
+    for (uint32_t i0 = blockIdx.x << lx; i0 < count; i0 += step, buf ^= 1) {
+      if (i0 + step < count) positions(i0 + step, P[buf ^ 1]);
+      __syncthreads();  // the tile's entries and weights
+      if (i0 + step < count) weights(P[buf ^ 1], E[buf ^ 1]);
     }
-    // entry `slot` (block slot >> lx, position slot mod X) of the tile of L,
-    // then of R
-    const int half = kBlocks << lx;
-    auto entry = [&](int slot, f128 *&at) {
-      const uint32_t i = i0 + (slot & (X - 1));
-      at = nullptr;
-      if (i < count)
-        at = (slot >= half ? c + n_half : c) + position(i) +
-             (size_t)((slot & (half - 1)) >> lx) * m;
-    };
-    if (b.k && lx <= kLaneTileLog) {
-      const int gl = b.k - 1;
-      for (int u = t; u < 2 * half << gl; u += kPassThreads) {
-        const int slot = u >> gl;
-        f128 *at;
-        entry(slot, at);
-        f128 v = pass_bind_lanes<false>(
-            [&](int j) { return at ? ld(at + j * n) : mk(0, 0); }, T, b.k, u & ((1 << gl) - 1));
-        if (u & ((1 << gl) - 1)) continue;
-        if (at) st(at, v);
-        (slot >= half ? R : G)[slot & (half - 1)] = v;
-      }
-    } else {
-      for (int slot = t; slot < 2 * half; slot += kPassThreads) {
-        f128 *at;
-        entry(slot, at);
-        f128 v = mk(0, 0);
-        if (at) {
-          v = pass_bind<false>([&](int j) { return ld(at + j * n); }, T, b.k);
-          if (b.k) st(at, v);
-        }
-        (slot >= half ? R : G)[slot & (half - 1)] = v;
-      }
-    }
-    __syncthreads();
-    for (int u = t; u < half; u += kPassThreads) G[u] = pass_mul(E[u & (X - 1)], G[u]);
-    __syncthreads();
+  } else {
+    int buf = 0;
+    int at_one[kTurns], at_inf[kTurns];  // a turn's point
 #pragma unroll
-    for (int q = 0; q < kTurns; q++) {
-      const int u = t + q * kPassThreads;
-      if (u < kPoints << lx) {
-        int one, inf;
-        point_bits<K, false>(u >> lx, one, inf);
-        const int x = u & (X - 1);
-        wacc(sum[q], pass_wide(point_value(G + x, X, one, inf), point_value(R + x, X, one, inf)));
+    for (int q = 0; q < kTurns; q++)
+      point_bits<K, false>((t + q * kPassThreads) >> lx, at_one[q], at_inf[q]);
+    for (uint32_t i0 = blockIdx.x << lx; i0 < count; i0 += step, buf ^= 1) {
+      // entry `slot` (block slot >> lx, position slot mod X) of the tile of L,
+      // then of R
+      const int half = kBlocks << lx;
+      auto entry = [&](int slot) -> f128 * {
+        const uint32_t x = P[buf][slot & (X - 1)];
+        if (x == kNone) return nullptr;
+        return (slot >= half ? c + n_half : c) + x + (size_t)((slot & (half - 1)) >> lx) * m;
+      };
+      if (K > 2 && b.k && lx <= kLaneTileLog) {
+        const int gl = b.k - 1;
+        for (int u = t; u < 2 * half << gl; u += kPassThreads) {
+          const int slot = u >> gl;
+          f128 *at = entry(slot);
+          f128 v = pass_bind_lanes<false>(
+              [&](int j) { return at ? ld(at + j * n) : mk(0, 0); }, T, b.k, u & ((1 << gl) - 1));
+          if (u & ((1 << gl) - 1)) continue;
+          if (at) st(at, v);
+          (slot >= half ? R : G)[slot & (half - 1)] = v;
+        }
+      } else {
+        for (int slot = t; slot < 2 * half; slot += kPassThreads) {
+          f128 *at = entry(slot);
+          f128 v = mk(0, 0);
+          if (at && K == 2) {
+            v = ld(at);
+          } else if (at) {
+            v = pass_bind<false>([&](int j) { return ld(at + j * n); }, T, b.k);
+            if (b.k) st(at, v);
+          }
+          (slot >= half ? R : G)[slot & (half - 1)] = v;
+        }
       }
+      __syncthreads();
+      for (int u = t; u < half; u += kPassThreads) G[u] = pass_mul(E[buf][u & (X - 1)], G[u]);
+      main_warps_sync();
+#pragma unroll
+      for (int q = 0; q < kTurns; q++) {
+        const int u = t + q * kPassThreads;
+        if (u < kPoints << lx) {
+          const int x = u & (X - 1);
+          wacc(sum[q], pass_wide(point_value(G + x, X, at_one[q], at_inf[q]),
+                                 point_value(R + x, X, at_one[q], at_inf[q])));
+        }
+      }
+      main_warps_sync();  // the tile's tables before the next tile's
     }
-    __syncthreads();  // the tile's tables before the next tile's
   }
   const bool direct = pass_direct(gridDim.x, kWords);
-  pass_reduce<kPoints, kTurns>(sum, lx, kWords, direct, post);
-  if (t >> 5 == kEqWarp) {
+  if (!eq_warp) {
+    pass_reduce<kPoints, kTurns>(sum, lx, kWords, direct, post);
+  } else {
     for (int off = 16; off > 0; off >>= 1) {
       sum_e.lo ^= __shfl_xor_sync(0xffffffffu, sum_e.lo, off);
       sum_e.hi ^= __shfl_xor_sync(0xffffffffu, sum_e.hi, off);
@@ -537,30 +592,34 @@ static_assert(4 << kHostLog <= kHandoverWords, "the last tables fit one handover
 constexpr int kFirstLog = 17;
 
 // Returns how many blocks post sums of their own.
-template <int K, int NF>
-static int launch_pass_nf(f128 *c, size_t n_half, int log_m, const PassBind &b, const EqHeap *heap,
-                           size_t colmask, uint32_t live, uint32_t count, const PassPost &post,
-                           cudaStream_t st) {
-  EqFactors<NF> eq;
-  for (int g = 0; g < NF; g++) {
-    const int have = std::min(kFacLog, std::max(0, log_m - g * kFacLog));
-    memcpy(eq.f[g], heap[g].prefix(have), sizeof(f128) << have);
+template <int K, bool kLow>
+static int launch_pass_as(f128 *c, size_t n_half, int log_m, const PassBind &b, const EqHeap *heap,
+                          const f128 *eq_low, size_t colmask, uint32_t live, uint32_t count,
+                          const PassPost &post, cudaStream_t st) {
+  using S = PassShape<K, kLow>;
+  EqFactors<S::kFactors> eq;
+  const int skip = kLow ? 2 : 0;  // factors that eq_low holds
+  for (int g = 0; g < S::kFactors; g++) {
+    const int have = std::min(kFacLog, std::max(0, log_m - (g + skip) * kFacLog));
+    memcpy(eq.f[g], heap[g + skip].prefix(have), sizeof(f128) << have);
   }
-  const int lx = pass_tile_log(count);
-  const unsigned int grid = pass_grid(count, lx);
-  gkr_pass<K, NF><<<grid, kPassThreads, 0, st>>>(c, n_half, log_m, b, eq, colmask, live, count, lx,
-                                                 post);
+  int lx = pass_tile_log(count);
+  if (lx == 5 && (count >> S::kMaxLx) >= 2u * kSMs) lx = S::kMaxLx;
+  const uint32_t tiles = (count + (1u << lx) - 1) >> lx;
+  const unsigned int grid =
+      std::max(1u, std::min(tiles, (unsigned int)(S::kBlocksPerSm * kSMs)));
+  gkr_pass<K, kLow><<<grid, S::kThreadsAll, 0, st>>>(c, n_half, log_m, b, eq, eq_low, colmask, live,
+                                                     count, lx, post);
   BZ_LAUNCH_CHECK();
   return pass_direct(grid, 2 * (pow3(K) + 1)) ? (int)grid : 1;
 }
 
 template <int K>
 static int launch_pass(f128 *c, size_t n_half, int log_m, const PassBind &b, const EqHeap *heap,
-                        size_t colmask, uint32_t live, uint32_t count, const PassPost &post,
-                        cudaStream_t st) {
-  if (log_m <= 2 * kFacLog)
-    return launch_pass_nf<K, 2>(c, n_half, log_m, b, heap, colmask, live, count, post, st);
-  return launch_pass_nf<K, 5>(c, n_half, log_m, b, heap, colmask, live, count, post, st);
+                       const f128 *eq_low, size_t colmask, uint32_t live, uint32_t count,
+                       const PassPost &post, cudaStream_t st) {
+  return (log_m <= kEqLowLog ? launch_pass_as<K, false> : launch_pass_as<K, true>)(
+      c, n_half, log_m, b, heap, eq_low, colmask, live, count, post, st);
 }
 
 void gkr_build(const f128 *cols, int s, const f128 *images, GkrScratch &sc, cudaStream_t st_) {
@@ -694,6 +753,12 @@ f128 gkr_prove(const f128 *cols, int s, const f128 *images, const f128 *zeta, ui
     for (int g = 0; g * kFacLog < n - 1 || g == 0; g++)
       heap[g].build(point + g * kFacLog, std::min(kFacLog, std::max(0, n - 1 - g * kFacLog)));
     for (int g = (n - 2) / kFacLog + 1; g < 5; g++) heap[g].v[1] = mk(1, 0);
+    if ((j >= 2 ? n : s) - 2 > kEqLowLog) {  // a pass of this layer has more coordinates below it
+      EqFactors<2> low;
+      for (int g = 0; g < 2; g++) memcpy(low.f[g], heap[g].prefix(kFacLog), sizeof(f128) << kFacLog);
+      gkr_eq_low<<<(1 << kEqLowLog) / kThreads, kThreads, 0, st_>>>(low, sc.eq_low);
+      BZ_LAUNCH_CHECK();
+    }
     LayerRounds rounds{point, next, grind_bits, ts};
     PassBind b{};
     int rem = n;  // coordinates not bound yet (b's are bound by the next pass)
@@ -745,7 +810,7 @@ f128 gkr_prove(const f128 *cols, int s, const f128 *images, const f128 *zeta, ui
       if (probed) probe.before(st_);
       const PassPost post{sc.acc, ch->counter, ch->handover_dev, ch->arm().seq};
       const int blocks = (k == 2 ? launch_pass<2> : launch_pass<3>)(
-          c, n_half, log_m, b, heap.data(), colmask, (uint32_t)live, count, post, st_);
+          c, n_half, log_m, b, heap.data(), sc.eq_low, colmask, (uint32_t)live, count, post, st_);
       if (probed) {
         // per live position: 2^(k+1) entries of the bound tables, each from
         // 2^kb read and one written (none written without a bind), 2^kb - 1
@@ -753,7 +818,7 @@ f128 gkr_prove(const f128 *cols, int s, const f128 *images, const f128 *zeta, ui
         // and 3^k wide ones
         const double e = (double)count * (2 << k), in = (double)(1 << b.k);
         probe.after(st_, "gkr_pass", 16.0 * e * (in + (b.k ? 1.0 : 0.0)),
-                    (double)count * ((1 << k) + (log_m - 1) / kFacLog), (double)count * points,
+                    (double)count * ((1 << k) + 1), (double)count * points,
                     e * (in - 1));
       }
       ch->wait_handover(st_, post.seq, words.data(), 2 * (points + 1) * blocks);
@@ -816,10 +881,11 @@ void preload_gkr_kernels() {
                 (const void *)gkr_moments<1>,
                 (const void *)gkr_bound_rows<0>,
                 (const void *)gkr_bound_rows<1>,
-                (const void *)gkr_pass<2, 2>,
-                (const void *)gkr_pass<2, 5>,
-                (const void *)gkr_pass<3, 2>,
-                (const void *)gkr_pass<3, 5>,
+                (const void *)gkr_eq_low,
+                (const void *)gkr_pass<2, false>,
+                (const void *)gkr_pass<2, true>,
+                (const void *)gkr_pass<3, false>,
+                (const void *)gkr_pass<3, true>,
                 (const void *)gkr_handover});
 }
 

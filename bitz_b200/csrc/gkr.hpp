@@ -14,6 +14,7 @@ struct GkrScratch {
   f128 *bound = nullptr;       // 2^(s+1): layers 0 and 1 once their rows are bound
   unsigned long long *gram = nullptr;  // gkr_gram_words() words
   f128 *mid = nullptr;                 // 2304 entries
+  f128 *eq_low = nullptr;              // 2^14 entries
   unsigned long long *acc = nullptr;  // a pass's sums: 56 words
   RoundChannel *channel = nullptr;    // carries the passes' sums and the last tables
   // Columns at or beyond live_cols hold no set bit (the padding of h), so

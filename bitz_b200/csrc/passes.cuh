@@ -242,11 +242,11 @@ static __device__ __forceinline__ void pass_reduce(const wide (&sum)[kTurns], in
     const int u = threadIdx.x + q * kPassThreads, p = u >> lx;
     if ((u & ~31) >= kPoints << lx) break;  // the whole warp
     f128 v = greduce(sum[q]);
-    for (int off = X >> 1; off > 0; off >>= 1) {
+    for (int off = (X < 32 ? X : 32) >> 1; off > 0; off >>= 1) {
       v.lo ^= __shfl_xor_sync(0xffffffffu, v.lo, off);
       v.hi ^= __shfl_xor_sync(0xffffffffu, v.hi, off);
     }
-    if (p < kPoints && (u & (X - 1)) == 0) {
+    if (p < kPoints && (u & (X < 32 ? X - 1 : 31)) == 0) {
       if (direct) {
         handover_post(post.handover, post.seq, blockIdx.x * words + 2 * p, v.lo);
         handover_post(post.handover, post.seq, blockIdx.x * words + 2 * p + 1, v.hi);

@@ -812,7 +812,7 @@ int ProofSystem::prove_after_commit(cudaStream_t s, std::vector<uint8_t> &proof)
   W.w0.resize(2);
   W.mt_dense.resize((size_t)128 << sc_cols);
   mt_transpose(dev_->csc_off.get(), dev_->csc_row.get(), S.f_bits + 1, W.u1.get(), W.u2.get(),
-               W.weights.get(), nbits, W.w0.get(), s, W.mt_dense.get(), sc_cols);
+               W.weights.get(), nbits, W.w0.get(), s, W.mt_dense.get(), sc_cols, S.h_len);
   f128 *w0_h = W.pin_small.get(kPinSmall) + kPinW0;
   // the inner-product statement's weight digest (opening.rs:337-368); the
   // weight of column 0 comes back with it

@@ -457,7 +457,7 @@ int ProofSystem::verify(const uint8_t *proof, size_t proof_len, Context *lane) {
   W.w0.resize(2);
   W.mt_dense.resize((size_t)128 << sc_cols);
   mt_transpose(dev_->csc_off.get(), dev_->csc_row.get(), S.f_bits + 1, W.u1.get(), W.u2.get(),
-               W.weights.get(), nbits, W.w0.get(), s, W.mt_dense.get(), sc_cols);
+               W.weights.get(), nbits, W.w0.get(), s, W.mt_dense.get(), sc_cols, S.h_len);
   // the weight digest (opening.rs:337-368): the weights' chunk tree on the
   // device, the trailing column weight [1] and the root here
   const size_t nchunks = nbits * 16 / 1024;
