@@ -24,13 +24,33 @@ namespace bz {
 
 // --------------------------------------------------------------- the fold
 
-__global__ void k_fold_columns(const f128 *__restrict__ cols, size_t ncols,
-                               const u128 *__restrict__ exps, u128 *__restrict__ folds) {
+// comb.pow(e): one multiply per non-zero 8-bit window (pow.rs:177-199)
+__device__ __forceinline__ f128 comb_power(const f128 *table, u128 e) {
+  f128 acc = mk(1, 0);
+  for (int w = 0; w < 16 && e; w++, e >>= 8) {
+    int d = (int)(e & 0xff);
+    if (d) acc = gmul(acc, ld(table + w * 256 + d));
+  }
+  return acc;
+}
+
+// The columns' folds by the 128 row exponents, and in the launch's last block
+// (when there is a table) the exponents' comb powers, which take as long as a
+// launch of their own but wait for nothing here.
+__global__ void __launch_bounds__(kThreads) k_fold_columns(
+    const f128 *__restrict__ cols, size_t ncols, const __grid_constant__ RowExponents exps,
+    u128 *__restrict__ folds, const f128 *__restrict__ table, f128 *__restrict__ images) {
+  const int blocks = gridDim.x - (table ? 1 : 0);
+  if ((int)blockIdx.x == blocks) {
+    if (threadIdx.x < 128)
+      st(images + threadIdx.x, comb_power(table, exps.e[threadIdx.x]));
+    return;
+  }
   __shared__ u128 e[128];
-  for (int i = threadIdx.x; i < 128; i += blockDim.x) e[i] = exps[i];
+  for (int i = threadIdx.x; i < 128; i += blockDim.x) e[i] = exps.e[i];
   __syncthreads();
   for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < ncols;
-       c += (size_t)gridDim.x * blockDim.x) {
+       c += (size_t)blocks * blockDim.x) {
     f128 w = ld(cols + c);
     u128 s = 0;
     uint64_t lo = w.lo, hi = w.hi;
@@ -46,22 +66,16 @@ __global__ void k_fold_columns(const f128 *__restrict__ cols, size_t ncols,
   }
 }
 
-// comb.pow(e): one multiply per non-zero 8-bit window (pow.rs:177-199)
 __global__ void k_comb_pow(const f128 *__restrict__ table, const u128 *__restrict__ exps, int n,
                            f128 *__restrict__ out) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  u128 e = exps[i];
-  f128 acc = mk(1, 0);
-  for (int w = 0; w < 16 && e; w++, e >>= 8) {
-    int d = (int)(e & 0xff);
-    if (d) acc = gmul(acc, ld(table + w * 256 + d));
-  }
-  st(out + i, acc);
+  if (i < n) st(out + i, comb_power(table, exps[i]));
 }
 
-void fold_columns(const f128 *cols, size_t ncols, const u128 *exps, u128 *folds, cudaStream_t s) {
-  k_fold_columns<<<grid_for(ncols), kThreads, 0, s>>>(cols, ncols, exps, folds);
+void fold_columns(const f128 *cols, size_t ncols, const RowExponents &exps, u128 *folds,
+                  const f128 *table, f128 *images, cudaStream_t s) {
+  k_fold_columns<<<grid_for(ncols) + (table ? 1 : 0), kThreads, 0, s>>>(cols, ncols, exps, folds,
+                                                                        table, images);
   BZ_LAUNCH_CHECK();
 }
 
@@ -72,99 +86,63 @@ void comb_pow(const f128 *table, const u128 *exps, int n, f128 *out, cudaStream_
 
 // -------------------------------------------------------------------- M^T
 
-// w[c] = sum over the rows of column c of u1[row & 127] * u2[row >> 7]; one
-// reduction per column. Column 0 (the constant) goes to w0, the others to
-// weights[c - 1]; weights beyond the last column are zero.
-__global__ void k_mt_transpose(const uint32_t *__restrict__ off, const uint32_t *__restrict__ row,
-                               size_t ncols, const f128 *__restrict__ u1,
-                               const f128 *__restrict__ u2, f128 *__restrict__ weights,
-                               size_t padded, f128 *w0) {
-  __shared__ f128 su1[128];
-  for (int i = threadIdx.x; i < 128; i += blockDim.x) su1[i] = u1[i];
-  __syncthreads();
-  for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c <= padded;
-       c += (size_t)gridDim.x * blockDim.x) {
-    if (c == 0) continue;  // the constant column: k_mt_col0
-    f128 v = mk(0, 0);
-    if (c < ncols) {
-      wide acc = wzero();
-      for (uint32_t e = off[c]; e < off[c + 1]; e++) {
-        uint32_t r = row[e];
-        wacc(acc, gmul_wide(su1[r & 127], ld(u2 + (r >> 7))));
-      }
-      v = greduce(acc);
-    }
-    st(weights + (c - 1), v);
-  }
-}
-
-// The constant column holds one entry per lift with a constant term (hundreds
-// where the others hold under ten), so one block shares it out.
-__global__ void k_mt_col0(const uint32_t *__restrict__ off, const uint32_t *__restrict__ row,
-                          const f128 *__restrict__ u1, const f128 *__restrict__ u2, f128 *w0) {
-  wide acc = wzero();
-  for (uint32_t e = off[0] + threadIdx.x; e < off[1]; e += blockDim.x) {
-    uint32_t r = row[e];
-    wacc(acc, gmul_wide(ld(u1 + (r & 127)), ld(u2 + (r >> 7))));
-  }
-  f128 v = greduce(acc);
-  uint64_t w[2] = {v.lo, v.hi};
-  block_xor_reduce<2>(w);
-  if (threadIdx.x == 0) st(w0, mk(w[0], w[1]));
-}
-
 // The dense eq table of the rows, dense[lo << log_u2 | hi] = u1[lo] * u2[hi]
 // (row r = hi * 128 + lo), for the `live` values of hi that rows exist for:
 // block (lo, part) takes a slice of hi through u1[lo]'s window table, writing
 // along hi. Bound by the table lookups (72 G/s), so rows that are only padding
 // are left out (38 % of them at 64 and 1024 blocks, 98 % at one) and the slices
 // are as many as keep the SMs level.
-__global__ void __launch_bounds__(kThreads) k_mt_dense(const f128 *__restrict__ u1,
+__global__ void __launch_bounds__(kThreads) k_mt_dense(const __grid_constant__ RowWeights128 u1,
                                                        const f128 *__restrict__ u2, int log_u2,
                                                        size_t live, f128 *__restrict__ dense) {
   __shared__ MulTable T;
   const int lo = blockIdx.x;
-  mul_table_build(T, ld(u1 + lo));
+  mul_table_build(T, u1.v[lo]);
   f128 *out = dense + ((size_t)lo << log_u2);
   for (size_t hi = blockIdx.y * (size_t)kThreads + threadIdx.x; hi < live;
        hi += (size_t)gridDim.y * kThreads)
     st(out + hi, mul_table(T, ld(u2 + hi)));
 }
 
-// k_mt_transpose over the dense table: each column XORs its rows' entries.
-__global__ void k_mt_gather(const uint32_t *__restrict__ off, const uint32_t *__restrict__ row,
-                            size_t ncols, const f128 *__restrict__ dense, int log_u2,
-                            f128 *__restrict__ weights, size_t padded) {
-  for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c <= padded;
-       c += (size_t)gridDim.x * blockDim.x) {
-    if (c == 0) continue;  // the constant column: k_mt_col0
+// w[c] = the sum over column c's rows of their table entries. The constant
+// column (an entry per lift with a constant term, hundreds where the others
+// hold under ten) is the launch's last block and goes to w0, the others to
+// weights[c - 1]; weights beyond the last column are zero.
+__global__ void __launch_bounds__(kThreads) k_mt_gather(
+    const uint32_t *__restrict__ off, const uint32_t *__restrict__ row, size_t ncols,
+    const f128 *__restrict__ dense, int log_u2, f128 *__restrict__ weights, size_t padded,
+    f128 *w0) {
+  auto entry = [&](uint32_t e) {
+    const uint32_t r = row[e];
+    return ld(dense + (((size_t)(r & 127) << log_u2) | (r >> 7)));
+  };
+  const int blocks = gridDim.x - 1;
+  if ((int)blockIdx.x == blocks) {
+    f128 v = mk(0, 0);
+    for (uint32_t e = off[0] + threadIdx.x; e < off[1]; e += blockDim.x) v = gadd(v, entry(e));
+    uint64_t w[2] = {v.lo, v.hi};
+    block_xor_reduce<2>(w);
+    if (threadIdx.x == 0) st(w0, mk(w[0], w[1]));
+    return;
+  }
+  for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x + 1; c <= padded;
+       c += (size_t)blocks * blockDim.x) {
     f128 v = mk(0, 0);
     if (c < ncols)
-      for (uint32_t e = off[c]; e < off[c + 1]; e++) {
-        const uint32_t r = row[e];
-        v = gadd(v, ld(dense + (((size_t)(r & 127) << log_u2) | (r >> 7))));
-      }
+      for (uint32_t e = off[c]; e < off[c + 1]; e++) v = gadd(v, entry(e));
     st(weights + (c - 1), v);
   }
 }
 
-void mt_transpose(const uint32_t *off, const uint32_t *row, size_t ncols, const f128 *u1,
+void mt_transpose(const uint32_t *off, const uint32_t *row, size_t ncols, const RowWeights128 &u1,
                   const f128 *u2, f128 *weights, size_t padded, f128 *w0, cudaStream_t s,
                   f128 *dense, int log_u2, size_t rows) {
-  if (dense && log_u2 >= 8) {
-    const size_t live = (rows + 127) / 128;
-    const dim3 grid(128, grid_for(live, kThreads, 8));
-    k_mt_dense<<<grid, kThreads, 0, s>>>(u1, u2, log_u2, live, dense);
-    BZ_LAUNCH_CHECK();
-    k_mt_gather<<<grid_for(padded + 1), kThreads, 0, s>>>(off, row, ncols, dense, log_u2, weights,
-                                                          padded);
-    BZ_LAUNCH_CHECK();
-  } else {
-    k_mt_transpose<<<grid_for(padded + 1), kThreads, 0, s>>>(off, row, ncols, u1, u2, weights,
-                                                             padded, w0);
-    BZ_LAUNCH_CHECK();
-  }
-  k_mt_col0<<<1, kThreads, 0, s>>>(off, row, u1, u2, w0);
+  const size_t live = (rows + 127) / 128;
+  const dim3 grid(128, grid_for(live, kThreads, 8));
+  k_mt_dense<<<grid, kThreads, 0, s>>>(u1, u2, log_u2, live, dense);
+  BZ_LAUNCH_CHECK();
+  k_mt_gather<<<grid_for(padded) + 1, kThreads, 0, s>>>(off, row, ncols, dense, log_u2, weights,
+                                                        padded, w0);
   BZ_LAUNCH_CHECK();
 }
 
@@ -201,6 +179,32 @@ __global__ void k_b3_parents(const uint32_t *__restrict__ in, size_t nout, Key8 
     b3_compress(key.k, m, 0, 64, flags | B3_PARENT, cv);
     for (int j = 0; j < 8; j++) out[8 * i + j] = cv[j];
   }
+}
+
+// Seven parent levels in one launch: a block reduces 128 chaining values to one
+// in shared memory.
+constexpr int kB3TreeLog = 7;
+__global__ void __launch_bounds__(1 << (kB3TreeLog - 1)) k_b3_tree(const uint32_t *__restrict__ in,
+                                                                   Key8 key, uint32_t flags,
+                                                                   uint32_t *__restrict__ out) {
+  __shared__ uint32_t cv[8 << kB3TreeLog];
+  const uint32_t *src = in + ((size_t)blockIdx.x << (kB3TreeLog + 3));
+  for (int i = threadIdx.x; i < 8 << kB3TreeLog; i += blockDim.x) cv[i] = src[i];
+  __syncthreads();
+  for (int m = 1 << (kB3TreeLog - 1); m >= 1; m /= 2) {
+    uint32_t o[8];
+    const bool mine = (int)threadIdx.x < m;
+    if (mine) {
+      uint32_t msg[16];
+      for (int j = 0; j < 16; j++) msg[j] = cv[16 * threadIdx.x + j];
+      b3_compress(key.k, msg, 0, 64, flags | B3_PARENT, o);
+    }
+    __syncthreads();  // every read of this level before any write
+    if (mine)
+      for (int j = 0; j < 8; j++) cv[8 * threadIdx.x + j] = o[j];
+    __syncthreads();
+  }
+  if (threadIdx.x < 8) out[8 * (size_t)blockIdx.x + threadIdx.x] = cv[threadIdx.x];
 }
 
 // The last parent levels of a tree in one block: n chaining values (a power
@@ -253,6 +257,13 @@ void blake3_tree_cv(const uint8_t *data, size_t nchunks, const uint32_t key[8], 
   BZ_LAUNCH_CHECK();
   size_t n = nchunks;
   while (n > 1 && (!ch || n > kB3BlockMax)) {
+    if (n >= (size_t)1 << kB3TreeLog) {
+      k_b3_tree<<<(unsigned int)(n >> kB3TreeLog), 1 << (kB3TreeLog - 1), 0, s>>>(a, k, flags, b);
+      BZ_LAUNCH_CHECK();
+      std::swap(a, b);
+      n >>= kB3TreeLog;
+      continue;
+    }
     k_b3_parents<<<grid_for(n / 2), kThreads, 0, s>>>(a, n / 2, k, flags, b);
     BZ_LAUNCH_CHECK();
     std::swap(a, b);
@@ -275,9 +286,11 @@ void blake3_tree_cv(const uint8_t *data, size_t nchunks, const uint32_t key[8], 
 // ----------------------------------------------------------- ring switch
 
 // claims[v] = sum over y with bit v of f[y] set of suffix[y]; block b covers
-// 64 consecutive y, thread v one bit position.
-__global__ void k_ring_claims(const f128 *__restrict__ f, const f128 *__restrict__ suffix,
-                              size_t n, unsigned long long *claims) {
+// 64 consecutive y, thread v one bit position. The last block posts the 256
+// words (acc is zero before and after).
+__global__ void __launch_bounds__(128) k_ring_claims(const f128 *__restrict__ f,
+                                                     const f128 *__restrict__ suffix, size_t n,
+                                                     PassPost post) {
   int v = threadIdx.x;
   uint64_t lo = 0, hi = 0;
   for (size_t y0 = blockIdx.x * (size_t)64; y0 < n; y0 += (size_t)gridDim.x * 64) {
@@ -291,17 +304,19 @@ __global__ void k_ring_claims(const f128 *__restrict__ f, const f128 *__restrict
       }
     }
   }
-  if (lo) atomicXor(claims + 2 * v, (unsigned long long)lo);
-  if (hi) atomicXor(claims + 2 * v + 1, (unsigned long long)hi);
+  if (lo) atomicXor(post.acc + 2 * v, (unsigned long long)lo);
+  if (hi) atomicXor(post.acc + 2 * v + 1, (unsigned long long)hi);
+  pass_publish(post.acc, 256, post.counter, post.handover, post.seq);
 }
 
 // B(y) = sum over u with bit u of suffix[y] set of bw[u] (the packed basis of
 // the batched ring-switch claim), plus coef * eq_ood[y] when eq_ood is given.
 __global__ void k_packed_basis(const f128 *__restrict__ suffix, size_t n,
-                               const f128 *__restrict__ bw, const f128 *__restrict__ eq_ood,
-                               f128 coef, f128 *__restrict__ basis) {
+                               const __grid_constant__ RowWeights128 bw,
+                               const f128 *__restrict__ eq_ood, f128 coef,
+                               f128 *__restrict__ basis) {
   __shared__ f128 w[128];
-  for (int i = threadIdx.x; i < 128; i += blockDim.x) w[i] = bw[i];
+  for (int i = threadIdx.x; i < 128; i += blockDim.x) w[i] = bw.v[i];
   __syncthreads();
   for (size_t y = blockIdx.x * (size_t)blockDim.x + threadIdx.x; y < n;
        y += (size_t)gridDim.x * blockDim.x) {
@@ -321,18 +336,6 @@ __global__ void k_packed_basis(const f128 *__restrict__ suffix, size_t n,
   }
 }
 
-// sum_y a[y] * b[y], XOR-reduced into acc[0..2).
-__global__ void k_dot(const f128 *__restrict__ a, const f128 *__restrict__ b, size_t n,
-                      unsigned long long *acc, Publish pub) {
-  wide s = wzero();
-  for (size_t y = blockIdx.x * (size_t)blockDim.x + threadIdx.x; y < n;
-       y += (size_t)gridDim.x * blockDim.x)
-    wacc(s, gmul_wide(ld(a + y), ld(b + y)));
-  f128 r = greduce(s);
-  uint64_t v[2] = {r.lo, r.hi};
-  block_xor_publish<2>(v, acc, pub);
-}
-
 __global__ void k_axpy(f128 *__restrict__ y, f128 a, const f128 *__restrict__ x, size_t n) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x)
@@ -344,23 +347,17 @@ void axpy(f128 *y, f128 a, const f128 *x, size_t n, cudaStream_t s) {
   BZ_LAUNCH_CHECK();
 }
 
-void ring_claims(const f128 *f, const f128 *suffix, size_t n, unsigned long long *claims,
+void ring_claims(const f128 *f, const f128 *suffix, size_t n, const PassPost &post,
                  cudaStream_t s) {
   int blocks = (int)((n + 63) / 64);
   if (blocks > kSMs * 4) blocks = kSMs * 4;
-  k_ring_claims<<<blocks, 128, 0, s>>>(f, suffix, n, claims);
+  k_ring_claims<<<blocks, 128, 0, s>>>(f, suffix, n, post);
   BZ_LAUNCH_CHECK();
 }
 
-void packed_basis(const f128 *suffix, size_t n, const f128 *bw, const f128 *eq_ood, f128 coef,
+void packed_basis(const f128 *suffix, size_t n, const RowWeights128 &bw, const f128 *eq_ood, f128 coef,
                   f128 *basis, cudaStream_t s) {
   k_packed_basis<<<grid_for(n), kThreads, 0, s>>>(suffix, n, bw, eq_ood, coef, basis);
-  BZ_LAUNCH_CHECK();
-}
-
-void dot(const f128 *a, const f128 *b, size_t n, unsigned long long *acc, Publish pub,
-         cudaStream_t s) {
-  k_dot<<<grid_for(n), kThreads, 0, s>>>(a, b, n, acc, pub);
   BZ_LAUNCH_CHECK();
 }
 
@@ -641,8 +638,8 @@ __global__ void k_merkle_parents(uint32_t *nodes, size_t lo, size_t hi) {
 constexpr int kOpeningThreads = 64;
 __global__ void __launch_bounds__(kOpeningThreads) k_check_openings(
     const uint32_t *__restrict__ proof, size_t at, int width, int depth,
-    const uint64_t *__restrict__ idx, int nq, const f128 *__restrict__ eqr, B3Root root,
-    f128 *__restrict__ vals, unsigned int *bad) {
+    const __grid_constant__ QueryRows queries, int nq, B3Root root, f128 *__restrict__ vals,
+    unsigned int *bad) {
   const uint32_t IV[8] = {0x6A09E667, 0xBB67AE85, 0x3C6EF372, 0xA54FF53A,
                           0x510E527F, 0x9B05688C, 0x1F83D9AB, 0x5BE0CD19};
   const int q = (blockIdx.x * kOpeningThreads + threadIdx.x) >> 5, lane = threadIdx.x & 31;
@@ -652,7 +649,7 @@ __global__ void __launch_bounds__(kOpeningThreads) k_check_openings(
   for (int c = lane; c < width; c += 32) {
     const uint32_t *p = row + 4 * c;
     wacc(sum, gmul_wide(mk((uint64_t)p[0] | (uint64_t)p[1] << 32, (uint64_t)p[2] | (uint64_t)p[3] << 32),
-                        ld(eqr + c)));
+                        queries.eqr[c]));
   }
   f128 v = greduce(sum);
   for (int off = 16; off > 0; off >>= 1) {
@@ -671,7 +668,7 @@ __global__ void __launch_bounds__(kOpeningThreads) k_check_openings(
     b3_compress(cv, m, 0, (uint32_t)(left < 16 ? 4 * left : 64), fl, cv);
   }
   const uint32_t *sib = row + 4 * width;
-  uint64_t node = idx[q];
+  uint64_t node = queries.idx[q];
   for (int d = 0; d < depth; d++, sib += 8, node >>= 1) {
     for (int j = 0; j < 8; j++) {
       m[(node & 1 ? 0 : 8) + j] = sib[j];
@@ -684,12 +681,14 @@ __global__ void __launch_bounds__(kOpeningThreads) k_check_openings(
   if (diff) *bad = 1;
 }
 
-void check_openings(const uint32_t *proof, size_t at, int width, int depth, const uint64_t *idx,
-                    int nq, const f128 *eqr, const B3Root &root, f128 *vals, unsigned int *bad,
-                    cudaStream_t s) {
-  if (16 * width > 1024) throw CudaError("check_openings: a row longer than one hash chunk");
+void check_openings(const uint32_t *proof, size_t at, int width, int depth,
+                    const QueryRows &queries, int nq, const B3Root &root, f128 *vals,
+                    unsigned int *bad, cudaStream_t s) {
+  // a row of kMaxQueryWidth entries is one hash chunk
+  if (nq > kMaxQueries || width > kMaxQueryWidth)
+    throw CudaError("check_openings: too many queries or too wide a row");
   k_check_openings<<<(32 * nq + kOpeningThreads - 1) / kOpeningThreads, kOpeningThreads, 0, s>>>(
-      proof, at, width, depth, idx, nq, eqr, root, vals, bad);
+      proof, at, width, depth, queries, nq, root, vals, bad);
   BZ_LAUNCH_CHECK();
 }
 
@@ -768,9 +767,8 @@ bool merkle_build_posted(const f128 *cw, size_t rows, int k, uint32_t *nodes, Pu
 // the subspace polynomials at the queried row: w[q][t] = Wh_t(x_q) = the sum
 // of Wh_t(X^s) over the set bits s >= t of idx[q] (wh is that table, t-major
 // with kMaxRsDim entries per t), formed by the block's first threads.
-__global__ void k_query_basis(const uint64_t *__restrict__ idx, const f128 *__restrict__ wh,
-                              const f128 *__restrict__ scale, int l,
-                              unsigned long long *basis) {
+__global__ void k_query_basis(const __grid_constant__ QueryTerms terms,
+                              const f128 *__restrict__ wh, int l, unsigned long long *basis) {
   extern __shared__ f128 tab[];
   __shared__ f128 w[kMaxRsDim];
   const int q = blockIdx.x;
@@ -778,11 +776,11 @@ __global__ void k_query_basis(const uint64_t *__restrict__ idx, const f128 *__re
     const int t = threadIdx.x;
     f128 v = mk(0, 0);
     // row indices stay below 2^kMaxRsDim; the mask keeps every read in wh
-    for (uint64_t bits = (idx[q] >> t) & ((1ull << (kMaxRsDim - t)) - 1); bits; bits &= bits - 1)
+    for (uint64_t bits = (terms.idx[q] >> t) & ((1ull << (kMaxRsDim - t)) - 1); bits; bits &= bits - 1)
       v = gadd(v, ld(wh + t * kMaxRsDim + t + __ffsll((long long)bits) - 1));
     w[t] = v;
   }
-  if (threadIdx.x == 0) tab[0] = scale[q];
+  if (threadIdx.x == 0) tab[0] = terms.scale[q];
   __syncthreads();
   for (int t = 0; t < l; t++) {
     int h = 1 << t;
@@ -797,37 +795,57 @@ __global__ void k_query_basis(const uint64_t *__restrict__ idx, const f128 *__re
   }
 }
 
-void query_basis(const uint64_t *idx, const f128 *wh, const f128 *scale, int nq, int l,
-                 f128 *basis, cudaStream_t s) {
+void query_basis(const QueryTerms &terms, const f128 *wh, int nq, int l, f128 *basis,
+                 cudaStream_t s) {
+  if (nq > kMaxQueries) throw CudaError("query basis: too many queries");
   if (l > kMaxRsDim || l > kThreads) throw CudaError("query basis dimension out of range");
   size_t smem = sizeof(f128) << l;
   if (smem > 48 * 1024 - sizeof(f128) * kMaxRsDim)
     BZ_CUDA(cudaFuncSetAttribute(k_query_basis, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)smem));
-  k_query_basis<<<nq, kThreads, smem, s>>>(idx, wh, scale, l, (unsigned long long *)basis);
+  k_query_basis<<<nq, kThreads, smem, s>>>(terms, wh, l, (unsigned long long *)basis);
   BZ_LAUNCH_CHECK();
 }
 
 // The opened rows and their Merkle paths, in proof order: per query the row
 // (width entries of 16 bytes), then the sibling of every node from the leaf
-// (rows + idx) up to the root's children (32 bytes each). One block per query.
-__global__ void k_gather_openings(const f128 *__restrict__ cw, const uint32_t *__restrict__ nodes,
-                                  size_t rows, int width, int depth,
-                                  const uint64_t *__restrict__ idx, f128 *__restrict__ out) {
+// (rows + idx) up to the root's children (32 bytes each); behind the last
+// query, the rows' combinations with eqr, which the host took 54 us for at 150
+// queries of 64 entries. One block of 64 threads per query.
+__global__ void __launch_bounds__(64) k_gather_openings(
+    const f128 *__restrict__ cw, const uint32_t *__restrict__ nodes, size_t rows, int width,
+    int depth, const __grid_constant__ QueryRows queries, f128 *__restrict__ out) {
+  __shared__ uint64_t other[2];
   const size_t stride = (size_t)width + 2 * (size_t)depth;  // in 16-byte units
-  f128 *o = out + blockIdx.x * stride;
-  const uint64_t id = idx[blockIdx.x];
-  for (int c = threadIdx.x; c < width; c += blockDim.x) st(o + c, ld(cw + id * width + c));
-  for (int k = threadIdx.x; k < 2 * depth; k += blockDim.x) {
+  const int q = blockIdx.x, t = threadIdx.x;
+  f128 *o = out + q * stride;
+  const uint64_t id = queries.idx[q];
+  wide sum = wzero();
+  for (int c = t; c < width; c += blockDim.x) {
+    const f128 v = ld(cw + id * width + c);
+    st(o + c, v);
+    wacc(sum, gmul_wide(v, queries.eqr[c]));
+  }
+  for (int k = t; k < 2 * depth; k += blockDim.x) {
     const int d = k >> 1, half = k & 1;
     const size_t sib = ((rows + id) >> d) ^ 1;
     st(o + width + k, ld(reinterpret_cast<const f128 *>(nodes + 8 * sib) + half));
   }
+  f128 v = greduce(sum);
+  for (int off = 16; off > 0; off >>= 1) {
+    v.lo ^= __shfl_xor_sync(0xffffffffu, v.lo, off);
+    v.hi ^= __shfl_xor_sync(0xffffffffu, v.hi, off);
+  }
+  if (t == 32) other[0] = v.lo, other[1] = v.hi;
+  __syncthreads();
+  if (t == 0) st(out + gridDim.x * stride + q, mk(v.lo ^ other[0], v.hi ^ other[1]));
 }
 
 void gather_openings(const f128 *cw, const uint32_t *nodes, size_t rows, int width, int depth,
-                     const uint64_t *idx, int nq, f128 *out, cudaStream_t s) {
-  k_gather_openings<<<nq, 64, 0, s>>>(cw, nodes, rows, width, depth, idx, out);
+                     const QueryRows &queries, int nq, f128 *out, cudaStream_t s) {
+  if (nq > kMaxQueries || width > kMaxQueryWidth)
+    throw CudaError("gather_openings: too many queries or too wide a row");
+  k_gather_openings<<<nq, 64, 0, s>>>(cw, nodes, rows, width, depth, queries, out);
   BZ_LAUNCH_CHECK();
 }
 
@@ -836,17 +854,15 @@ void gather_openings(const f128 *cw, const uint32_t *nodes, size_t rows, int wid
 void preload_pcs_kernels() {
   load_kernels({(const void *)k_fold_columns,
                 (const void *)k_comb_pow,
-                (const void *)k_mt_transpose,
-                (const void *)k_mt_col0,
                 (const void *)k_mt_dense,
                 (const void *)k_mt_gather,
                 (const void *)k_b3_chunks,
                 (const void *)k_b3_parents,
                 (const void *)k_b3_top,
+                (const void *)k_b3_tree,
                 (const void *)k_check_openings,
                 (const void *)k_ring_claims,
                 (const void *)k_packed_basis,
-                (const void *)k_dot,
                 (const void *)k_axpy,
                 (const void *)k_rs_pass,
                 (const void *)k_rs_encode_block,

@@ -286,6 +286,8 @@ int ProofSystem::witness(cudaStream_t s) {
   const CircuitSetup &S = *dev_->host;
   Workspace &W = workspace(*lane_);
   W.acc.resize(512);
+  // the sums of the proof's kernels: each leaves them zero again
+  BZ_CUDA(cudaMemsetAsync(W.acc.get(), 0, 512 * sizeof(unsigned long long), s));
   size_t n_in = inputs_.size();
   size_t fwords = ((size_t)1 << S.committed_m) / 32;
   size_t hwords = ((size_t)1 << (S.claim_log_cols + 7)) / 32;
@@ -418,12 +420,8 @@ int ProofSystem::commit(cudaStream_t s) {
     for (int i = 0; i < log_n; i++) ood_point_.push_back(t.challenge_f128());
     size_t n = (size_t)1 << log_n;
     W.eq_ood.resize(n);
-    W.eqs.resize(eq_scratch_entries(log_n));
-    eq_table_device(ood_point_.data(), log_n, W.eq_ood.get(), W.eqs.get(), s);
-    W.acc.resize(512);
-    BZ_CUDA(cudaMemsetAsync(W.acc.get(), 0, 16, s));
     RoundChannel *ch = lane_->channel();
-    dot(W.eq_ood.get(), fpk, n, W.acc.get(), ch->arm(), s);
+    eq_table_dot(ood_point_.data(), log_n, W.eq_ood.get(), fpk, W.acc.get(), ch->arm(), s);
     ch->wait(s, W.host_acc, 2);
     ood_value_ = mk(W.host_acc[0], W.host_acc[1]);
     t.prover_f128(ood_value_);
@@ -487,7 +485,6 @@ std::vector<uint8_t> ProofSystem::ligerito(cudaStream_t s, f128 target) {
     const PcsLevel &L = cfg.levels[i];
     std::vector<f128> rs;
     // the level's folds in passes of up to three rounds; the last binds without sums
-    BZ_CUDA(cudaMemsetAsync(acc, 0, 2 * pow3(kPassMaxK) * sizeof(unsigned long long), s));
     PassBind pb{};
     for (int r = 0; r < L.k;) {
       const int k = std::min(kPassMaxK, L.k - r), points = pow3(k);
@@ -549,10 +546,7 @@ std::vector<uint8_t> ProofSystem::ligerito(cudaStream_t s, f128 target) {
       t.prover_message(root, 36);
       if (N.ood_samples) {
         std::vector<f128> pt = sample_vec((size_t)l);
-        W.eqs.resize(eq_scratch_entries(l));
-        eq_table_device(pt.data(), l, W.eq.get(), W.eqs.get(), s);
-        BZ_CUDA(cudaMemsetAsync(acc, 0, 16, s));
-        dot(W.eq.get(), f, n, acc, ch->arm(), s);
+        eq_table_dot(pt.data(), l, W.eq.get(), f, acc, ch->arm(), s);
         ch->wait(s, W.host_acc, 2);
         f128 v = mk(W.host_acc[0], W.host_acc[1]);
         t.prover_f128(v);
@@ -576,28 +570,25 @@ std::vector<uint8_t> ProofSystem::ligerito(cudaStream_t s, f128 target) {
     int width = 1 << cur_k;
     int depth = ceil_log2(cur_rows);
     const size_t stride = (size_t)width + 2 * (size_t)depth;  // 16-byte units per query
-    uint64_t *idx = W.pin_idx.get(L.queries);
-    for (int q = 0; q < L.queries; q++) idx[q] = qs[q].lo & (cur_rows - 1);
-    W.qidx.resize(L.queries);
-    BZ_CUDA(cudaMemcpyAsync(W.qidx.get(), idx, (size_t)L.queries * 8, cudaMemcpyHostToDevice, s));
-    W.openings.resize(stride * L.queries);
-    gather_openings(cw, nodes, cur_rows, width, depth, W.qidx.get(), L.queries, W.openings.get(), s);
-    f128 *opened = W.pin_open.get(stride * L.queries);
-    BZ_CUDA(cudaMemcpyAsync(opened, W.openings.get(), stride * L.queries * 16,
+    std::vector<f128> eqr((size_t)1 << L.k);
+    eq_table_host(rs.data(), L.k, eqr.data());
+    QueryRows rows;
+    QueryTerms terms;
+    if (L.queries > kMaxQueries || width > kMaxQueryWidth)
+      throw std::runtime_error("ligerito: too many queries or too wide a row");
+    for (int q = 0; q < L.queries; q++) rows.idx[q] = terms.idx[q] = qs[q].lo & (cur_rows - 1);
+    std::copy(eqr.begin(), eqr.begin() + width, rows.eqr);
+    const size_t opened_units = stride * L.queries;
+    W.openings.resize(opened_units + L.queries);
+    gather_openings(cw, nodes, cur_rows, width, depth, rows, L.queries, W.openings.get(), s);
+    f128 *opened = W.pin_open.get(opened_units + L.queries);
+    BZ_CUDA(cudaMemcpyAsync(opened, W.openings.get(), (opened_units + L.queries) * 16,
                             cudaMemcpyDeviceToHost, s));
     BZ_CUDA(stream_wait(s));
     put_u64(proof, (uint64_t)L.queries);
     const uint8_t *ob = reinterpret_cast<const uint8_t *>(opened);
-    proof.insert(proof.end(), ob, ob + stride * L.queries * 16);
-    std::vector<f128> eqr((size_t)1 << L.k);
-    eq_table_host(rs.data(), L.k, eqr.data());
-    std::vector<f128> vals(L.queries);
-    for (int q = 0; q < L.queries; q++) {
-      const f128 *row = opened + q * stride;
-      wide v = wzero();
-      for (int c = 0; c < width; c++) wacc(v, gmul_wide(row[c], eqr[c]));
-      vals[q] = greduce(v);
-    }
+    proof.insert(proof.end(), ob, ob + opened_units * 16);
+    const f128 *vals = opened + opened_units;
     int av = ceil_log2((size_t)L.queries);
     std::vector<f128> alpha = sample_vec((size_t)av);
     f128 mu = t.challenge_f128();
@@ -605,14 +596,11 @@ std::vector<uint8_t> ProofSystem::ligerito(cudaStream_t s, f128 target) {
     eq_table_host(alpha.data(), av, beta.data());
     // glue: basis += sum_q s_q X(x_q) with X_j(x) = prod_{t in j} Wh_t(x);
     // the kernel forms Wh_t(x_q) from the uploaded row indices
-    f128 *sq = W.pin_qw.get(L.queries);
     for (int q = 0; q < L.queries; q++) {
-      sq[q] = gmul(mu, beta[q]);
-      claim = gadd(claim, gmul(sq[q], vals[q]));
+      terms.scale[q] = gmul(mu, beta[q]);
+      claim = gadd(claim, gmul(terms.scale[q], vals[q]));
     }
-    W.qs.resize(L.queries);
-    BZ_CUDA(cudaMemcpyAsync(W.qs.get(), sq, (size_t)L.queries * 16, cudaMemcpyHostToDevice, s));
-    query_basis(W.qidx.get(), T.wh.get(), W.qs.get(), L.queries, l, b, s);
+    query_basis(terms, T.wh.get(), L.queries, l, b, s);
     ph.mark("lig queries+glue");
     if (!last) {
       cw = next_cw[flip].get();
@@ -669,7 +657,6 @@ int ProofSystem::prove_after_commit(cudaStream_t s, std::vector<uint8_t> &proof)
   size_t R = (size_t)1 << nr, Cn = (size_t)1 << nc;
   W.sp_t.resize(8 * R);
   W.sp_d.resize(4 * Cn);
-  W.sp_eqs.resize(4096 * 2 + ((size_t)1 << ((std::max(nr, nc) + 1) / 2 + 1)));
   W.sp_part.resize(kSpPartials);
   W.sp_sums.resize(4);
   W.sp_tab.resize(dev_->ntab + 1);
@@ -680,7 +667,7 @@ int ProofSystem::prove_after_commit(cudaStream_t s, std::vector<uint8_t> &proof)
   SpartanScratch sc;
   for (int i = 0; i < 8; i++) sc.t[i] = W.sp_t.get() + i * R;
   for (int i = 0; i < 4; i++) sc.d[i] = W.sp_d.get() + i * Cn;
-  sc.eq_scratch = W.sp_eqs.get();
+  sc.counter = ctx.channel()->counter;
   sc.partial = W.sp_part.get();
   sc.sums = W.sp_sums.get();
   sc.tab = W.sp_tab.get();
@@ -737,26 +724,25 @@ int ProofSystem::prove_after_commit(cudaStream_t s, std::vector<uint8_t> &proof)
   // the column folds and row images, and the GKR product layers.
   W.cols_fp.resize(ncol + 2);
   W.cols_canon.resize(ncol);
-  fp_eq_table(pt.data() + 7, sc_cols, fc, W.cols_fp.get(), sc.eq_scratch, s);
+  fp_eq_table(pt.data() + 7, sc_cols, fc, W.cols_fp.get(), s);
   fp_canonical_device(W.cols_fp.get(), ncol, fc, W.cols_canon.get(), s);
   u128 *cols_h = W.host_cols.get(ncol);
   BZ_CUDA(cudaMemcpyAsync(cols_h, W.cols_canon.get(), ncol * 16, cudaMemcpyDeviceToHost, s));
   BZ_CUDA(cudaEventRecord(W.ev_cols, s));
   // send_fold (crates/prover/src/fold.rs:38-75) and the GKR build
-  W.exps.upload(rows_w.data(), 128, s);
-  W.folds.resize(ncol);
+  RowExponents exps;
+  for (int i = 0; i < 128; i++) exps.e[i] = rows_w[i];
+  W.folds.resize(ncol + 128);  // the folds, then the 128 row images
+  f128 *images = reinterpret_cast<f128 *>(W.folds.get() + ncol);
   const f128 *hpk = reinterpret_cast<const f128 *>(h_->get());
-  fold_columns(hpk, ncol, W.exps.get(), W.folds.get(), s);
-  u128 *folds_h = W.host_folds.get(ncol + 128);  // the folds, then the 128 row images
-  BZ_CUDA(cudaMemcpyAsync(folds_h, W.folds.get(), ncol * 16, cudaMemcpyDeviceToHost, s));
-  W.images.resize(128);
-  comb_pow(T.comb.get(), W.exps.get(), 128, W.images.get(), s);
+  fold_columns(hpk, ncol, exps, W.folds.get(), T.comb.get(), images, s);
+  u128 *folds_h = W.host_folds.get(ncol + 128);
+  BZ_CUDA(cudaMemcpyAsync(folds_h, W.folds.get(), (ncol + 128) * 16, cudaMemcpyDeviceToHost, s));
   f128 *row_images_h = reinterpret_cast<f128 *>(folds_h + ncol);
-  BZ_CUDA(cudaMemcpyAsync(row_images_h, W.images.get(), 128 * 16, cudaMemcpyDeviceToHost, s));
   BZ_CUDA(cudaEventRecord(W.ev_folds, s));
   GkrScratch &gs = ctx.gkr_scratch(sc_cols);
   gs.live_cols = (S.h_len + 127) / 128;  // packed columns past h's last bit are all zero
-  gkr_build(hpk, sc_cols, W.images.get(), gs, s);
+  gkr_build(hpk, sc_cols, images, gs, s);
   u128 target_p = fp_canonical(so.final_claim, fc);
   // prove_virtual (crates/prover/src/prove.rs:96-152)
   t.public_message("bitz/virtual-statement/v1", 25);
@@ -795,23 +781,22 @@ int ProofSystem::prove_after_commit(cudaStream_t s, std::vector<uint8_t> &proof)
   ph.mark("fold");
   // gkr_reduce (crates/prover/src/reduce.rs:17-47); the layers were built above
   std::vector<f128> gpt(sc_cols + 7);
-  f128 gclaim = gkr_prove(hpk, sc_cols, W.images.get(), zeta.data(),
+  f128 gclaim = gkr_prove(hpk, sc_cols, images, zeta.data(),
                           grinding_bits((uint32_t)security_, 3), t, gs, s, gpt.data());
   f128 ip_target = gadd(gclaim, mk(1, 0));
   ph.mark("gkr");
-  std::vector<f128> eqb(128), u1(128);
+  std::vector<f128> eqb(128);
+  RowWeights128 u1;
   eq_table_host(gpt.data() + sc_cols, 7, eqb.data());
-  for (int b = 0; b < 128; b++) u1[b] = gmul(gadd(row_images[b], mk(1, 0)), eqb[b]);
-  W.u1.upload(u1.data(), 128, s);
+  for (int b = 0; b < 128; b++) u1.v[b] = gmul(gadd(row_images[b], mk(1, 0)), eqb[b]);
   W.u2.resize(ncol);
-  W.eqs.resize(eq_scratch_entries(sc_cols));
-  eq_table_device(gpt.data(), sc_cols, W.u2.get(), W.eqs.get(), s);
+  eq_table_device(gpt.data(), sc_cols, W.u2.get(), s);
   // transpose_query (crates/common/src/virtual_map.rs:174-223)
   size_t nbits = (size_t)1 << S.committed_m;
   W.weights.resize(nbits);
   W.w0.resize(2);
   W.mt_dense.resize((size_t)128 << sc_cols);
-  mt_transpose(dev_->csc_off.get(), dev_->csc_row.get(), S.f_bits + 1, W.u1.get(), W.u2.get(),
+  mt_transpose(dev_->csc_off.get(), dev_->csc_row.get(), S.f_bits + 1, u1, W.u2.get(),
                W.weights.get(), nbits, W.w0.get(), s, W.mt_dense.get(), sc_cols, S.h_len);
   f128 *w0_h = W.pin_small.get(kPinSmall) + kPinW0;
   // the inner-product statement's weight digest (opening.rs:337-368); the
@@ -879,14 +864,12 @@ int ProofSystem::prove_after_commit(cudaStream_t s, std::vector<uint8_t> &proof)
   int log_n = pcs_.log_n;
   size_t np = (size_t)1 << log_n;
   W.suffix.resize(np);
-  W.eqs.resize(eq_scratch_entries(log_n));
-  eq_table_device(rho.data() + 7, log_n, W.suffix.get(), W.eqs.get(), s);
-  BZ_CUDA(cudaMemsetAsync(W.acc.get(), 0, 256 * 8, s));
-  ring_claims(pa.packed, W.suffix.get(), np, W.acc.get(), s);
-  f128 *claims_h = W.pin_small.get(kPinSmall) + kPinClaims;
-  BZ_CUDA(cudaMemcpyAsync(claims_h, W.acc.get(), 128 * 16, cudaMemcpyDeviceToHost, s));
-  BZ_CUDA(stream_wait(s));
-  std::vector<f128> claims(claims_h, claims_h + 128);
+  eq_table_device(rho.data() + 7, log_n, W.suffix.get(), s);
+  RoundChannel *rch = ctx.channel();
+  const PassPost ring_post{W.acc.get(), rch->counter, rch->handover_dev, rch->arm().seq};
+  ring_claims(pa.packed, W.suffix.get(), np, ring_post, s);
+  std::vector<f128> claims(128);
+  rch->wait_handover(s, ring_post.seq, reinterpret_cast<uint64_t *>(claims.data()), 256);
   {
     std::vector<f128> pre(128);
     eq_table_host(rho.data(), 7, pre.data());
@@ -904,8 +887,9 @@ int ProofSystem::prove_after_commit(cudaStream_t s, std::vector<uint8_t> &proof)
   t.public_message("bitz/pcs/ring-switch-challenges/v1", 34);
   std::vector<f128> bpt(7);
   for (auto &c : bpt) c = t.challenge_f128();
-  std::vector<f128> bw(128);
-  eq_table_host(bpt.data(), 7, bw.data());
+  RowWeights128 basis_weights;
+  f128 *bw = basis_weights.v;
+  eq_table_host(bpt.data(), 7, bw);
   // transpose.rs:14: out[u].bit(v) = claims[v].bit(u), and the target is
   // sum over u of out[u] bw[u] = sum over v of X^v (sum over the set bits u
   // of claims[v] of bw[u]): one XOR per set bit and one shift per claim
@@ -916,7 +900,6 @@ int ProofSystem::prove_after_commit(cudaStream_t s, std::vector<uint8_t> &proof)
     for (uint64_t m = claims[vv].hi; m; m &= m - 1) sv = gadd(sv, bw[64 + __builtin_ctzll(m)]);
     ptarget = gadd(ptarget, gmul_xk(sv, vv));
   }
-  W.bw.upload(bw.data(), 128, s);
   W.lb.resize(np);
   W.lf.resize(np);
   W.lb2.resize(np);
@@ -928,7 +911,7 @@ int ProofSystem::prove_after_commit(cudaStream_t s, std::vector<uint8_t> &proof)
     coef = t.challenge_f128();
     ptarget = gadd(ptarget, gmul(coef, ood_value_));
   }
-  packed_basis(W.suffix.get(), np, W.bw.get(), security_ == 100 ? W.eq_ood.get() : nullptr, coef,
+  packed_basis(W.suffix.get(), np, basis_weights, security_ == 100 ? W.eq_ood.get() : nullptr, coef,
                W.lb.get(), s);
   BZ_CUDA(cudaMemcpyAsync(W.lf.get(), f_->get(), np * 16, cudaMemcpyDeviceToDevice, s));
   ph.mark("ring_switch");

@@ -39,12 +39,11 @@ constexpr size_t kPinFlag = 0, kPinRoot = 1, kPinLevelRoot = 3, kPinW0 = 5, kPin
 // Per-lane device workspace, grown on demand.
 struct Workspace {
   DeviceBuffer<int> flag;
-  DeviceBuffer<fp> sp_t, sp_d, sp_eqs, sp_part, sp_sums, sp_tab;
+  DeviceBuffer<fp> sp_t, sp_d, sp_part, sp_sums, sp_tab;
   DeviceBuffer<fp> cols_fp;
   DeviceBuffer<u128> exps, folds;
-  DeviceBuffer<f128> images, u1, u2, weights, w0, ones, eq, eqs, suffix, basis, eq_ood, lf, lb,
-      lf2, lb2, qs, level_cw, bw;
-  DeviceBuffer<uint32_t> b3, level_nodes;
+  DeviceBuffer<f128> images, u2, weights, w0, ones, eq, suffix, eq_ood, lf, lb, lf2, lb2;
+  DeviceBuffer<uint32_t> b3;
   DeviceBuffer<unsigned long long> acc;
   fp *host_fp = nullptr;
   uint64_t *host_acc = nullptr;
@@ -52,21 +51,19 @@ struct Workspace {
   // while the host absorbs earlier messages
   DeviceBuffer<fp> cols_canon;
   PinnedBuffer<u128> host_cols, host_folds;
-  // Ligerito: the next levels' codewords and trees, the query indices and the
+  // Ligerito: the next levels' codewords and trees, the
   // gathered openings, with their host copies
   DeviceBuffer<f128> lig_cw[2], openings;
   DeviceBuffer<uint32_t> lig_nodes[2];
-  DeviceBuffer<uint64_t> qidx;
   // the verifier: the hint bytes, the openings' combinations and each level's
   // path flag
   DeviceBuffer<uint32_t> v_hints;
-  DeviceBuffer<f128> v_vals, v_eqr;
+  DeviceBuffer<f128> v_vals;
   DeviceBuffer<unsigned int> v_bad;
   PinnedBuffer<uint32_t> pin_hints;
   PinnedBuffer<f128> pin_vals;
   PinnedBuffer<unsigned int> pin_bad;
-  PinnedBuffer<uint64_t> pin_idx;
-  PinnedBuffer<f128> pin_open, pin_f, pin_b, pin_qw, pin_small;
+  PinnedBuffer<f128> pin_open, pin_f, pin_b, pin_small;
   // the proof's own state: the staged statement, the witness, the level-0
   // codeword and tree
   DeviceBuffer<uint32_t> states, msgs, fin, f, h, bit_rows, nodes0;

@@ -23,43 +23,66 @@
 
 namespace bz {
 
-// Both factor tables in one launch: block 0 the low a coordinates, block 1
-// the high b.
-__global__ void k_fp_eq_factor(FpPoint p, int a, int b, FpCtx c, fp *lo, fp *hi) {
-  const int first = blockIdx.x == 0 ? 0 : a, n = blockIdx.x == 0 ? a : b;
-  fp *out = blockIdx.x == 0 ? lo : hi;
-  if (threadIdx.x == 0) out[0] = c.one;
-  __syncthreads();
-  for (int i = 0; i < n; i++) {
-    fp z = p.c[first + i];
-    int half = 1 << i;
-    for (int k = threadIdx.x; k < half; k += blockDim.x) {
-      fp par = out[k];
-      fp one = fp_mul(par, z, c);
-      out[k] = fp_sub(par, one, c);
-      out[k + half] = one;
+// eq over n coordinates (Montgomery) in one launch, as eq.cu's: the factors of
+// seven coordinates come from the host, a run of 128 entries shares the product
+// of the upper ones.
+struct FpEqFactors {
+  fp f[5][1 << kFacLog];
+};
+
+__global__ void __launch_bounds__(kThreads) k_fp_eq(const __grid_constant__ FpEqFactors eq, int n,
+                                                    int per, FpCtx c, fp *__restrict__ out) {
+  __shared__ fp H[16];
+  const int t = threadIdx.x;
+  const size_t total = (size_t)1 << n, step = (size_t)per * kThreads;
+  constexpr int kMask = (1 << kFacLog) - 1;
+  for (size_t base = blockIdx.x * step; base < total; base += gridDim.x * step) {
+    if (t < 2 * per) {
+      const size_t run = (base >> kFacLog) + t;
+      fp h = eq.f[1][run & kMask];
+#pragma unroll 1
+      for (int g = 2; g * kFacLog < n; g++)
+        h = fp_mul(h, eq.f[g][(run >> ((g - 1) * kFacLog)) & kMask], c);
+      H[t] = h;
     }
     __syncthreads();
+    for (int k = 0; k < per; k++) {
+      const size_t x = base + (size_t)k * kThreads + t;
+      if (x >= total) break;
+      out[x] = fp_mul(eq.f[0][x & kMask], H[(k * kThreads + t) >> kFacLog], c);
+    }
+    __syncthreads();  // the runs before the next ones
   }
 }
 
-__global__ void k_fp_eq_expand(const fp *__restrict__ lo, int a, const fp *__restrict__ hi,
-                               FpCtx c, fp *__restrict__ out, size_t total) {
-  size_t mask = ((size_t)1 << a) - 1;
-  for (size_t x = blockIdx.x * (size_t)blockDim.x + threadIdx.x; x < total;
-       x += (size_t)gridDim.x * blockDim.x)
-    out[x] = fp_mul(lo[x & mask], hi[x >> a], c);
+// eq over a run of coordinates, coordinate 0 in the lowest bit.
+static std::vector<fp> sp_eq(const fp *z, int n, const FpCtx &c, fp scale) {
+  std::vector<fp> e{scale};
+  e.reserve((size_t)1 << n);
+  for (int i = 0; i < n; i++) {
+    const size_t h = e.size();
+    e.resize(2 * h);
+    for (size_t k = 0; k < h; k++) {
+      const fp one = fp_mul(e[k], z[i], c);
+      e[k + h] = one;
+      e[k] = fp_sub(e[k], one, c);
+    }
+  }
+  return e;
 }
 
-void fp_eq_table(const fp *point, int n, const FpCtx &c, fp *out, fp *scratch, cudaStream_t s) {
-  FpPoint p;
-  for (int i = 0; i < n; i++) p.c[i] = point[i];
-  int a = n / 2, b = n - a;
-  fp *lo = scratch, *hi = scratch + ((size_t)1 << a);
-  k_fp_eq_factor<<<2, kThreads, 0, s>>>(p, a, b, c, lo, hi);
-  BZ_LAUNCH_CHECK();
-  size_t total = (size_t)1 << n;
-  k_fp_eq_expand<<<grid_for(total), kThreads, 0, s>>>(lo, a, hi, c, out, total);
+void fp_eq_table(const fp *point, int n, const FpCtx &c, fp *out, cudaStream_t s) {
+  if (n > 5 * kFacLog) throw CudaError("fp_eq_table: point too long");
+  FpEqFactors f{};
+  for (int g = 0; g < 5; g++) {
+    const std::vector<fp> e = sp_eq(point + g * kFacLog, std::min(kFacLog, std::max(0, n - g * kFacLog)),
+                                    c, c.one);
+    std::copy(e.begin(), e.end(), f.f[g]);
+  }
+  const size_t total = (size_t)1 << n;
+  int per = 1;
+  while (per < 8 && total / ((size_t)per * kThreads) >= 4 * kSMs) per *= 2;
+  k_fp_eq<<<grid_for(total, per * kThreads), kThreads, 0, s>>>(f, n, per, c, out);
   BZ_LAUNCH_CHECK();
 }
 
@@ -127,49 +150,60 @@ __global__ void k_bind_table(const int64_t *__restrict__ vals, const uint8_t *__
 
 // bind_and_batch (matrix.rs:429-467) as a gather over the column-major copy of
 // A, B and C: D(y) = sum over column y's entries of eq(r_x, row) * table[idx].
-// Column 0 (the constant, one entry per round constant and bit constraint)
-// is left to k_bind_col0, which spreads it over a whole grid.
-__global__ void k_bind(const uint32_t *__restrict__ off, const uint32_t *__restrict__ row,
-                       const uint16_t *__restrict__ idx, const fp *__restrict__ tab,
-                       const fp *__restrict__ eq, size_t cols, size_t padded, FpCtx c, fp *D) {
-  for (size_t y = blockIdx.x * (size_t)blockDim.x + threadIdx.x; y < padded;
-       y += (size_t)gridDim.x * blockDim.x) {
-    fp acc = fp_zero();
-    if (y > 0 && y < cols)
-      for (uint32_t e = off[y]; e < off[y + 1]; e++) acc = fp_add(acc, fp_mul(eq[row[e]], tab[idx[e]], c), c);
-    D[y] = acc;
+// Column 0 (the constant) has an entry per round constant and bit constraint,
+// so the launch's last `col0_blocks` blocks share it out, and with it the
+// statement-dependent part of C there: the bit constraints whose expected value
+// is one put rho^2 eq(r_x, row) there (each thread scales its share of those
+// rows, which sums to the same total mod q). The last of them to finish adds
+// the blocks' sums up.
+__global__ void __launch_bounds__(kThreads) k_bind(
+    const uint32_t *__restrict__ off, const uint32_t *__restrict__ row,
+    const uint16_t *__restrict__ idx, const fp *__restrict__ tab, const fp *__restrict__ eq,
+    size_t cols, size_t padded, const uint32_t *__restrict__ bit_rows, int n_bits, fp rho2,
+    int col0_blocks, FpCtx c, fp *partial, unsigned int *counter, fp *D) {
+  const int blocks = gridDim.x - col0_blocks;
+  if ((int)blockIdx.x < blocks) {
+    for (size_t y = blockIdx.x * (size_t)blockDim.x + threadIdx.x; y < padded;
+         y += (size_t)blocks * blockDim.x) {
+      if (y == 0) continue;
+      fp acc = fp_zero();
+      if (y < cols)
+        for (uint32_t e = off[y]; e < off[y + 1]; e++)
+          acc = fp_add(acc, fp_mul(eq[row[e]], tab[idx[e]], c), c);
+      D[y] = acc;
+    }
+    return;
   }
-}
-
-// Column 0's entries [0, n) split across blocks, and with them the
-// statement-dependent part of C on column 0: the bit constraints whose
-// expected value is one put rho^2 eq(r_x, row) there (each thread scales its
-// share of those rows, which sums to the same total mod q). Per-block
-// partial sums.
-__global__ void k_bind_col0(const uint32_t *__restrict__ row, const uint16_t *__restrict__ idx,
-                            const fp *__restrict__ tab, const fp *__restrict__ eq, uint32_t n,
-                            const uint32_t *__restrict__ bit_rows, int n_bits, fp rho2, FpCtx c,
-                            fp *partial) {
+  __shared__ bool last;
+  __shared__ fp total[1];
+  const int b = blockIdx.x - blocks, stride = col0_blocks * kThreads;
+  const uint32_t n = off[1];
   fp acc[1] = {fp_zero()};
-  for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x)
+  for (uint32_t e = b * kThreads + threadIdx.x; e < n; e += stride)
     acc[0] = fp_add(acc[0], fp_mul(eq[row[e]], tab[idx[e]], c), c);
   fp bits = fp_zero();
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_bits; i += gridDim.x * blockDim.x)
+  for (int i = b * kThreads + threadIdx.x; i < n_bits; i += stride)
     bits = fp_add(bits, eq[bit_rows[i]], c);
   acc[0] = fp_add(acc[0], fp_mul(bits, rho2, c), c);
-  block_fp_sum<1>(acc, c, partial);
-}
-
-// D[0] = the column-0 partial sums.
-__global__ void k_bind_col0_finish(const fp *partial, int nblocks, FpCtx c, fp *D) {
-  fp acc[1] = {fp_zero()};
-  for (int b = threadIdx.x; b < nblocks; b += blockDim.x) acc[0] = fp_add(acc[0], partial[b], c);
-  __shared__ fp out[1];
-  block_fp_sum<1>(acc, c, out);
+  block_fp_sum<1>(acc, c, partial + b - blockIdx.x);
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(counter, 1u) == (unsigned)col0_blocks - 1;
+    __threadfence();
+  }
   __syncthreads();
-  if (threadIdx.x == 0) D[0] = out[0];
+  if (!last) return;
+  acc[0] = fp_zero();
+  for (int k = threadIdx.x; k < col0_blocks; k += kThreads) {
+    const ulonglong2 w = __ldcg(reinterpret_cast<const ulonglong2 *>(partial + k));
+    acc[0] = fp_add(acc[0], fp{w.x, w.y}, c);
+  }
+  block_fp_sum<1>(acc, c, total - blockIdx.x);
+  if (threadIdx.x == 0) {
+    D[0] = total[0];
+    *counter = 0;
+  }
 }
-
 
 // ------------------------------------------------------------------ passes
 
@@ -594,21 +628,6 @@ static void sp_fold_points(std::vector<fp> &F, fp r, const FpCtx &c) {
   F.resize(block);
 }
 
-// eq over a run of coordinates, coordinate 0 in the lowest bit.
-static std::vector<fp> sp_eq(const fp *z, int n, const FpCtx &c, fp scale) {
-  std::vector<fp> e{scale};
-  for (int i = 0; i < n; i++) {
-    const size_t h = e.size();
-    e.resize(2 * h);
-    for (size_t k = 0; k < h; k++) {
-      const fp one = fp_mul(e[k], z[i], c);
-      e[k + h] = one;
-      e[k] = fp_sub(e[k], one, c);
-    }
-  }
-  return e;
-}
-
 static FpBind sp_bind_weights(const fp *r, int k, const FpCtx &c) {
   FpBind b{};
   const std::vector<fp> e = sp_eq(r, k, c, c.one);
@@ -643,6 +662,16 @@ static fp round_message(Transcript &ts, const FpCtx &c, fp &claim, const fp *wl,
   claim = v;
   for (int i = 0; i < ncoef; i++) coefs_out[i] = co[i];
   return r;
+}
+
+static void launch_bind(const SpartanArgs &a, const fp *tab, const fp *eq, fp rho2, size_t padded,
+                        const FpCtx &c, fp *partial, unsigned int *counter, fp *D,
+                        cudaStream_t s) {
+  const int col0 = grid_for(std::max<size_t>(a.col0_nnz, (size_t)a.n_bit_rows), 4 * kThreads, kSMs);
+  k_bind<<<grid_for(padded) + col0, kThreads, 0, s>>>(
+      a.csc_off, a.csc_row, a.csc_idx, tab, eq, a.cols, padded, a.bit_rows, a.n_bit_rows, rho2, col0,
+      c, partial, counter, D);
+  BZ_LAUNCH_CHECK();
 }
 
 void spartan_prove(const SpartanArgs &a, Transcript &ts, SpartanScratch &sc, cudaStream_t s,
@@ -795,22 +824,12 @@ void spartan_prove(const SpartanArgs &a, Transcript &ts, SpartanScratch &sc, cud
   claim = fp_add(fp_add(fin[0], fp_mul(rho, fin[1], c), c), fp_mul(rho2, fin[2], c), c);
   // bind: eq(r_x) over the rows, then the column gather
   fp *eq = sc.t[0];
-  fp_eq_table(out.rx.data(), nr, c, eq, sc.eq_scratch, s);
+  fp_eq_table(out.rx.data(), nr, c, eq, s);
   k_bind_table<<<(a.ntab + 127) / 128, 128, 0, s>>>(a.tab_vals, a.tab_which, a.ntab, rho, rho2, c,
                                                      sc.tab);
   BZ_LAUNCH_CHECK();
   fp *D = sc.d[0];
-  k_bind<<<grid_for(Cn), kThreads, 0, s>>>(a.csc_off, a.csc_row, a.csc_idx, sc.tab, eq, a.cols, Cn,
-                                           c, D);
-  BZ_LAUNCH_CHECK();
-  {
-    int g = grid_for(std::max<size_t>(a.col0_nnz, (size_t)a.n_bit_rows));
-    k_bind_col0<<<g, kThreads, 0, s>>>(a.csc_row, a.csc_idx, sc.tab, eq, a.col0_nnz, a.bit_rows,
-                                       a.n_bit_rows, rho2, c, sc.partial);
-    BZ_LAUNCH_CHECK();
-    k_bind_col0_finish<<<1, kThreads, 0, s>>>(sc.partial, g, c, D);
-    BZ_LAUNCH_CHECK();
-  }
+  launch_bind(a, sc.tab, eq, rho2, Cn, c, sc.partial, sc.counter, D, s);
   // inner sumcheck
   out.inner.resize(3 * (size_t)nc);
   out.ry.resize(nc);
@@ -952,24 +971,14 @@ fp spartan_matrix_eval(const SpartanArgs &a, const fp *rx, fp rho, const fp *ry,
   const fp rho2 = fp_mul(rho, rho, c);
   // the prover's bind at (r_x, rho): D(y) for every column y
   fp *eq = sc.t[0];
-  fp_eq_table(rx, nr, c, eq, sc.eq_scratch, s);
+  fp_eq_table(rx, nr, c, eq, s);
   k_bind_table<<<(a.ntab + 127) / 128, 128, 0, s>>>(a.tab_vals, a.tab_which, a.ntab, rho, rho2, c,
                                                      sc.tab);
   BZ_LAUNCH_CHECK();
   fp *D = sc.d[0], *EY = sc.d[1];
-  k_bind<<<grid_for(Cn), kThreads, 0, s>>>(a.csc_off, a.csc_row, a.csc_idx, sc.tab, eq, a.cols, Cn,
-                                           c, D);
-  BZ_LAUNCH_CHECK();
-  {
-    int g = grid_for(std::max<size_t>(a.col0_nnz, (size_t)a.n_bit_rows));
-    k_bind_col0<<<g, kThreads, 0, s>>>(a.csc_row, a.csc_idx, sc.tab, eq, a.col0_nnz, a.bit_rows,
-                                       a.n_bit_rows, rho2, c, sc.partial);
-    BZ_LAUNCH_CHECK();
-    k_bind_col0_finish<<<1, kThreads, 0, s>>>(sc.partial, g, c, D);
-    BZ_LAUNCH_CHECK();
-  }
+  launch_bind(a, sc.tab, eq, rho2, Cn, c, sc.partial, sc.counter, D, s);
   // then sum_y D(y) eq(r_y, y)
-  fp_eq_table(ry, nc, c, EY, sc.eq_scratch, s);
+  fp_eq_table(ry, nc, c, EY, s);
   const int g = grid_for(Cn);
   k_fp_dot<<<g, kThreads, 0, s>>>(D, EY, Cn, c, sc.partial);
   BZ_LAUNCH_CHECK();
@@ -1044,8 +1053,7 @@ fp fp_to_mont(u128 v, const FpCtx &c) { return fp_mul(fp{(uint64_t)v, (uint64_t)
 // Every kernel of this file, loaded when the process's first lane on a device
 // is made (lane_bootstrap, context.cpp).
 void preload_spartan_kernels() {
-  load_kernels({(const void *)k_fp_eq_factor,
-                (const void *)k_fp_eq_expand,
+  load_kernels({(const void *)k_fp_eq,
                 (const void *)k_products_to_fp,
                 (const void *)k_fp_finalize,
                 (const void *)sp_outer_pass<3>,
@@ -1056,8 +1064,6 @@ void preload_spartan_kernels() {
                 (const void *)sp_handover<false>,
                 (const void *)k_bind_table,
                 (const void *)k_bind,
-                (const void *)k_bind_col0,
-                (const void *)k_bind_col0_finish,
                 (const void *)k_fp_dot,
                 (const void *)k_fold_claim,
                 (const void *)k_fp_canonical});

@@ -36,11 +36,11 @@ struct SpartanArgs {
 struct SpartanScratch {
   fp *t[8];        // eq over the rows (0), A, B, C (1-3) and their bound forms (4-6), 2^rows each
   fp *d[4];        // D (0) and the bound D and W (2, 3, then 0, 1), 2^cols each
-  fp *eq_scratch;  // factor tables
   fp *partial;     // per-block partial sums, kSpPartials entries
   fp *sums;        // device, 3 entries
   fp *tab;         // coefficient table, ntab entries
   fp *host;        // pinned, 4 entries
+  unsigned int *counter = nullptr;  // finished blocks: zero before and after a kernel
   RoundChannel *channel = nullptr;  // carries the passes' sums and the last tables
 };
 
@@ -59,7 +59,8 @@ u128 fp_canonical(fp mont, const FpCtx &c);
 // out[k] = canonical value of in[k] (as two LE words), on the device.
 void fp_canonical_device(const fp *in, size_t n, const FpCtx &c, fp *out, cudaStream_t s);
 fp fp_to_mont(u128 v, const FpCtx &c);
-void fp_eq_table(const fp *point, int n, const FpCtx &c, fp *out, fp *scratch, cudaStream_t s);
+// out[x] = eq(point, x) for x < 2^n (Montgomery).
+void fp_eq_table(const fp *point, int n, const FpCtx &c, fp *out, cudaStream_t s);
 
 void spartan_prove(const SpartanArgs &a, Transcript &ts, SpartanScratch &sc, cudaStream_t s,
                    SpartanOut &out);
@@ -67,7 +68,7 @@ void spartan_prove(const SpartanArgs &a, Transcript &ts, SpartanScratch &sc, cud
 // rho^2 C (with the statement's bit constants in C) of eq(r_x, row) eq(r_y,
 // col) times the entry, on the device through the prover's bind (the dense
 // D(y) over the columns) and a dot product with eq(r_y). Montgomery in and
-// out; uses sc.t[0], sc.d[0..1], eq_scratch, partial, sums, tab and host.
+// out; uses sc.t[0], sc.d[0..1], partial, sums, tab, counter and host.
 fp spartan_matrix_eval(const SpartanArgs &a, const fp *rx, fp rho, const fp *ry,
                        SpartanScratch &sc, cudaStream_t s);
 

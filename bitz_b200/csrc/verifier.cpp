@@ -290,7 +290,6 @@ int ProofSystem::verify(const uint8_t *proof, size_t proof_len, Context *lane) {
   const size_t R = (size_t)1 << nr, Cn = (size_t)1 << nc;
   W.sp_t.resize(8 * R);
   W.sp_d.resize(4 * Cn);
-  W.sp_eqs.resize(4096 * 2 + ((size_t)1 << ((std::max(nr, nc) + 1) / 2 + 1)));
   W.sp_part.resize(kSpPartials);
   W.sp_sums.resize(4);
   W.sp_tab.resize(dev_->ntab + 1);
@@ -301,7 +300,7 @@ int ProofSystem::verify(const uint8_t *proof, size_t proof_len, Context *lane) {
   SpartanScratch sc;
   for (int i = 0; i < 8; i++) sc.t[i] = W.sp_t.get() + i * R;
   for (int i = 0; i < 4; i++) sc.d[i] = W.sp_d.get() + i * Cn;
-  sc.eq_scratch = W.sp_eqs.get();
+  sc.counter = ctx.channel()->counter;
   sc.partial = W.sp_part.get();
   sc.sums = W.sp_sums.get();
   sc.tab = W.sp_tab.get();
@@ -336,7 +335,7 @@ int ProofSystem::verify(const uint8_t *proof, size_t proof_len, Context *lane) {
   }
   W.cols_fp.resize(ncol + 2);
   W.cols_canon.resize(ncol);
-  fp_eq_table(pt.data() + 7, sc_cols, fc, W.cols_fp.get(), sc.eq_scratch, s);
+  fp_eq_table(pt.data() + 7, sc_cols, fc, W.cols_fp.get(), s);
   fp_canonical_device(W.cols_fp.get(), ncol, fc, W.cols_canon.get(), s);
   u128 *cols_w = W.host_cols.get(ncol);
   BZ_CUDA(cudaMemcpyAsync(cols_w, W.cols_canon.get(), ncol * 16, cudaMemcpyDeviceToHost, s));
@@ -392,11 +391,10 @@ int ProofSystem::verify(const uint8_t *proof, size_t proof_len, Context *lane) {
   for (auto &z : point) z = t.challenge_f128();
   // ---- gpgkr_verify (crates/gkr/src/lib.rs:717-772) from e0 = MLE(images)(zeta)
   W.u2.resize(ncol);
-  W.eqs.resize(eq_scratch_entries(std::max(sc_cols, std::max(m, log_n))));
   W.acc.resize(512);
-  eq_table_device(point.data(), sc_cols, W.u2.get(), W.eqs.get(), s);
   BZ_CUDA(cudaMemsetAsync(W.acc.get(), 0, 16, s));
-  dot(W.u2.get(), W.images.get() + 128, ncol, W.acc.get(), Publish{nullptr, nullptr, 0}, s);
+  eq_table_dot(point.data(), sc_cols, W.u2.get(), W.images.get() + 128, W.acc.get(),
+               Publish{nullptr, nullptr, 0}, s);
   BZ_CUDA(cudaMemcpyAsync(W.host_acc, W.acc.get(), 16, cudaMemcpyDeviceToHost, s));
   BZ_CUDA(stream_wait(s));
   BZ_VERIFY(fp_canonical(sc.host[0], fc) == fin_c, "the column folds do not meet the Spartan claim");
@@ -447,16 +445,16 @@ int ProofSystem::verify(const uint8_t *proof, size_t proof_len, Context *lane) {
   // ---- gkr_reduce's claim (crates/verifier/src/reduce.rs:27-54) and the
   // transposed query (virtual_map.rs:174-223), on the device as the prover
   const f128 ip_target = gadd(gclaim, kOne);
-  std::vector<f128> eqb(128), u1(128);
+  std::vector<f128> eqb(128);
+  RowWeights128 u1;
   eq_table_host(point.data() + sc_cols, 7, eqb.data());
-  for (int b = 0; b < 128; b++) u1[b] = gmul(gadd(row_images[b], kOne), eqb[b]);
-  W.u1.upload(u1.data(), 128, s);
-  eq_table_device(point.data(), sc_cols, W.u2.get(), W.eqs.get(), s);
+  for (int b = 0; b < 128; b++) u1.v[b] = gmul(gadd(row_images[b], kOne), eqb[b]);
+  eq_table_device(point.data(), sc_cols, W.u2.get(), s);
   const size_t nbits = (size_t)1 << m;
   W.weights.resize(nbits);
   W.w0.resize(2);
   W.mt_dense.resize((size_t)128 << sc_cols);
-  mt_transpose(dev_->csc_off.get(), dev_->csc_row.get(), S.f_bits + 1, W.u1.get(), W.u2.get(),
+  mt_transpose(dev_->csc_off.get(), dev_->csc_row.get(), S.f_bits + 1, u1, W.u2.get(),
                W.weights.get(), nbits, W.w0.get(), s, W.mt_dense.get(), sc_cols, S.h_len);
   // the weight digest (opening.rs:337-368): the weights' chunk tree on the
   // device, the trailing column weight [1] and the root here
@@ -504,9 +502,9 @@ int ProofSystem::verify(const uint8_t *proof, size_t proof_len, Context *lane) {
   {
     // MLE(weights)(rho) on the device: eq(rho, .) against the weights
     W.eq.resize(nbits);
-    eq_table_device(rho_pt.data(), m, W.eq.get(), W.eqs.get(), s);
     BZ_CUDA(cudaMemsetAsync(W.acc.get(), 0, 16, s));
-    dot(W.eq.get(), W.weights.get(), nbits, W.acc.get(), Publish{nullptr, nullptr, 0}, s);
+    eq_table_dot(rho_pt.data(), m, W.eq.get(), W.weights.get(), W.acc.get(),
+                 Publish{nullptr, nullptr, 0}, s);
     BZ_CUDA(cudaMemcpyAsync(W.host_acc, W.acc.get(), 16, cudaMemcpyDeviceToHost, s));
     BZ_CUDA(stream_wait(s));
     const f128 wv = mk(W.host_acc[0], W.host_acc[1]);
@@ -534,9 +532,11 @@ int ProofSystem::verify(const uint8_t *proof, size_t proof_len, Context *lane) {
                      grinding_bits((uint32_t)security_, 7 + (security_ == 100 ? 1 : 0))),
             "ring-switch grinding nonce");
   t.public_message("bitz/pcs/ring-switch-challenges/v1", 34);
-  std::vector<f128> bpt(7), bw(128);
+  std::vector<f128> bpt(7);
   for (auto &c : bpt) c = t.challenge_f128();
-  eq_table_host(bpt.data(), 7, bw.data());
+  RowWeights128 basis_weights;
+  f128 *bw = basis_weights.v;
+  eq_table_host(bpt.data(), 7, bw);
   // transpose.rs:14: the target is sum over v of X^v (sum over the set bits
   // u of claims[v] of bw[u])
   f128 ptarget = mk(0, 0);
@@ -548,8 +548,7 @@ int ProofSystem::verify(const uint8_t *proof, size_t proof_len, Context *lane) {
   }
   const size_t np = (size_t)1 << log_n;
   W.suffix.resize(np);
-  eq_table_device(rho_pt.data() + 7, log_n, W.suffix.get(), W.eqs.get(), s);
-  W.bw.upload(bw.data(), 128, s);
+  eq_table_device(rho_pt.data() + 7, log_n, W.suffix.get(), s);
   W.lb.resize(np);
   W.lb2.resize(np);
   W.eq.resize(np);
@@ -559,9 +558,9 @@ int ProofSystem::verify(const uint8_t *proof, size_t proof_len, Context *lane) {
     coef = t.challenge_f128();
     ptarget = gadd(ptarget, gmul(coef, ood_val));
     W.eq_ood.resize(np);
-    eq_table_device(ood_pt.data(), log_n, W.eq_ood.get(), W.eqs.get(), s);
+    eq_table_device(ood_pt.data(), log_n, W.eq_ood.get(), s);
   }
-  packed_basis(W.suffix.get(), np, W.bw.get(), security_ == 100 ? W.eq_ood.get() : nullptr, coef,
+  packed_basis(W.suffix.get(), np, basis_weights, security_ == 100 ? W.eq_ood.get() : nullptr, coef,
                W.lb.get(), s);
   // ---- the Ligerito opening (this library's construction, prover.cpp)
   const uint8_t *lhead = hs.take(4);
@@ -678,7 +677,7 @@ int ProofSystem::verify(const uint8_t *proof, size_t proof_len, Context *lane) {
         const std::vector<f128> opt = sample_vec((size_t)l);
         const f128 ov = rd.f();
         const f128 mu = t.challenge_f128();
-        eq_table_device(opt.data(), l, W.eq.get(), W.eqs.get(), s);
+        eq_table_device(opt.data(), l, W.eq.get(), s);
         axpy(b, mu, W.eq.get(), n, s);  // basis += mu eq(point, .)
         lclaim = gadd(lclaim, gmul(mu, ov));
       }
@@ -702,8 +701,13 @@ int ProofSystem::verify(const uint8_t *proof, size_t proof_len, Context *lane) {
     BZ_VERIFY_OPENING(nq == (uint64_t)L.queries, "a level's query count");
     std::vector<f128> eqr((size_t)1 << L.k);
     eq_table_host(rs.data(), L.k, eqr.data());
-    std::vector<uint64_t> idx(L.queries);
-    for (int qi = 0; qi < L.queries; qi++) idx[qi] = qs[qi].lo & (rows - 1);
+    if (L.queries > kMaxQueries || width > kMaxQueryWidth)
+      throw std::runtime_error("ligerito: too many queries or too wide a row");
+    QueryRows queried;
+    QueryTerms terms;
+    for (int qi = 0; qi < L.queries; qi++)
+      queried.idx[qi] = terms.idx[qi] = qs[qi].lo & (rows - 1);
+    std::copy(eqr.begin(), eqr.begin() + width, queried.eqr);
     const size_t level_at = hs.pos, row_bytes = (size_t)width * 16;
     const size_t whole = (hs.len - hs.pos) / (row_bytes + 32 * (size_t)depth);
     if (whole < (size_t)L.queries) {  // the stream ends at an opening's row or path
@@ -712,12 +716,10 @@ int ProofSystem::verify(const uint8_t *proof, size_t proof_len, Context *lane) {
       BZ_VERIFY_OPENING(false, "the hint stream ends inside a Merkle path");
     }
     hs.take((size_t)L.queries * (row_bytes + 32 * (size_t)depth));
-    W.qidx.upload(idx.data(), idx.size(), s);
-    W.v_eqr.upload(eqr.data(), eqr.size(), s);
     B3Root want;
     b3_load_le(cur_root, want.w, 8);
-    check_openings(W.v_hints.get(), level_at / 4, width, depth, W.qidx.get(), L.queries,
-                   W.v_eqr.get(), want, W.v_vals.get() + opened_queries, W.v_bad.get() + i, s);
+    check_openings(W.v_hints.get(), level_at / 4, width, depth, queried, L.queries, want,
+                   W.v_vals.get() + opened_queries, W.v_bad.get() + i, s);
     const int av = ceil_log2((size_t)L.queries);
     const std::vector<f128> alpha = sample_vec((size_t)av);
     const f128 mu = t.challenge_f128();
@@ -725,8 +727,8 @@ int ProofSystem::verify(const uint8_t *proof, size_t proof_len, Context *lane) {
     eq_table_host(alpha.data(), av, beta.data());
     for (int qi = 0; qi < L.queries; qi++) sq[qi] = gmul(mu, beta[qi]);
     // the glue on the device: basis += sum_q s_q X(x_q)
-    W.qs.upload(sq.data(), sq.size(), s);
-    query_basis(W.qidx.get(), T.wh.get(), W.qs.get(), L.queries, l, b, s);
+    std::copy(sq.begin(), sq.end(), terms.scale);
+    query_basis(terms, T.wh.get(), L.queries, l, b, s);
     opened.push_back(Opened{std::move(sq), opened_queries, kOne});
     opened_queries += (size_t)L.queries;
     if (!last) {
