@@ -250,6 +250,10 @@ AllocScope::~AllocScope() {
   if (on_ && --gate_depth().alloc == 0) DeviceGate::get().leave_alloc();
 }
 
+// Tiles of a small pass on a pooled lane (pass_tile_log); the default lane has
+// one per SM.
+constexpr int kPoolPassBlocks = 32;
+
 Context::Context() {
   AllocScope gate;
   BZ_CUDA(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
@@ -277,6 +281,7 @@ Context::Context() {
   channel_.handover_dev = (unsigned long long *)((char *)mbd + 4096);
   counter_.resize(1);
   BZ_CUDA(cudaMemset(counter_.get(), 0, sizeof(unsigned int)));
+  channel_.pass_blocks = kPoolPassBlocks;
   channel_.counter = counter_.get();
   pg_.channel = &channel_;
   gk_.channel = &channel_;
@@ -305,6 +310,7 @@ Context &Context::get() {
   // launches (or 32-block grids with BITZ_POOL_MID=1).
   static Context *ctx = [] {
     Context *c = new Context();
+    c->channel_.pass_blocks = kSMs;
     return c;
   }();
   return *ctx;

@@ -229,6 +229,8 @@ struct RoundChannel {
   // the host's challenge between them: same tagged format, host to device.
   Mailbox *down_host = nullptr, *down_dev = nullptr;
   unsigned long long down_next = 0;
+  // Tiles a sumcheck pass of this lane is split into where its size allows.
+  int pass_blocks = kSMs;
   // host time spent inside wait() and the number of waits (phase timer)
   unsigned long long wait_ns = 0, waits = 0;
   // A word in the same mapped page that the lane's kernels set when a bounded

@@ -595,7 +595,7 @@ constexpr int kFirstLog = 17;
 template <int K, bool kLow>
 static int launch_pass_as(f128 *c, size_t n_half, int log_m, const PassBind &b, const EqHeap *heap,
                           const f128 *eq_low, size_t colmask, uint32_t live, uint32_t count,
-                          const PassPost &post, cudaStream_t st) {
+                          int spread, const PassPost &post, cudaStream_t st) {
   using S = PassShape<K, kLow>;
   EqFactors<S::kFactors> eq;
   const int skip = kLow ? 2 : 0;  // factors that eq_low holds
@@ -603,7 +603,7 @@ static int launch_pass_as(f128 *c, size_t n_half, int log_m, const PassBind &b, 
     const int have = std::min(kFacLog, std::max(0, log_m - (g + skip) * kFacLog));
     memcpy(eq.f[g], heap[g + skip].prefix(have), sizeof(f128) << have);
   }
-  int lx = pass_tile_log(count);
+  int lx = pass_tile_log(count, spread);
   if (lx == 5 && (count >> S::kMaxLx) >= 2u * kSMs) lx = S::kMaxLx;
   const uint32_t tiles = (count + (1u << lx) - 1) >> lx;
   const unsigned int grid =
@@ -617,9 +617,9 @@ static int launch_pass_as(f128 *c, size_t n_half, int log_m, const PassBind &b, 
 template <int K>
 static int launch_pass(f128 *c, size_t n_half, int log_m, const PassBind &b, const EqHeap *heap,
                        const f128 *eq_low, size_t colmask, uint32_t live, uint32_t count,
-                       const PassPost &post, cudaStream_t st) {
+                       int spread, const PassPost &post, cudaStream_t st) {
   return (log_m <= kEqLowLog ? launch_pass_as<K, false> : launch_pass_as<K, true>)(
-      c, n_half, log_m, b, heap, eq_low, colmask, live, count, post, st);
+      c, n_half, log_m, b, heap, eq_low, colmask, live, count, spread, post, st);
 }
 
 void gkr_build(const f128 *cols, int s, const f128 *images, GkrScratch &sc, cudaStream_t st_) {
@@ -810,7 +810,8 @@ f128 gkr_prove(const f128 *cols, int s, const f128 *images, const f128 *zeta, ui
       if (probed) probe.before(st_);
       const PassPost post{sc.acc, ch->counter, ch->handover_dev, ch->arm().seq};
       const int blocks = (k == 2 ? launch_pass<2> : launch_pass<3>)(
-          c, n_half, log_m, b, heap.data(), sc.eq_low, colmask, (uint32_t)live, count, post, st_);
+          c, n_half, log_m, b, heap.data(), sc.eq_low, colmask, (uint32_t)live, count, ch->pass_blocks,
+          post, st_);
       if (probed) {
         // per live position: 2^(k+1) entries of the bound tables, each from
         // 2^kb read and one written (none written without a bind), 2^kb - 1

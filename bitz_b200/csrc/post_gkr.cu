@@ -354,7 +354,7 @@ static int launch_quad(const f128 *w, const f128 *v, f128 *w2, f128 *v2, size_t 
                         const PassBind &b, const BitWeights &e8, const PassPost &post,
                         cudaStream_t s) {
   const uint32_t count = (uint32_t)(n >> K);
-  const int lx = pass_tile_log(count);
+  const int lx = pass_tile_log(count, post.blocks);
   const unsigned int grid = pass_grid(count, lx);
   pg_pass<K, kBits><<<grid, kPassThreads, 0, s>>>(w, v, w2, v2, count, b, e8, lx, post);
   BZ_LAUNCH_CHECK();
@@ -417,8 +417,8 @@ struct PostGkrRun {
   PassPost arm() {
     if (sc.channel)
       return PassPost{sc.acc, sc.channel->counter, sc.channel->handover_dev,
-                      sc.channel->arm().seq};
-    return PassPost{sc.acc, sc.counter, sc.handover, ++sc.seq};
+                      sc.channel->arm().seq, sc.channel->pass_blocks};
+    return PassPost{sc.acc, sc.counter, sc.handover, ++sc.seq, kSMs};
   }
   void wait(const PassPost &post, int n) {
     if (sc.channel) {

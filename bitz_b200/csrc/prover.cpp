@@ -488,7 +488,7 @@ std::vector<uint8_t> ProofSystem::ligerito(cudaStream_t s, f128 target) {
     PassBind pb{};
     for (int r = 0; r < L.k;) {
       const int k = std::min(kPassMaxK, L.k - r), points = pow3(k);
-      const PassPost post{acc, ch->counter, ch->handover_dev, ch->arm().seq};
+      const PassPost post{acc, ch->counter, ch->handover_dev, ch->arm().seq, ch->pass_blocks};
       n >>= pb.k;
       const int blocks = quad_pass(k, b, f, b2, f2, n, pb, post, s);
       if (pb.k) {

@@ -755,7 +755,7 @@ void spartan_prove(const SpartanArgs &a, Transcript &ts, SpartanScratch &sc, cud
       const size_t live_out = (live + (((size_t)1 << b.k) - 1)) >> b.k;
       // positions past the live entries add nothing
       const uint32_t count = (uint32_t)((live_out + ((size_t)1 << k) - 1) >> k);
-      const int lx = pass_tile_log(count);
+      const int lx = pass_tile_log(count, ch->pass_blocks);
       const unsigned int grid = pass_grid(count, lx);
       const bool probed = probe.on("sp_outer_pass");
       if (probed) probe.before(s);
@@ -895,7 +895,7 @@ void spartan_prove(const SpartanArgs &a, Transcript &ts, SpartanScratch &sc, cud
       const int k = kPassMaxK, points = pow3(k);
       const size_t live_out = (live + (((size_t)1 << b.k) - 1)) >> b.k;
       const uint32_t count = (uint32_t)((live_out + ((size_t)1 << k) - 1) >> k);
-      const int lx = pass_tile_log(count);
+      const int lx = pass_tile_log(count, ch->pass_blocks);
       const unsigned int grid = pass_grid(count, lx);
       const bool probed = probe.on("sp_inner_pass");
       if (probed) probe.before(s);
