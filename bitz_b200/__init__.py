@@ -90,10 +90,10 @@ def round_wait_stats():
 
 
 def gate_stats():
-    """The device gate since the process started: lanes whose kernels may wait
-    for their host thread hold it as resident stretches; device and pinned
-    allocations wait until none is held. Returns a dict of the allocation and
-    resident stretch counts and the seconds each kind waited."""
+    """The device gate since the process started: device and pinned
+    allocations pass it one at a time. Returns a dict of the allocation
+    stretches and the seconds they waited; the resident entries (kernels that
+    wait for their host thread) are zero, no proof launches such a kernel."""
     out = (ctypes.c_ulonglong * 4)()
     _check(_lib.load().bitz_gate_stats(out))
     return {"allocs": int(out[0]), "alloc_wait_s": out[1] * 1e-9,

@@ -5,7 +5,7 @@
 // the buffers of the lane that computed them, so a staged proof holds that
 // lane from bitz_witness until bitz_prove consumes it (or a handle is freed).
 // The lane is the process's default lane when no other staged proof or
-// single-call proof holds it (it keeps the middle sumcheck rounds resident),
+// single-call proof holds it (its passes use a tile per SM),
 // else one from the lane pool.
 #include <stdlib.h>
 #include <string.h>

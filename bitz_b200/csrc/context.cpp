@@ -171,48 +171,22 @@ static unsigned long long ns_since(std::chrono::steady_clock::time_point t0) {
       .count();
 }
 
-void DeviceGate::enter_resident() {
-  std::unique_lock<std::mutex> lk(mu_);
-  resident_n_++;
-  if (alloc_ || allocs_waiting_ != 0) {
-    const auto t0 = std::chrono::steady_clock::now();
-    if (in_fiber()) {
-      while (alloc_ || allocs_waiting_ != 0) {
-        lk.unlock();
-        fiber_yield();
-        lk.lock();
-      }
-    } else {
-      cv_.wait(lk, [&] { return !alloc_ && allocs_waiting_ == 0; });
-    }
-    resident_wait_ns_ += ns_since(t0);
-  }
-  residents_++;
-}
-
-void DeviceGate::leave_resident() {
-  std::lock_guard<std::mutex> lk(mu_);
-  if (--residents_ == 0) cv_.notify_all();
-}
-
 void DeviceGate::enter_alloc() {
   std::unique_lock<std::mutex> lk(mu_);
   alloc_n_++;
-  allocs_waiting_++;
-  if (alloc_ || residents_ != 0) {
+  if (alloc_) {
     const auto t0 = std::chrono::steady_clock::now();
     if (in_fiber()) {
-      while (alloc_ || residents_ != 0) {
+      while (alloc_) {
         lk.unlock();
         fiber_yield();
         lk.lock();
       }
     } else {
-      cv_.wait(lk, [&] { return !alloc_ && residents_ == 0; });
+      cv_.wait(lk, [&] { return !alloc_; });
     }
     alloc_wait_ns_ += ns_since(t0);
   }
-  allocs_waiting_--;
   alloc_ = true;
 }
 
@@ -225,29 +199,15 @@ void DeviceGate::leave_alloc() {
 void DeviceGate::stats(unsigned long long out[4]) const {
   out[0] = alloc_n_.load();
   out[1] = alloc_wait_ns_.load();
-  out[2] = resident_n_.load();
-  out[3] = resident_wait_ns_.load();
+  out[2] = out[3] = 0;
 }
 
-ResidentScope::ResidentScope(bool on) : on_(on) {
-  if (on_ && gate_depth().resident++ == 0) DeviceGate::get().enter_resident();
-}
-
-ResidentScope::~ResidentScope() {
-  if (on_ && --gate_depth().resident == 0) DeviceGate::get().leave_resident();
-}
-
-AllocScope::AllocScope(bool strict) {
-  if (gate_depth().resident > 0) {
-    if (strict) throw CudaError("device allocation while a round kernel of this lane may wait");
-    return;  // unwinding out of a resident stretch: free without the gate
-  }
-  on_ = true;
+AllocScope::AllocScope() {
   if (gate_depth().alloc++ == 0) DeviceGate::get().enter_alloc();
 }
 
 AllocScope::~AllocScope() {
-  if (on_ && --gate_depth().alloc == 0) DeviceGate::get().leave_alloc();
+  if (--gate_depth().alloc == 0) DeviceGate::get().leave_alloc();
 }
 
 // Tiles of a small pass on a pooled lane (pass_tile_log); the default lane has
@@ -258,10 +218,8 @@ Context::Context() {
   AllocScope gate;
   BZ_CUDA(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
   acc_.resize(8 * 128);
-  BZ_CUDA(cudaMallocHost(&host_, 64 * sizeof(uint64_t)));
   pg_.acc = acc_.get();
   gk_.acc = acc_.get();
-  gk_ctl_.resize(kMaxPointGkr);
   // the round mailbox: one mapped pinned page and a device block counter
   void *mb = nullptr;
   // one mapped allocation: mailbox (0), downbox (512), error word (1024),
@@ -291,9 +249,8 @@ Context::Context() {
 Context::~Context() {
   if (stream_) cudaStreamSynchronize(stream_);
   workspace.reset();
-  AllocScope gate(false);
+  AllocScope gate;
   if (channel_.host) cudaFreeHost(channel_.host);
-  if (host_) cudaFreeHost(host_);
   if (stream_) cudaStreamDestroy(stream_);
 }
 
@@ -304,10 +261,8 @@ std::atomic<unsigned long long> &launch_counter() {
 
 Context &Context::get() {
   // One default lane per process, created on first use on the current device.
-  // It proves one statement at a time with the GPU to itself, so its resident
-  // middle rounds (Spartan) use grids of 128
-  // blocks; pool lanes, which share the GPU, run those rounds as queued
-  // launches (or 32-block grids with BITZ_POOL_MID=1).
+  // It proves one statement at a time with the GPU to itself, so its passes use
+  // a tile per SM; pool lanes share the GPU and use kPoolPassBlocks.
   static Context *ctx = [] {
     Context *c = new Context();
     c->channel_.pass_blocks = kSMs;

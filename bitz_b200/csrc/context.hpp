@@ -41,7 +41,7 @@ class DeviceBuffer {
   }
   void release() {
     if (p_) {
-      AllocScope gate(false);
+      AllocScope gate;
       cudaFree(p_);
     }
     p_ = nullptr;
@@ -69,7 +69,7 @@ class PinnedBuffer {
   PinnedBuffer() = default;
   ~PinnedBuffer() {
     if (p_) {
-      AllocScope gate(false);
+      AllocScope gate;
       cudaFreeHost(p_);
     }
   }
@@ -109,8 +109,6 @@ class Context {
 
   cudaStream_t stream() const { return stream_; }
   RoundChannel *channel() { return &channel_; }
-  // The lane's round controls (kMaxPointGkr entries), used by one phase at a time.
-  RoundCtl *round_ctl() { return gk_ctl_.get(); }
   // Prover workspace slot, owned by the lane (created by the prover).
   std::shared_ptr<Workspace> workspace;
 
@@ -165,18 +163,15 @@ class Context {
   PostGkrScratch pg_;
   DeviceBuffer<f128> pg_w0_, pg_v0_, pg_w1_, pg_v1_;
   DeviceBuffer<unsigned long long> acc_;
-  uint64_t *host_ = nullptr;
   GkrScratch gk_;
   DeviceBuffer<f128> gk_layers_, gk_mid_;
   DeviceBuffer<unsigned long long> gk_gram_;
-  DeviceBuffer<RoundCtl> gk_ctl_;
   RoundChannel channel_;
   DeviceBuffer<unsigned int> counter_;
 };
 
 // Loads kernels now (cudaFuncGetAttributes), so no kernel is loaded on its
-// first launch while a kernel that waits for a host thread is in flight: a
-// load may wait for the running kernels to finish.
+// first launch inside a proof: a load may wait for the running kernels to finish.
 void load_kernels(std::initializer_list<const void *> kernels);
 
 // A lane held for one proof: the process's default lane when no other proof

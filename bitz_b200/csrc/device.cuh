@@ -255,96 +255,40 @@ struct RoundChannel {
   void clear_down();
 };
 
-// Queued sumcheck rounds. With the host's challenges delivered to the
-// device, the rounds of a sumcheck can all be queued at its start, so no
-// round waits for a launch from the host: the last block of each round
-// kernel posts the round's message, then waits (bounded) for the next
-// challenge in the lane's downbox and leaves it in `out` for the next kernel
-// in the stream, which reads it from `in`. Only that one block waits; the
-// next kernel starts when it has left. A missing challenge (time limit or
-// the host's abort marker) leaves flag 2, and every later kernel of the chain
-// passes it on and does no work.
-//
-// RoundCtl: one challenge in device memory (flag 1: valid, 2: the chain
-// stopped); `done` counts the blocks of a resident kernel through a round.
-struct RoundCtl {
-  unsigned long long r_lo, r_hi;
-  unsigned int flag, done;
-  unsigned long long pad;
-};
-
-struct RoundLink {
-  const RoundCtl *in;       // this round's challenge; null: the launch argument
-  RoundCtl *out;            // the next challenge; null: no wait
-  const Mailbox *down;      // the host's downbox
-  unsigned long long dseq;  // the host's publication of the next challenge
-};
-constexpr unsigned long long kRoundWaitNs = 2000000000ull;  // 2 s per challenge
-
-// Whether kernels that wait for their lane's host thread may run (resident
-// tails, queued rounds, the resident middle rounds). BITZ_RESIDENT_ROUNDS=0
-// turns them off and =1 on. Otherwise they are off when a CUDA injection tool
-// announces itself (CUDA_INJECTION64_PATH), or when the process's first lane
-// found that its host thread cannot reach a running kernel (a kernel that
-// waits up to 100 ms for one word from the host got none): a kernel profiler
-// holds the host at every launch until the kernel has finished, so a kernel
-// that waits for the host would sit out its time limit. The proof bytes are
-// the same either way.
+// Whether kernels that wait for their lane's host thread could run here.
+// BITZ_RESIDENT_ROUNDS=0 says no and =1 yes. Otherwise no when a CUDA injection
+// tool announces itself (CUDA_INJECTION64_PATH), or when the process's first
+// lane found that its host thread cannot reach a running kernel (a kernel that
+// waits up to 100 ms for one word from the host got none), as under a kernel
+// profiler. The sumchecks need no such kernel: a pass hands its sums over and
+// ends, so the proof and the launches are the same either way.
 bool resident_rounds_enabled();
 
-// Kernels that wait for their lane's host thread, and calls that wait for the
-// whole device. Such a kernel must never be in flight while another thread
-// is inside cudaFree, cudaFreeHost, cudaMalloc, cudaMallocHost or
-// cudaHostAlloc: the call waits for the kernel, the driver can hold the
-// lane's host thread (its next launch or stream query) behind the call, and
-// neither moves until the kernel's time limit ends the proof. A lane holds a
-// ResidentScope from before it launches the first such kernel of a stretch
-// until the stretch has ended; those calls run under an AllocScope, which
-// waits until no ResidentScope is held and holds new ones back meanwhile.
-// Scopes nest within a thread; an allocation inside a ResidentScope of its
-// own thread is a bug and throws.
+// One device or pinned allocation (or free) at a time: those calls wait for
+// the whole device, so lanes that grow their scratch together would queue up
+// inside the driver. They run under an AllocScope, which nests in a thread.
 class DeviceGate {
  public:
   static DeviceGate &get();
-  void enter_resident();
-  void leave_resident();
   void enter_alloc();
   void leave_alloc();
   // Since the process started: allocation stretches and the nanoseconds they
-  // waited for the gate, resident stretches and the nanoseconds they waited.
+  // waited for the gate; then two zeros (no kernel waits for its host thread).
   void stats(unsigned long long out[4]) const;
 
  private:
   std::mutex mu_;
   std::condition_variable cv_;
-  int residents_ = 0, allocs_waiting_ = 0;
   bool alloc_ = false;
-  std::atomic<unsigned long long> alloc_n_{0}, alloc_wait_ns_{0}, resident_n_{0},
-      resident_wait_ns_{0};
-};
-
-class ResidentScope {
- public:
-  explicit ResidentScope(bool on = true);
-  ~ResidentScope();
-  ResidentScope(const ResidentScope &) = delete;
-  ResidentScope &operator=(const ResidentScope &) = delete;
-
- private:
-  bool on_;
+  std::atomic<unsigned long long> alloc_n_{0}, alloc_wait_ns_{0};
 };
 
 class AllocScope {
  public:
-  // `strict`: throw when this thread holds a ResidentScope (false in
-  // destructors, which must not throw and then free without the gate).
-  explicit AllocScope(bool strict = true);
+  AllocScope();
   ~AllocScope();
   AllocScope(const AllocScope &) = delete;
   AllocScope &operator=(const AllocScope &) = delete;
-
- private:
-  bool on_ = false;
 };
 
 #if defined(__CUDACC__)
@@ -395,108 +339,6 @@ __device__ __forceinline__ bool mailbox_wait_device(const Mailbox *mb, unsigned 
     }
     if (globaltimer_ns() - t0 > limit_ns) return false;
     __nanosleep(32);
-  }
-}
-
-// Every thread calls it: the challenge words from lk.in (lk.in not null);
-// false when the chain has stopped, which block 0 passes on to lk.out.
-__device__ __forceinline__ bool link_begin(const RoundLink &lk, unsigned long long &w0,
-                                           unsigned long long &w1) {
-  __shared__ unsigned long long s[3];
-  if (threadIdx.x == 0) {
-    s[0] = lk.in->r_lo;
-    s[1] = lk.in->r_hi;
-    s[2] = lk.in->flag;
-  }
-  __syncthreads();
-  w0 = s[0];
-  w1 = s[1];
-  if (s[2] == 1) return true;
-  if (blockIdx.x == 0 && threadIdx.x == 0 && lk.out) lk.out->flag = 2;
-  return false;
-}
-
-// One thread of a round's last block, after its post: the next challenge
-// from the downbox into lk.out (nothing without lk.out).
-__device__ __forceinline__ void link_fetch(const RoundLink &lk) {
-  if (!lk.out) return;
-  unsigned long long w[2] = {0, 0};
-  const bool ok = mailbox_wait_device(lk.down, lk.dseq, 2, w, kRoundWaitNs);
-  lk.out->r_lo = w[0];
-  lk.out->r_hi = w[1];
-  lk.out->flag = ok ? 1u : 2u;
-}
-
-// Block 0's relay of a challenge to the other blocks of a resident kernel:
-// flag written last with release semantics, read with acquire (bounded).
-__device__ __forceinline__ void relay_post(RoundCtl *cl, const unsigned long long w[2], bool ok) {
-  cl->r_lo = w[0];
-  cl->r_hi = w[1];
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(&cl->flag), "r"(ok ? 1u : 2u)
-               : "memory");
-}
-
-__device__ __forceinline__ bool relay_wait(const RoundCtl *cl, unsigned long long w[2]) {
-  const unsigned long long t0 = globaltimer_ns();
-  for (;;) {
-    unsigned int f;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(f) : "l"(&cl->flag) : "memory");
-    if (f == 1) {
-      asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w[0]) : "l"(&cl->r_lo) : "memory");
-      asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w[1]) : "l"(&cl->r_hi) : "memory");
-      return true;
-    }
-    if (f == 2 || globaltimer_ns() - t0 > kRoundWaitNs) return false;
-    __nanosleep(64);
-  }
-}
-
-// Every thread of every block of a resident kernel calls it: block 0 waits
-// for host publication dseq in the downbox and relays it through cl; the
-// other blocks read the relay. The challenge words land in w (every thread);
-// false when it did not come (time limit or abort marker).
-__device__ __forceinline__ bool resident_challenge(const Mailbox *down, unsigned long long dseq,
-                                                   RoundCtl *cl, unsigned long long w[2]) {
-  __shared__ unsigned long long rs[2];
-  __shared__ int ok_s;
-  if (threadIdx.x == 0) {
-    unsigned long long v[2] = {0, 0};
-    bool ok;
-    if (blockIdx.x == 0) {
-      ok = mailbox_wait_device(down, dseq, 2, v, kRoundWaitNs);
-      relay_post(cl, v, ok);
-    } else {
-      ok = relay_wait(cl, v);
-    }
-    rs[0] = v[0];
-    rs[1] = v[1];
-    ok_s = ok;
-  }
-  __syncthreads();
-  w[0] = rs[0];
-  w[1] = rs[1];
-  const bool ok = ok_s;
-  __syncthreads();
-  return ok;
-}
-
-// publish<N> (after the block's atomics), then the last block fetches the
-// next challenge for the round link.
-template <int N>
-__device__ __forceinline__ void publish_link(unsigned long long *acc, const Publish &p,
-                                             const RoundLink &lk) {
-  static_assert(N <= kMailboxWords, "mailbox too small");
-  if (!p.counter) return;
-  if (threadIdx.x == 0) {
-    __threadfence();
-    const unsigned int prev = atomicAdd(p.counter, 1u);
-    if (prev == gridDim.x - 1) {
-      __threadfence();
-#pragma unroll
-      for (int k = 0; k < N; k++) mailbox_post(p.mailbox, p.seq, k, atomicExch(acc + k, 0ull));
-      *p.counter = 0;
-      link_fetch(lk);
-    }
   }
 }
 #endif

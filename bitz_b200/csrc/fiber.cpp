@@ -156,11 +156,11 @@ unsigned long long fiber_selftest(int threads, int fibers, int yields, bool *ok)
     for (int i = 0; i < fibers; i++) {
       loop.add([&, i] {
         for (int k = 0; k < yields; k++) {
-          gate_depth().resident += i + 1;
+          gate_depth().alloc += i + 1;
           h = (h ^ (unsigned long long)(i * 1000003 + k)) * 1099511628211ull;
           fiber_yield();
-          if (gate_depth().resident != i + 1) good[t] = 0;  // another fiber's count leaked in
-          gate_depth().resident -= i + 1;
+          if (gate_depth().alloc != i + 1) good[t] = 0;  // another fiber's count leaked in
+          gate_depth().alloc -= i + 1;
           if (k == yields / 2) {
             try {
               volatile double x = 1.0 / (k + 3);
@@ -176,7 +176,7 @@ unsigned long long fiber_selftest(int threads, int fibers, int yields, bool *ok)
     }
     loop.run();
     for (int v : finished) good[t] &= v;
-    if (gate_depth().resident != 0) good[t] = 0;  // the thread's own counter untouched
+    if (gate_depth().alloc != 0) good[t] = 0;  // the thread's own counter untouched
     sums[t] = h;
   };
   std::vector<std::thread> ts;

@@ -20,10 +20,10 @@ namespace bz {
 
 struct Fiber;
 
-// Per-fiber (or, outside fibers, per-thread) counters of the device gate's
+// Per-fiber (or, outside fibers, per-thread) depth of the device gate's
 // scopes (context.cpp).
 struct GateDepth {
-  int resident = 0, alloc = 0;
+  int alloc = 0;
 };
 
 class FiberLoop {

@@ -25,8 +25,8 @@
 // three rounds make 4 (4 + 2 + 1) = 28, so a turn per three rounds is the
 // better split at every size. Tables of 2^kHostLog entries or fewer go to the
 // host, which runs the remaining rounds. Measured for the seven layers, a
-// round a turn before and passes now: s = 18 8.59 -> 3.91 ms, s = 14 in a
-// proof of 64 blocks 1.52 -> 0.93 ms (77 turns -> 29).
+// round a turn before and passes now: s = 18 8.57 -> 3.3 ms, s = 14 in a
+// proof of 64 blocks 1.52 -> 0.75 ms (77 turns -> 29).
 #include <algorithm>
 #include <chrono>
 #include <cstdio>

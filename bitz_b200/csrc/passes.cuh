@@ -210,9 +210,10 @@ static __device__ __forceinline__ f128 pass_bind(In in, const MulTable *T, int k
 }
 
 // The same by 2^(k-1) neighbouring lanes, lane q of them: one pair per lane,
-// then joined by exchanges. Three products deep instead of seven (0.9 against
-// 6.2 us for a small pass); it makes 12 lane products for 7, so only where a
-// block has few entries. k >= 1, every lane of the warp.
+// then joined by exchanges. Three products deep instead of seven, which took
+// 11,900 cycles of a 64-block pass; it makes 12 lane products for 7, so only
+// where a block has few entries. One call per level for both halves: the seven
+// layers over 2^10 columns 393 -> 371 us. k >= 1, every lane of the warp.
 template <bool kLowFirst, class In>
 static __device__ __forceinline__ f128 pass_bind_lanes(In in, const MulTable *T, int k, int q) {
   const int g = 1 << (k - 1);

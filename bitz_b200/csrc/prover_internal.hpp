@@ -82,7 +82,7 @@ struct Workspace {
     BZ_CUDA(cudaEventCreateWithFlags(&ev_folds, cudaEventDisableTiming));
   }
   ~Workspace() {
-    AllocScope gate(false);
+    AllocScope gate;
     if (host_fp) cudaFreeHost(host_fp);
     if (host_acc) cudaFreeHost(host_acc);
     if (ev_cols) cudaEventDestroy(ev_cols);

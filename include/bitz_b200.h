@@ -180,13 +180,13 @@ void bitz_committed_witness_free(bitz_committed_witness *com);
  * library since the process started. */
 unsigned long long bitz_launch_count(void);
 /* Diagnostic (no reference counterpart): 1 when kernels that wait for the
- * host thread (resident and queued sumcheck rounds) are in use, 0 when every
- * round is its own launch. BITZ_RESIDENT_ROUNDS=0/1 forces the mode; unset,
- * it is off when a CUDA injection tool announces itself
+ * host thread could run here, 0 when not. BITZ_RESIDENT_ROUNDS=0/1 forces the
+ * answer; unset, it is 0 when a CUDA injection tool announces itself
  * (CUDA_INJECTION64_PATH) or when the first prover lane found that the host
  * cannot reach a running kernel (a kernel profiler holds the host at every
- * launch). Proof bytes are the same in both modes. Needs no GPU (before the
- * first lane exists it reports the environment's answer). */
+ * launch). The provers launch no such kernel, so proofs and launches are the
+ * same with either answer. Needs no GPU (before the first lane exists it
+ * reports the environment's answer). */
 int bitz_resident_rounds(void);
 /* Diagnostic (no reference counterpart): on the default lane since the
  * process started, out[0] the nanoseconds the host spent waiting for round
@@ -195,11 +195,10 @@ int bitz_resident_rounds(void);
  * work. */
 int bitz_round_wait_stats(unsigned long long out[2]);
 /* Diagnostic (no reference counterpart): the process's device gate since it
- * started. A lane whose kernels may wait for its host thread holds the gate
- * as a resident stretch; a device or pinned allocation (a lane's scratch
- * growing, a new circuit shape) waits until no stretch is held and holds new
- * ones back meanwhile. out[0] allocation stretches, out[1] nanoseconds they
- * waited, out[2] resident stretches, out[3] nanoseconds they waited. */
+ * started. Device and pinned allocations (a lane's scratch growing, a new
+ * circuit shape) pass it one at a time. out[0] allocation stretches, out[1]
+ * nanoseconds they waited; out[2] and out[3] (stretches of kernels that wait
+ * for their host thread, nanoseconds) are zero: no proof launches one. */
 int bitz_gate_stats(unsigned long long out[4]);
 /* Diagnostic (no reference counterpart): the last proof's packed witness f,
  * packed h = M (1 || f) and the exact products (A h, B h, C h per row). */
