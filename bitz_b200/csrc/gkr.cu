@@ -26,7 +26,7 @@
 // better split at every size. Tables of 2^kHostLog entries or fewer go to the
 // host, which runs the remaining rounds. Measured for the seven layers, a
 // round a turn before and passes now: s = 18 8.57 -> 3.3 ms, s = 14 in a
-// proof of 64 blocks 1.52 -> 0.75 ms (77 turns -> 29).
+// proof of 64 blocks 1.52 -> 0.75 ms (77 turns -> 25).
 #include <algorithm>
 #include <chrono>
 #include <cstdio>
