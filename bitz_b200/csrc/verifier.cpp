@@ -611,11 +611,22 @@ int ProofSystem::verify(const uint8_t *proof, size_t proof_len, Context *lane) {
   };
   std::vector<Opened> opened;
   size_t opened_queries = 0;
-  const size_t hint_words = (hs.len + 3) / 4;
   {
-    uint32_t *ph = W.pin_hints.get(hint_words);
-    memcpy(ph, hs.p, hs.len);
-    W.v_hints.upload(ph, hint_words, s);
+    // The openings' bytes to the device. The configuration fixes how many an
+    // accepted proof has (per level a count, then a row and a path for every
+    // query), so the buffers take that size; what a longer stream holds behind
+    // them is left where it is and refused as leftover bytes.
+    size_t want = hs.pos;
+    for (int i = 0; i < cfg.nlevels; i++) {
+      const PcsLevel &L = cfg.levels[i];
+      want += 8 + (size_t)L.queries *
+                      (((size_t)16 << L.k) + 32 * (size_t)(L.log_msg_cols + L.log_inv_rate));
+    }
+    const size_t have = std::min(hs.len, want);
+    uint32_t *ph = W.pin_hints.get((want + 3) / 4);
+    memcpy(ph, hs.p, have);
+    W.v_hints.resize((want + 3) / 4);
+    W.v_hints.upload(ph, (have + 3) / 4, s);
     W.v_vals.resize(total_queries);
     W.v_bad.resize((size_t)cfg.nlevels);
     BZ_CUDA(cudaMemsetAsync(W.v_bad.get(), 0, sizeof(unsigned int) * (size_t)cfg.nlevels, s));

@@ -9,6 +9,7 @@ import struct
 import pytest
 
 import bitz_b200 as bz
+import test_pcs_pins as pcs
 from bitz_b200 import statements as ci
 from oracle import ffi as of
 
@@ -118,3 +119,46 @@ def test_rejects_swapped_proofs(proofs):
     b = proofs[("sha256-chain", 2, 100)]
     rejects(a[0], b[3])
     rejects(b[0], a[3])
+
+
+def with_hints(proof, body):
+    """The proof with another hint body, its prefix and container lengths to match."""
+    i, n0, n1, _ = sections(proof)
+    return (proof[:i + 16] + struct.pack("<QQ", n1 - n0, 4 + len(body)) + proof[i + 32:n1]
+            + struct.pack("<I", len(body)) + body)
+
+
+def last_level(ps, security):
+    """Bytes of an opened row, of its path, and the queries, at the last level."""
+    _, levels = pcs.config(ps.stats()["padded_committed_bits"].bit_length() - 1, security)
+    lv = levels[-1]
+    return 16 << lv.k, 32 * (lv.log_msg_cols + lv.log_inv_rate), lv.queries
+
+
+def test_padded_hints_are_refused_and_take_no_memory(proofs):
+    """Hints longer than the statement's, with every length agreeing: leftover
+    bytes, and the device memory held does not grow with them."""
+    import torch
+    ps, _, _, proof = proofs[("sha256-compression", 1, 100)]
+    body = proof[sections(proof)[2] + 4:]
+    assert with_hints(proof, body) == proof
+    ps.verify(proof)
+    torch.cuda.synchronize()
+    for extra in (1, 4, 256 << 20):
+        bad = with_hints(proof, body + bytes(extra))
+        free = torch.cuda.mem_get_info()[0]
+        assert "leftover proof bytes" in str(rejects(ps, bad))
+        assert free - torch.cuda.mem_get_info()[0] < 16 << 20
+    ps.verify(proof)
+
+
+def test_shortened_hints_are_refused(proofs):
+    ps, _, _, proof = proofs[("sha256-compression", 1, 100)]
+    body = proof[sections(proof)[2] + 4:]
+    row, path, queries = last_level(ps, 100)
+    for cut, what in ((1, "inside a Merkle path"), (path, "inside a Merkle path"),
+                      (path + 1, "inside an opened row"), (path + row, "inside an opened row"),
+                      (queries * (row + path) + 1, "before a level's openings"),
+                      (len(body), "before a level's openings")):
+        assert what in str(rejects(ps, with_hints(proof, body[:len(body) - cut]))), cut
+    ps.verify(proof)
