@@ -20,12 +20,17 @@ struct CudaError : std::runtime_error {
   explicit CudaError(const std::string &s) : std::runtime_error(s) {}
 };
 
+// A failed call's error is taken out of the runtime's last-error slot with it: one that
+// leaves the context usable (an allocation that did not fit) would otherwise be reported
+// again by the next launch check, in a call that it has nothing to do with.
 #define BZ_CUDA(call)                                                                          \
   do {                                                                                         \
     cudaError_t e_ = (call);                                                                   \
-    if (e_ != cudaSuccess)                                                                     \
+    if (e_ != cudaSuccess) {                                                                   \
+      (void)cudaGetLastError();                                                                \
       throw ::bz::CudaError(std::string(#call) + ": " + cudaGetErrorString(e_) + " at " +     \
                             __FILE__ + ":" + std::to_string(__LINE__));                        \
+    }                                                                                          \
   } while (0)
 
 // Every launch site ends in BZ_LAUNCH_CHECK(), which also counts the launch
