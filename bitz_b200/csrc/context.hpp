@@ -114,6 +114,7 @@ class Context {
 
   PostGkrScratch &post_gkr_scratch(size_t entries) {
     if (pg_.capacity < entries) {
+      pg_.capacity = 0;  // nothing is usable if an allocation throws half-way
       pg_w0_.resize(entries);
       pg_v0_.resize(entries);
       pg_w1_.resize(entries);
@@ -139,6 +140,7 @@ class Context {
   GkrScratch &gkr_scratch(int s) {
     size_t leaves = (size_t)128 << s;
     if (gk_.capacity < leaves) {
+      gk_.capacity = 0;  // nothing is usable if an allocation throws half-way
       size_t total = leaves >> 6;
       for (int j = 2; j < 8; j++) total += leaves >> j;
       gk_layers_.resize(total);
