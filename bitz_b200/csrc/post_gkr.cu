@@ -418,7 +418,7 @@ struct PostGkrRun {
     if (sc.channel)
       return PassPost{sc.acc, sc.channel->counter, sc.channel->handover_dev,
                       sc.channel->arm().seq, sc.channel->pass_blocks};
-    return PassPost{sc.acc, sc.counter, sc.handover, ++sc.seq, kSMs};
+    return PassPost{sc.acc, sc.counter, sc.handover, ++*sc.seq, kSMs};
   }
   void wait(const PassPost &post, int n) {
     if (sc.channel) {

@@ -32,7 +32,9 @@ struct PostGkrScratch {
   RoundChannel *channel = nullptr;
   unsigned int *counter = nullptr;         // without a channel
   unsigned long long *handover = nullptr;  // 2 kHandoverWords slots
-  unsigned long long seq = 0;
+  // the last publication in those slots, kept between calls: a tag is not used
+  // again while the words of an earlier call may still be there
+  unsigned long long *seq = nullptr;
 };
 
 // The quadratic sumcheck of <W, V> (shared with the Ligerito folds), low
@@ -54,5 +56,7 @@ int post_gkr_prove(const PostGkrArgs &a, Transcript &ts, PostGkrScratch &sc, cud
 // Claims up to 2^20 bits; see post_gkr_noalloc.cu for the sharing rules.
 int post_gkr_prove_noalloc(const PostGkrArgs &a, Transcript &ts, cudaStream_t s, f128 *point_out,
                            f128 *value_out, std::string &err);
+// The tag of that call's last publication on the device (for tests).
+unsigned long long noalloc_last_publication(int device);
 
 }  // namespace bz

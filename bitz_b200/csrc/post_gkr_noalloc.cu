@@ -41,6 +41,9 @@ constexpr int kMaxDevices = 64;
 static f128 *s_tables[kMaxDevices];
 static unsigned long long *s_acc[kMaxDevices];
 static void *s_context[kMaxDevices];  // the context the addresses belong to
+// The last publication that a call on the device asked for.
+static unsigned long long s_seq[kMaxDevices];
+unsigned long long noalloc_last_publication(int device) { return s_seq[device]; }
 static std::mutex s_setup_mu;
 
 // The calling thread's current context (the device's primary context once
@@ -112,6 +115,7 @@ int post_gkr_prove_noalloc(const PostGkrArgs &a, Transcript &ts, cudaStream_t s,
   sc.acc = s_acc[dev];  // zeroed by post_gkr_prove before its first pass
   sc.counter = reinterpret_cast<unsigned int *>(s_acc[dev] + kNoAllocSums - 1);
   sc.handover = s_acc[dev] + kNoAllocSums;
+  sc.seq = &s_seq[dev];
   return post_gkr_prove(a, ts, sc, s, point_out, value_out);
 }
 

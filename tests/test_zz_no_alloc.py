@@ -106,3 +106,17 @@ def test_noalloc_takes_no_device_memory():
     assert np.array_equal(results[0][0], results[1][0])
     assert np.array_equal(results[0][1], results[1][1])
     assert results[0][2] == results[1][2]
+
+
+def test_publications_are_not_numbered_anew_by_each_call():
+    """The slots that the host copies keep the words of earlier calls. A pass is told from
+    them by its number, so a later call of the same shape must not count from one again."""
+    last = _lib.load()["_ZN2bz24noalloc_last_publicationEi"]
+    last.restype, last.argtypes = ctypes.c_ulonglong, [ctypes.c_int]
+    rows, cols, packed, target = _claim(17, 14, 0)
+    seen = []
+    for _ in range(3):
+        rc, _, _ = _noalloc(rows, cols, packed, target, 100, bz.build_prover(b"s", b"i"))
+        assert rc == 0, _lib.load().bitz_last_error()
+        seen.append(last(0))
+    assert seen[1] - seen[0] == seen[2] - seen[1] > 1
