@@ -123,7 +123,13 @@ void bitz_free(void *p) { free(p); }
 
 unsigned long long bitz_launch_count(void) { return launch_counter(); }
 
-int bitz_resident_rounds(void) { return resident_rounds_enabled() ? 1 : 0; }
+int bitz_resident_rounds(void) {
+  try {
+    return resident_rounds_enabled() ? 1 : 0;
+  } catch (...) {  // no lane to probe with
+    return 0;
+  }
+}
 
 int bitz_round_wait_stats(unsigned long long out[2]) {
   if (!out) return capi_fail(BZ_ERR_ARGUMENT, "null argument");

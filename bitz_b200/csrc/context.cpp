@@ -102,9 +102,27 @@ void RoundChannel::clear_down() {
   for (int k = 0; k < 2 * kMailboxWords; k++) s[k] = 0;
 }
 
-// The probe's result, set when the process's first lane is made: -1 not
-// yet probed, 0 the host cannot reach a running kernel, 1 it can.
-static std::atomic<int> g_host_reaches_kernel{-1};
+bool host_reaches_running_kernel(Context &lane);
+std::unique_ptr<Context> take_lane(int device);
+void give_lane(int device, std::unique_ptr<Context> lane);
+
+static std::atomic<bool> g_lane_made{false};
+
+// Whether this host can reach a running kernel, probed on a pool lane the first
+// time it is asked once the process has a lane. No proof asks.
+static bool host_reaches_kernels() {
+  static std::mutex mu;
+  static int known = -1;
+  std::lock_guard<std::mutex> lk(mu);
+  if (known < 0) {
+    int dev = 0;
+    BZ_CUDA(cudaGetDevice(&dev));
+    std::unique_ptr<Context> lane = take_lane(dev);
+    known = host_reaches_running_kernel(*lane) ? 1 : 0;
+    give_lane(dev, std::move(lane));
+  }
+  return known == 1;
+}
 
 bool resident_rounds_enabled() {
   static const int forced = [] {
@@ -114,9 +132,9 @@ bool resident_rounds_enabled() {
     const char *inj = getenv("CUDA_INJECTION64_PATH");
     return (inj && inj[0]) ? 0 : -1;
   }();
-  const bool on = forced >= 0 ? forced == 1 : g_host_reaches_kernel.load() != 0;
-  // probed launches are timed one by one, each its own round
-  return on && !KernelProbe::get().active();
+  if (KernelProbe::get().active()) return false;
+  if (forced >= 0) return forced == 1;
+  return !g_lane_made.load() || host_reaches_kernels();
 }
 
 void load_kernels(std::initializer_list<const void *> kernels) {
@@ -131,13 +149,10 @@ void preload_post_gkr_kernels();
 void preload_spartan_kernels();
 void preload_witness_kernels();
 void preload_diag_kernels();
-bool host_reaches_running_kernel(Context &lane);
 
 // Once per device, when its first lane is made: every kernel of the library
-// is loaded; and once per process, whether this host can reach a running
-// kernel is probed on that lane (a tool that holds the host at every launch
-// cannot run the kernels that wait for the host).
-static void lane_bootstrap(Context &lane) {
+// is loaded.
+static void lane_bootstrap() {
   static std::mutex mu;
   static std::set<int> loaded;
   std::lock_guard<std::mutex> lk(mu);
@@ -152,8 +167,7 @@ static void lane_bootstrap(Context &lane) {
     preload_witness_kernels();
     preload_diag_kernels();
   }
-  if (g_host_reaches_kernel.load() < 0)
-    g_host_reaches_kernel.store(host_reaches_running_kernel(lane) ? 1 : 0);
+  g_lane_made.store(true);
 }
 
 // ------------------------------------------------------------ DeviceGate
@@ -243,7 +257,7 @@ Context::Context() {
   channel_.counter = counter_.get();
   pg_.channel = &channel_;
   gk_.channel = &channel_;
-  lane_bootstrap(*this);
+  lane_bootstrap();
 }
 
 Context::~Context() {

@@ -262,11 +262,11 @@ struct RoundChannel {
 
 // Whether kernels that wait for their lane's host thread could run here.
 // BITZ_RESIDENT_ROUNDS=0 says no and =1 yes. Otherwise no when a CUDA injection
-// tool announces itself (CUDA_INJECTION64_PATH), or when the process's first
-// lane found that its host thread cannot reach a running kernel (a kernel that
-// waits up to 100 ms for one word from the host got none), as under a kernel
-// profiler. The sumchecks need no such kernel: a pass hands its sums over and
-// ends, so the proof and the launches are the same either way.
+// tool announces itself (CUDA_INJECTION64_PATH), or when a host thread cannot
+// reach a running kernel (a kernel that waits up to 100 ms for one word from the
+// host got none), as under a kernel profiler: tried when this is first asked
+// once a lane exists. The sumchecks need no such kernel: a pass hands its sums
+// over and ends, so the proof and the launches are the same either way.
 bool resident_rounds_enabled();
 
 // One device or pinned allocation (or free) at a time: those calls wait for

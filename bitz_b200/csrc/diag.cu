@@ -1,6 +1,7 @@
 // Measurement aids: the round-trip floor of the two ways a round's result
-// reaches the host and its challenge reaches the device. Not on the proving
-// path; exported through bitz_diag_round_trip.
+// reaches the host and its challenge reaches the device, and whether the host
+// can reach a running kernel. Not on the proving path; exported through
+// bitz_diag_round_trip and bitz_resident_rounds.
 #include <chrono>
 
 #include "context.hpp"

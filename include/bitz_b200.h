@@ -182,11 +182,12 @@ unsigned long long bitz_launch_count(void);
 /* Diagnostic (no reference counterpart): 1 when kernels that wait for the
  * host thread could run here, 0 when not. BITZ_RESIDENT_ROUNDS=0/1 forces the
  * answer; unset, it is 0 when a CUDA injection tool announces itself
- * (CUDA_INJECTION64_PATH) or when the first prover lane found that the host
- * cannot reach a running kernel (a kernel profiler holds the host at every
- * launch). The provers launch no such kernel, so proofs and launches are the
- * same with either answer. Needs no GPU (before the first lane exists it
- * reports the environment's answer). */
+ * (CUDA_INJECTION64_PATH) or when the host cannot reach a running kernel (a
+ * kernel profiler holds the host at every launch), which the first call made
+ * once a prover lane exists finds out with a kernel of at most 100 ms. The
+ * provers launch no such kernel, so proofs and launches are the same with
+ * either answer. Needs no GPU (before the first lane exists it reports the
+ * environment's answer). */
 int bitz_resident_rounds(void);
 /* Diagnostic (no reference counterpart): on the default lane since the
  * process started, out[0] the nanoseconds the host spent waiting for round

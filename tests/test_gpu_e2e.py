@@ -146,3 +146,29 @@ def test_large_proof_is_accepted_by_the_restated_verifier():
     inp, out, _ = ci.instance("sha256-chain", 1024, 2)
     proof, _ = bz.CircuitProofSystem("sha256-chain", inp, out, 128).prove()
     assert of.verify(ci.KINDS["sha256-chain"], inp, out, 128, proof) == 0
+
+
+def test_the_first_lane_launches_nothing_of_its_own():
+    """A process's first call launches the same kernels as its second; whether the host
+    reaches a running kernel is only tried when bitz_resident_rounds asks."""
+    import os
+    import subprocess
+    import sys
+    code = ("import numpy as np\n"
+            "import bitz_b200 as bz\n"
+            "from bitz_b200 import _lib\n"
+            "x = np.ones((128, 2), dtype=np.uint64)\n"
+            "n = [bz.launch_count()]\n"
+            "for _ in range(2):\n"
+            "    bz.gkr_outputs(x, x)\n"
+            "    n.append(bz.launch_count())\n"
+            "answers = [_lib.load().bitz_resident_rounds() for _ in range(2)]\n"
+            "n.append(bz.launch_count())\n"
+            "print(n[1] - n[0], n[2] - n[1], n[3] - n[2], *answers)\n")
+    env = {k: v for k, v in os.environ.items()
+           if k not in ("BITZ_RESIDENT_ROUNDS", "CUDA_INJECTION64_PATH")}
+    r = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True,
+                       timeout=300, cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert r.returncode == 0, r.stderr[-2000:]
+    first, second, asked, *answers = map(int, r.stdout.split())
+    assert first == second > 0 and asked == 1 and answers == [1, 1]
