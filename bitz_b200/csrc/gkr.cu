@@ -853,7 +853,7 @@ f128 gkr_prove(const f128 *cols, int s, const f128 *images, const f128 *zeta, ui
       R[k] = mk(words[2 * (len + k)], words[2 * (len + k) + 1]);
     }
     f128 lr[2];
-        std::vector<f128> prefix((size_t)1 << std::max(1, rem));
+    std::vector<f128> prefix((size_t)1 << std::max(1, rem));
     prefix[1] = mk(1, 0);
     for (int i = 0; i + 1 < rem; i++) eq_double(prefix.data() + ((size_t)1 << i), (size_t)1 << i, point[i]);
     rounds.from_tables(L.data(), R.data(), rem, prefix.data(), lr);

@@ -655,7 +655,7 @@ int ProofSystem::prove_after_commit(cudaStream_t s, std::vector<uint8_t> &proof)
   // Spartan
   int nr = ceil_log2(S.rows ? S.rows : 1), nc = ceil_log2(S.h_len);
   size_t R = (size_t)1 << nr, Cn = (size_t)1 << nc;
-  W.sp_t.resize(8 * R);
+  W.sp_t.resize(7 * R);
   W.sp_d.resize(4 * Cn);
   W.sp_part.resize(kSpPartials);
   W.sp_sums.resize(4);
@@ -665,7 +665,7 @@ int ProofSystem::prove_after_commit(cudaStream_t s, std::vector<uint8_t> &proof)
   else
     d_bit_rows_->upload(bit_rows_.data(), bit_rows_.size(), s);
   SpartanScratch sc;
-  for (int i = 0; i < 8; i++) sc.t[i] = W.sp_t.get() + i * R;
+  for (int i = 0; i < 7; i++) sc.t[i] = W.sp_t.get() + i * R;
   for (int i = 0; i < 4; i++) sc.d[i] = W.sp_d.get() + i * Cn;
   sc.counter = ctx.channel()->counter;
   sc.partial = W.sp_part.get();

@@ -118,18 +118,6 @@ BZ_HD fp interp(fp a, fp b, fp r, const FpCtx &c) {
   return fp_add(a, fp_mul(r, fp_sub(b, a, c), c), c);
 }
 
-// cubic_contribution (sumcheck.rs:724-746): [e0 r0, e0 rq + ed rl, ed rq]
-BZ_HD void cubic(fp e0, fp e1, fp a0, fp a1, fp b0, fp b1, fp c0, fp c1, const FpCtx &c,
-                 fp (&acc)[3]) {
-  fp ed = fp_sub(e1, e0, c), ad = fp_sub(a1, a0, c), bd = fp_sub(b1, b0, c), cd = fp_sub(c1, c0, c);
-  fp r0 = fp_sub(fp_mul(a0, b0, c), c0, c);
-  fp rl = fp_sub(fp_add(fp_mul(a0, bd, c), fp_mul(ad, b0, c), c), cd, c);
-  fp rq = fp_mul(ad, bd, c);
-  acc[0] = fp_add(acc[0], fp_mul(e0, r0, c), c);
-  acc[1] = fp_add(acc[1], fp_add(fp_mul(e0, rq, c), fp_mul(ed, rl, c), c), c);
-  acc[2] = fp_add(acc[2], fp_mul(ed, rq, c), c);
-}
-
 // One block adds the per-block partials into out.
 __global__ void k_fp_finalize(const fp *partial, int nblocks, FpCtx c, fp *out) {
   fp acc[1] = {fp_zero()};
@@ -547,25 +535,14 @@ __global__ void __launch_bounds__(kThreads) sp_bits(const fp *__restrict__ D,
   if (t == 0) *post.counter = 0;
 }
 
-// The last tables to the host, `tables` of n entries each after the binds; W
-// from h's bytes with kBits (then b.k = 3) or from its bits (w_bits).
-template <bool kBits>
+// The last tables to the host, `tables` of n entries each after the binds.
 __global__ void __launch_bounds__(64) sp_handover(SpTabs in, int tables, int n, size_t live,
-                                                  const uint32_t *w_bits,
                                                   const __grid_constant__ FpBind b, FpCtx c,
                                                   unsigned long long *handover,
                                                   unsigned long long seq) {
   const int k = blockIdx.x * 64 + threadIdx.x, tab = k / n, o = k % n;
   if (tab >= tables) return;
-  fp v = fp_zero();
-  if (kBits && tab == 1) {
-    const int byte = reinterpret_cast<const uint8_t *>(w_bits)[o];
-#pragma unroll 1
-    for (int j = 0; j < 8; j++)
-      if ((byte >> j) & 1) v = fp_add(v, b.e[j], c);
-  } else {
-    v = fp_bound(in.t[tab], o, live, b, c);
-  }
+  const fp v = fp_bound(in.t[tab], o, live, b, c);
   handover_post(handover, seq, 2 * k, v.lo);
   handover_post(handover, seq, 2 * k + 1, v.hi);
 }
@@ -717,9 +694,9 @@ void spartan_prove(const SpartanArgs &a, Transcript &ts, SpartanScratch &sc, cud
       const int lo = std::max(0, hi - kFacLog);
       for (int at = hi; at >= lo; at--) group[g].push_back(sp_eq(tau + at, hi - at, c, c.one));
     }
-    auto factors = [&](int n) {  // over the top n coordinates
+    auto factors = [&](int n) {  // over the top n > 0 coordinates
       FpFactors f{};
-      const int groups = n == 0 ? 1 : (n + kFacLog - 1) / kFacLog;
+      const int groups = (n + kFacLog - 1) / kFacLog;
       f.n = groups;
       f.low = n - kFacLog * (groups - 1);
       for (int g = 0; g < groups; g++) {
@@ -751,7 +728,7 @@ void spartan_prove(const SpartanArgs &a, Transcript &ts, SpartanScratch &sc, cud
     FpBind b{};
     int rem = nr;
     while (rem > kSpHostLog) {
-      const int k = std::min(kPassMaxK, rem), points = pow3(k);
+      const int k = kPassMaxK, points = pow3(k);
       const size_t live_out = (live + (((size_t)1 << b.k) - 1)) >> b.k;
       // positions past the live entries add nothing
       const uint32_t count = (uint32_t)((live_out + ((size_t)1 << k) - 1) >> k);
@@ -788,8 +765,7 @@ void spartan_prove(const SpartanArgs &a, Transcript &ts, SpartanScratch &sc, cud
     }
     const int n = 1 << rem;
     const PassPost post = arm();
-    sp_handover<false><<<(3 * n + 63) / 64, 64, 0, s>>>(in, 3, n, live, nullptr, b, c,
-                                                        post.handover, post.seq);
+    sp_handover<<<(3 * n + 63) / 64, 64, 0, s>>>(in, 3, n, live, b, c, post.handover, post.seq);
     BZ_LAUNCH_CHECK();
     ch->wait_handover(s, post.seq, words.data(), 6 * n);
     mark("outer tables", rem);
@@ -859,7 +835,8 @@ void spartan_prove(const SpartanArgs &a, Transcript &ts, SpartanScratch &sc, cud
     size_t live = a.cols;
     bool bits = true;
     const fp *d = D, *w = nullptr;
-    // every circuit has a compression's 20,456 columns
+    // every circuit has a compression's 20,456 columns, so the bits' rounds are
+    // followed by a pass
     if (rem <= kSpHostLog + kPassMaxK) throw CudaError("spartan: too few columns");
     {
       const PassPost post = arm();
@@ -926,8 +903,7 @@ void spartan_prove(const SpartanArgs &a, Transcript &ts, SpartanScratch &sc, cud
     const int n = 1 << rem;
     const PassPost post = arm();
     const SpTabs last{{const_cast<fp *>(d), const_cast<fp *>(w), nullptr}};
-    (bits ? sp_handover<true> : sp_handover<false>)<<<(2 * n + 63) / 64, 64, 0, s>>>(
-        last, 2, n, live, a.hbits, b, c, post.handover, post.seq);
+    sp_handover<<<(2 * n + 63) / 64, 64, 0, s>>>(last, 2, n, live, b, c, post.handover, post.seq);
     BZ_LAUNCH_CHECK();
     ch->wait_handover(s, post.seq, words.data(), 4 * n);
     mark("inner tables", rem);
@@ -1060,8 +1036,7 @@ void preload_spartan_kernels() {
                 (const void *)sp_inner_pass<3, true>,
                 (const void *)sp_inner_pass<3, false>,
                 (const void *)sp_bits,
-                (const void *)sp_handover<true>,
-                (const void *)sp_handover<false>,
+                (const void *)sp_handover,
                 (const void *)k_bind_table,
                 (const void *)k_bind,
                 (const void *)k_fp_dot,

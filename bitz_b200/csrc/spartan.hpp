@@ -10,9 +10,6 @@
 namespace bz {
 
 constexpr int kMaxFpPoint = 40;
-struct FpPoint {
-  fp c[kMaxFpPoint];
-};
 
 struct SpartanArgs {
   FpCtx ctx;
@@ -34,7 +31,7 @@ struct SpartanArgs {
 };
 
 struct SpartanScratch {
-  fp *t[8];        // eq over the rows (0), A, B, C (1-3) and their bound forms (4-6), 2^rows each
+  fp *t[7];        // eq over the rows (0), A, B, C (1-3) and their bound forms (4-6), 2^rows each
   fp *d[4];        // D (0) and the bound D and W (2, 3, then 0, 1), 2^cols each
   fp *partial;     // per-block partial sums, kSpPartials entries
   fp *sums;        // device, 3 entries

@@ -288,7 +288,7 @@ int ProofSystem::verify(const uint8_t *proof, size_t proof_len, Context *lane) {
   const fp fin = claim;
   // D(r_y) on the device
   const size_t R = (size_t)1 << nr, Cn = (size_t)1 << nc;
-  W.sp_t.resize(8 * R);
+  W.sp_t.resize(7 * R);
   W.sp_d.resize(4 * Cn);
   W.sp_part.resize(kSpPartials);
   W.sp_sums.resize(4);
@@ -298,7 +298,7 @@ int ProofSystem::verify(const uint8_t *proof, size_t proof_len, Context *lane) {
   else
     W.bit_rows.upload(bit_rows_.data(), bit_rows_.size(), s);
   SpartanScratch sc;
-  for (int i = 0; i < 8; i++) sc.t[i] = W.sp_t.get() + i * R;
+  for (int i = 0; i < 7; i++) sc.t[i] = W.sp_t.get() + i * R;
   for (int i = 0; i < 4; i++) sc.d[i] = W.sp_d.get() + i * Cn;
   sc.counter = ctx.channel()->counter;
   sc.partial = W.sp_part.get();
