@@ -60,6 +60,30 @@ def test_zero_and_one_coordinates(s, at):
     assert gt.narg() == ot.narg() and np.array_equal(gclaim, oclaim)
 
 
+@pytest.mark.parametrize("s,fill,zero", [
+    (15, "random", 14), (16, "full", 0), (16, "random", 15), (17, "sparse", 3), (20, "random", 19),
+])
+def test_large_schedules_match_oracle(s, fill, zero):
+    """Column counts with 16 sums a thread (2^16 columns on), weights of three factors above
+    the lowest 14 coordinates (2^20), a zero coordinate in a round that a pass sums, and a
+    one above it."""
+    rng = np.random.default_rng(5000 + s)
+    images, cols, zeta = rand_f128(rng, 128), rand_f128(rng, 1 << s), rand_f128(rng, s)
+    if fill == "sparse":
+        cols &= rand_f128(rng, 1 << s) & rand_f128(rng, 1 << s)
+        cols[(1 << s) * 3 // 4:] = 0
+    elif fill == "full":
+        cols[:] = np.uint64(2**64 - 1)
+    zeta[zero] = 0
+    zeta[(zero + 1) % s] = (1, 0)
+    ot = of.Transcript(b"gkr-passes", b"large")
+    opoint, oclaim = of.gkr_prove(images, cols, zeta, 0, ot)
+    gt = bz.build_prover(b"gkr-passes", b"large")
+    gpoint, gclaim = bz.gkr_prove(images, cols, zeta, 100, gt)
+    assert gt.narg() == ot.narg()
+    assert np.array_equal(gpoint, opoint) and np.array_equal(gclaim, oclaim)
+
+
 def test_scalar_host_rounds_give_the_same_transcript():
     """BITZ_HOST_SIMD=0 runs the host's last rounds with one product at a time."""
     import hashlib

@@ -162,3 +162,20 @@ def test_shortened_hints_are_refused(proofs):
                       (len(body), "before a level's openings")):
         assert what in str(rejects(ps, with_hints(proof, body[:len(body) - cut]))), cut
     ps.verify(proof)
+
+
+def test_a_failed_path_comes_before_later_failures(proofs):
+    """Paths are checked on the device while the replay goes on; the error is the first one
+    in the proof's order."""
+    ps, _, _, proof = proofs[("sha256-compression", 1, 100)]
+    body = bytearray(proof[sections(proof)[2] + 4:])
+    cut = with_hints(proof, bytes(body[:-1]))
+    assert "inside a Merkle path" in str(rejects(ps, cut))
+    body[8 + 3] ^= 1  # the first level's first opened row
+    assert "does not reach the root" in str(rejects(ps, with_hints(proof, bytes(body[:-1]))))
+    assert "does not reach the root" in str(rejects(ps, with_hints(proof, bytes(body))))
+    assert "does not reach the root" in str(rejects(ps, with_hints(proof, bytes(body) + bytes(5))))
+    late = bytearray(with_hints(proof, bytes(body)))
+    late[sections(proof)[2] - 1] ^= 1  # and the last nonce
+    assert "does not reach the root" in str(rejects(ps, bytes(late)))
+    ps.verify(proof)

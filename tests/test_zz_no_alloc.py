@@ -120,3 +120,32 @@ def test_publications_are_not_numbered_anew_by_each_call():
         assert rc == 0, _lib.load().bitz_last_error()
         seen.append(last(0))
     assert seen[1] - seen[0] == seen[2] - seen[1] > 1
+
+
+@pytest.mark.parametrize("lr,lc", [(8, 0), (13, 0), (14, 0), (17, 0), (20, 0), (7, 13), (13, 7), (9, 1)])
+def test_noalloc_shapes_match_allocating_entry_point(lr, lc):
+    """One column (rounds from the bits) and many, the smallest claim and the largest, on a
+    stream of the caller's."""
+    import torch
+    of.lib().o_set_clmul_mode(1)
+    rows, cols, packed, target = _claim(300 + lr, lr, lc)
+    of.lib().o_set_clmul_mode(0)
+    ref_ts, ts = bz.build_prover(b"no-alloc", b"shape"), bz.build_prover(b"no-alloc", b"shape")
+    ref_point, ref_value = bz.post_gkr_prove(rows, cols, target, packed, 100, ref_ts)
+    dev = [torch.from_numpy(x.view(np.int64)).cuda() for x in (rows, cols, packed)]
+    torch.cuda.synchronize()
+    stream = torch.cuda.Stream()
+    point, value = np.zeros((lr + lc, 2), dtype=np.uint64), np.zeros(2, dtype=np.uint64)
+
+    def call(tgt, transcript):
+        return _lib.load().bitz_post_gkr_prove_noalloc(
+            dev[0].data_ptr(), lr, dev[1].data_ptr(), lc, tgt.ctypes.data_as(_u64p), dev[2].data_ptr(),
+            100, transcript.handle, stream.cuda_stream, point.ctypes.data_as(_u64p),
+            value.ctypes.data_as(_u64p))
+
+    tgt = np.array(target, dtype=np.uint64)
+    assert call(tgt, ts) == 0, _lib.load().bitz_last_error()
+    assert np.array_equal(point, ref_point) and np.array_equal(value, ref_value)
+    assert ts.narg() == ref_ts.narg()
+    tgt[0] ^= np.uint64(1)
+    assert call(tgt, bz.build_prover(b"s", b"i")) != 0
