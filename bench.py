@@ -188,7 +188,7 @@ def profile_figure(summary, key, tag="sha256-chain-n64"):
 
 def roofline(bz, ps, steps, hbm_gbs, pk_kind, tag="sha256-chain-n64"):
     """Times every launch of the instrumented kernels with CUDA events over
-    ``steps`` proofs (every round its own launch, as under a kernel profiler),
+    ``steps`` proofs (each launch between two events of its own),
     picks the kernel with the largest share of the proofs' device time, and
     holds it to its roofline: its algorithmic bytes at the measured HBM
     bandwidth and its GF(2^128) products at the GPU's measured product
@@ -249,7 +249,7 @@ def roofline(bz, ps, steps, hbm_gbs, pk_kind, tag="sha256-chain-n64"):
             "share_note": "share_of_device_span: this run's CUDA-event kernel time over the proofs' "
                           "device span (host waits included); share_of_kernel_time_ncu: the "
                           "committed ncu launch list's share of summed kernel time",
-            "mode": "every sumcheck round its own launch (as under ncu), events per launch",
+            "mode": "the proof's own launches, events around each",
             "kernels": rows[:8]}
 
 
@@ -371,8 +371,8 @@ def batched(args, bz):
 
 def gate_delta(g0, g1):
     """Device-gate activity between two gate_stats() readings: allocations
-    (scratch growth) and the seconds allocations and resident stretches
-    waited for each other."""
+    (scratch growth) and the seconds they waited. No proof launches a kernel that
+    waits for its host thread, so the resident entry stays zero."""
     return {"allocs": g1["allocs"] - g0["allocs"],
             "alloc_wait_s": round(g1["alloc_wait_s"] - g0["alloc_wait_s"], 6),
             "resident_wait_s": round(g1["resident_wait_s"] - g0["resident_wait_s"], 6)}

@@ -421,7 +421,7 @@ class ProveServer:
 def probe_kernel(spec):
     """Times every launch of the probed kernels with CUDA events: None turns
     the probe off, "*" probes every instrumented kernel, else a
-    comma-separated list of names. While on, every round is its own launch."""
+    comma-separated list of names. The launches are the same while it is on."""
     _check(_lib.load().bitz_probe_kernel(spec.encode() if spec else None))
 
 

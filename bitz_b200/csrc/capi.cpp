@@ -19,10 +19,9 @@ struct bitz_transcript {
   Transcript t;
 };
 
-// Prover lanes are streams that each keep a round kernel waiting for their
-// host thread; with the CUDA default of 8 hardware work queues, lanes past 8
-// share queues, and a waiting kernel at the head of a queue holds back the
-// other lanes' launches behind it. When the library is loaded before the
+// Prover lanes are streams with short launches; with the CUDA default of 8
+// hardware work queues, lanes past 8 share queues, and a kernel at the head of
+// a queue holds back the other lanes' launches behind it. When the library is loaded before the
 // process creates its CUDA context and the caller has not chosen, ask for 32
 // queues (the most the driver gives). A caller's own setting is kept.
 __attribute__((constructor)) static void bz_default_work_queues() {

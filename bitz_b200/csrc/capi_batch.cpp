@@ -279,10 +279,9 @@ int bitz_batch_prove(bitz_system *const *systems, size_t n, int lanes, uint8_t *
     return capi_fail(BZ_ERR_CUDA, e.what());
   }
   // Largest statements first. A lane's first proof is then the largest it
-  // proves in the batch, so its scratch grows at most once per batch (a
-  // growth allocation waits until no lane has a kernel waiting for its host
-  // thread and holds every lane back meanwhile), and the batch ends on its
-  // shortest proofs. The proofs come back in the callers' order.
+  // proves in the batch, so its scratch grows at most once per batch (an
+  // allocation waits for the whole device, and they pass one at a time), and
+  // the batch ends on its shortest proofs. The proofs come back in the callers' order.
   std::vector<size_t> order(n);
   std::iota(order.begin(), order.end(), (size_t)0);
   {

@@ -198,8 +198,8 @@ class LaneLease {
 // algorithmic bytes each launch moves and the GF(2^128) products it computes
 // (a measurement aid; off by default). Events are recorded on the launching
 // stream; totals are collected once the stream has synchronised. While the
-// probe is on, every sumcheck round runs as its own launch (as under a kernel
-// profiler), so each probed launch is timed alone.
+// probe is on each probed launch (a sumcheck pass, say) lies between two events
+// of its own; the launches are the same as without it.
 class KernelProbe {
  public:
   static KernelProbe &get();

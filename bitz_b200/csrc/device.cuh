@@ -230,8 +230,8 @@ struct RoundChannel {
   Mailbox *dev = nullptr;   // device view
   unsigned int *counter = nullptr;
   unsigned long long next = 0;
-  // The reverse direction, for kernels that run several rounds and wait for
-  // the host's challenge between them: same tagged format, host to device.
+  // The reverse direction, for the diagnostics' kernels that wait for a word of
+  // the host (diag.cu): same tagged format, host to device.
   Mailbox *down_host = nullptr, *down_dev = nullptr;
   unsigned long long down_next = 0;
   // Tiles a sumcheck pass of this lane is split into where its size allows.
@@ -354,7 +354,8 @@ __device__ __forceinline__ bool mailbox_wait_device(const Mailbox *mb, unsigned 
 // r v_j X^(4j). The 32 x 16 entries live in shared memory as separate low and
 // high 64-bit words: a row of 16 words spans the 32 banks once, so the lanes
 // of a half-warp never conflict, whatever nibbles they look up. A product is
-// 32 independent lookups instead of about 550 dependent integer instructions.
+// 32 independent lookups instead of about 430 integer instructions, 144 of them
+// wide multiplies.
 struct MulTable {
   uint64_t lo[32][16], hi[32][16];
 };

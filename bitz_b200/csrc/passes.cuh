@@ -86,6 +86,10 @@ inline void quad_rounds(std::vector<f128> &F, int k, f128 *r, Round round) {
 // are three per thread), narrow ones the chip. A lane proving alone wants a tile
 // for every SM; lanes that share the GPU want few SMs each: 48 proofs on 24
 // lanes take 18.3 ms with 148 tiles, 17.6 with 74, 17.2 with 32, 18.0 with 16.
+// The line is drawn by the kind of lane, not by how many prove: a pooled lane at
+// work alone takes 32 tiles too, which costs it 1 to 2 % (64 blocks 2.91 ms
+// against 2.85 on the default lane, 201 6.53 against 6.46, 1024 22.5 against
+// 22.4, the batch call's own thread included).
 inline int pass_tile_log(uint32_t count, int blocks) {
   int lx = 5;
   while (lx > 2 && (count >> lx) < (uint32_t)blocks) lx--;

@@ -6,9 +6,7 @@ single proof or capturing its kernels under a profiler.
                                   [--seed 77] [--security 100] [--proofs 2]
 
 Messages come from the SplitMix64 stream of ``--seed`` (the bench's
-generator). With a kernel profiler attached the library runs every sumcheck
-round as its own launch by itself; BITZ_RESIDENT_ROUNDS=0 asks for the same
-explicitly.
+generator). The launches are the same with and without a profiler.
 """
 import argparse
 import json
